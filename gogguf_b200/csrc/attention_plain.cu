@@ -13,9 +13,15 @@
 // restates ops.AttentionScoresInto (pkg/ops/attention.go:10-47) and replaces the reference's
 // attn_qk / softmax / attn_v PTX kernels (pkg/gpu/cuda/ptx.go:679-889), which the host loops
 // over heads.
+//
+// What bounds it is latency: a key costs a table read, a row read and a reduction over the warp before its
+// exponential is known.  So a warp takes eight neighbouring keys at a time (eight rows in flight, eight reductions side
+// by side, one running maximum and one rescaling for the eight), and eight warps share a token's keys: a decode step has
+// few (token, head) pairs.  Keys are given out by position alone, so the result does not depend on the batch.
 #include "common.cuh"
 
-#define ATT_WARPS 4
+#define ATT_WARPS 8
+#define ATT_KEYS 8
 #define ATT_MAXD 256
 
 template <typename T>
@@ -53,22 +59,44 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_plain_kernel(
     for (int j = 0; j < ATT_MAXD / 32; ++j) acc[j] = 0.f;
     float m = -INFINITY, l = 0.f;
     const int* pt = page_table + (size_t)b * max_pages;
-    for (int j = lo + warp; j <= pos; j += ATT_WARPS) {
-        const int page = gg_page(pt, j / page_size, max_pages, pb, 41);
-        const size_t base = ((size_t)page * nkv + g) * page_size + (j % page_size);
-        const T* kp = k_pool + base * d;
-        const T* vp = v_pool + base * dv;
-        float dot = 0.f;
-        for (int i = lane; i < d; i += 32) dot = fmaf(qs[i], to_f<T>(kp[i]), dot);
-        dot = warp_sum(dot) * scale;
-        const float mn = fmaxf(m, dot);
+    for (int j0 = lo + warp * ATT_KEYS; j0 <= pos; j0 += ATT_WARPS * ATT_KEYS) {
+        size_t base[ATT_KEYS];
+        float dot[ATT_KEYS];
+#pragma unroll
+        for (int u = 0; u < ATT_KEYS; ++u) {
+            const int j = min(j0 + u, pos);              // past the last key: its row again, with weight zero
+            const int page = gg_page(pt, j / page_size, max_pages, pb, 41);
+            base[u] = ((size_t)page * nkv + g) * page_size + (j % page_size);
+            dot[u] = 0.f;
+        }
+#pragma unroll 4
+        for (int i = lane; i < d; i += 32) {
+            const float qv = qs[i];
+#pragma unroll
+            for (int u = 0; u < ATT_KEYS; ++u) dot[u] = fmaf(qv, to_f<T>(k_pool[base[u] * d + i]), dot[u]);
+        }
+        float mn = m;
+#pragma unroll
+        for (int u = 0; u < ATT_KEYS; ++u) {
+            dot[u] = j0 + u <= pos ? warp_sum(dot[u]) * scale : -INFINITY;
+            mn = fmaxf(mn, dot[u]);
+        }
         const float corr = expf(m - mn);
-        const float p = expf(dot - mn);
-        l = l * corr + p;
+        l *= corr;
+#pragma unroll
+        for (int u = 0; u < ATT_KEYS; ++u) {
+            dot[u] = j0 + u <= pos ? expf(dot[u] - mn) : 0.f;
+            l += dot[u];
+        }
 #pragma unroll
         for (int jj = 0; jj < ATT_MAXD / 32; ++jj) {
             const int i = lane + 32 * jj;
-            if (i < dv) acc[jj] = acc[jj] * corr + p * to_f<T>(vp[i]);
+            if (i < dv) {
+                acc[jj] *= corr;
+#pragma unroll
+                for (int u = 0; u < ATT_KEYS; ++u)
+                    if (j0 + u <= pos) acc[jj] = fmaf(dot[u], to_f<T>(v_pool[base[u] * dv + i]), acc[jj]);
+            }
         }
         m = mn;
     }

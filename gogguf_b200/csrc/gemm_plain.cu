@@ -3,93 +3,211 @@
 // This is the true 32-bit path of every projection (no tensor cores, no reduced
 // precision mode) and the plain twin the tensor-core kernels are checked against.
 // It also serves mixed operands (bfloat16 activations with a matrix that is stored
-// in 32-bit and stays so).  Each output element is accumulated over k in a fixed
-// order that does not depend on M, so a token's result does not depend on the batch.
-// The reference's counterpart is the one-thread-per-row matmul_vec PTX kernel
-// (pkg/gpu/cuda/ptx.go:67-129) and ops.MatMulVecInto (pkg/ops/ops.go:30-53).
+// in 32-bit and stays so).  The reference's counterpart is the one-thread-per-row matmul_vec PTX
+// kernel (pkg/gpu/cuda/ptx.go:67-129) and ops.MatMulVecInto (pkg/ops/ops.go:30-53).
+//
+// The order of the additions depends on K alone, so a token's result does not depend on the batch:
+// K is cut into four slices of equal length (a multiple of 32, the last may be short or empty), a slice
+// is summed with one fused multiply-add after another in ascending k, and the four sums are added as
+// (s0 + s1) + (s2 + s3).  Every tile size below keeps this order, so the same bits come from all of them.
+//
+// A CTA owns a BM x BN tile of the output and has G groups of threads; a group sums 4 / G neighbouring
+// slices of its whole tile, with TM x TN outputs per thread, from a ring of STAGES shared-memory stages of
+// its own (BK columns of x and W as float32, rows padded by 16 bytes: the float4 reads along k of eight
+// neighbouring rows touch all banks once).  Four slices side by side are what keeps a CTA's loads of
+// W in flight when M is small and the time is that of reading W; at large M the arithmetic bounds.
 #include "common.cuh"
 
-#define BM 64
-#define BN 64
-#define BK 16
+#define SLICES 4
 
-template <typename TX, typename TW, typename TO, bool ACC>
-__global__ void __launch_bounds__(256) gemm_plain_kernel(const TX* x, const TW* __restrict__ w,
-                                                         TO* __restrict__ out, int M, int N, int K,
-                                                         long long ldx, long long ldo, const float* __restrict__ bias) {
-    pdl_launch();
-    pdl_wait();
-    __shared__ float xs[BK][BM + 1];
-    __shared__ float ws[BK][BN + 1];
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int tid = threadIdx.x;
-    const int tm = (tid / 16) * 4, tn = (tid % 16) * 4;
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+__device__ __forceinline__ void gp_cp16(float* smem, const float* gmem) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(gmem) : "memory");
+}
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        // 64 rows x 16 k = 1024 elements per operand, 4 per thread
+template <int THREADS>
+__device__ __forceinline__ void group_sync(int g) {
+    if (THREADS == 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(THREADS) : "memory");
+}
+
+// Rows r0.. of a row-major operand into [R][BK + 4] floats; rows from `rows` on and columns from `k_end` on are zero.
+// ASYNC (float32 on 16-byte boundaries, K a multiple of 4): copies are issued and not waited for.
+template <typename T, int R, int BK, int THREADS>
+__device__ __forceinline__ void stage_rows(float* dst, const T* src, long long ld, int r0, int rows, int k0, int k_end, int tid,
+                                           bool async) {
+    if (sizeof(T) == 4 && async) {
+        constexpr int V = BK / 4;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int idx = tid + e * 256;
-            const int r = idx / BK, kk = idx % BK;
-            const int gk = k0 + kk;
-            float xv = 0.f, wv = 0.f;
-            if (gk < K) {
-                if (m0 + r < M) xv = to_f<TX>(x[(size_t)(m0 + r) * ldx + gk]);
-                if (n0 + r < N) wv = to_f<TW>(w[(size_t)(n0 + r) * K + gk]);
-            }
-            xs[kk][r] = xv;
-            ws[kk][r] = wv;
+        for (int c = tid; c < R * V; c += THREADS) {
+            const int r = c / V, kk = (c % V) * 4;
+            float* d = dst + r * (BK + 4) + kk;
+            if (r0 + r < rows && k0 + kk < k_end) gp_cp16(d, reinterpret_cast<const float*>(src) + (size_t)(r0 + r) * ld + k0 + kk);
+            else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = xs[kk][tm + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = ws[kk][tn + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + tm + i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tn + j;
-            if (n >= N) continue;
-            TO* o = out + (size_t)m * ldo + n;
-            if (bias != nullptr) acc[i][j] += bias[n];
-            if (ACC) *o = from_f<TO>(to_f<TO>(*o) + acc[i][j]);
-            else *o = from_f<TO>(acc[i][j]);
+    } else {
+#pragma unroll 4
+        for (int c = tid; c < R * BK; c += THREADS) {
+            const int r = c / BK, kk = c % BK;
+            float v = 0.f;
+            if (r0 + r < rows && k0 + kk < k_end) v = to_f<T>(src[(size_t)(r0 + r) * ld + k0 + kk]);
+            dst[r * (BK + 4) + kk] = v;
         }
     }
 }
 
-template <typename TX, typename TW>
-static int launch(const void* x, const void* w, void* out, int out_dtype, int accumulate,
-                  int M, int N, int K, long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    if (out_dtype == GG_F32) {
-        if (accumulate) gg_launch(gemm_plain_kernel<TX, TW, float, true>, dim3(grid), dim3(256), 0, stream, 1, (const TX*)x, (const TW*)w, (float*)out, M, N, K, ldx, ldo, bias);
-        else gg_launch(gemm_plain_kernel<TX, TW, float, false>, dim3(grid), dim3(256), 0, stream, 1, (const TX*)x, (const TW*)w, (float*)out, M, N, K, ldx, ldo, bias);
-    } else if (out_dtype == GG_BF16) {
-        if (accumulate) return GG_ERR_DTYPE;  // sums are kept in float32
-        gg_launch(gemm_plain_kernel<TX, TW, bf16, false>, dim3(grid), dim3(256), 0, stream, 1, (const TX*)x, (const TW*)w, (bf16*)out, M, N, K, ldx, ldo, bias);
-    } else {
-        return GG_ERR_DTYPE;
+template <typename TX, typename TW, int BM, int BN, int TM, int TN, int G, int BK, int STAGES>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
+    const TX* x, const TW* __restrict__ w, void* out, int out_bf16, int accumulate, int M, int N, int K, long long ldx,
+    long long ldo, const float* __restrict__ bias, int m_tiles, int async_x, int async_w, int early) {
+    constexpr int THN = BN / TN, THM = BM / TM, THREADS = THN * THM;
+    constexpr int STAGE = (BM + BN) * (BK + 4), PER = SLICES / G;
+    extern __shared__ __align__(16) float sm[];
+    if (early) pdl_launch();
+    const int g = threadIdx.x / THREADS, tid = threadIdx.x % THREADS;
+    const int tx = tid % THN, ty = tid / THN;
+    const int m0 = (int)(blockIdx.x % m_tiles) * BM, n0 = (int)(blockIdx.x / m_tiles) * BN;
+    const int len = ((K + SLICES - 1) / SLICES + 31) / 32 * 32;         // a slice
+    const int k_begin = min(K, g * PER * len), k_end = min(K, (g + 1) * PER * len);
+    const int steps = (k_end - k_begin + BK - 1) / BK;
+    float* ring = sm + (size_t)g * STAGES * STAGE;
+    auto load_w = [&](int it) {
+        if (it < steps) stage_rows<TW, BN, BK, THREADS>(ring + (it % STAGES) * STAGE + BM * (BK + 4), w, K, n0, N, k_begin + it * BK, k_end, tid, async_w);
+    };
+    auto load_x = [&](int it) {
+        if (it < steps) stage_rows<TX, BM, BK, THREADS>(ring + (it % STAGES) * STAGE, x, ldx, m0, M, k_begin + it * BK, k_end, tid, async_x);
+    };
+#pragma unroll 1
+    for (int s = 0; s < STAGES - 1; ++s) load_w(s);     // weights: nothing before this kernel writes them
+    pdl_wait();
+#pragma unroll 1
+    for (int s = 0; s < STAGES - 1; ++s) {
+        load_x(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    return gg_last_error();
+    float acc[TM][TN], run[PER > 1 ? TM : 1][PER > 1 ? TN : 1];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    const int per_slice = len / BK;
+#pragma unroll 1
+    for (int it = 0; it < steps; ++it) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        group_sync<THREADS>(g);                          // stage `it` is there, and nobody reads stage it - 1 any more
+        load_w(it + STAGES - 1);
+        load_x(it + STAGES - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (PER > 1 && it == per_slice) {                // the first of the group's two slices is done
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) { run[PER > 1 ? i : 0][PER > 1 ? j : 0] = acc[i][j]; acc[i][j] = 0.f; }
+        }
+        const float* xs = ring + (it % STAGES) * STAGE + ty * (BK + 4);
+        const float* ws = ring + (it % STAGES) * STAGE + (BM + tx) * (BK + 4);
+#pragma unroll
+        for (int kk = 0; kk < BK; kk += 4) {
+            float4 b[TN];
+#pragma unroll
+            for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(ws + j * THN * (BK + 4) + kk);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(xs + i * THM * (BK + 4) + kk);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.x, b[j].x, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.y, b[j].y, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.z, b[j].z, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.w, b[j].w, acc[i][j]);
+            }
+        }
+    }
+    if (PER > 1 && steps > per_slice) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) acc[i][j] = run[PER > 1 ? i : 0][PER > 1 ? j : 0] + acc[i][j];
+    }
+    // the groups' sums through shared memory: (s0 + s1) + (s2 + s3)
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (g > 0) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) sm[((g - 1) * TM * TN + i * TN + j) * THREADS + tid] = acc[i][j];
+    }
+    __syncthreads();
+    if (g > 0) return;
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + ty + i * THM;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + tx + j * THN;
+            if (m >= M || n >= N) continue;
+            const float* o = sm + (i * TN + j) * THREADS + tid;
+            float v = acc[i][j] + o[0];
+            if (G == 4) v += o[TM * TN * THREADS] + o[2 * TM * TN * THREADS];
+            if (bias != nullptr) v += bias[n];
+            if (out_bf16) reinterpret_cast<bf16*>(out)[(size_t)m * ldo + n] = __float2bfloat16_rn(v);
+            else {
+                float* p = reinterpret_cast<float*>(out) + (size_t)m * ldo + n;
+                *p = accumulate ? *p + v : v;
+            }
+        }
+    }
+}
+
+template <typename TX, typename TW, int BM, int BN, int TM, int TN, int G, int BK, int STAGES>
+static int launch_tile(const TX* x, const TW* w, void* out, int out_bf16, int accumulate, int M, int N, int K,
+                       long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
+    constexpr int threads = (BM / TM) * (BN / TN) * G;
+    constexpr size_t ring = (size_t)G * STAGES * (BM + BN) * (BK + 4) * sizeof(float);
+    static_assert(ring <= 227 * 1024 && ring >= (size_t)(G - 1) * BM * BN * sizeof(float), "shared memory");
+    auto kern = gemm_plain_kernel<TX, TW, BM, BN, TM, TN, G, BK, STAGES>;
+    static int resident = 0;                 // CTAs that the device holds at once (any thread computes the same number)
+    if (resident == 0) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
+        if (e != cudaSuccess) return (int)e;
+        int per = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, ring);
+        if (e != cudaSuccess) return (int)e;
+        resident = 148 * per;
+    }
+    const int m_tiles = (M + BM - 1) / BM;
+    const long long tiles = (long long)m_tiles * ((N + BN - 1) / BN);
+    if (tiles > 0x7fffffffLL) return GG_ERR_ARG;
+    const int async_x = sizeof(TX) == 4 && K % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & 15) == 0;
+    const int async_w = sizeof(TW) == 4 && K % 4 == 0 && ((uintptr_t)w & 15) == 0;
+    // the successor may start early only where no CTA of this grid still waits for an SM (see common.cuh)
+    return gg_launch(kern, dim3((unsigned)tiles), dim3(threads), ring, stream, 1, x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo,
+                     bias, m_tiles, async_x, async_w, (int)(tiles <= resident));
+}
+
+template <typename TX, typename TW>
+static int launch(const void* xv, const void* wv, void* out, int out_bf16, int accumulate,
+                  int M, int N, int K, long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
+    const TX* x = (const TX*)xv;
+    const TW* w = (const TW*)wv;
+#define GP(BM, BN, TM, TN, G, BK, ST) return launch_tile<TX, TW, BM, BN, TM, TN, G, BK, ST>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream)
+    if (M <= 2) GP(2, 16, 1, 1, 4, 32, 6);
+    if (M <= 4) GP(4, 16, 2, 1, 4, 32, 6);
+    if (M <= 8) GP(8, 16, 2, 2, 4, 32, 6);
+    if (M <= 16) GP(16, 16, 4, 2, 4, 32, 4);
+    // cycles of an SM per column of k, as its multipliers (128 a cycle) and each tile's measured share of them give
+    auto cost = [&](int bm, int bn, double share) {
+        const long long t = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+        return (double)((t + 147) / 148) * bm * bn / (128.0 * share);
+    };
+    const double small = cost(32, 16, 0.5), mid = cost(64, 32, 0.75), large = cost(128, 64, 0.88);
+    if (small <= mid && small <= large) GP(32, 16, 4, 4, 4, 32, 4);
+    if (mid <= large) GP(64, 32, 8, 4, 4, 16, 3);
+    GP(128, 64, 8, 8, 2, 16, 3);
+#undef GP
 }
 
 // x[M, K] with row stride ldx (elements), w[N, K] contiguous, out[M, N] with row stride ldo.
@@ -99,10 +217,13 @@ GG_API gg_gemm_plain(const void* x, int x_dtype, const void* w, int w_dtype, voi
                      cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || ldx < K || ldo < N) return GG_ERR_ARG;
-    if ((M + BM - 1) / BM > 65535) return GG_ERR_ARG;
-    if (x_dtype == GG_F32 && w_dtype == GG_F32) return launch<float, float>(x, w, out, out_dtype, accumulate, M, N, K, ldx, ldo, bias, stream);
-    if (x_dtype == GG_BF16 && w_dtype == GG_BF16) return launch<bf16, bf16>(x, w, out, out_dtype, accumulate, M, N, K, ldx, ldo, bias, stream);
-    if (x_dtype == GG_BF16 && w_dtype == GG_F32) return launch<bf16, float>(x, w, out, out_dtype, accumulate, M, N, K, ldx, ldo, bias, stream);
-    if (x_dtype == GG_F32 && w_dtype == GG_BF16) return launch<float, bf16>(x, w, out, out_dtype, accumulate, M, N, K, ldx, ldo, bias, stream);
+    if ((M + 63) / 64 > 65535) return GG_ERR_ARG;
+    if (out_dtype != GG_F32 && out_dtype != GG_BF16) return GG_ERR_DTYPE;
+    if (out_dtype == GG_BF16 && accumulate) return GG_ERR_DTYPE;  // sums are kept in float32
+    const int ob = out_dtype == GG_BF16;
+    if (x_dtype == GG_F32 && w_dtype == GG_F32) return launch<float, float>(x, w, out, ob, accumulate, M, N, K, ldx, ldo, bias, stream);
+    if (x_dtype == GG_BF16 && w_dtype == GG_BF16) return launch<bf16, bf16>(x, w, out, ob, accumulate, M, N, K, ldx, ldo, bias, stream);
+    if (x_dtype == GG_BF16 && w_dtype == GG_F32) return launch<bf16, float>(x, w, out, ob, accumulate, M, N, K, ldx, ldo, bias, stream);
+    if (x_dtype == GG_F32 && w_dtype == GG_BF16) return launch<float, bf16>(x, w, out, ob, accumulate, M, N, K, ldx, ldo, bias, stream);
     return GG_ERR_DTYPE;
 }
