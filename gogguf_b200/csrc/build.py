@@ -56,6 +56,7 @@ MODULES: Dict[str, str] = {
     "attention_plain": "attention_plain.cu",
     "latent_attention": "latent_attention.cu",
     "moe": "moe.cu",
+    "moe_grouped": "moe_grouped.cu",
     "retention": "retention.cu",
     "recurrence": "recurrence.cu",
     "diag_recurrence": "diag_recurrence.cu",
@@ -79,6 +80,7 @@ _INCLUDES: Dict[str, List[str]] = {
     "attention_fast.cu": ["tma_util.cuh"],
     "mixed_head_prompt.cu": ["tma_util.cuh"],
     "gemm_tcgen05.cu": ["tma_util.cuh"],
+    "moe_grouped.cu": ["tma_util.cuh"],
     "gemm_tcgen05_static.cu": ["gemm_tcgen05.cu", "gemm_tcgen05_static.h", "tma_util.cuh"],
     "diagnostics.cu": ["tma_util.cuh"],
 }

@@ -1216,6 +1216,47 @@ def moe_expert_mma(x: torch.Tensor, w: torch.Tensor, idx: torch.Tensor, n_pairs:
                                         float(slope), float(up_offset), float(out_scale), _p(wts), _stream())
 
 
+MOE_GROUPED_MAX_EXPERTS = 1024      # csrc/moe_grouped.cu keeps the experts' ranges in shared memory
+
+
+def moe_place_gather(h: torch.Tensor, wts: torch.Tensor, idx: torch.Tensor, n_pairs: int, n_experts: int, top: int,
+                     weight_on_input: bool, offsets: torch.Tensor, place: torch.Tensor, row_wts: torch.Tensor,
+                     xs: torch.Tensor) -> None:
+    """The pairs in the order (expert, pair): offsets[E + 1] the experts' row ranges, place[p] the row of pair p, row_wts
+    its weight, xs its input row (times the weight if that sits on the input).  Negative indices come last."""
+    _need(h, torch.bfloat16, "h")
+    _need(xs, torch.bfloat16, "xs")
+    for t, what in ((idx, "idx"), (offsets, "offsets"), (place, "place")):
+        _need(t, torch.int32, what)
+    for t, what in ((wts, "wts"), (row_wts, "row_wts")):
+        _need(t, torch.float32, what)
+    W = h.shape[-1]
+    if (xs.shape[-1] != W or xs.shape[0] < n_pairs or offsets.numel() < n_experts + 1
+            or min(idx.numel(), wts.numel(), place.numel(), row_wts.numel(), h.shape[0] * top) < n_pairs):
+        raise KernelError("moe_place_gather: shapes disagree")
+    kernel("moe_grouped", "gg_moe_place_gather")(_p(h), _p(wts), _p(idx), int(n_pairs), int(n_experts), W, int(top),
+                                                  int(weight_on_input), _p(offsets), _p(place), _p(row_wts), _p(xs), _stream())
+
+
+def moe_grouped(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, n_pairs: int, out: torch.Tensor, gated: bool,
+                limit: float = 0.0, slope: float = 1.0, out_scale: float = 1.0, row_wts: Optional[torch.Tensor] = None,
+                up_offset: float = 1.0) -> None:
+    """Rows offsets[e] .. offsets[e + 1] of x [P, K] times expert e's matrix, on the tcgen05 tensor cores.  gated: w
+    [E, 2, N, K], out bfloat16 [P, N] = out_scale * act(gate, up) (* row_wts[row]); else w [E, N, K], out float32."""
+    from .tcgen05_gemm import status_word
+    _need(x, torch.bfloat16, "x")
+    _need(w, torch.bfloat16, "w")
+    _need(out, torch.bfloat16 if gated else torch.float32, "out")
+    _need(offsets, torch.int32, "offsets")
+    E, N, K = w.shape[0], w.shape[-2], w.shape[-1]
+    if (x.shape[-1] != K or out.shape[-1] != N or x.shape[0] < n_pairs or out.shape[0] < n_pairs or offsets.numel() < E + 1
+            or w.dim() != (4 if gated else 3) or (gated and w.shape[1] != 2)):
+        raise KernelError("moe_grouped: shapes disagree")
+    kernel("moe_grouped", "gg_moe_grouped")(_p(x), _p(w), _p(offsets), int(n_pairs), E, _p(out), N, K, int(gated), float(limit),
+                                             float(slope), float(up_offset), float(out_scale), _p(row_wts),
+                                             _p(status_word(x.device)), _stream())
+
+
 def wait_probe(limit_cycles: int, code: int, status: torch.Tensor) -> torch.Tensor:
     """Run the package's bounded wait on a barrier nothing arrives at (csrc/diagnostics.cu) and return the
     kernel's report (5 int32 on the device): both roles' return values, their elapsed cycles / 1024, the

@@ -13,42 +13,85 @@
 #include "common.cuh"
 
 // ----------------------------------------------------------------------------- router logits
-// z[t, e] = Wr[e] . h[t] in float32: a warp per (token, expert), the token's row in shared memory.  A product of so
-// few output columns would be one or two CTAs of the tiled kernels; this one has a CTA per token and 8 experts.
-template <typename TX, typename TW>
-__global__ void __launch_bounds__(256) moe_router_logits_kernel(const TX* h, const TW* __restrict__ wr, float* z, int W, int E) {
+// z[t, e] = Wr[e] . h[t] in float32: a warp per expert, TB tokens' rows in shared memory.  A product of so few output
+// columns would be one or two CTAs of the tiled kernels; this one has a CTA per TB tokens and 8 experts.  A lane takes
+// eight neighbouring elements of every 256 (16-byte loads where the row allows them; one token a CTA and 2-byte loads
+// took 43 us for 2,048 tokens of width 2,048 and 16 experts); the order of the sums depends on neither TB nor the loads.
+template <typename T>
+__device__ __forceinline__ void load8(const T* p, int left, bool vec, float* v) {
+    if (vec && left >= 8) {
+        if (sizeof(T) == 2) {
+            const uint4 u = *reinterpret_cast<const uint4*>(p);
+            const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(b[j]); v[2 * j] = f.x; v[2 * j + 1] = f.y; }
+        } else {
+            const float4 a = reinterpret_cast<const float4*>(p)[0], c = reinterpret_cast<const float4*>(p)[1];
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = j < left ? to_f<T>(p[j]) : 0.f;
+    }
+}
+
+template <typename TX, typename TW, int TB>
+__global__ void __launch_bounds__(256) moe_router_logits_kernel(const TX* h, const TW* __restrict__ wr, float* z, int T, int W, int E) {
     pdl_launch();
     pdl_wait();
-    extern __shared__ float rx[];
-    const int t = blockIdx.x;
-    const TX* ht = h + (size_t)t * W;
-    for (int i = threadIdx.x; i < W; i += blockDim.x) rx[i] = to_f<TX>(ht[i]);
+    extern __shared__ __align__(16) float rx[];          // [TB][W8], zeros from W on
+    const int t0 = blockIdx.x * TB, W8 = (W + 7) / 8 * 8;
+    const bool vec = W % 8 == 0 && (((uintptr_t)h | (uintptr_t)wr) & 15) == 0;
+    for (int i = threadIdx.x * 8; i < TB * W8; i += 256 * 8) {
+        const int t = t0 + i / W8, k = i % W8;
+        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (t < T) load8<TX>(h + (size_t)t * W + k, W - k, vec, v);
+        reinterpret_cast<float4*>(rx + i)[0] = make_float4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<float4*>(rx + i)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = blockIdx.y * 8 + warp;
     if (e >= E) return;
     const TW* w = wr + (size_t)e * W;
-    float s = 0.f;
-    for (int i = lane; i < W; i += 32) s = fmaf(to_f<TW>(w[i]), rx[i], s);
-    s = warp_sum(s);
-    if (lane == 0) z[(size_t)t * E + e] = s;
+    float s[TB];
+#pragma unroll
+    for (int u = 0; u < TB; ++u) s[u] = 0.f;
+#pragma unroll 2
+    for (int i = lane * 8; i < W; i += 256) {
+        float v[8];
+        load8<TW>(w + i, W - i, vec, v);
+#pragma unroll
+        for (int u = 0; u < TB; ++u) {
+            const float4 a = reinterpret_cast<const float4*>(rx + u * W8 + i)[0], c = reinterpret_cast<const float4*>(rx + u * W8 + i)[1];
+            s[u] = fmaf(v[0], a.x, s[u]); s[u] = fmaf(v[1], a.y, s[u]); s[u] = fmaf(v[2], a.z, s[u]); s[u] = fmaf(v[3], a.w, s[u]);
+            s[u] = fmaf(v[4], c.x, s[u]); s[u] = fmaf(v[5], c.y, s[u]); s[u] = fmaf(v[6], c.z, s[u]); s[u] = fmaf(v[7], c.w, s[u]);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < TB; ++u) {
+        const float r = warp_sum(s[u]);
+        if (lane == 0 && t0 + u < T) z[(size_t)(t0 + u) * E + e] = r;
+    }
 }
 
 GG_API gg_moe_router_logits(const void* h, int h_dtype, const void* wr, int w_dtype, float* z, int T, int W, int E,
                             cudaStream_t stream) {
     if (T <= 0) return 0;
     if (W <= 0 || E <= 0 || (size_t)W * 4 > 48 * 1024 || (E + 7) / 8 > 65535) return GG_ERR_ARG;
-    dim3 grid(T, (E + 7) / 8);
-    const size_t smem = (size_t)W * sizeof(float);
-#define GG_RL(TX, TW) gg_launch(moe_router_logits_kernel<TX, TW>, dim3(grid), dim3(256), smem, stream, 1, (const TX*)h, \
-        (const TW*)wr, z, W, E)
-    if (h_dtype == GG_F32 && w_dtype == GG_F32) GG_RL(float, float);
-    else if (h_dtype == GG_BF16 && w_dtype == GG_BF16) GG_RL(bf16, bf16);
-    else if (h_dtype == GG_BF16 && w_dtype == GG_F32) GG_RL(bf16, float);
-    else if (h_dtype == GG_F32 && w_dtype == GG_BF16) GG_RL(float, bf16);
-    else return GG_ERR_DTYPE;
+    // four tokens a CTA share the reads of the router's rows once there are CTAs enough for the chip (8 experts: 592 tokens)
+    const size_t row = (size_t)((W + 7) / 8 * 8) * sizeof(float);
+    const int tb = (long long)T * ((E + 7) / 8) >= 592 && 4 * row <= 48 * 1024 ? 4 : 1;
+    dim3 grid((T + tb - 1) / tb, (E + 7) / 8);
+#define GG_RL(TX, TW) (tb == 4 ? gg_launch(moe_router_logits_kernel<TX, TW, 4>, dim3(grid), dim3(256), 4 * row, stream, 1, (const TX*)h, \
+        (const TW*)wr, z, T, W, E) : gg_launch(moe_router_logits_kernel<TX, TW, 1>, dim3(grid), dim3(256), row, stream, 1, (const TX*)h, \
+        (const TW*)wr, z, T, W, E))
+    if (h_dtype == GG_F32 && w_dtype == GG_F32) return GG_RL(float, float);
+    if (h_dtype == GG_BF16 && w_dtype == GG_BF16) return GG_RL(bf16, bf16);
+    if (h_dtype == GG_BF16 && w_dtype == GG_F32) return GG_RL(bf16, float);
+    if (h_dtype == GG_F32 && w_dtype == GG_BF16) return GG_RL(float, bf16);
+    return GG_ERR_DTYPE;
 #undef GG_RL
-    return gg_last_error();
 }
 
 // ----------------------------------------------------------------------------- route
@@ -422,21 +465,33 @@ GG_API gg_moe_invert(const int* place, int* pair_of, int P, cudaStream_t stream)
     return gg_last_error();
 }
 
-// residual[t, :] += sum_k rows[place[t * top + k], :]  (without `place`: the rows are in pair order)
+// residual[t, :] += sum_k rows[place[t * top + k], :]  (without `place`: the rows are in pair order).  VEC: four
+// neighbouring columns a thread, W a multiple of 4 and both buffers on 16-byte boundaries.
+template <bool VEC>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* rows, const int* place, float* residual, int W,
                                                           int top, const int* __restrict__ seq_of_token, const int* idx) {
     pdl_launch();
     pdl_wait();
     const int t = blockIdx.x;
     if (seq_of_token != nullptr && seq_of_token[t] < 0) return;
-    for (int i = threadIdx.x; i < W; i += blockDim.x) {
-        float s = 0.f;
+    constexpr int V = VEC ? 4 : 1;
+    for (int i = threadIdx.x * V; i < W; i += blockDim.x * V) {
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
         for (int k = 0; k < top; ++k) {
             const size_t p = (size_t)t * top + k;
             if (idx != nullptr && idx[p] < 0) continue;      // a choice without an expert left no row
-            s += rows[(place != nullptr ? (size_t)place[p] : p) * W + i];
+            const float* r = rows + (place != nullptr ? (size_t)place[p] : p) * W + i;
+            if (VEC) {
+                const float4 v = *reinterpret_cast<const float4*>(r);
+                s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w;
+            } else s[0] += *r;
         }
-        residual[(size_t)t * W + i] += s;
+        float* o = residual + (size_t)t * W + i;
+        if (VEC) {
+            float4 v = *reinterpret_cast<const float4*>(o);
+            v.x += s[0]; v.y += s[1]; v.z += s[2]; v.w += s[3];
+            *reinterpret_cast<float4*>(o) = v;
+        } else *o += s[0];
     }
 }
 
@@ -444,8 +499,9 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* rows, con
 GG_API gg_moe_combine(const float* rows, const int* place, float* residual, int T, int W, int top,
                       const int* seq_of_token, const int* idx, cudaStream_t stream) {
     if (T <= 0) return 0;
-    gg_launch(moe_combine_kernel, dim3(T), dim3(256), 0, stream, 1, rows, place, residual, W, top, seq_of_token, idx);
-    return gg_last_error();
+    if (W % 4 == 0 && (((uintptr_t)rows | (uintptr_t)residual) & 15) == 0)
+        return gg_launch(moe_combine_kernel<true>, dim3(T), dim3(256), 0, stream, 1, rows, place, residual, W, top, seq_of_token, idx);
+    return gg_launch(moe_combine_kernel<false>, dim3(T), dim3(256), 0, stream, 1, rows, place, residual, W, top, seq_of_token, idx);
 }
 
 // ----------------------------------------------------------------------------- identity experts

@@ -232,13 +232,23 @@ class RoutedExperts:
             self._grouped.run(h, idx, wts, residual, ctx)
             return
         if self._mma and h.dtype == torch.bfloat16 and (P <= K.MOE_MMA_MAX_PAIRS or self._grouped is None):
-            # few pairs in bfloat16: the experts' rows stream once through mma.sync, the pairs' rows as the operand
-            # (more pairs than one launch takes, where the sorted form does not serve: a launch per slice of pairs)
             xs = ctx.ws.get("moe_rows_in", (P, self.hidden), torch.bfloat16)
-            K.moe_gather(h, wts, None, xs, P, self.top, self.on_input)
             yb = ctx.ws.get("moe_act_rows", (P, self.inter), torch.bfloat16)
             rows = ctx.ws.get("moe_rows_out", (P, self.hidden), torch.float32)
             flat_idx, flat_wts = idx.view(-1), wts.view(-1)
+            if self.E <= K.MOE_GROUPED_MAX_EXPERTS:
+                # every expert's rows side by side, one tcgen05 launch per matrix for all experts
+                offsets = ctx.ws.get("moe_offsets", (self.E + 1,), torch.int32)
+                place = ctx.ws.get("moe_place", (P,), torch.int32)
+                row_wts = ctx.ws.get("moe_row_wts", (P,), torch.float32)
+                K.moe_place_gather(h, flat_wts, flat_idx, P, self.E, self.top, self.on_input, offsets, place, row_wts, xs)
+                K.moe_grouped(xs, self.w_gu, offsets, P, yb, True, self.limit, self.slope, self.out_scale,
+                              None if self.on_input else row_wts, up_offset=self.up_offset)
+                K.moe_grouped(yb, self.w_d, offsets, P, rows, False)
+                K.moe_combine(rows, place, residual, T, self.top, ctx.seq_of_token, idx=idx if self.identity else None)
+                return
+            # more experts than that kernel keeps ranges for: their rows stream through mma.sync (a launch per slice of pairs)
+            K.moe_gather(h, wts, None, xs, P, self.top, self.on_input)
             for p0 in range(0, P, K.MOE_MMA_MAX_PAIRS):
                 p1 = min(P, p0 + K.MOE_MMA_MAX_PAIRS)
                 K.moe_expert_mma(xs[p0:p1], self.w_gu, flat_idx[p0:p1], p1 - p0, yb[p0:p1], True, self.limit, self.slope,
