@@ -78,7 +78,9 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_plain_kernel(
         float mn = m;
 #pragma unroll
         for (int u = 0; u < ATT_KEYS; ++u) {
-            dot[u] = j0 + u <= pos ? warp_sum(dot[u]) * scale : -INFINITY;
+            // (no branch: the eight reductions run side by side)
+            const float r = warp_sum(dot[u]) * scale;
+            dot[u] = j0 + u <= pos ? r : -INFINITY;
             mn = fmaxf(mn, dot[u]);
         }
         const float corr = expf(m - mn);
@@ -92,10 +94,12 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_plain_kernel(
         for (int jj = 0; jj < ATT_MAXD / 32; ++jj) {
             const int i = lane + 32 * jj;
             if (i < dv) {
+                float v[ATT_KEYS];
+#pragma unroll
+                for (int u = 0; u < ATT_KEYS; ++u) v[u] = to_f<T>(v_pool[base[u] * dv + i]);
                 acc[jj] *= corr;
 #pragma unroll
-                for (int u = 0; u < ATT_KEYS; ++u)
-                    if (j0 + u <= pos) acc[jj] = fmaf(dot[u], to_f<T>(v_pool[base[u] * dv + i]), acc[jj]);
+                for (int u = 0; u < ATT_KEYS; ++u) acc[jj] = fmaf(dot[u], j0 + u <= pos ? v[u] : 0.f, acc[jj]);
             }
         }
         m = mn;

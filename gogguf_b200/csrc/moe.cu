@@ -13,78 +13,78 @@
 #include "common.cuh"
 
 // ----------------------------------------------------------------------------- router logits
-// z[t, e] = Wr[e] . h[t] in float32: a warp per expert, TB tokens' rows in shared memory.  A product of so few output
-// columns would be one or two CTAs of the tiled kernels; this one has a CTA per TB tokens and 8 experts.  A lane takes
-// eight neighbouring elements of every 256 (16-byte loads where the row allows them; one token a CTA and 2-byte loads
-// took 43 us for 2,048 tokens of width 2,048 and 16 experts); the order of the sums depends on neither TB nor the loads.
+// z[t, e] = Wr[e] . h[t] in float32: a CTA has 8 warps, TB tokens' rows in shared memory and EB experts a warp.  A product
+// of so few output columns would be one or two CTAs of the tiled kernels.  A lane takes four neighbouring elements of every
+// 128 (8- or 16-byte loads where the row allows them, shared-memory reads without bank conflicts); the order of the sums
+// depends on neither TB, EB nor the loads.
 template <typename T>
-__device__ __forceinline__ void load8(const T* p, int left, bool vec, float* v) {
-    if (vec && left >= 8) {
-        if (sizeof(T) == 2) {
-            const uint4 u = *reinterpret_cast<const uint4*>(p);
-            const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(b[j]); v[2 * j] = f.x; v[2 * j + 1] = f.y; }
-        } else {
-            const float4 a = reinterpret_cast<const float4*>(p)[0], c = reinterpret_cast<const float4*>(p)[1];
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = j < left ? to_f<T>(p[j]) : 0.f;
+__device__ __forceinline__ float4 load4(const T* p, int left, bool vec) {
+    float v[4];
+    if (vec && left >= 4) {
+        if (sizeof(T) == 4) return *reinterpret_cast<const float4*>(p);
+        const uint2 u = *reinterpret_cast<const uint2*>(p);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+        return make_float4(a.x, a.y, b.x, b.y);
     }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = j < left ? to_f<T>(p[j]) : 0.f;
+    return make_float4(v[0], v[1], v[2], v[3]);
 }
 
-template <typename TX, typename TW, int TB>
+template <typename TX, typename TW, int TB, int EB>
 __global__ void __launch_bounds__(256) moe_router_logits_kernel(const TX* h, const TW* __restrict__ wr, float* z, int T, int W, int E) {
     pdl_launch();
     pdl_wait();
-    extern __shared__ __align__(16) float rx[];          // [TB][W8], zeros from W on
-    const int t0 = blockIdx.x * TB, W8 = (W + 7) / 8 * 8;
-    const bool vec = W % 8 == 0 && (((uintptr_t)h | (uintptr_t)wr) & 15) == 0;
-    for (int i = threadIdx.x * 8; i < TB * W8; i += 256 * 8) {
-        const int t = t0 + i / W8, k = i % W8;
-        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (t < T) load8<TX>(h + (size_t)t * W + k, W - k, vec, v);
-        reinterpret_cast<float4*>(rx + i)[0] = make_float4(v[0], v[1], v[2], v[3]);
-        reinterpret_cast<float4*>(rx + i)[1] = make_float4(v[4], v[5], v[6], v[7]);
-    }
+    extern __shared__ __align__(16) float rx[];          // [TB][W4], zeros from W on
+    const int t0 = blockIdx.x * TB, W4 = (W + 3) / 4 * 4;
+    const bool vec = W % 4 == 0 && (((uintptr_t)h | (uintptr_t)wr) & 15) == 0;
+#pragma unroll
+    for (int u = 0; u < TB; ++u)
+        for (int k = threadIdx.x * 4; k < W4; k += 256 * 4)
+            *reinterpret_cast<float4*>(rx + u * W4 + k) =
+                t0 + u < T ? load4<TX>(h + (size_t)(t0 + u) * W + k, W - k, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int e = blockIdx.y * 8 + warp;
-    if (e >= E) return;
-    const TW* w = wr + (size_t)e * W;
-    float s[TB];
+    const int e0 = (blockIdx.y * 8 + warp) * EB;
+    if (e0 >= E) return;
+    float s[EB][TB];
 #pragma unroll
-    for (int u = 0; u < TB; ++u) s[u] = 0.f;
-#pragma unroll 2
-    for (int i = lane * 8; i < W; i += 256) {
-        float v[8];
-        load8<TW>(w + i, W - i, vec, v);
+    for (int v = 0; v < EB; ++v)
+#pragma unroll
+        for (int u = 0; u < TB; ++u) s[v][u] = 0.f;
+#pragma unroll 4
+    for (int i = lane * 4; i < W; i += 128) {
+        float4 w[EB];
+#pragma unroll
+        for (int v = 0; v < EB; ++v) w[v] = load4<TW>(wr + (size_t)min(e0 + v, E - 1) * W + i, W - i, vec);
 #pragma unroll
         for (int u = 0; u < TB; ++u) {
-            const float4 a = reinterpret_cast<const float4*>(rx + u * W8 + i)[0], c = reinterpret_cast<const float4*>(rx + u * W8 + i)[1];
-            s[u] = fmaf(v[0], a.x, s[u]); s[u] = fmaf(v[1], a.y, s[u]); s[u] = fmaf(v[2], a.z, s[u]); s[u] = fmaf(v[3], a.w, s[u]);
-            s[u] = fmaf(v[4], c.x, s[u]); s[u] = fmaf(v[5], c.y, s[u]); s[u] = fmaf(v[6], c.z, s[u]); s[u] = fmaf(v[7], c.w, s[u]);
+            const float4 a = *reinterpret_cast<const float4*>(rx + u * W4 + i);
+#pragma unroll
+            for (int v = 0; v < EB; ++v)
+                s[v][u] = fmaf(w[v].w, a.w, fmaf(w[v].z, a.z, fmaf(w[v].y, a.y, fmaf(w[v].x, a.x, s[v][u]))));
         }
     }
 #pragma unroll
-    for (int u = 0; u < TB; ++u) {
-        const float r = warp_sum(s[u]);
-        if (lane == 0 && t0 + u < T) z[(size_t)(t0 + u) * E + e] = r;
-    }
+    for (int v = 0; v < EB; ++v)
+#pragma unroll
+        for (int u = 0; u < TB; ++u) {
+            const float r = warp_sum(s[v][u]);
+            if (lane == 0 && t0 + u < T && e0 + v < E) z[(size_t)(t0 + u) * E + e0 + v] = r;
+        }
 }
 
 GG_API gg_moe_router_logits(const void* h, int h_dtype, const void* wr, int w_dtype, float* z, int T, int W, int E,
                             cudaStream_t stream) {
     if (T <= 0) return 0;
     if (W <= 0 || E <= 0 || (size_t)W * 4 > 48 * 1024 || (E + 7) / 8 > 65535) return GG_ERR_ARG;
-    // four tokens a CTA share the reads of the router's rows once there are CTAs enough for the chip (8 experts: 592 tokens)
-    const size_t row = (size_t)((W + 7) / 8 * 8) * sizeof(float);
-    const int tb = (long long)T * ((E + 7) / 8) >= 592 && 4 * row <= 48 * 1024 ? 4 : 1;
-    dim3 grid((T + tb - 1) / tb, (E + 7) / 8);
-#define GG_RL(TX, TW) (tb == 4 ? gg_launch(moe_router_logits_kernel<TX, TW, 4>, dim3(grid), dim3(256), 4 * row, stream, 1, (const TX*)h, \
-        (const TW*)wr, z, T, W, E) : gg_launch(moe_router_logits_kernel<TX, TW, 1>, dim3(grid), dim3(256), row, stream, 1, (const TX*)h, \
+    // four tokens and two experts a warp share what is read, once that leaves CTAs enough for the chip
+    const size_t row = (size_t)((W + 3) / 4 * 4) * sizeof(float);
+    const bool many = (long long)T * ((E + 15) / 16) >= 4 * 148 && 4 * row <= 48 * 1024;
+    const dim3 grid = many ? dim3((T + 3) / 4, (E + 15) / 16) : dim3(T, (E + 7) / 8);
+#define GG_RL(TX, TW) (many ? gg_launch(moe_router_logits_kernel<TX, TW, 4, 2>, grid, dim3(256), 4 * row, stream, 1, (const TX*)h, \
+        (const TW*)wr, z, T, W, E) : gg_launch(moe_router_logits_kernel<TX, TW, 1, 1>, grid, dim3(256), row, stream, 1, (const TX*)h, \
         (const TW*)wr, z, T, W, E))
     if (h_dtype == GG_F32 && w_dtype == GG_F32) return GG_RL(float, float);
     if (h_dtype == GG_BF16 && w_dtype == GG_BF16) return GG_RL(bf16, bf16);

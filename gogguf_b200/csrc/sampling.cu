@@ -442,15 +442,25 @@ __device__ unsigned long long block_kth_largest(int n_mine, KeyOf key_of, int k,
 
 // Stage one: grid (slices, rows), 256 threads with 32 logits each (the per-pass cost of a thread is mostly fixed:
 // shuffles, the barrier, the decision).  cand[(row * slices + slice) * k + j]: the slice's k best keys (0 = none).
+//
+// Walking the digits of all 8,192 keys costs 32 keys a thread and pass, which is what bounds this kernel.  So for k up to
+// SAMP_SIEVE_K a threshold comes first: a thread's 32 keys make four groups of eight, and the k-th best of the 1,024
+// groups' best is a key that at least k keys reach (one per group), so the k best are among the keys that reach it.  In
+// a row without order those are k to 1.4 k of the 8,192; they go to shared memory and the digits of only these, at most
+// four a thread, are walked.  Where more than SAMP_SIEVE_ROOM reach it (large logits side by side) all keys are walked as for
+// larger k, where the sieve would let most keys through.
 #define SAMP_SLICE_THREADS 256
 #define SAMP_SLICE_PER (SAMP_SLICE / SAMP_SLICE_THREADS)
+#define SAMP_SIEVE_K 512
+#define SAMP_SIEVE_ROOM 1024
 
 __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const float* logits, long long ld, int V, float temp,
                                                                         int k, unsigned long long* __restrict__ cand) {
     pdl_launch();
     pdl_wait();
     __shared__ unsigned long long tot[3][4];
-    __shared__ int n_out;
+    __shared__ unsigned long long room[SAMP_SIEVE_ROOM];
+    __shared__ int n_out, n_room;
     const int row = blockIdx.y, slice = blockIdx.x, tid = threadIdx.x;
     const float* x = logits + (size_t)row * ld;
     const bool scale = temp > 0.f && temp != 1.f;
@@ -463,9 +473,41 @@ __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const fl
         if (scale) v = (float)((double)v * inv_temp);
         keys[u] = i < V ? best_key(v, i) : 0ull;
     }
-    if (tid == 0) n_out = 0;
-    const unsigned long long thr = block_kth_largest(SAMP_SLICE_PER, [&](int j) { return keys[j]; }, k, tot);
+    if (tid == 0) { n_out = 0; n_room = 0; }
     unsigned long long* dst = cand + ((size_t)row * gridDim.x + slice) * k;
+    unsigned long long thr;
+    bool sieved = false;
+    if (k <= SAMP_SIEVE_K) {
+        unsigned long long best[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+        for (int u = 0; u < SAMP_SLICE_PER; ++u) best[u & 3] = best[u & 3] > keys[u] ? best[u & 3] : keys[u];
+        const unsigned long long sieve = block_kth_largest(4, [&](int j) { return best[j]; }, k, tot);
+        // (0: fewer than k groups hold a key, as in a short last slice: every key passes)
+#pragma unroll
+        for (int u = 0; u < SAMP_SLICE_PER; ++u) {
+            if (keys[u] != 0ull && keys[u] >= sieve) {
+                const int at = atomicAdd(&n_room, 1);
+                if (at < SAMP_SIEVE_ROOM) room[at] = keys[u];
+            }
+        }
+        __syncthreads();
+        sieved = n_room <= SAMP_SIEVE_ROOM;
+    }
+    if (sieved) {
+        const int n = n_room;
+        unsigned long long mine[SAMP_SIEVE_ROOM / SAMP_SLICE_THREADS];
+#pragma unroll
+        for (int u = 0; u < SAMP_SIEVE_ROOM / SAMP_SLICE_THREADS; ++u)
+            mine[u] = u * SAMP_SLICE_THREADS + tid < n ? room[u * SAMP_SLICE_THREADS + tid] : 0ull;
+        thr = block_kth_largest((n + SAMP_SLICE_THREADS - 1) / SAMP_SLICE_THREADS, [&](int j) { return j == 0 ? mine[0] : (j == 1 ? mine[1] : (j == 2 ? mine[2] : mine[3])); }, k, tot);
+        for (int j = tid; j < k; j += SAMP_SLICE_THREADS) dst[j] = 0ull;
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < SAMP_SIEVE_ROOM / SAMP_SLICE_THREADS; ++u)
+            if (mine[u] != 0ull && mine[u] >= thr) dst[atomicAdd(&n_out, 1)] = mine[u];
+        return;
+    }
+    thr = block_kth_largest(SAMP_SLICE_PER, [&](int j) { return keys[j]; }, k, tot);
     for (int j = tid; j < k; j += SAMP_SLICE_THREADS) dst[j] = 0ull;
     __syncthreads();
 #pragma unroll

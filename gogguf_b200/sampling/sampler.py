@@ -42,6 +42,23 @@ def uniform01(seed: int, stream: int, step: int) -> float:
     return (z >> 11) / float(1 << 53)
 
 
+def _uniforms(seed: int, streams: Sequence[int], steps: Sequence[int]) -> List[float]:
+    """`uniform01(seed, s, k)` for every pair, the same bits: a batch's numbers in one go (64 rows one by one took 0.1 ms
+    of the host's time)."""
+    def mix(z):
+        z = z + np.uint64(0x9E3779B97F4A7C15)
+        z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+        z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+        return z ^ (z >> np.uint64(31))
+
+    pairs = list(zip(streams, steps))
+    if len(pairs) < 4:
+        return [uniform01(seed, s, k) for s, k in pairs]
+    a = np.array([[s & _M64 for s, _ in pairs], [k & _M64 for _, k in pairs]], dtype=np.uint64)
+    z = mix(mix(np.uint64(_mix64(seed & _M64)) ^ a[0]) ^ a[1])
+    return ((z >> np.uint64(11)).astype(np.float64) / float(1 << 53)).tolist()
+
+
 @dataclass(frozen=True)
 class SamplerConfig:
     """pkg/sampler/chain.go:9-15."""
@@ -221,8 +238,7 @@ class Sampler:
         if self.cfg.greedy:
             K.argmax(logits, out, rows)
         else:
-            u_host[:rows] = torch.tensor([uniform01(self.cfg.seed, s, k) for s, k in zip(streams, steps)],
-                                         dtype=torch.float64)
+            u_host[:rows] = torch.tensor(_uniforms(self.cfg.seed, streams, steps), dtype=torch.float64)
             u_dev[:rows].copy_(u_host[:rows], non_blocking=True)
             if self.device_chain:
                 K.sample_topk(logits, self.cfg.temp, self.cfg.top_k, self.cfg.top_p, self.cfg.min_p, u_dev, out, rows)
@@ -245,7 +261,7 @@ class Sampler:
         """`streams[r]`: request index of row r; `steps[r]`: tokens it has generated so far;
         `histories[r]`: prompt + generated ids (only read when a repeat penalty is set)."""
         rows = len(streams)
-        us = [uniform01(self.cfg.seed, s, k) for s, k in zip(streams, steps)]
+        us = _uniforms(self.cfg.seed, streams, steps)
         if logits.is_cuda and self.on_device and not self.penalised:
             from ..csrc import kernels as K
             if self._out is None or self._out.numel() < rows:
