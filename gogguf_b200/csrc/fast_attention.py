@@ -7,7 +7,7 @@ from typing import Callable, Optional
 import torch
 
 from . import kernels as K
-from .build import kernel, module
+from .build import kernel, module, stream_ptr
 
 
 def decode_splits(n_tokens: int, nkv: int, max_ctx: int) -> int:
@@ -26,7 +26,7 @@ def attn_decode(q, k_pool, v_pool, out, positions, seq_of_token, table, page_siz
         part_o.data_ptr() if part_o is not None else 0, part_ml.data_ptr() if part_ml is not None else 0,
         positions.data_ptr(), seq_of_token.data_ptr(), table.data_ptr(), table.shape[-1], page_size,
         k_pool.shape[0], n_tokens, nq, nkv, d, float(scale), int(window), int(splits),
-        status_word(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+        status_word(q.device).data_ptr(), stream_ptr())
 
 
 def decode_tma_splits(n_tokens: int, nkv: int, max_ctx: int, cluster: bool = False) -> int:
@@ -49,7 +49,7 @@ def attn_decode_tma(q, k_pool, v_pool, out, positions, seq_of_token, table, page
         positions.data_ptr(), seq_of_token.data_ptr(), table.data_ptr(), table.shape[-1], page_size,
         k_pool.shape[0], n_tokens, nq, nkv, d, d if dv is None else int(dv), float(scale), int(window), int(chunk), int(splits),
         int(bool(cluster)), sink.data_ptr() if sink is not None else 0, float(out_scale), *_gate(gate),
-        status_word(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+        status_word(q.device).data_ptr(), stream_ptr())
 
 
 def attn_prefill(q, k_pool, v_pool, out, cu_seqlens, ctx_lens, seq_of_token, table, page_size, n_seqs,
@@ -61,7 +61,7 @@ def attn_prefill(q, k_pool, v_pool, out, cu_seqlens, ctx_lens, seq_of_token, tab
         ctx_lens.data_ptr(), seq_of_token.data_ptr(), table.data_ptr(), table.shape[-1], page_size,
         k_pool.shape[0], n_seqs, max_tiles, nq, nkv, d, d if dv is None else int(dv), float(scale), int(window), int(chunk),
         sink.data_ptr() if sink is not None else 0, float(out_scale), *_gate(gate),
-        status_word(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+        status_word(q.device).data_ptr(), stream_ptr())
 
 
 def attn_prefill_tc(q, k_pool, v_pool, out, cu_seqlens, ctx_lens, seq_of_token, table, page_size, n_tokens,
@@ -74,7 +74,7 @@ def attn_prefill_tc(q, k_pool, v_pool, out, cu_seqlens, ctx_lens, seq_of_token, 
         ctx_lens.data_ptr(), seq_of_token.data_ptr(), table.data_ptr(), table.shape[-1], page_size,
         k_pool.shape[0], n_tokens, n_seqs, max_tiles, nq, nkv, d, d if dv is None else int(dv), float(scale), int(window),
         int(chunk), sink.data_ptr() if sink is not None else 0, float(out_scale), *_gate(gate),
-        status_word(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+        status_word(q.device).data_ptr(), stream_ptr())
 
 
 def takes(nq: int, nkv: int, d: int, dv: int) -> bool:

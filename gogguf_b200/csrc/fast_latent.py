@@ -6,7 +6,7 @@ from typing import Optional
 
 import torch
 
-from .build import KernelError, kernel, module
+from .build import KernelError, kernel, module, stream_ptr
 
 
 def headwise_gemm_mma(x: torch.Tensor, ldx: int, hx: int, w: torch.Tensor, out: torch.Tensor, ldo: int, ho: int,
@@ -23,7 +23,7 @@ def headwise_gemm_mma(x: torch.Tensor, ldx: int, hx: int, w: torch.Tensor, out: 
     kernel("latent_attention", "gg_headwise_gemm_mma")(
         x.data_ptr(), int(ldx), int(hx), w.data_ptr(), out.data_ptr(), dtype_code(out.dtype), int(ldo), int(ho),
         int(m), N, K, H, float(alpha), gate.data_ptr() if gate is not None else 0,
-        gate.stride(0) if gate is not None else 0, torch.cuda.current_stream().cuda_stream)
+        gate.stride(0) if gate is not None else 0, stream_ptr())
 
 
 def latent_attention_mma(qcat: torch.Tensor, pool: torch.Tensor, out: torch.Tensor, cu_seqlens: torch.Tensor,
@@ -47,7 +47,7 @@ def latent_attention_mma(qcat: torch.Tensor, pool: torch.Tensor, out: torch.Tens
         part_o.data_ptr() if part_o is not None else 0, part_ml.data_ptr() if part_ml is not None else 0,
         int(max_new) if max_new is not None else int(n_tokens), sink.data_ptr() if sink is not None else 0,
         status_word(qcat.device).data_ptr(),
-        torch.cuda.current_stream().cuda_stream)
+        stream_ptr())
 
 
 def mma_splits(n_seqs: int, n_tokens: int, heads: int, R: int, r: int, window: int, max_ctx: int) -> int:
@@ -74,7 +74,7 @@ def latent_prompt_mma(qd: torch.Tensor, qcat: torch.Tensor, kv: torch.Tensor, ck
         av.data_ptr(), cu_seqlens.data_ptr(), seq_of_token.data_ptr(), int(n_seqs), int(n_tokens), heads, d, r, dv, R,
         float(scale), int(window), float(out_scale), sink.data_ptr() if sink is not None else 0,
         gate.data_ptr() if gate is not None else 0, gate.stride(0) if gate is not None else 0,
-        torch.cuda.current_stream().cuda_stream)
+        stream_ptr())
 
 
 def prompt_takes(d: int, r: int, dv: int) -> bool:

@@ -188,6 +188,206 @@ static int launch_tile(const TX* x, const TW* w, void* out, int out_bf16, int ac
                      bias, m_tiles, async_x, async_w, (int)(tiles <= resident));
 }
 
+// ----------------------------------------------------------------------------- the tile for many rows
+// BM x 64 outputs, two groups of BM threads with two slices each, 8 x 8 outputs a thread.  Here the multipliers bound, and
+// on sm_100a they reach their rate only with the packed form (measured, registers only: fma.rn.f32 60 TFLOP/s,
+// fma.rn.f32x2 74): a thread's sums are pairs of neighbouring columns.  So x and W lie in shared memory with k as the
+// slow index, four columns or rows a 16-byte read, and come there through registers (the next stage's loads are
+// issued before this stage's arithmetic).  Both halves of a packed multiply-add are rounded as fma.rn.f32, so the bits
+// are those of the other tiles.
+#define WIDE_BN 64
+#define WIDE_BK 16
+
+template <typename T>
+__device__ __forceinline__ float4 gp_load4(const T* p, int left, bool vec) {
+    if (vec) {
+        if (left <= 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+        if (sizeof(T) == 4) return *reinterpret_cast<const float4*>(p);
+        const uint2 u = *reinterpret_cast<const uint2*>(p);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+        return make_float4(a.x, a.y, b.x, b.y);
+    }
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (left > 0) v.x = to_f<T>(p[0]);
+    if (left > 1) v.y = to_f<T>(p[1]);
+    if (left > 2) v.z = to_f<T>(p[2]);
+    if (left > 3) v.w = to_f<T>(p[3]);
+    return v;
+}
+__device__ __forceinline__ unsigned long long gp_pack(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 gp_unpack(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+template <typename TX, typename TW, int BM>
+__global__ void __launch_bounds__(2 * BM) gemm_plain_wide_kernel(
+    const TX* x, const TW* __restrict__ w, void* out, int out_bf16, int accumulate, int M, int N, int K, long long ldx,
+    long long ldo, const float* __restrict__ bias, int m_tiles, int vec_x, int vec_w, int early) {
+    constexpr int BN = WIDE_BN, BK = WIDE_BK, LX = BM + 4, LW = BN + 4, STAGE = BK * (LX + LW);
+    constexpr int WROWS = BN * 4 / BM;                  // float4s of W a thread loads per stage (of x: 4)
+    extern __shared__ __align__(16) float sm[];
+    if (early) pdl_launch();
+    const int g = threadIdx.x / BM, tid = threadIdx.x % BM;
+    const int tx = tid % 8, ty = tid / 8;               // columns 4 tx + {0..3, 32..35}, rows 4 ty + {0..3, BM/2..}
+    const int m0 = (int)(blockIdx.x % m_tiles) * BM, n0 = (int)(blockIdx.x / m_tiles) * BN;
+    const int len = ((K + SLICES - 1) / SLICES + 31) / 32 * 32;
+    const int k_begin = min(K, g * 2 * len), k_end = min(K, (g + 1) * 2 * len);
+    const int steps = (k_end - k_begin + BK - 1) / BK, per_slice = len / BK;
+    float* ring = sm + (size_t)g * 2 * STAGE;
+    const int lr = tid / 4, lk = (tid % 4) * 4;         // this thread's loads: rows lr + (BM / 4) i, columns lk .. lk + 3 of the stage
+    float4 xr[4], wr[WROWS];
+    auto load_w = [&](int it) {
+        const int k = k_begin + it * BK + lk;
+#pragma unroll
+        for (int i = 0; i < WROWS; ++i) {
+            const int n = n0 + lr + BM / 4 * i;
+            wr[i] = gp_load4<TW>(w + (size_t)(n < N ? n : 0) * K + k, n < N ? k_end - k : 0, vec_w);
+        }
+    };
+    auto load_x = [&](int it) {
+        const int k = k_begin + it * BK + lk;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int m = m0 + lr + BM / 4 * i;
+            xr[i] = gp_load4<TX>(x + (size_t)(m < M ? m : 0) * ldx + k, m < M ? k_end - k : 0, vec_x);
+        }
+    };
+    auto store = [&](int it) {
+        float* xs = ring + (it & 1) * STAGE;
+        float* ws = xs + BK * LX;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float* d = xs + lk * LX + lr + BM / 4 * i;
+            d[0] = xr[i].x; d[LX] = xr[i].y; d[2 * LX] = xr[i].z; d[3 * LX] = xr[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < WROWS; ++i) {
+            float* d = ws + lk * LW + lr + BM / 4 * i;
+            d[0] = wr[i].x; d[LW] = wr[i].y; d[2 * LW] = wr[i].z; d[3 * LW] = wr[i].w;
+        }
+    };
+    unsigned long long acc[8][4], run[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    if (steps > 0) load_w(0);
+    pdl_wait();
+    if (steps > 0) { load_x(0); store(0); }
+    group_sync<BM>(g);
+#pragma unroll 1
+    for (int it = 0; it < steps; ++it) {
+        if (it + 1 < steps) { load_w(it + 1); load_x(it + 1); }
+        if (it == per_slice) {                           // the first of the group's two slices is done
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { run[i][j] = acc[i][j]; acc[i][j] = 0ull; }
+        }
+        const float* xs = ring + (it & 1) * STAGE + 4 * ty;
+        const float* ws = ring + (it & 1) * STAGE + BK * LX + 4 * tx;
+#pragma unroll
+        for (int k = 0; k < BK; ++k) {
+            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(ws + k * LW), b1 = *reinterpret_cast<const ulonglong2*>(ws + k * LW + 32);
+            const unsigned long long b[4] = {b0.x, b0.y, b1.x, b1.y};
+            const float4 a0 = *reinterpret_cast<const float4*>(xs + k * LX), a1 = *reinterpret_cast<const float4*>(xs + k * LX + BM / 2);
+            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const unsigned long long aa = gp_pack(a[i], a[i]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(aa), "l"(b[j]));
+            }
+        }
+        if (it + 1 < steps) store(it + 1);               // (its last readers left it a barrier ago)
+        group_sync<BM>(g);
+    }
+    float f[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float2 v = gp_unpack(acc[i][j]);
+            if (steps > per_slice) {
+                const float2 r = gp_unpack(run[i][j]);
+                v.x = r.x + v.x; v.y = r.y + v.y;
+            }
+            f[i][2 * j] = v.x; f[i][2 * j + 1] = v.y;
+        }
+    __syncthreads();
+    if (g > 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sm[(i * 8 + j) * BM + tid] = f[i][j];
+    }
+    __syncthreads();
+    if (g > 0) return;
+    const bool vec_o = !out_bf16 && (ldo & 3) == 0 && (((uintptr_t)out) & 15) == 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + 4 * ty + (i & 3) + (i >> 2) * (BM / 2);
+        if (m >= M) continue;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int n = n0 + 4 * tx + 32 * h;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[j] = f[i][4 * h + j] + sm[(i * 8 + 4 * h + j) * BM + tid];
+                if (bias != nullptr && n + j < N) v[j] += bias[n + j];
+            }
+            if (vec_o && n + 4 <= N) {
+                float4* p = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + (size_t)m * ldo + n);
+                float4 r = make_float4(v[0], v[1], v[2], v[3]);
+                if (accumulate) { const float4 o = *p; r.x += o.x; r.y += o.y; r.z += o.z; r.w += o.w; }
+                *p = r;
+                continue;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (n + j >= N) continue;
+                if (out_bf16) reinterpret_cast<bf16*>(out)[(size_t)m * ldo + n + j] = __float2bfloat16_rn(v[j]);
+                else {
+                    float* p = reinterpret_cast<float*>(out) + (size_t)m * ldo + n + j;
+                    *p = accumulate ? *p + v[j] : v[j];
+                }
+            }
+        }
+    }
+}
+
+template <typename TX, typename TW, int BM>
+static int launch_wide(const TX* x, const TW* w, void* out, int out_bf16, int accumulate, int M, int N, int K,
+                       long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
+    constexpr size_t ring = (size_t)4 * WIDE_BK * (BM + WIDE_BN + 8) * sizeof(float);
+    static_assert(ring >= (size_t)64 * BM * sizeof(float), "the second group's sums go through the stages");
+    auto kern = gemm_plain_wide_kernel<TX, TW, BM>;
+    static int resident = 0;
+    if (resident == 0) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
+        if (e != cudaSuccess) return (int)e;
+        int per = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 2 * BM, ring);
+        if (e != cudaSuccess) return (int)e;
+        resident = 148 * per;
+    }
+    const int m_tiles = (M + BM - 1) / BM;
+    const long long tiles = (long long)m_tiles * ((N + WIDE_BN - 1) / WIDE_BN);
+    if (tiles > 0x7fffffffLL) return GG_ERR_ARG;
+    const int vec_x = K % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & (sizeof(TX) * 4 - 1)) == 0;
+    const int vec_w = K % 4 == 0 && ((uintptr_t)w & (sizeof(TW) * 4 - 1)) == 0;
+    return gg_launch(kern, dim3((unsigned)tiles), dim3(2 * BM), ring, stream, 1, x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo,
+                     bias, m_tiles, vec_x, vec_w, (int)(tiles <= resident));
+}
+
 template <typename TX, typename TW>
 static int launch(const void* xv, const void* wv, void* out, int out_bf16, int accumulate,
                   int M, int N, int K, long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
@@ -203,10 +403,11 @@ static int launch(const void* xv, const void* wv, void* out, int out_bf16, int a
         const long long t = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
         return (double)((t + 147) / 148) * bm * bn / (128.0 * share);
     };
-    const double small = cost(32, 16, 0.5), mid = cost(64, 32, 0.75), large = cost(128, 64, 0.88);
-    if (small <= mid && small <= large) GP(32, 16, 4, 4, 4, 32, 4);
-    if (mid <= large) GP(64, 32, 8, 4, 4, 16, 3);
-    GP(128, 64, 8, 8, 2, 16, 3);
+    const double small = cost(32, 16, 0.5), mid = cost(64, 32, 0.6), tall = cost(64, 64, 0.7), large = cost(128, 64, 0.8);
+    if (small <= mid && small <= large && small <= tall) GP(32, 16, 4, 4, 4, 32, 4);
+    if (mid <= large && mid <= tall) GP(64, 32, 8, 4, 4, 16, 3);
+    if (tall <= large) return launch_wide<TX, TW, 64>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream);
+    return launch_wide<TX, TW, 128>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream);
 #undef GP
 }
 

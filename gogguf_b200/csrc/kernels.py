@@ -10,7 +10,7 @@ from typing import Optional
 
 import torch
 
-from .build import KernelError, kernel
+from .build import KernelError, kernel, stream_ptr
 
 F32, BF16 = 0, 1
 
@@ -31,8 +31,7 @@ def _p(t: Optional[torch.Tensor]) -> int:
     return t.data_ptr()
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+_stream = stream_ptr
 
 
 def _need(t: torch.Tensor, dt: torch.dtype, what: str) -> None:

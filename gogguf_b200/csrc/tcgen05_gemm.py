@@ -5,7 +5,7 @@ from typing import Callable, Dict, Optional
 
 import torch
 
-from .build import KernelError, kernel, module
+from .build import KernelError, kernel, module, stream_ptr
 
 OUT_BF16, OUT_F32, OUT_F32_ACC, OUT_SWIGLU = 0, 1, 2, 3
 
@@ -15,8 +15,10 @@ _status: Dict[torch.device, torch.Tensor] = {}
 def status_word(device: torch.device) -> torch.Tensor:
     """One int32 on the device that kernels write to when a bounded wait runs out or, in the debug build,
     when a page table holds an index or page id out of range."""
-    device = torch.device(device)
     t = _status.get(device)
+    if t is None:
+        device = torch.device(device)
+        t = _status.get(device)
     if t is None:
         t = _status[device] = torch.zeros(1, dtype=torch.int32, device=device)
     return t
@@ -101,7 +103,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: boo
     kernel("gemm_tcgen05", "gg_gemm_tc")(
         x.data_ptr(), w.data_ptr(), out.data_ptr(), mode, M, N, K, x.stride(0), out.stride(0),
         scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
-        int(bool(cluster)), st.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        int(bool(cluster)), st.data_ptr(), stream_ptr())
 
 
 def gemm_tc_norm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
@@ -165,7 +167,7 @@ def gemm_tc_norm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate
         bias.data_ptr() if bias is not None else 0, out_norm[1].data_ptr() if out_norm is not None else 0,
         out_norm[2].data_ptr() if out_norm is not None else 0, float(out_norm[0]) if out_norm is not None else 0.0, int(glu_act),
         scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
-        st.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        st.data_ptr(), stream_ptr())
 
 
 def gemm_tc_qkv_rope(x: torch.Tensor, w: torch.Tensor, m: int, q_out: torch.Tensor, qw: Optional[torch.Tensor],
@@ -204,7 +206,7 @@ def gemm_tc_qkv_rope(x: torch.Tensor, w: torch.Tensor, m: int, q_out: torch.Tens
         page_table.data_ptr(), page_table.shape[-1], int(page_size), k_pool.shape[0] if k_pool is not None else 0,
         k_pool.data_ptr() if k_pool is not None else 0, v_pool.data_ptr() if v_pool is not None else 0,
         nq, nkv, scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
-        st.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        st.data_ptr(), stream_ptr())
 
 
 def make_linear(weight: torch.Tensor, swiglu: bool = False, glu_act: int = 0) -> Optional[Callable]:

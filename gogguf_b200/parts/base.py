@@ -42,11 +42,18 @@ class Runtime:
 class Workspace:
     """Named scratch buffers that are reused from step to step and grow on demand."""
 
+    MAX_VIEWS = 1024     # views kept ready (a few dozen per length of a step); then they are made anew
+
     def __init__(self, device):
         self.device = device
         self._bufs: Dict[Tuple[str, torch.dtype], torch.Tensor] = {}
+        self._views: Dict[Tuple[str, Tuple[int, ...], torch.dtype], torch.Tensor] = {}
 
     def get(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+        asked = (name, shape, dtype)
+        view = self._views.get(asked)
+        if view is not None:
+            return view
         n = 1
         for s in shape:
             n *= int(s)
@@ -55,7 +62,11 @@ class Workspace:
         if buf is None or buf.numel() < n:
             buf = torch.empty(max(n, 1), dtype=dtype, device=self.device)
             self._bufs[key] = buf
-        return buf[:n].view(*shape)
+            self._views.clear()          # (some were views of the buffer that this one replaces)
+        if len(self._views) >= self.MAX_VIEWS:
+            self._views.clear()
+        view = self._views[asked] = buf[:n].view(*shape)
+        return view
 
 
 @dataclass

@@ -7,14 +7,13 @@ from typing import List, Optional
 
 import torch
 
-from ..csrc.build import kernel
+from ..csrc.build import kernel, stream_ptr
 from .base import Linear, StepContext
 
 MIN_PAIRS = 512       # below this the experts are reached through the index (nothing is read back)
 
 
-def _s() -> int:
-    return torch.cuda.current_stream().cuda_stream
+_s = stream_ptr
 
 
 class _Grouped:
