@@ -20,6 +20,8 @@
 
 #define SLICES 4
 
+__device__ __forceinline__ int slice_len(int K) { return ((K + SLICES - 1) / SLICES + 31) / 32 * 32; }
+
 __device__ __forceinline__ void gp_cp16(float* smem, const float* gmem) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(gmem) : "memory");
@@ -67,7 +69,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
     const int g = threadIdx.x / THREADS, tid = threadIdx.x % THREADS;
     const int tx = tid % THN, ty = tid / THN;
     const int m0 = (int)(blockIdx.x % m_tiles) * BM, n0 = (int)(blockIdx.x / m_tiles) * BN;
-    const int len = ((K + SLICES - 1) / SLICES + 31) / 32 * 32;         // a slice
+    const int len = slice_len(K);
     const int k_begin = min(K, g * PER * len), k_end = min(K, (g + 1) * PER * len);
     const int steps = (k_end - k_begin + BK - 1) / BK;
     float* ring = sm + (size_t)g * STAGES * STAGE;
@@ -237,7 +239,7 @@ __global__ void __launch_bounds__(2 * BM) gemm_plain_wide_kernel(
     const int g = threadIdx.x / BM, tid = threadIdx.x % BM;
     const int tx = tid % 8, ty = tid / 8;               // columns 4 tx + {0..3, 32..35}, rows 4 ty + {0..3, BM/2..}
     const int m0 = (int)(blockIdx.x % m_tiles) * BM, n0 = (int)(blockIdx.x / m_tiles) * BN;
-    const int len = ((K + SLICES - 1) / SLICES + 31) / 32 * 32;
+    const int len = slice_len(K);
     const int k_begin = min(K, g * 2 * len), k_end = min(K, (g + 1) * 2 * len);
     const int steps = (k_end - k_begin + BK - 1) / BK, per_slice = len / BK;
     float* ring = sm + (size_t)g * 2 * STAGE;
@@ -394,10 +396,32 @@ static int launch(const void* xv, const void* wv, void* out, int out_bf16, int a
     const TX* x = (const TX*)xv;
     const TW* w = (const TW*)wv;
 #define GP(BM, BN, TM, TN, G, BK, ST) return launch_tile<TX, TW, BM, BN, TM, TN, G, BK, ST>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream)
-    if (M <= 2) GP(2, 16, 1, 1, 4, 32, 6);
-    if (M <= 4) GP(4, 16, 2, 1, 4, 32, 6);
-    if (M <= 8) GP(8, 16, 2, 2, 4, 32, 6);
-    if (M <= 16) GP(16, 16, 4, 2, 4, 32, 4);
+    // Up to 16 rows the time is that of reading W, and what counts is how much of it is asked for at a time.  With a CTA an SM
+    // or less, deep rings of wide stages; with more tiles, the ring that lets most of them be resident.  Measured, M = 4
+    // (us; BK 32 in 6 stages for all | as below): 2,048 x 2,048 10.7 | 6.4, 2,048 x 5,376 25.4 | 13.6, 4,096 x 2,048 11.6 | 9.3,
+    // 10,752 x 2,048 25.2 | 22.2, 65,536 x 2,048 106 | 98 (5.5 TB/s).
+    const long long tiles = (long long)((N + 15) / 16) * ((M + 15) / 16);
+    if (M <= 2) {
+        if (tiles <= 148) GP(2, 16, 1, 1, 4, 128, 4);
+        if (tiles <= 296) GP(2, 16, 1, 1, 4, 64, 4);
+        GP(2, 16, 1, 1, 4, 64, 2);
+    }
+    if (M <= 4) {
+        if (tiles <= 148) GP(4, 16, 2, 1, 4, 128, 4);
+        if (tiles <= 296) GP(4, 16, 2, 1, 4, 64, 4);
+        GP(4, 16, 2, 1, 4, 64, 2);
+    }
+    if (M <= 8) {
+        if (tiles <= 74) GP(8, 8, 2, 1, 4, 128, 3);
+        if (tiles <= 148) GP(8, 16, 2, 2, 4, 64, 6);
+        if (tiles <= 296) GP(8, 16, 2, 2, 4, 64, 4);
+        GP(8, 16, 2, 2, 4, 64, 2);
+    }
+    if (M <= 16) {
+        if (tiles <= 148) GP(16, 8, 2, 2, 4, 64, 3);
+        if (tiles <= 296) GP(16, 16, 4, 2, 4, 64, 3);
+        GP(16, 16, 4, 2, 4, 64, 2);
+    }
     // cycles of an SM per column of k, as its multipliers (128 a cycle) and each tile's measured share of them give
     auto cost = [&](int bm, int bn, double share) {
         const long long t = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);

@@ -15,12 +15,13 @@
 // ----------------------------------------------------------------------------- router logits
 // z[t, e] = Wr[e] . h[t] in float32: a CTA has 8 warps, TB tokens' rows in shared memory and EB experts a warp.  A product
 // of so few output columns would be one or two CTAs of the tiled kernels.  A lane takes four neighbouring elements of every
-// 128 (8- or 16-byte loads where the row allows them, shared-memory reads without bank conflicts); the order of the sums
-// depends on neither TB, EB nor the loads.
-template <typename T>
-__device__ __forceinline__ float4 load4(const T* p, int left, bool vec) {
+// 128 (VEC: 8- or 16-byte loads, W a multiple of 4 and aligned rows; shared-memory reads without bank conflicts); the order
+// of the sums depends on neither TB, EB nor VEC.  (The form of the loads is no run-time branch: behind one, a warp's sixteen
+// loads of a row of 2,048 waited for one another, 11 us for 8 tokens.)
+template <typename T, bool VEC>
+__device__ __forceinline__ float4 load4(const T* p, int left) {
     float v[4];
-    if (vec && left >= 4) {
+    if (VEC) {
         if (sizeof(T) == 4) return *reinterpret_cast<const float4*>(p);
         const uint2 u = *reinterpret_cast<const uint2*>(p);
         const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
@@ -32,18 +33,17 @@ __device__ __forceinline__ float4 load4(const T* p, int left, bool vec) {
     return make_float4(v[0], v[1], v[2], v[3]);
 }
 
-template <typename TX, typename TW, int TB, int EB>
+template <typename TX, typename TW, int TB, int EB, bool VEC>
 __global__ void __launch_bounds__(256) moe_router_logits_kernel(const TX* h, const TW* __restrict__ wr, float* z, int T, int W, int E) {
     pdl_launch();
     pdl_wait();
     extern __shared__ __align__(16) float rx[];          // [TB][W4], zeros from W on
     const int t0 = blockIdx.x * TB, W4 = (W + 3) / 4 * 4;
-    const bool vec = W % 4 == 0 && (((uintptr_t)h | (uintptr_t)wr) & 15) == 0;
 #pragma unroll
     for (int u = 0; u < TB; ++u)
         for (int k = threadIdx.x * 4; k < W4; k += 256 * 4)
             *reinterpret_cast<float4*>(rx + u * W4 + k) =
-                t0 + u < T ? load4<TX>(h + (size_t)(t0 + u) * W + k, W - k, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+                t0 + u < T ? load4<TX, VEC>(h + (size_t)(t0 + u) * W + k, W - k) : make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e0 = (blockIdx.y * 8 + warp) * EB;
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(256) moe_router_logits_kernel(const TX* h, con
     for (int i = lane * 4; i < W; i += 128) {
         float4 w[EB];
 #pragma unroll
-        for (int v = 0; v < EB; ++v) w[v] = load4<TW>(wr + (size_t)min(e0 + v, E - 1) * W + i, W - i, vec);
+        for (int v = 0; v < EB; ++v) w[v] = load4<TW, VEC>(wr + (size_t)min(e0 + v, E - 1) * W + i, W - i);
 #pragma unroll
         for (int u = 0; u < TB; ++u) {
             const float4 a = *reinterpret_cast<const float4*>(rx + u * W4 + i);
@@ -83,15 +83,18 @@ GG_API gg_moe_router_logits(const void* h, int h_dtype, const void* wr, int w_dt
     const size_t row = (size_t)((W + 3) / 4 * 4) * sizeof(float);
     const bool many = (long long)T * ((E + 15) / 16) >= 4 * 148 && 4 * row <= 48 * 1024;
     const dim3 grid = many ? dim3((T + 3) / 4, (E + 15) / 16) : dim3(T, (E + 7) / 8);
-#define GG_RL(TX, TW) (many ? gg_launch(moe_router_logits_kernel<TX, TW, 4, 2>, grid, dim3(256), 4 * row, stream, 1, (const TX*)h, \
-        (const TW*)wr, z, T, W, E) : gg_launch(moe_router_logits_kernel<TX, TW, 1, 1>, grid, dim3(256), row, stream, 1, (const TX*)h, \
-        (const TW*)wr, z, T, W, E))
+    const bool vec = W % 4 == 0 && (((uintptr_t)h | (uintptr_t)wr) & 15) == 0;
+#define GG_RL1(TX, TW, TB, EB, VEC) gg_launch(moe_router_logits_kernel<TX, TW, TB, EB, VEC>, grid, dim3(256), TB * row, stream, 1, \
+        (const TX*)h, (const TW*)wr, z, T, W, E)
+#define GG_RL(TX, TW) (many ? (vec ? GG_RL1(TX, TW, 4, 2, true) : GG_RL1(TX, TW, 4, 2, false)) \
+                            : (vec ? GG_RL1(TX, TW, 1, 1, true) : GG_RL1(TX, TW, 1, 1, false)))
     if (h_dtype == GG_F32 && w_dtype == GG_F32) return GG_RL(float, float);
     if (h_dtype == GG_BF16 && w_dtype == GG_BF16) return GG_RL(bf16, bf16);
     if (h_dtype == GG_BF16 && w_dtype == GG_F32) return GG_RL(bf16, float);
     if (h_dtype == GG_F32 && w_dtype == GG_BF16) return GG_RL(float, bf16);
     return GG_ERR_DTYPE;
 #undef GG_RL
+#undef GG_RL1
 }
 
 // ----------------------------------------------------------------------------- route

@@ -13,7 +13,9 @@
 // store them.
 //
 // What bounds it: with few rows per expert the weights' bytes (each touched expert's matrix is read once), with hundreds
-// the tensor cores.  BN = 128 with two CTAs an SM for the first, BN = 256 for the second; see the rule at the launcher.
+// the tensor cores.  BN = 128 with two CTAs an SM for the first, BN = 256 for the second; see the rule at the launcher.  A
+// stage holds as many rows of x as a tile can need (AROWS: the multiplication always reads 128, the others are what lies
+// behind them in shared memory and end in rows that are not stored), so that with few pairs the ring is full of weights.
 // Every mbarrier wait is bounded (tma_util.cuh).
 #include "common.cuh"
 #include "tma_util.cuh"
@@ -21,7 +23,6 @@
 namespace {
 
 constexpr int BM = 128, BK = 64, UMMA_K = 16, NUM_THREADS = 192, MAX_E = 1024;
-constexpr int A_BYTES = BM * BK * 2;
 
 __device__ __forceinline__ float clamped_glu(float g, float u, float limit, float slope, float up_offset) {
     g = fminf(g, limit);
@@ -97,13 +98,14 @@ __global__ void __launch_bounds__(256) moe_place_gather_kernel(const bf16* h, co
 }
 
 // ----------------------------------------------------------------------------- the products
-template <int BN, int STAGES, int MINB>
+template <int BN, int STAGES, int MINB, int AROWS>
 __global__ void __launch_bounds__(NUM_THREADS, MINB) moe_grouped_kernel(
-    const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int box_rows, const int* offsets, int E,
+    const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const int* offsets, int E,
     void* out, int N, int K, int gated, float limit, float slope, float up_offset, float out_scale, const float* row_wts,
     int* __restrict__ status) {
     constexpr int HALF = BN / 2;
-    constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2;
+    constexpr int A_BYTES = AROWS * BK * 2, STAGE_BYTES = A_BYTES + BN * BK * 2;
+    static_assert(A_BYTES % 1024 == 0 && STAGE_BYTES >= BM * BK * 2, "the last stage's 128 rows end inside it");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = (uint64_t*)(smem + STAGES * STAGE_BYTES);
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(NUM_THREADS, MINB) moe_grouped_kernel(
 
     if (warp == 0) {
         if (lane == 0) {
-            const uint32_t tx = (uint32_t)(box_rows * BK * 2 + BN * BK * 2);
+            const uint32_t tx = (uint32_t)STAGE_BYTES;
             int it = 0, e = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
@@ -290,23 +292,26 @@ __global__ void __launch_bounds__(NUM_THREADS, MINB) moe_grouped_kernel(
     }
 }
 
-template <int BN, int STAGES, int MINB>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, int box_rows, const int* offsets, int P, int E, void* out, int N, int K,
+template <int BN, int STAGES, int MINB, int AROWS>
+int launch(const void* x, const CUtensorMap& tb, const int* offsets, int P, int E, void* out, int N, int K,
            int gated, float limit, float slope, float up_offset, float out_scale, const float* row_wts, int* status,
            cudaStream_t stream) {
-    constexpr int fixed = STAGES * (A_BYTES + BN * BK * 2) + 1024 + 256;
+    constexpr int fixed = STAGES * (AROWS + BN) * BK * 2 + 1024 + 256;
     const int smem = fixed + 8 * (E + 1);
-    auto kern = moe_grouped_kernel<BN, STAGES, MINB>;
+    auto kern = moe_grouped_kernel<BN, STAGES, MINB, AROWS>;
     static bool configured = false;
     if (!configured) {
         cudaError_t er = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fixed + 8 * (MAX_E + 1));
         if (er != cudaSuccess) return (int)er;
         configured = true;
     }
+    CUtensorMap ta;
+    const int rc = tma::make_map_bf16(&ta, x, (unsigned long long)P, K, K, AROWS);
+    if (rc != 0) return rc;
     const int feat = gated ? BN / 2 : BN;
     const long long most = ((long long)(P < E ? P : E) + P / BM) * ((N + feat - 1) / feat);      // tiles, at most
     const int grid = (int)(most < 148LL * MINB ? most : 148LL * MINB);
-    return gg_launch(kern, dim3(grid), dim3(NUM_THREADS), smem, stream, 1, ta, tb, box_rows, offsets, E, out, N, K, gated, limit,
+    return gg_launch(kern, dim3(grid), dim3(NUM_THREADS), smem, stream, 1, ta, tb, offsets, E, out, N, K, gated, limit,
                      slope, up_offset, out_scale, row_wts, status);
 }
 
@@ -331,15 +336,18 @@ GG_API gg_moe_grouped(const void* x, const void* w, const int* offsets, int P, i
     if (E <= 0 || E > MAX_E || N <= 0 || K <= 0 || (K % 8) || status == nullptr || (((uintptr_t)x | (uintptr_t)w) & 15) ||
         (long long)E * 2 * N > 0x7fffffffLL)
         return GG_ERR_ARG;
-    // rows of x that one tile can need: fewer than 128 are copied where there are no more (an expert may have all P: the
-    // rows of a padded batch all go to the first)
-    const int box = P <= 16 ? 16 : (P <= 32 ? 32 : (P <= 64 ? 64 : 128));
+    // Measured (16 experts of 2,048 x 1,024, two a token, gate/up + down): 4,096 pairs 95 us on 256-wide tiles; 994 pairs 53 us
+    // on 128-wide ones, where each expert's weights are read for some sixty rows.  Few pairs: an expert may have all of them (the rows of a
+    // padded batch all go to the first), so P bounds the rows of a tile.
     const bool wide = P >= 128LL * E;
-    const int bn = wide ? 256 : 128;
-    CUtensorMap ta, tb;
-    int rc;
-    if ((rc = tma::make_map_bf16(&ta, x, (unsigned long long)P, K, K, box)) != 0) return rc;
-    if ((rc = tma::make_map_bf16(&tb, w, (unsigned long long)E * (gated ? 2 : 1) * N, K, K, bn / 2)) != 0) return rc;
-    if (wide) return launch<256, 4, 1>(ta, tb, box, offsets, P, E, out, N, K, gated, limit, slope, up_offset, out_scale, row_wts, status, stream);
-    return launch<128, 3, 2>(ta, tb, box, offsets, P, E, out, N, K, gated, limit, slope, up_offset, out_scale, row_wts, status, stream);
+    CUtensorMap tb;
+    const int rc = tma::make_map_bf16(&tb, w, (unsigned long long)E * (gated ? 2 : 1) * N, K, K, wide ? 128 : 64);
+    if (rc != 0) return rc;
+#define GG_MG(BN, ST, MINB, AR) return launch<BN, ST, MINB, AR>(x, tb, offsets, P, E, out, N, K, gated, limit, slope, up_offset, \
+                                                                out_scale, row_wts, status, stream)
+    if (wide) GG_MG(256, 4, 1, 128);
+    if (P <= 16) GG_MG(128, 5, 2, 16);
+    if (P <= 64) GG_MG(128, 4, 2, 64);
+    GG_MG(128, 3, 2, 128);
+#undef GG_MG
 }

@@ -16,7 +16,7 @@ def bound(k):
     return 3.0 * (k ** 0.5 / 2 + 4) * 2.0 ** -24
 
 
-@pytest.mark.parametrize("N,K_", [(16, 4), (130, 36), (49, 129), (2048, 260), (700, 1800)])
+@pytest.mark.parametrize("N,K_", [(16, 4), (130, 36), (49, 129), (2048, 260), (700, 1800), (2500, 96), (5000, 200)])
 @pytest.mark.parametrize("dtypes", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32)])
 def test_rows_of_every_tile(N, K_, dtypes):
     g = torch.Generator(device="cuda").manual_seed(3)
@@ -26,7 +26,7 @@ def test_rows_of_every_tile(N, K_, dtypes):
     first = None
     for off in (0, 1):                          # (rows that start off a 16-byte boundary take element loads)
         x = wide[:, off:off + K_]
-        for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 65, 129, 300, 700):
+        for M in (1, 2, 3, 4, 5, 8, 9, 12, 16, 17, 32, 33, 65, 129, 300, 700):
             out = torch.full((M, N), float("nan"), device="cuda")
             K().gemm_plain(x[:M], w, out)
             want = x[:M].double() @ w.double().T
@@ -60,3 +60,20 @@ def test_attention_keys_in_groups(pos):
         want = torch.einsum("hk,hkd->hd", p, vals)
         # (a weight's relative error is the score's absolute one: d terms of size about 1, three times their rounding)
         assert (out[0].double() - want).abs().max() <= 3 * (d + 8) * 2.0 ** -24 * vals.abs().max()
+
+
+@pytest.mark.parametrize("d,dv", [(128, 128), (120, 64), (36, 132), (256, 256), (30, 30)])
+def test_attention_head_sizes(d, dv):
+    """Lanes with four columns and one or two groups of them, sizes that leave lanes without columns, element loads."""
+    g = torch.Generator(device="cuda").manual_seed(d)
+    nq, nkv, ps, pos = 2, 1, 64, 150
+    for dt, tol in ((torch.float32, 3 * (d + 8) * 2.0 ** -24), (torch.bfloat16, 2.0 ** -8)):
+        q = torch.randn(1, nq, d, device="cuda", generator=g).to(dt)
+        kp, vp = (torch.randn(3, nkv, ps, n, device="cuda", generator=g).to(dt) for n in (d, dv))
+        table = torch.tensor([[2, 0, 1]], device="cuda", dtype=torch.int32)
+        out = torch.empty(1, nq, dv, device="cuda", dtype=dt)
+        K().attention_plain(q, kp, vp, out, torch.tensor([pos], device="cuda", dtype=torch.int32),
+                            torch.zeros(1, device="cuda", dtype=torch.int32), table, ps, 1, nq, nkv, d, d ** -0.5, 0, dv=dv)
+        keys, vals = (t[[2, 0, 1], 0].reshape(-1, t.shape[-1])[:pos + 1].double() for t in (kp, vp))
+        want = torch.softmax(q[0].double() @ keys.T * d ** -0.5, -1) @ vals
+        assert (out[0].double() - want).abs().max() <= tol * vals.abs().max()
