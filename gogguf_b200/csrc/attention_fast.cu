@@ -885,8 +885,26 @@ int launch_decode_tma(const CUtensorMap& tk, const CUtensorMap& tv, const void* 
 // by more than 2^8, and compute the page again.
 // Two CTAs share an SM (96 KB of shared memory and 256 tensor-memory columns each): while one runs
 // its softmax the other's MMAs keep the tensor pipe busy.
+// A step of few tokens on a long history has few (tile, head) pairs: 333 tokens and 32 heads are 96 CTAs for 296 places, and
+// each walks all pages of its history (84 us for 6,433).  So the pages of a tile may be split over the CTAs of a
+// cluster (grid z): each leaves its O, maximum and sum in its own shared memory, and the cluster adds them row by row, a
+// share of the rows per CTA, read through distributed shared memory and always in rank order.
 // All exponentials go to the special-function unit: computing a share of them as polynomials on the FMA pipe,
 // and a pass over the scores for their maximum, cost more issue slots than the unit's time they saved.
+// from the shared memory of CTA `rank` of the cluster, at the address that `local` is in this CTA
+__device__ __forceinline__ void attn_remote(uint32_t local, int rank, float& a, float& b) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(remote) : "memory");
+}
+__device__ __forceinline__ float4 attn_remote4(uint32_t local, int rank) {
+    uint32_t remote;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+    return v;
+}
+
 template <int DK, int DV, bool EXACT>
 __global__ void __launch_bounds__(192) attn_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -965,8 +983,10 @@ __global__ void __launch_bounds__(192) attn_prefill_tc_kernel(
     const int rows = active ? min(128, n_new - row0) : 0;
     const int pos0 = active ? ctx_lens[b] - n_new + row0 : 0;
     const int lo = attn_first(pos0, window, sh.chunk);
-    const int kt_first = lo / PAGE, kt_last = active ? (pos0 + rows - 1) / PAGE : -1;
-    const int ntiles = kt_last - kt_first + 1;
+    const int kt_begin = lo / PAGE, kt_last = active ? (pos0 + rows - 1) / PAGE : -1;
+    const int splits = (int)gridDim.z, all_tiles = kt_last - kt_begin + 1, per = (all_tiles + splits - 1) / splits;
+    const int kt_first = kt_begin + (int)blockIdx.z * per;                       // this CTA's share of the pages
+    const int ntiles = max(0, min(per, kt_last - kt_first + 1));
     // tensor memory: two score buffers of 64 columns (the scores of page j + 1 are computed while the softmax
     // of page j runs), then the output accumulator
     const uint32_t S_t = tmem_base, O_t = tmem_base + 128;
@@ -1142,6 +1162,27 @@ __global__ void __launch_bounds__(192) attn_prefill_tc_kernel(
             __syncwarp();
             if (lane == 0) tma::mbar_arrive(&p_ready[j & 1]);
         }
+        if (splits > 1) {
+            // O as it is, with the maximum it was taken against and its sum, for the cluster (Q, K and V are free once
+            // every product is done); 16-byte chunk c of row r lies at place c ^ (r & 7)
+            if (ok) ok = tma::mbar_wait(o_done, 0, abort_flag, status, 28);
+            if (ok) {
+                tc5::fence_after();
+                uint4* os = reinterpret_cast<uint4*>(smem) + row * (DV / 4);
+#pragma unroll 1
+                for (int c0 = 0; c0 < DV; c0 += 32) {
+                    uint32_t orow[32];
+                    tc5::ld32(O_t + lane_off + c0, orow);
+                    tc5::wait_ld();
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        os[(c0 / 4 + c) ^ (row & 7)] = ntiles > 0 ? make_uint4(orow[4 * c], orow[4 * c + 1], orow[4 * c + 2], orow[4 * c + 3])
+                                                                  : make_uint4(0u, 0u, 0u, 0u);
+                }
+            }
+            reinterpret_cast<float2*>(bars + 32)[row] = make_float2(m_used, l);
+            ok = false;                                      // what follows is the end of a tile that is not split
+        }
         // the gates of the row's next 32 columns, asked for ahead
         uint4 gates[4];
         const bf16* grow = sh.gate != nullptr && row < rows ? sh.gate + (size_t)(tok0 + row0 + row) * sh.ldg + h * dv : nullptr;
@@ -1190,6 +1231,46 @@ __global__ void __launch_bounds__(192) attn_prefill_tc_kernel(
     }
     tc5::fence_before();
     __syncthreads();
+    if (splits > 1) {
+        // (every CTA of the cluster passes both barriers, whatever happened before: they share the tile)
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (active && !*abort_flag) {
+            const uint32_t os = tma::smem_u32(smem), ml = tma::smem_u32(bars + 32);
+            const int share = (rows + splits - 1) / splits, r1 = min(rows, ((int)blockIdx.z + 1) * share);
+            for (int r = (int)blockIdx.z * share + warp; r < r1; r += 6) {
+                float m[8], l[8], M = -INFINITY;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    m[q] = -INFINITY; l[q] = 0.f;
+                    if (q < splits) attn_remote(ml + 8u * (uint32_t)r, q, m[q], l[q]);
+                    M = fmaxf(M, m[q]);
+                }
+                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                float ls = 0.f;
+                if (lane < DV / 4) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        if (q >= splits) break;
+                        const float f = m[q] == -INFINITY ? 0.f : fast_exp2(m[q] - M);
+                        const float4 v = attn_remote4(os + 16u * (uint32_t)(r * (DV / 4) + (lane ^ (r & 7))), q);
+                        ls = fmaf(l[q], f, ls);
+                        acc.x = fmaf(v.x, f, acc.x); acc.y = fmaf(v.y, f, acc.y); acc.z = fmaf(v.z, f, acc.z); acc.w = fmaf(v.w, f, acc.w);
+                    }
+                }
+                ls = attn_sink_sum(ls, M, sink, h);
+                const float inv = ls > 0.f ? out_scale / ls : 0.f;
+                const int tok = tok0 + row0 + r, c = 4 * lane;
+                if (c < dv && lane < DV / 4) {
+                    const float x = attn_gate(acc.x * inv, sh, tok, h * dv + c), y = attn_gate(acc.y * inv, sh, tok, h * dv + c + 1);
+                    const float z = attn_gate(acc.z * inv, sh, tok, h * dv + c + 2), w = attn_gate(acc.w * inv, sh, tok, h * dv + c + 3);
+                    *reinterpret_cast<uint2*>(out + ((size_t)tok * nq + h) * dv + c) = make_uint2(pack_bf16(x, y), pack_bf16(z, w));
+                }
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
     if (*abort_flag) {
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000LL) { }
@@ -1364,28 +1445,30 @@ static int launch_attn_prefill_tc(const CUtensorMap& tq, const CUtensorMap& tk, 
                                   const int* cu_seqlens, const int* ctx_lens, const int* seq_of_token, const int* page_table,
                                   int max_pages, int n_seqs, int nq, int nkv, float scale_log2, int window, const float* sink,
                                   float out_scale, int n_pages, int* status, const AttnShape& sh, cudaStream_t stream) {
-    // Q, K x 2, V x 2 (boxes of 64 columns: 16 KB of Q, 8 KB of K or V), barriers
-    constexpr int smem = (DK / 64) * (16384 + 2 * 8192) + (DV / 64) * 2 * 8192 + 256;
+    // Q, K x 2, V x 2 (boxes of 64 columns: 16 KB of Q, 8 KB of K or V), barriers, the rows' maxima and sums
+    constexpr int smem = (DK / 64) * (16384 + 2 * 8192) + (DV / 64) * 2 * 8192 + 256 + 1024;
+    static_assert(smem - 1280 >= 128 * DV * 4, "the float32 rows that a cluster adds lie where Q, K and V were");
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<DK, DV, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    return gg_launch(attn_prefill_tc_kernel<DK, DV, EXACT>, grid, dim3(192), smem, stream, 1, tq, tk, tv, (bf16*)out, cu_seqlens,
+    return gg_launch(attn_prefill_tc_kernel<DK, DV, EXACT>, grid, dim3(192), smem, stream, (int)grid.z, tq, tk, tv, (bf16*)out, cu_seqlens,
                      ctx_lens, seq_of_token, page_table, max_pages, n_seqs, nq, nkv, scale_log2, window, sink, out_scale, n_pages,
                      status, sh);
 }
 
 // Prefill attention on tcgen05 (see attn_prefill_tc_kernel).  q [n_tokens, nq, d], out [n_tokens, nq, dv] bf16; pools
 // [page][nkv][64][d] and [..][dv]; max_tiles >= sum over sequences of ceil(new tokens / 128); status as in the
-// tensor-core product (codes 21-28 name the wait that ran out).
+// tensor-core product (codes 21-28 name the wait that ran out).  splits (1 to 8): CTAs that share a tile's pages.
 GG_API gg_attn_prefill_tc(const void* q, const void* k_pool, const void* v_pool, void* out, const int* cu_seqlens,
                           const int* ctx_lens, const int* seq_of_token, const int* page_table, int max_pages,
                           int page_size, int n_pages, int n_tokens, int n_seqs, int max_tiles, int nq, int nkv, int d, int dv,
-                          float scale, int window, int chunk, const float* sink, float out_scale, const void* gate, long long ldg,
+                          float scale, int window, int chunk, int splits, const float* sink, float out_scale, const void* gate, long long ldg,
                           int* status, cudaStream_t stream) {
     if (n_seqs <= 0 || max_tiles <= 0 || n_tokens <= 0) return 0;
+    if (splits < 1 || splits > 8) return GG_ERR_ARG;
     if (page_size != PAGE || nq <= 0 || nkv <= 0 || nq % nkv || nq > 65535 || max_tiles > 65535 ||
         n_pages <= 0 || status == nullptr || !attn_shape_ok(d, dv, chunk, gate, ldg))
         return GG_ERR_ARG;
@@ -1398,7 +1481,7 @@ GG_API gg_attn_prefill_tc(const void* q, const void* k_pool, const void* v_pool,
     if ((rc = tma::make_map_bf16(&tv, v_pool, rows, dv, dv, PAGE)) != 0) return rc;
     const float scale_log2 = scale * 1.4426950408889634f;
     const AttnShape sh = {d, dv, chunk, (const bf16*)gate, ldg};
-    GG_ATTN_SIZES(launch_attn_prefill_tc, tq, tk, tv, dim3(nq, max_tiles), out, cu_seqlens, ctx_lens, seq_of_token, page_table,
+    GG_ATTN_SIZES(launch_attn_prefill_tc, tq, tk, tv, dim3(nq, max_tiles, splits), out, cu_seqlens, ctx_lens, seq_of_token, page_table,
                   max_pages, n_seqs, nq, nkv, scale_log2, window, sink, out_scale, n_pages, status, sh, stream);
 }
 

@@ -66,15 +66,25 @@ def attn_prefill(q, k_pool, v_pool, out, cu_seqlens, ctx_lens, seq_of_token, tab
 
 def attn_prefill_tc(q, k_pool, v_pool, out, cu_seqlens, ctx_lens, seq_of_token, table, page_size, n_tokens,
                     n_seqs, max_tiles, nq, nkv, d, scale, window, sink=None, out_scale: float = 1.0,
-                    dv: Optional[int] = None, chunk: int = 0, gate=None) -> None:
-    """Prefill attention on tcgen05: 128-query tiles, S and O in tensor memory."""
+                    dv: Optional[int] = None, chunk: int = 0, gate=None, splits: int = 1) -> None:
+    """Prefill attention on tcgen05: 128-query tiles, S and O in tensor memory; the pages of a tile shared by `splits` CTAs."""
     from .tcgen05_gemm import status_word
     kernel("attention_fast", "gg_attn_prefill_tc")(
         q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(), cu_seqlens.data_ptr(),
         ctx_lens.data_ptr(), seq_of_token.data_ptr(), table.data_ptr(), table.shape[-1], page_size,
         k_pool.shape[0], n_tokens, n_seqs, max_tiles, nq, nkv, d, d if dv is None else int(dv), float(scale), int(window),
-        int(chunk), sink.data_ptr() if sink is not None else 0, float(out_scale), *_gate(gate),
+        int(chunk), int(splits), sink.data_ptr() if sink is not None else 0, float(out_scale), *_gate(gate),
         status_word(q.device).data_ptr(), stream_ptr())
+
+
+def prefill_splits(n_tokens: int, n_seqs: int, nq: int, reach: int) -> int:
+    """CTAs that share the pages of a query tile which reads up to `reach` positions.  The device holds 296 CTAs; where the
+    (tile, head) pairs leave places free and a share keeps four pages, the pages are split.  Powers of two only: clusters of
+    three or six filled the chip worse than two or four (16 heads, 333 tokens, 6,433 positions, in 1 / 3 / 4 / 6 shares:
+    84 / 43 / 37 / 52 us; 32 heads in 1 / 2 / 3 / 4: 84 / 60 / 74 / 64)."""
+    tiles = -(-n_tokens // 128) if n_seqs == 1 else n_tokens // 128 + n_seqs
+    most = min(296 // (tiles * nq), reach // 256, 8)
+    return 1 << (most.bit_length() - 1) if most > 1 else 1
 
 
 def takes(nq: int, nkv: int, d: int, dv: int) -> bool:
@@ -107,11 +117,14 @@ def try_make(nq: int, nkv: int, d: int, scale: float, window: int, dv: Optional[
                 splits = min(splits, 8)
             attn_decode_tma(q, k_pool, v_pool, out, ctx.positions, ctx.seq_of_token, table, page_size, T, nq, nkv, d,
                             scale, window, splits, cluster=True, **kw)
-        elif ctx.max_new >= 32:
-            # 128-query tiles on tcgen05 (S and O in tensor memory)
-            max_tiles = T // 128 + ctx.n_seqs
+            return
+        splits = prefill_splits(T, ctx.n_seqs, nq, min([ctx.max_ctx] + [n + 192 for n in (window, chunk) if n]))
+        if ctx.max_new >= 32 or splits > 1:
+            # 128-query tiles on tcgen05 (S and O in tensor memory); a few tokens per sequence too where their history is long
+            # enough to be shared (10 tokens on 6,000, 32 heads: 25 us against 187)
+            max_tiles = -(-T // 128) if ctx.n_seqs == 1 else T // 128 + ctx.n_seqs
             attn_prefill_tc(q, k_pool, v_pool, out, ctx.cu_seqlens, ctx.ctx_lens, ctx.seq_of_token, table, page_size,
-                            T, ctx.n_seqs, max_tiles, nq, nkv, d, scale, window, **kw)
+                            T, ctx.n_seqs, max_tiles, nq, nkv, d, scale, window, splits=splits, **kw)
         else:
             # a few tokens per sequence: 64-query tiles on mma.sync waste less
             max_tiles = T // 64 + ctx.n_seqs
