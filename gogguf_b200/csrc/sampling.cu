@@ -384,7 +384,8 @@ __device__ __forceinline__ unsigned long long best_key(float x, int id) {
 // warp's words into one of three rotating sets in shared memory, and after one barrier every thread reads
 // the totals and takes the same decision.  The low 32 bits (the ids) are only walked when the k-th place
 // falls among equal values.
-template <typename KeyOf>
+// N > 0: that many keys for every thread, known here (keys in registers need it), else n_mine.
+template <int N = 0, typename KeyOf>
 __device__ unsigned long long block_kth_largest(int n_mine, KeyOf key_of, int k, unsigned long long (*tot)[4]) {
     const int lane = threadIdx.x & 31;
     unsigned long long prefix = 0;
@@ -399,7 +400,8 @@ __device__ unsigned long long block_kth_largest(int n_mine, KeyOf key_of, int k,
         const uint32_t mask_above = shift == 28 ? 0u : (0xffffffffu << (shift + 4));     // the digits decided in this word
         if (threadIdx.x < 4) tot[(pass + 1) % 3][threadIdx.x] = 0ull;     // last read two passes ago
         unsigned long long c4[4] = {0ull, 0ull, 0ull, 0ull};
-        for (int j = 0; j < n_mine; ++j) {
+#pragma unroll
+        for (int j = 0; j < (N > 0 ? N : n_mine); ++j) {
             const unsigned long long key = key_of(j);
             const uint32_t hi = (uint32_t)(key >> 32), lo = (uint32_t)key;
             const uint32_t word = pass < 8 ? hi : lo;
@@ -443,15 +445,18 @@ __device__ unsigned long long block_kth_largest(int n_mine, KeyOf key_of, int k,
 // Stage one: grid (slices, rows), 256 threads with 32 logits each (the per-pass cost of a thread is mostly fixed:
 // shuffles, the barrier, the decision).  cand[(row * slices + slice) * k + j]: the slice's k best keys (0 = none).
 //
-// Walking the digits of all 8,192 keys costs 32 keys a thread and pass, which is what bounds this kernel.  So for k up to
-// SAMP_SIEVE_K a threshold comes first: a thread's 32 keys make four groups of eight, and the k-th best of the 1,024
-// groups' best is a key that at least k keys reach (one per group), so the k best are among the keys that reach it.  In
-// a row without order those are k to 1.4 k of the 8,192; they go to shared memory and the digits of only these, at most
-// four a thread, are walked.  Where more than SAMP_SIEVE_ROOM reach it (large logits side by side) all keys are walked as for
-// larger k, where the sieve would let most keys through.
+// What bounds it is instructions: a pass over the digits is some 300 a thread with four keys, several times that with 32.  So a
+// threshold on the value comes first: the keys form groups, and at least k keys reach the k-th largest of the groups'
+// largest (one per group), so the k best are among the keys that reach it.  In a row without order those are k to
+// 1.4 k of the 8,192.  For k up to 64: 128 groups of 64 (two threads each), the k-th found by counting, and the survivors ranked by
+// counting too.  Up to SAMP_SIEVE_K: 1,024 groups of eight, the k-th and then the survivors' k-th by digits, at most four keys
+// a thread.  Where more than SAMP_SIEVE_ROOM pass (large logits side by side) the digits of all keys are walked, as for larger k,
+// where the sieve would let most through.  64 rows of 151,936, k = 20: all keys by digits 187 us, the larger sieve alone
+// 121, as it is 19.
 #define SAMP_SLICE_THREADS 256
 #define SAMP_SLICE_PER (SAMP_SLICE / SAMP_SLICE_THREADS)
 #define SAMP_SIEVE_K 512
+#define SAMP_COUNT_K 64
 #define SAMP_SIEVE_ROOM 1024
 
 __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const float* logits, long long ld, int V, float temp,
@@ -460,34 +465,66 @@ __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const fl
     pdl_wait();
     __shared__ unsigned long long tot[3][4];
     __shared__ unsigned long long room[SAMP_SIEVE_ROOM];
+    __shared__ __align__(16) uint32_t tops[SAMP_SLICE_THREADS / 2];
     __shared__ int n_out, n_room;
-    const int row = blockIdx.y, slice = blockIdx.x, tid = threadIdx.x;
+    __shared__ uint32_t at_least;
+    const int row = blockIdx.y, slice = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const float* x = logits + (size_t)row * ld;
     const bool scale = temp > 0.f && temp != 1.f;
     const double inv_temp = scale ? 1.0 / (double)temp : 1.0;
-    unsigned long long keys[SAMP_SLICE_PER];
+    const int id0 = slice * SAMP_SLICE + tid;                // this thread's logits: id0 + 256 u
+    float raw[SAMP_SLICE_PER];
 #pragma unroll
-    for (int u = 0; u < SAMP_SLICE_PER; ++u) {
-        const int i = slice * SAMP_SLICE + u * SAMP_SLICE_THREADS + tid;
-        float v = i < V ? x[i] : 0.f;
-        if (scale) v = (float)((double)v * inv_temp);
-        keys[u] = i < V ? best_key(v, i) : 0ull;
+    for (int u = 0; u < SAMP_SLICE_PER; ++u) raw[u] = id0 + u * SAMP_SLICE_THREADS < V ? x[id0 + u * SAMP_SLICE_THREADS] : 0.f;
+    uint32_t val[SAMP_SLICE_PER];                            // ordered values; 0 beyond the row
+    if (scale) {
+#pragma unroll
+        for (int u = 0; u < SAMP_SLICE_PER; ++u) raw[u] = (float)((double)raw[u] * inv_temp);
     }
-    if (tid == 0) { n_out = 0; n_room = 0; }
+#pragma unroll
+    for (int u = 0; u < SAMP_SLICE_PER; ++u) val[u] = id0 + u * SAMP_SLICE_THREADS < V ? order_key(raw[u]) : 0u;
+    auto key_of = [&](int u) -> unsigned long long {
+        const int id = id0 + u * SAMP_SLICE_THREADS;
+        return id < V ? ((unsigned long long)val[u] << 32) | (unsigned long long)(0xffffffffu - (uint32_t)id) : 0ull;
+    };
+    if (tid == 0) { n_out = 0; n_room = 0; at_least = 0xffffffffu; }
     unsigned long long* dst = cand + ((size_t)row * gridDim.x + slice) * k;
-    unsigned long long thr;
     bool sieved = false;
     if (k <= SAMP_SIEVE_K) {
-        unsigned long long best[4] = {0ull, 0ull, 0ull, 0ull};
+        uint32_t sieve;
+        if (k <= SAMP_COUNT_K) {
+            uint32_t top = 0u;
 #pragma unroll
-        for (int u = 0; u < SAMP_SLICE_PER; ++u) best[u & 3] = best[u & 3] > keys[u] ? best[u & 3] : keys[u];
-        const unsigned long long sieve = block_kth_largest(4, [&](int j) { return best[j]; }, k, tot);
-        // (0: fewer than k groups hold a key, as in a short last slice: every key passes)
+            for (int u = 0; u < SAMP_SLICE_PER; ++u) top = max(top, val[u]);
+            top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+            if ((lane & 1) == 0) tops[tid >> 1] = top;
+            __syncthreads();
+            if (tid < SAMP_SLICE_THREADS / 2) {
+                const uint32_t mine = tops[tid];
+                int above = 0;
+#pragma unroll 8
+                for (int j = 0; j < SAMP_SLICE_THREADS / 2; j += 4) {
+                    const uint4 t = *reinterpret_cast<const uint4*>(tops + j);
+                    above += (t.x > mine) + (t.y > mine) + (t.z > mine) + (t.w > mine);
+                }
+                // (the smallest value that fewer than k others exceed is the k-th largest)
+                const uint32_t least = __reduce_min_sync(0xffffffffu, above < k ? mine : 0xffffffffu);
+                if (lane == 0) atomicMin(&at_least, least);
+            }
+            __syncthreads();
+            sieve = at_least;
+        } else {
+            uint32_t best[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int u = 0; u < SAMP_SLICE_PER; ++u) best[u & 3] = max(best[u & 3], val[u]);
+            // (equal values are fine here: only the threshold is asked for; 0: fewer than k groups, every key passes)
+            sieve = (uint32_t)(block_kth_largest<4>(4, [&](int j) { return best[j] != 0u ? ((unsigned long long)best[j] << 32) | 1ull : 0ull; }, k, tot) >> 32);
+        }
 #pragma unroll
         for (int u = 0; u < SAMP_SLICE_PER; ++u) {
-            if (keys[u] != 0ull && keys[u] >= sieve) {
+            if (val[u] >= sieve && id0 + u * SAMP_SLICE_THREADS < V) {
                 const int at = atomicAdd(&n_room, 1);
-                if (at < SAMP_SIEVE_ROOM) room[at] = keys[u];
+                if (at < SAMP_SIEVE_ROOM) room[at] = key_of(u);
             }
         }
         __syncthreads();
@@ -495,11 +532,22 @@ __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const fl
     }
     if (sieved) {
         const int n = n_room;
+        if (n <= SAMP_SLICE_THREADS) {                       // ranks by counting: no two keys are equal
+            if (tid < n) {
+                const unsigned long long mine = room[tid];
+                int above = 0;
+                for (int j = 0; j < n; ++j) above += room[j] > mine;
+                if (above < k) dst[above] = mine;
+            }
+            for (int j = n + tid; j < k; j += SAMP_SLICE_THREADS) dst[j] = 0ull;
+            return;
+        }
         unsigned long long mine[SAMP_SIEVE_ROOM / SAMP_SLICE_THREADS];
 #pragma unroll
         for (int u = 0; u < SAMP_SIEVE_ROOM / SAMP_SLICE_THREADS; ++u)
             mine[u] = u * SAMP_SLICE_THREADS + tid < n ? room[u * SAMP_SLICE_THREADS + tid] : 0ull;
-        thr = block_kth_largest((n + SAMP_SLICE_THREADS - 1) / SAMP_SLICE_THREADS, [&](int j) { return j == 0 ? mine[0] : (j == 1 ? mine[1] : (j == 2 ? mine[2] : mine[3])); }, k, tot);
+        const unsigned long long thr = block_kth_largest((n + SAMP_SLICE_THREADS - 1) / SAMP_SLICE_THREADS,
+            [&](int j) { return j == 0 ? mine[0] : (j == 1 ? mine[1] : (j == 2 ? mine[2] : mine[3])); }, k, tot);
         for (int j = tid; j < k; j += SAMP_SLICE_THREADS) dst[j] = 0ull;
         __syncthreads();
 #pragma unroll
@@ -507,12 +555,12 @@ __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const fl
             if (mine[u] != 0ull && mine[u] >= thr) dst[atomicAdd(&n_out, 1)] = mine[u];
         return;
     }
-    thr = block_kth_largest(SAMP_SLICE_PER, [&](int j) { return keys[j]; }, k, tot);
+    const unsigned long long thr = block_kth_largest<SAMP_SLICE_PER>(SAMP_SLICE_PER, key_of, k, tot);
     for (int j = tid; j < k; j += SAMP_SLICE_THREADS) dst[j] = 0ull;
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < SAMP_SLICE_PER; ++u)
-        if (keys[u] != 0ull && keys[u] >= thr) dst[atomicAdd(&n_out, 1)] = keys[u];
+        if (key_of(u) != 0ull && key_of(u) >= thr) dst[atomicAdd(&n_out, 1)] = key_of(u);
 }
 
 // Inclusive prefix sums of one double per thread over the block, in thread order; *total gets the block's sum.

@@ -15,7 +15,7 @@ def test_uniforms_of_a_batch():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("V", [40, 8192, 8200, 30011])
-@pytest.mark.parametrize("top_k", [1, 20, 511, 512, 513])
+@pytest.mark.parametrize("top_k", [1, 20, 64, 65, 511, 512, 513])
 def test_rows_through_the_sieve(V, top_k):
     from gogguf_b200.sampling.sampler import Sampler, SamplerConfig, sample_host, uniform01
     g = torch.Generator().manual_seed(V + top_k)
