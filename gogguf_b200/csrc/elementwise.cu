@@ -449,9 +449,10 @@ __global__ void qk_norm_rope_cache_kernel(
     }
 }
 
-// bfloat16 form for a full rotation (rot == d) and d = 64, 128 or 256.  D / 16 lanes share one head: a lane
-// owns eight pairs (i, i + d/2), i = 8 * sub .. + 8, so both halves of a pair sit in the same thread and
-// every access to the head is 16 bytes wide; a warp handles 32 / (D / 16) heads at once (four of size 128),
+// bfloat16 form for d = 64, 128 or 256 and rotations of a multiple of 16 elements.  D / 16 lanes share one head: the
+// first rot / 16 of them own eight pairs (i, i + rot/2), i = 8 * sub .. + 8, so both halves of a pair sit in the same thread,
+// the others 16 neighbouring elements behind the rotated ones (2,048 tokens, 32 heads of 128, of which 64 turn: 25 us in
+// the form with a lane per element, 13 here), and every access to the head is 16 bytes wide; a warp handles 32 / (D / 16) heads at once (four of size 128),
 // which keeps 1 KB in flight per warp.  The head's sum of squares is added over its lanes by shuffles.
 template <int D>
 __global__ void __launch_bounds__(128) qk_norm_rope_cache_vec_kernel(
@@ -460,10 +461,10 @@ __global__ void __launch_bounds__(128) qk_norm_rope_cache_vec_kernel(
     const float* cosv, const float* sinv,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token,
     const int* __restrict__ page_table, int max_pages, int page_size,
-    bf16* __restrict__ k_pool, bf16* __restrict__ v_pool, int ntok, int nq, int nkv, const PageBounds pb) {
+    bf16* __restrict__ k_pool, bf16* __restrict__ v_pool, int ntok, int nq, int nkv, int rot, const PageBounds pb) {
     pdl_launch();
     pdl_wait();
-    constexpr int HALF = D / 2, LPH = D / 16, HPW = 32 / LPH;      // lanes per head, heads per warp
+    constexpr int LPH = D / 16, HPW = 32 / LPH;      // lanes per head, heads per warp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nheads = nq + 2 * nkv;
     const long long item = ((long long)blockIdx.x * (blockDim.x >> 5) + warp) * HPW + lane / LPH;
@@ -486,26 +487,31 @@ __global__ void __launch_bounds__(128) qk_norm_rope_cache_vec_kernel(
             else dst = (is_k ? k_pool : v_pool) + (((size_t)page * nkv + kvh) * page_size + (pos % page_size)) * D;
         }
     }
-    const int i0 = sub * 8;             // first index of this lane in the low half
+    const bool turns = sub < rot / 16;
+    const int i0 = turns ? sub * 8 : rot + 16 * (sub - rot / 16), i1 = turns ? i0 + rot / 2 : i0 + 8;     // this lane's two runs of eight
     uint4 lo4 = make_uint4(0, 0, 0, 0), hi4 = make_uint4(0, 0, 0, 0);
     if (live) {
         lo4 = *reinterpret_cast<const uint4*>(src + i0);
-        hi4 = *reinterpret_cast<const uint4*>(src + i0 + HALF);
+        hi4 = *reinterpret_cast<const uint4*>(src + i1);
     }
     if (live && !is_q && !is_k) {       // value head: plain copy
         *reinterpret_cast<uint4*>(dst + i0) = lo4;
-        *reinterpret_cast<uint4*>(dst + i0 + HALF) = hi4;
+        *reinterpret_cast<uint4*>(dst + i1) = hi4;
     }
     const bool rotate = live && (is_q || is_k);
     const float* w = is_q ? qw : kw;
     float4 cs[2], sn[2], wl[2], wh[2];
     if (rotate) {                       // asked for before the sum of squares is known
-        const float4* cp = reinterpret_cast<const float4*>(cosv + (size_t)t * HALF + i0);
-        const float4* sp = reinterpret_cast<const float4*>(sinv + (size_t)t * HALF + i0);
-        cs[0] = cp[0]; cs[1] = cp[1]; sn[0] = sp[0]; sn[1] = sp[1];
+        cs[0] = cs[1] = make_float4(1.f, 1.f, 1.f, 1.f);
+        sn[0] = sn[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (turns) {
+            const float4* cp = reinterpret_cast<const float4*>(cosv + (size_t)t * (rot / 2) + i0);
+            const float4* sp = reinterpret_cast<const float4*>(sinv + (size_t)t * (rot / 2) + i0);
+            cs[0] = cp[0]; cs[1] = cp[1]; sn[0] = sp[0]; sn[1] = sp[1];
+        }
         if (w != nullptr) {
             wl[0] = reinterpret_cast<const float4*>(w + i0)[0]; wl[1] = reinterpret_cast<const float4*>(w + i0)[1];
-            wh[0] = reinterpret_cast<const float4*>(w + i0 + HALF)[0]; wh[1] = reinterpret_cast<const float4*>(w + i0 + HALF)[1];
+            wh[0] = reinterpret_cast<const float4*>(w + i1)[0]; wh[1] = reinterpret_cast<const float4*>(w + i1)[1];
         }
     }
     const bf16* lo = reinterpret_cast<const bf16*>(&lo4);
@@ -531,11 +537,11 @@ __global__ void __launch_bounds__(128) qk_norm_rope_cache_vec_kernel(
     for (int k = 0; k < 8; ++k) {
         const float x0 = a[k] * scale * (w != nullptr ? wlf[k] : 1.f);
         const float x1 = c[k] * scale * (w != nullptr ? whf[k] : 1.f);
-        ol[k] = __float2bfloat16_rn(x0 * csf[k] - x1 * snf[k]);
-        oh[k] = __float2bfloat16_rn(x0 * snf[k] + x1 * csf[k]);
+        ol[k] = __float2bfloat16_rn(turns ? x0 * csf[k] - x1 * snf[k] : x0);
+        oh[k] = __float2bfloat16_rn(turns ? x0 * snf[k] + x1 * csf[k] : x1);
     }
     *reinterpret_cast<uint4*>(dst + i0) = olo;
-    *reinterpret_cast<uint4*>(dst + i0 + HALF) = ohi;
+    *reinterpret_cast<uint4*>(dst + i1) = ohi;
 }
 
 GG_API gg_qk_norm_rope_cache(const void* qkv, int dtype, void* q_out, const float* qw, const float* kw, float eps,
@@ -549,12 +555,12 @@ GG_API gg_qk_norm_rope_cache(const void* qkv, int dtype, void* q_out, const floa
     const unsigned grid = (unsigned)((total + warps - 1) / warps);
     const bool al = ((((uintptr_t)qkv) | ((uintptr_t)q_out) | ((uintptr_t)k_pool) | ((uintptr_t)v_pool) |
                       ((uintptr_t)cosv) | ((uintptr_t)sinv) | ((uintptr_t)qw) | ((uintptr_t)kw)) & 15) == 0;
-    if (dtype == GG_BF16 && rot == d && al && (d == 64 || d == 128 || d == 256)) {
+    if (dtype == GG_BF16 && rot % 16 == 0 && al && (d == 64 || d == 128 || d == 256)) {
         const int per_block = warps * (32 / (d / 16));          // heads a block of four warps handles
         const unsigned vgrid = (unsigned)((total + per_block - 1) / per_block);
 #define GG_QK_VEC(D_) gg_launch(qk_norm_rope_cache_vec_kernel<D_>, dim3(vgrid), dim3(warps * 32), 0, stream, 1,  \
             (const bf16*)qkv, (bf16*)q_out, qw, kw, eps, cosv, sinv, positions, seq_of_token, page_table, max_pages, \
-            page_size, (bf16*)k_pool, (bf16*)v_pool, ntok, nq, nkv, PageBounds{n_pages, status})
+            page_size, (bf16*)k_pool, (bf16*)v_pool, ntok, nq, nkv, rot, PageBounds{n_pages, status})
         if (d == 64) GG_QK_VEC(64); else if (d == 128) GG_QK_VEC(128); else GG_QK_VEC(256);
 #undef GG_QK_VEC
         return gg_last_error();

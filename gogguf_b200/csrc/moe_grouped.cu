@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(256) moe_place_gather_kernel(const bf16* h, co
             tie[j] = 0;
         }
     }
+#pragma unroll 4
     for (int q = threadIdx.x; q < P; q += 256) {
         const int v = idx[q], e = v < 0 ? E : v;
 #pragma unroll
@@ -83,17 +84,22 @@ __global__ void __launch_bounds__(256) moe_place_gather_kernel(const bf16* h, co
     if (idx[p] < 0) return;                               // no product reads its row
     const uint4* src = reinterpret_cast<const uint4*>(h + (size_t)(p / top) * W);
     uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)at * W);
-    for (int i = lane; i < W / 8; i += 32) {
-        uint4 v = src[i];
-        if (weight_on_input) {
-            __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&v);
+    for (int i0 = lane; i0 < W / 8; i0 += 4 * 32) {           // four loads, then four stores
+        uint4 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float2 f = __bfloat1622float2(b[u]);
-                b[u] = __floats2bfloat162_rn(f.x * wt, f.y * wt);
+        for (int k = 0; k < 4; ++k) v[k] = src[min(i0 + 32 * k, W / 8 - 1)];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (weight_on_input) {
+                __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&v[k]);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float2 f = __bfloat1622float2(b[u]);
+                    b[u] = __floats2bfloat162_rn(f.x * wt, f.y * wt);
+                }
             }
+            if (i0 + 32 * k < W / 8) dst[i0 + 32 * k] = v[k];
         }
-        dst[i] = v;
     }
 }
 

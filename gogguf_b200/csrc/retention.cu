@@ -597,6 +597,263 @@ __global__ void __launch_bounds__(256, 2) ret_chunk_out_kernel(
     }
 }
 
+// ----------------------------------------------------------------------------- chunks, four elements an access
+// The same two kernels for d in multiples of 32 (whole groups of eight chunks), dv and rot of eight, rows on 16-byte boundaries.  A prompt of 2,048 tokens and 8
+// heads is 256 CTAs, all resident at once, so what counts is how long one takes: element loads one after another behind
+// integer divisions, and a shared-memory read for every two multiply-adds.  Here a thread asks for all of its rows' pieces at
+// once (four times eight elements), operands come 16 bytes a read (a thread's columns and rows are runs of four), and rows
+// that are read across have their 16-byte chunks at place c ^ (row & 7).  Same sums in the same order.  2,048 tokens, 8 heads of
+// 128 x 128: states 57 -> 20 us, outputs 101 -> 49 us.
+template <typename T> __device__ __forceinline__ float4 ret_ld4(const T* p);
+template <> __device__ __forceinline__ float4 ret_ld4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 ret_ld4<bf16>(const bf16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float4 f4_mul(float4 a, float f) { return make_float4(a.x * f, a.y * f, a.z * f, a.w * f); }
+// place of 16-byte chunk c of row r, in floats
+template <bool SWZ> __device__ __forceinline__ int ret_place(int r, int c, int stride) { return r * stride + 4 * (SWZ ? c ^ (r & 7) : c); }
+
+// Rotated q (WITH_Q) and k (times kscale and wk[j], where given) and v of the n tokens from t0 on; q and k rows of d floats
+// (chunks swizzled with SWZ), v rows of dv.  256 threads; a piece is eight elements of q and k: two runs of four that turn
+// together, or eight neighbours behind the rotated ones.
+template <typename T, bool WITH_Q, bool SWZ>
+__device__ __forceinline__ void ret_stage_vec(const T* qkvg, int ld, int t0, int n, int h, int H, int d, int dv, int rot, float kscale,
+                                              const float* cosv, const float* sinv, float* qs, float* ks, float* vs, const float* wk) {
+    constexpr int IT = RET_PC * RET_PMAX / 8 / 256;          // pieces a thread has at most: 4
+    const int per = d / 8, half = rot / 2, rp = rot / 8;
+    float4 q0[WITH_Q ? IT : 1], q1[WITH_Q ? IT : 1], k0[IT], k1[IT], cs[IT], sn[IT];
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+        const int idx = min((int)threadIdx.x + 256 * it, n * per - 1), tt = idx / per, m = idx - tt * per;
+        const bool turns = m < rp;
+        const int i0 = turns ? 4 * m : 8 * m, i1 = turns ? half + 4 * m : 8 * m + 4;
+        const T* qp = qkvg + (size_t)(t0 + tt) * ld + h * d;
+        const T* kp = qp + (size_t)H * d;
+        if (WITH_Q) { q0[it] = ret_ld4<T>(qp + i0); q1[it] = ret_ld4<T>(qp + i1); }
+        k0[it] = ret_ld4<T>(kp + i0); k1[it] = ret_ld4<T>(kp + i1);
+        cs[it] = make_float4(1.f, 1.f, 1.f, 1.f); sn[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (turns) {
+            cs[it] = *reinterpret_cast<const float4*>(cosv + (size_t)(t0 + tt) * half + i0);
+            sn[it] = *reinterpret_cast<const float4*>(sinv + (size_t)(t0 + tt) * half + i0);
+        }
+    }
+    auto lo = [](float4 a, float4 b, float4 c, float4 s) { return make_float4(a.x * c.x - b.x * s.x, a.y * c.y - b.y * s.y, a.z * c.z - b.z * s.z, a.w * c.w - b.w * s.w); };
+    auto hi = [](float4 a, float4 b, float4 c, float4 s) { return make_float4(a.x * s.x + b.x * c.x, a.y * s.y + b.y * c.y, a.z * s.z + b.z * c.z, a.w * s.w + b.w * c.w); };
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+        const int idx = (int)threadIdx.x + 256 * it;
+        if (idx < n * per) {
+            const int tt = idx / per, m = idx - tt * per;
+            const bool turns = m < rp;
+            const int i0 = turns ? 4 * m : 8 * m, i1 = turns ? half + 4 * m : 8 * m + 4;
+            if (WITH_Q) {
+                *reinterpret_cast<float4*>(qs + ret_place<SWZ>(tt, i0 / 4, d)) = turns ? lo(q0[it], q1[it], cs[it], sn[it]) : q0[it];
+                *reinterpret_cast<float4*>(qs + ret_place<SWZ>(tt, i1 / 4, d)) = turns ? hi(q0[it], q1[it], cs[it], sn[it]) : q1[it];
+            }
+            const float w = wk != nullptr ? wk[tt] : 1.f;
+            *reinterpret_cast<float4*>(ks + ret_place<SWZ>(tt, i0 / 4, d)) = f4_mul(f4_mul(turns ? lo(k0[it], k1[it], cs[it], sn[it]) : k0[it], kscale), w);
+            *reinterpret_cast<float4*>(ks + ret_place<SWZ>(tt, i1 / 4, d)) = f4_mul(f4_mul(turns ? hi(k0[it], k1[it], cs[it], sn[it]) : k1[it], kscale), w);
+        }
+    }
+    const int vper = dv / 4;
+    float4 v[2 * IT];
+#pragma unroll
+    for (int it = 0; it < 2 * IT; ++it) {
+        const int idx = min((int)threadIdx.x + 256 * it, n * vper - 1), tt = idx / vper, m = idx - tt * vper;
+        v[it] = ret_ld4<T>(qkvg + (size_t)(t0 + tt) * ld + (size_t)2 * H * d + h * dv + 4 * m);
+    }
+#pragma unroll
+    for (int it = 0; it < 2 * IT; ++it) {
+        const int idx = (int)threadIdx.x + 256 * it;
+        if (idx < n * vper) *reinterpret_cast<float4*>(vs + (size_t)idx * 4) = v[it];
+    }
+}
+
+// acc[4 rows or runs][4 columns] += a (four scalars) times b (a run of four)
+__device__ __forceinline__ void f4_fma(float4& o, float a, float4 b) {
+    o.x = fmaf(a, b.x, o.x); o.y = fmaf(a, b.y, o.y); o.z = fmaf(a, b.z, o.z); o.w = fmaf(a, b.w, o.w);
+}
+
+// a thread: rows 4 ty + {0..3} and 64 + 4 ty + {0..3} of the state, columns 4 tx + {0..3} and 64 + 4 tx + {0..3}
+template <typename T>
+__global__ void __launch_bounds__(256, 2) ret_chunk_state_vec_kernel(
+    const T* qkvg, int ld, float* U, const float* cosv, const float* sinv, const int* __restrict__ cu_seqlens,
+    const int* __restrict__ seq_of_token, const float* __restrict__ decay, int n_seqs, int H, int d, int dv, int rot, float kscale) {
+    pdl_launch();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    int b, t0, n;
+    if (!ret_find_chunk(blockIdx.x, cu_seqlens, seq_of_token, n_seqs, b, t0, n)) return;
+    const int h = blockIdx.y;
+    float* ks = sm;                        // [PC][d], already times decay^(n-1-j)
+    float* vs = ks + RET_PC * d;           // [PC][dv]
+    float* wk = vs + RET_PC * dv;          // [PC]
+    const float a = decay[h];
+    if (threadIdx.x < n) {
+        float p = 1.f;
+        for (int i = 0; i < n - 1 - (int)threadIdx.x; ++i) p *= a;
+        wk[threadIdx.x] = p;
+    }
+    __syncthreads();
+    ret_stage_vec<T, false, false>(qkvg, ld, t0, n, h, H, d, dv, rot, kscale, cosv, sinv, nullptr, ks, vs, wk);
+    __syncthreads();
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    float4 acc[8][2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    // (runs beyond d or dv read some other row and are not stored)
+    const float* kr = ks + (4 * ty < d ? 4 * ty : 0), *kr2 = ks + (64 + 4 * ty < d ? 64 + 4 * ty : 0);
+    const float* vr = vs + (4 * tx < dv ? 4 * tx : 0), *vr2 = vs + (64 + 4 * tx < dv ? 64 + 4 * tx : 0);
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+        const float4 k0 = *reinterpret_cast<const float4*>(kr + j * d), k1 = *reinterpret_cast<const float4*>(kr2 + j * d);
+        const float4 v0 = *reinterpret_cast<const float4*>(vr + j * dv), v1 = *reinterpret_cast<const float4*>(vr2 + j * dv);
+        const float kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { f4_fma(acc[i][0], kk[i], v0); f4_fma(acc[i][1], kk[i], v1); }
+    }
+    float* up = U + ((size_t)blockIdx.x * H + h) * d * dv;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = 4 * ty + (i & 3) + (i >> 2) * 64;
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            if (r < d && 4 * tx + 64 * c < dv) *reinterpret_cast<float4*>(up + (size_t)r * dv + 4 * tx + 64 * c) = acc[i][c];
+    }
+}
+
+// a thread: rows ty + 16 i of the chunk, columns 4 tx + {0..3} and 64 + 4 tx + {0..3} of the output
+template <typename T>
+__global__ void __launch_bounds__(256, 2) ret_chunk_out_vec_kernel(
+    const T* qkvg, int ld, T* out, const float* Sin, const float* cosv, const float* sinv,
+    const int* __restrict__ cu_seqlens, const int* __restrict__ seq_of_token, const float* __restrict__ decay,
+    int n_seqs, int H, int d, int dv, int rot, float kscale, float eps, float out_scale) {
+    pdl_launch();
+    pdl_wait();
+    extern __shared__ __align__(16) float sm[];
+    int b, t0, n;
+    if (!ret_find_chunk(blockIdx.x, cu_seqlens, seq_of_token, n_seqs, b, t0, n)) return;
+    const int h = blockIdx.y, wide = max(d, dv);
+    float* qs = sm;                           // [PC][wide]: q rows (stride d), later the raw outputs (stride dv)
+    float* ks = qs + RET_PC * wide;           // [PC][d]
+    float* vs = ks + RET_PC * d;              // [PC][dv]
+    float* A = vs + RET_PC * dv;              // [PC][PC]
+    float* pw = A + RET_PC * RET_PC;          // [PC + 1]
+    const float a = decay[h];
+    if (threadIdx.x <= RET_PC) {
+        float p = 1.f;
+        for (int i = 0; i < (int)threadIdx.x; ++i) p *= a;
+        pw[threadIdx.x] = p;
+    }
+    ret_stage_vec<T, true, true>(qkvg, ld, t0, n, h, H, d, dv, rot, kscale, cosv, sinv, qs, ks, vs, nullptr);
+    __syncthreads();
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    int qrow[4], krow[4];                     // (rows beyond the chunk read its last one and are not used)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { qrow[i] = min(ty + 16 * i, n - 1); krow[i] = min(tx + 16 * i, n - 1); }
+    {   // A[i][j] = decay^(i-j) (q_i . k_j) for j <= i < n, else 0
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll 2
+        for (int c = 0; c < d / 4; ++c) {
+            float4 k4[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) k4[j] = *reinterpret_cast<const float4*>(ks + ret_place<true>(krow[j], c, d));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 q4 = *reinterpret_cast<const float4*>(qs + ret_place<true>(qrow[i], c, d));
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    acc[i][j] = fmaf(q4.w, k4[j].w, fmaf(q4.z, k4[j].z, fmaf(q4.y, k4[j].y, fmaf(q4.x, k4[j].x, acc[i][j]))));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int qi = ty + 16 * i, kj = tx + 16 * j;
+                A[qi * RET_PC + kj] = (kj <= qi && qi < n) ? acc[i][j] * pw[qi - kj] : 0.f;
+            }
+    }
+    float4 o[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i][0] = o[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool in0 = 4 * tx < dv, in1 = 64 + 4 * tx < dv;
+    const float* S = Sin + ((size_t)blockIdx.x * H + h) * d * dv;
+    const float* S0 = S + (in0 ? 4 * tx : 0), *S1 = S + (in1 ? 64 + 4 * tx : 0);
+    // the state's rows come from global memory: the next four are asked for before these four are used
+    float4 s0[4], s1[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { s0[u] = *reinterpret_cast<const float4*>(S0 + (size_t)u * dv); s1[u] = *reinterpret_cast<const float4*>(S1 + (size_t)u * dv); }
+#pragma unroll 1
+    for (int c = 0; c < d / 4; ++c) {
+        float4 n0[4], n1[4];
+        const int nx = c + 1 < d / 4 ? 4 * (c + 1) : 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            n0[u] = *reinterpret_cast<const float4*>(S0 + (size_t)(nx + u) * dv);
+            n1[u] = *reinterpret_cast<const float4*>(S1 + (size_t)(nx + u) * dv);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 q4 = *reinterpret_cast<const float4*>(qs + ret_place<true>(qrow[i], c, d));
+            f4_fma(o[i][0], q4.x, s0[0]); f4_fma(o[i][1], q4.x, s1[0]);
+            f4_fma(o[i][0], q4.y, s0[1]); f4_fma(o[i][1], q4.y, s1[1]);
+            f4_fma(o[i][0], q4.z, s0[2]); f4_fma(o[i][1], q4.z, s1[2]);
+            f4_fma(o[i][0], q4.w, s0[3]); f4_fma(o[i][1], q4.w, s1[3]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { s0[u] = n0[u]; s1[u] = n1[u]; }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float f = pw[min(ty + 16 * i + 1, RET_PC)];
+        o[i][0] = f4_mul(o[i][0], f);
+        o[i][1] = f4_mul(o[i][1], f);
+    }
+    __syncthreads();                          // A is whole; every thread is done with the q rows
+    const float* v0p = vs + (in0 ? 4 * tx : 0), *v1p = vs + (in1 ? 64 + 4 * tx : 0);
+#pragma unroll 2
+    for (int j = 0; j < n; ++j) {
+        const float4 v0 = *reinterpret_cast<const float4*>(v0p + j * dv), v1 = *reinterpret_cast<const float4*>(v1p + j * dv);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float av = A[(ty + 16 * i) * RET_PC + j];
+            f4_fma(o[i][0], av, v0);
+            f4_fma(o[i][1], av, v1);
+        }
+    }
+    float* os = qs;                           // raw outputs [PC][dv]
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = ty + 16 * i;
+        if (r < n && in0) *reinterpret_cast<float4*>(os + r * dv + 4 * tx) = o[i][0];
+        if (r < n && in1) *reinterpret_cast<float4*>(os + r * dv + 64 + 4 * tx) = o[i][1];
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool has = 4 * lane < dv;
+#pragma unroll 2
+    for (int i = warp; i < n; i += 8) {
+        const float4 x = has ? *reinterpret_cast<const float4*>(os + i * dv + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (has) g = ret_ld4<T>(qkvg + (size_t)(t0 + i) * ld + (size_t)2 * H * d + (size_t)H * dv + h * dv + 4 * lane);
+        const float ss = warp_sum(fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w))));
+        const float f = out_scale / sqrtf(ss / (float)dv + eps);
+        if (has) {
+            T* op = out + (size_t)(t0 + i) * H * dv + h * dv + 4 * lane;
+            op[0] = from_f<T>(x.x * f * silu_f(g.x)); op[1] = from_f<T>(x.y * f * silu_f(g.y));
+            op[2] = from_f<T>(x.z * f * silu_f(g.z)); op[3] = from_f<T>(x.w * f * silu_f(g.w));
+        }
+    }
+}
+
 // Zero rows for the padding sequences of a replayed batch (the chunk kernels skip them).
 template <typename T>
 __global__ void ret_zero_padding_kernel(T* out, const int* __restrict__ seq_of_token, int ntok, int width) {
@@ -619,18 +876,24 @@ GG_API gg_retention_chunks(const void* qkvg, int dtype, int ld, void* out, float
     const int chunks = ntok / RET_PC + n_seqs, ds = d + 1, wide = d > dv ? d : dv;
     const size_t smem_a = ((size_t)RET_PC * (ds + dv + 1)) * sizeof(float);
     const size_t smem_c = ((size_t)RET_PC * (wide + ((d & 31) == 0 ? d : d + 1) + dv + RET_PC) + RET_PC + 1) * sizeof(float);
+    const bool vec = d % 32 == 0 && dv % 8 == 0 && rot % 8 == 0 && ld % 8 == 0 &&
+                     (((uintptr_t)qkvg | (uintptr_t)scratch | (uintptr_t)cosv | (uintptr_t)sinv) & 15) == 0;
+#define GG_RET(STATE, OUT) \
+        if (smem_a > 48 * 1024) \
+            cudaFuncSetAttribute(STATE<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a); \
+        if (smem_c > 48 * 1024) \
+            cudaFuncSetAttribute(OUT<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c); \
+        gg_launch(STATE<T>, dim3(chunks, H), dim3(256), smem_a, stream, 1, (const T*)qkvg, ld, scratch, \
+                  cosv, sinv, cu_seqlens, seq_of_token, decay, n_seqs, H, d, dv, rot, kscale); \
+        gg_launch(ret_chunk_scan_kernel, dim3(n_seqs, H, (d * dv + 255) / 256), dim3(256), 0, stream, 1, scratch, state, \
+                  cu_seqlens, slots, seq_of_token, decay, H, d, dv); \
+        gg_launch(OUT<T>, dim3(chunks, H), dim3(256), smem_c, stream, 1, (const T*)qkvg, ld, (T*)out, \
+                  (const float*)scratch, cosv, sinv, cu_seqlens, seq_of_token, decay, n_seqs, H, d, dv, rot, kscale, eps, \
+                  out_scale)
     GG_DISPATCH_DTYPE(dtype, T,
-        if (smem_a > 48 * 1024)
-            cudaFuncSetAttribute(ret_chunk_state_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a);
-        if (smem_c > 48 * 1024)
-            cudaFuncSetAttribute(ret_chunk_out_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c);
-        gg_launch(ret_chunk_state_kernel<T>, dim3(chunks, H), dim3(256), smem_a, stream, 1, (const T*)qkvg, ld, scratch,
-                  cosv, sinv, cu_seqlens, seq_of_token, decay, n_seqs, H, d, dv, rot, kscale);
-        gg_launch(ret_chunk_scan_kernel, dim3(n_seqs, H, (d * dv + 255) / 256), dim3(256), 0, stream, 1, scratch, state,
-                  cu_seqlens, slots, seq_of_token, decay, H, d, dv);
-        gg_launch(ret_chunk_out_kernel<T>, dim3(chunks, H), dim3(256), smem_c, stream, 1, (const T*)qkvg, ld, (T*)out,
-                  (const float*)scratch, cosv, sinv, cu_seqlens, seq_of_token, decay, n_seqs, H, d, dv, rot, kscale, eps,
-                  out_scale);
+        if (vec) { GG_RET(ret_chunk_state_vec_kernel, ret_chunk_out_vec_kernel); }
+        else { GG_RET(ret_chunk_state_kernel, ret_chunk_out_kernel); }
         gg_launch(ret_zero_padding_kernel<T>, dim3(ntok), dim3(128), 0, stream, 1, (T*)out, seq_of_token, ntok, H * dv));
+#undef GG_RET
     return gg_last_error();
 }
