@@ -808,21 +808,29 @@ __global__ void __launch_bounds__(128) latent_prompt_mma_kernel(
         bf16* kd = ks + (size_t)stage * KT * LQ;
         bf16* vd = vs + (size_t)stage * KT * LV;
         const int j0 = tile * KT;
-        for (int kk = warp; kk < KT; kk += 4) {
+        // a thread copies one 16-byte chunk in 128, rows one after another: with a warp per row, twelve of its lanes had a
+        // chunk of a key of 96 elements and eight one of a value of 64 (with that and a test per score in every tile, 1,276
+        // tokens of 4 prompts and 16 heads took 57.6 us, now 43.6)
+        int kk = tid / cq, c = tid - kk * cq;
+        for (; kk < KT;) {
+            bf16* dst = kd + kk * LQ + c * 8;
             const int j = j0 + kk;
-            bf16* dk = kd + kk * LQ;
-            bf16* dvp = vd + kk * LV;
-            if (j <= p1) {
-                const bf16* kp = kv + (size_t)(t0 + j) * ldkv + (size_t)h * d;           // this head's plain key
-                const bf16* kr = ckr + (size_t)(t0 + j) * ldc + R;                       // the shared rotated part
-                const bf16* vp = kv + (size_t)(t0 + j) * ldkv + (size_t)H * d + (size_t)h * dv;
-                for (int c = lane; c < cq; c += 32)
-                    cp_async16(dk + c * 8, c < cq_plain ? kp + c * 8 : kr + (c - cq_plain) * 8);
-                for (int c = lane; c < cv; c += 32) cp_async16(dvp + c * 8, vp + c * 8);
-            } else {
-                for (int c = lane; c < cq; c += 32) zero16(dk + c * 8);
-                for (int c = lane; c < cv; c += 32) zero16(dvp + c * 8);
-            }
+            if (j > p1) zero16(dst);
+            else if (c < cq_plain) cp_async16(dst, kv + (size_t)(t0 + j) * ldkv + (size_t)h * d + c * 8);      // this head's plain key
+            else cp_async16(dst, ckr + (size_t)(t0 + j) * ldc + R + (c - cq_plain) * 8);                        // the shared rotated part
+            kk += 128 / cq;
+            c += 128 % cq;
+            if (c >= cq) { c -= cq; ++kk; }
+        }
+        kk = tid / cv; c = tid - kk * cv;
+        for (; kk < KT;) {
+            bf16* dst = vd + kk * LV + c * 8;
+            const int j = j0 + kk;
+            if (j > p1) zero16(dst);
+            else cp_async16(dst, kv + (size_t)(t0 + j) * ldkv + (size_t)H * d + (size_t)h * dv + c * 8);
+            kk += 128 / cv;
+            c += 128 % cv;
+            if (c >= cv) { c -= cv; ++kk; }
         }
     };
     for (int row = warp; row < 64; row += 4) {           // queries: plain part from the product, rotated part from prep
@@ -885,13 +893,15 @@ __global__ void __launch_bounds__(128) latent_prompt_mma_kernel(
             }
             const int j0 = (tile0 + it) * KT;
             float mnew[2] = {mrow[0], mrow[1]};
+            // a tile that all 64 queries see whole needs no test per score (rows beyond the chunk are not stored)
+            const bool inside = rows_here == 64 && j0 + KT - 1 <= p0 && (window <= 0 || j0 > p0 + 63 - window);
 #pragma unroll
             for (int nt = 0; nt < KT / 8; ++nt)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int i = e >> 1;
                     const int j = j0 + nt * 8 + 2 * q4 + (e & 1);
-                    const bool see = valid[i] && j <= prow[i] && (window <= 0 || j > prow[i] - window);
+                    const bool see = inside || (valid[i] && j <= prow[i] && (window <= 0 || j > prow[i] - window));
                     const float v = see ? s[nt][e] * scale_log2 : -INFINITY;
                     s[nt][e] = v;
                     mnew[i] = fmaxf(mnew[i], v);

@@ -400,8 +400,7 @@ __device__ unsigned long long block_kth_largest(int n_mine, KeyOf key_of, int k,
         const uint32_t mask_above = shift == 28 ? 0u : (0xffffffffu << (shift + 4));     // the digits decided in this word
         if (threadIdx.x < 4) tot[(pass + 1) % 3][threadIdx.x] = 0ull;     // last read two passes ago
         unsigned long long c4[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-        for (int j = 0; j < (N > 0 ? N : n_mine); ++j) {
+        auto count = [&](int j) {
             const unsigned long long key = key_of(j);
             const uint32_t hi = (uint32_t)(key >> 32), lo = (uint32_t)key;
             const uint32_t word = pass < 8 ? hi : lo;
@@ -411,6 +410,12 @@ __device__ unsigned long long block_kth_largest(int n_mine, KeyOf key_of, int k,
             const unsigned long long inc = in ? (1ull << (16 * (b & 3))) : 0ull;
 #pragma unroll
             for (int q = 0; q < 4; ++q) c4[q] += (q == (b >> 2)) ? inc : 0ull;
+        };
+        if constexpr (N > 0) {
+#pragma unroll
+            for (int j = 0; j < N; ++j) count(j);
+        } else {
+            for (int j = 0; j < n_mine; ++j) count(j);
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -459,6 +464,9 @@ __device__ unsigned long long block_kth_largest(int n_mine, KeyOf key_of, int k,
 #define SAMP_COUNT_K 64
 #define SAMP_SIEVE_ROOM 1024
 
+// SIEVE: k up to SAMP_SIEVE_K (a kernel of its own, so that the walk over all keys, which it takes only where its sieve fails,
+// need not keep them in registers).
+template <bool SIEVE>
 __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const float* logits, long long ld, int V, float temp,
                                                                         int k, unsigned long long* __restrict__ cand) {
     pdl_launch();
@@ -490,7 +498,7 @@ __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const fl
     if (tid == 0) { n_out = 0; n_room = 0; at_least = 0xffffffffu; }
     unsigned long long* dst = cand + ((size_t)row * gridDim.x + slice) * k;
     bool sieved = false;
-    if (k <= SAMP_SIEVE_K) {
+    if (SIEVE) {
         uint32_t sieve;
         if (k <= SAMP_COUNT_K) {
             uint32_t top = 0u;
@@ -555,7 +563,7 @@ __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const fl
             if (mine[u] != 0ull && mine[u] >= thr) dst[atomicAdd(&n_out, 1)] = mine[u];
         return;
     }
-    const unsigned long long thr = block_kth_largest<SAMP_SLICE_PER>(SAMP_SLICE_PER, key_of, k, tot);
+    const unsigned long long thr = block_kth_largest<SIEVE ? 0 : SAMP_SLICE_PER>(SAMP_SLICE_PER, key_of, k, tot);
     for (int j = tid; j < k; j += SAMP_SLICE_THREADS) dst[j] = 0ull;
     __syncthreads();
 #pragma unroll
@@ -738,7 +746,7 @@ GG_API gg_sample_topk(const float* logits, long long ld, float temp, int top_k, 
         if (e != cudaSuccess) return (int)e;
         configured = smem;
     }
-    int rc = gg_launch(topk_slice_kernel, dim3(slices, R), dim3(SAMP_SLICE_THREADS), 0, stream, 1, logits, ld, V, temp, k,
+    int rc = gg_launch(k <= SAMP_SIEVE_K ? topk_slice_kernel<true> : topk_slice_kernel<false>, dim3(slices, R), dim3(SAMP_SLICE_THREADS), 0, stream, 1, logits, ld, V, temp, k,
                        (unsigned long long*)scratch);
     if (rc != 0) return rc;
     return gg_launch(sample_topk_kernel, dim3(R), dim3(SAMP_THREADS), smem, stream, 1,
@@ -777,7 +785,7 @@ GG_API gg_sample_nucleus(const float* logits, long long ld, float temp, float to
     rc = gg_launch(sample_slice_sum_uniform_kernel, dim3(slices, R), dim3(SAMP_THREADS), 0, stream, 1, logits, ld, temp,
                    (const int*)best, zs, V);
     if (rc != 0) return rc;
-    rc = gg_launch(topk_slice_kernel, dim3(slices, R), dim3(SAMP_SLICE_THREADS), 0, stream, 1, logits, ld, V, temp, k, cand);
+    rc = gg_launch(k <= SAMP_SIEVE_K ? topk_slice_kernel<true> : topk_slice_kernel<false>, dim3(slices, R), dim3(SAMP_SLICE_THREADS), 0, stream, 1, logits, ld, V, temp, k, cand);
     if (rc != 0) return rc;
     return gg_launch(sample_topk_kernel, dim3(R), dim3(SAMP_THREADS), smem, stream, 1, (const unsigned long long*)cand,
                      (int)per_row, k, top_p, min_p, uniforms, out, (const double*)zs, slices, flags, V);
