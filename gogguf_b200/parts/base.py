@@ -50,7 +50,7 @@ class Workspace:
         self._views: Dict[Tuple[str, Tuple[int, ...], torch.dtype], torch.Tensor] = {}
 
     def get(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
-        asked = (name, shape, dtype)
+        asked = (name, tuple(shape), dtype)
         view = self._views.get(asked)
         if view is not None:
             return view

@@ -17,9 +17,10 @@ outputs beyond `num_experts` with no matrices behind them; choosing one adds the
 weight.  `weight_scale` multiplies the weights after the renormalisation (which divides by the chosen scores' sum
 + 1e-20).
 The experts' matrices are reached through the chosen index with nothing read back: on the CUDA cores pair by pair
-(the 32-bit path, sizes the tensor-core forms do not take), or in bfloat16 on mma.sync, a CTA per expert and 64
-output rows with the expert's pairs as the operand (decode steps, short prompts).  Steps of many tokens in
-bfloat16 sort the (token, choice) pairs by expert and run one tcgen05 product per expert on its rows.
+(the 32-bit path, sizes the tensor-core forms do not take), or in bfloat16 with the pairs' rows placed expert by expert
+and one tcgen05 launch per matrix for all experts (decode steps, prompts; beyond 1,024 experts on mma.sync, a CTA per
+expert and 64 output rows).  Steps whose experts have very many rows each sort the pairs, read the ranges back and run one
+tcgen05 product per expert.
 """
 from __future__ import annotations
 
