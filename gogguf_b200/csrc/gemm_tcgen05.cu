@@ -547,7 +547,8 @@ __device__ __forceinline__ void epilogue_row_qkv(uint32_t taddr, int gi, int tn,
 // residual 28.3 and 28.7 us, gated unit 39.7 and 41.6; they read or compute between the loads and the stores.)
 constexpr int ROWBUF_BYTES = 32 * 128;
 
-__device__ __forceinline__ void store_partial_rows(uint32_t taddr, int gi0, int tn, int M, int NS, float* out, uint4* buf, int lane) {
+// (not inlined: inside the kernel its registers spilled)
+__device__ __noinline__ void store_partial_rows(uint32_t taddr, int gi0, int tn, int M, int NS, float* out, uint4* buf, int lane) {
     constexpr int BN = 256;
     if (gi0 >= M) return;
     const int rr = lane >> 3, ch = lane & 7;                 // round i of 8 below: row 4 i + rr, chunk ch
@@ -1578,11 +1579,14 @@ PairPlan pair_plan(int M, int N, int K, bool uneven_ok) {
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out_mode, long long ldo, int M, int N,
                 int K, int* status, const NormIO& nio, const QkvIO& qio, PairPlan plan, float* partial, cudaStream_t stream) {
     constexpr int STAGES = 6;
-    constexpr int smem = STAGES * (A_BYTES + 128 * BK * 2) + 1024 + 256 + 4 * ROWBUF_BYTES;
+    // the warps' buffers for partial tiles only where there are any: the other epilogues read a thread's row 16 bytes at a
+    // time through what shared memory leaves of the L1, and with 16 KB less of it the product that adds 2,048 tokens of
+    // 4,096 columns into the residual took 65 us instead of 62.5
+    constexpr int smem_whole = STAGES * (A_BYTES + 128 * BK * 2) + 1024 + 256, smem_split = smem_whole + 4 * ROWBUF_BYTES;
     static int sms = 0;
     auto kern = gemm_tc_pair_kernel<STAGES>;
     if (sms == 0) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_split);
         if (e != cudaSuccess) return (int)e;
         int dev = 0, n = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
@@ -1598,7 +1602,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out
     const int total = whole + (tiles - whole) * used;
     int pairs = sms / 2;
     if (pairs > total) pairs = total;
-    int rc = gg_launch2(kern, dim3(2 * pairs), dim3(NUM_THREADS), smem, stream, ta, tb, out, out_mode, ldo, M, N, K, status, nio,
+    int rc = gg_launch2(kern, dim3(2 * pairs), dim3(NUM_THREADS), used > 1 ? smem_split : smem_whole, stream, ta, tb, out, out_mode, ldo, M, N, K, status, nio,
                         used, whole, per, partial, qio);
     if (rc != 0 || used == 1) return rc;
     const int col0 = (whole / tiles_m) * 256, NS = N - col0;
