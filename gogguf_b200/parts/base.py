@@ -40,7 +40,12 @@ class Runtime:
 
 
 class Workspace:
-    """Named scratch buffers that are reused from step to step and grow on demand."""
+    """Named scratch buffers that are reused from step to step and grow on demand.
+
+    `get` returns a tensor object of the caller's own over the buffer: launchers take a row's stride from the tensor they
+    are given, and tensors leave the library (a step's logits) or go to registered parts, which may reshape them in place.
+    The view that is kept per shape (making one from the buffer is two operations, 2.5 us on the host) never leaves; a
+    caller gets an alias of it (0.7 us)."""
 
     MAX_VIEWS = 1024     # views kept ready (a few dozen per length of a step); then they are made anew
 
@@ -53,7 +58,7 @@ class Workspace:
         asked = (name, tuple(shape), dtype)
         view = self._views.get(asked)
         if view is not None:
-            return view
+            return view[...]
         n = 1
         for s in shape:
             n *= int(s)
@@ -66,7 +71,7 @@ class Workspace:
         if len(self._views) >= self.MAX_VIEWS:
             self._views.clear()
         view = self._views[asked] = buf[:n].view(*shape)
-        return view
+        return view[...]
 
 
 @dataclass
