@@ -307,6 +307,16 @@ def stream_ptr() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
+def need_rows(out: torch.Tensor, m: int, n: int, what: str) -> None:
+    """Refuse an output in which m rows of n elements, `out.stride(0)` apart, do not end inside the tensor: a launcher sees
+    a pointer and a stride only."""
+    if out.dim() == 2 and out.shape[0] >= m and out.shape[1] >= n:
+        return
+    end = 1 + sum((size - 1) * stride for size, stride in zip(out.shape, out.stride())) if out.numel() else 0
+    if m > 0 and (out.dim() == 0 or (m - 1) * out.stride(0) + n > end):
+        raise KernelError(f"{what}: an output of shape {tuple(out.shape)}, strides {out.stride()} has no room for {m} rows of {n}")
+
+
 _STATUS = {
     -1: "unsupported size or argument (the launcher refused it)",
     -2: "unsupported dtype combination",

@@ -10,7 +10,7 @@ from typing import Optional
 
 import torch
 
-from .build import KernelError, kernel, stream_ptr
+from .build import KernelError, kernel, need_rows, stream_ptr
 
 F32, BF16 = 0, 1
 
@@ -408,6 +408,7 @@ def gemm_plain(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: 
         raise KernelError(f"gemm: x{tuple(x.shape)} w{tuple(w.shape)} out{tuple(out.shape)} disagree")
     if x.stride(-1) != 1 or out.stride(-1) != 1 or not w.is_contiguous():
         raise KernelError("gemm: operands must be row-major")
+    need_rows(out, M, N, "gemm")
     if bias is not None:
         _need(bias, torch.float32, "bias")
         if bias.numel() != N:

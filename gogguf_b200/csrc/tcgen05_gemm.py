@@ -5,7 +5,7 @@ from typing import Callable, Dict, Optional
 
 import torch
 
-from .build import KernelError, kernel, module, stream_ptr
+from .build import KernelError, kernel, module, need_rows, stream_ptr
 
 OUT_BF16, OUT_F32, OUT_F32_ACC, OUT_SWIGLU = 0, 1, 2, 3
 
@@ -99,6 +99,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: boo
         raise KernelError(f"gemm_tc: output dtype {out.dtype}")
     if x.stride(-1) != 1 or out.stride(-1) != 1 or not w.is_contiguous():
         raise KernelError("gemm_tc: operands must be row-major")
+    need_rows(out, M, N // 2 if swiglu else N, "gemm_tc")
     st = status_word(x.device)
     kernel("gemm_tcgen05", "gg_gemm_tc")(
         x.data_ptr(), w.data_ptr(), out.data_ptr(), mode, M, N, K, x.stride(0), out.stride(0),
@@ -137,6 +138,7 @@ def gemm_tc_norm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate
         raise KernelError(f"gemm_tc_norm: output dtype {out.dtype}")
     if x.stride(-1) != 1 or out.stride(-1) != 1 or not w.is_contiguous():
         raise KernelError("gemm_tc_norm: operands must be row-major")
+    need_rows(out, M, N // 2 if swiglu else N, "gemm_tc_norm")
     in_parts = 0
     if in_ssq is not None:
         in_parts = (K + 127) // 128
