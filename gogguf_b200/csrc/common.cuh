@@ -190,6 +190,24 @@ static inline int gg_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     return (int)cudaGetLastError();
 }
 
+// How many CTAs of `kernel` the current device holds at once, its limit of dynamic shared memory there raised to `smem`.
+// Both belong to a device, not to the process: `known` (zeros at first) keeps the answer of each device, one beyond its places
+// is asked every time.  (Threads that meet here at first write the same numbers.)
+#define GG_MAX_DEVICES 64
+template <typename... KArgs>
+static inline int gg_resident(void (*kernel)(KArgs...), int threads, size_t smem, int (&known)[GG_MAX_DEVICES], int& resident) {
+    int dev = 0, sms = 0, per = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < GG_MAX_DEVICES && known[dev] > 0) { resident = known[dev]; return 0; }
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return (int)e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem)) != cudaSuccess) return (int)e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
+    resident = sms * per;
+    if (dev < GG_MAX_DEVICES) known[dev] = resident;
+    return 0;
+}
+
 // As gg_launch, with clusters of (2, 1, 1): pairs of CTAs with consecutive blockIdx.x.
 template <typename... KArgs, typename... Args>
 static inline int gg_launch2(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -171,15 +171,10 @@ static int launch_tile(const TX* x, const TW* w, void* out, int out_bf16, int ac
     constexpr size_t ring = (size_t)G * STAGES * (BM + BN) * (BK + 4) * sizeof(float);
     static_assert(ring <= 227 * 1024 && ring >= (size_t)(G - 1) * BM * BN * sizeof(float), "shared memory");
     auto kern = gemm_plain_kernel<TX, TW, BM, BN, TM, TN, G, BK, STAGES>;
-    static int resident = 0;                 // CTAs that the device holds at once (any thread computes the same number)
-    if (resident == 0) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
-        if (e != cudaSuccess) return (int)e;
-        int per = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, ring);
-        if (e != cudaSuccess) return (int)e;
-        resident = 148 * per;
-    }
+    static int known[GG_MAX_DEVICES] = {};
+    int resident = 0;
+    const int rc = gg_resident(kern, threads, ring, known, resident);
+    if (rc != 0) return rc;
     const int m_tiles = (M + BM - 1) / BM;
     const long long tiles = (long long)m_tiles * ((N + BN - 1) / BN);
     if (tiles > 0x7fffffffLL) return GG_ERR_ARG;
@@ -373,15 +368,10 @@ static int launch_wide(const TX* x, const TW* w, void* out, int out_bf16, int ac
     constexpr size_t ring = (size_t)4 * WIDE_BK * (BM + WIDE_BN + 8) * sizeof(float);
     static_assert(ring >= (size_t)64 * BM * sizeof(float), "the second group's sums go through the stages");
     auto kern = gemm_plain_wide_kernel<TX, TW, BM>;
-    static int resident = 0;
-    if (resident == 0) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
-        if (e != cudaSuccess) return (int)e;
-        int per = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 2 * BM, ring);
-        if (e != cudaSuccess) return (int)e;
-        resident = 148 * per;
-    }
+    static int known[GG_MAX_DEVICES] = {};
+    int resident = 0;
+    const int rc = gg_resident(kern, 2 * BM, ring, known, resident);
+    if (rc != 0) return rc;
     const int m_tiles = (M + BM - 1) / BM;
     const long long tiles = (long long)m_tiles * ((N + WIDE_BN - 1) / WIDE_BN);
     if (tiles > 0x7fffffffLL) return GG_ERR_ARG;
