@@ -77,14 +77,35 @@ def attn_prefill_tc(q, k_pool, v_pool, out, cu_seqlens, ctx_lens, seq_of_token, 
         status_word(q.device).data_ptr(), stream_ptr())
 
 
-def prefill_splits(n_tokens: int, n_seqs: int, nq: int, reach: int) -> int:
-    """CTAs that share the pages of a query tile which reads up to `reach` positions.  The device holds 296 CTAs; where the
-    (tile, head) pairs leave places free and a share keeps four pages, the pages are split.  Powers of two only: clusters of
-    three or six filled the chip worse than two or four (16 heads, 333 tokens, 6,433 positions, in 1 / 3 / 4 / 6 shares:
-    84 / 43 / 37 / 52 us; 32 heads in 1 / 2 / 3 / 4: 84 / 60 / 74 / 64)."""
-    tiles = -(-n_tokens // 128) if n_seqs == 1 else n_tokens // 128 + n_seqs
-    most = min(296 // (tiles * nq), reach // 256, 8)
-    return 1 << (most.bit_length() - 1) if most > 1 else 1
+# (query tile, head) pairs whose shares are all on the device at once, by the CTAs of a cluster: pairs fill all 296 places, larger
+# clusters do not (64 clusters of four run side by side and 72 do not; 32 of eight do).
+_RESIDENT = {2: 148, 4: 66, 8: 32}
+
+
+def prefill_tiles(n_tokens: int, n_seqs: int, max_new: int) -> int:
+    """At least as many 128-query tiles as the sequences of a step have."""
+    return min(n_tokens // 128 + n_seqs, n_seqs * -(-max_new // 128))
+
+
+def prefill_splits(n_tokens: int, n_seqs: int, nq: int, reach: int, max_new: Optional[int] = None, wide: int = 128) -> int:
+    """CTAs that share the pages of a query tile which reads up to `reach` positions: the 1, 2, 4 or 8 that a few constants
+    call quickest, of those that fit the device and leave a share two pages, from 512 positions on.  A page takes a CTA 0.55 us; a cluster that adds up its
+    shares takes 2 us, 0.065 us for every row that a CTA adds up (0.1 with rows of up to 64 values), and 2 us more
+    where the shares are what puts two CTAs on an SM.  Measured (us, in 1 / 2 / 4 / 8 shares): 333 tokens of 16 heads of
+    64 on 520 positions 10.4 / 14.8 / 13.4, of 32 heads of 128 on 1,024 16.8 / 17.5, on 6,400 79 / 51; 128 tokens of 16 heads of 64 on
+    1,024 14.4 / 17.6 / 13.7 / 12.1.  A sequence's shares depend on the whole step, and with them the order in which its
+    values are added."""
+    rows = n_tokens if max_new is None else max_new
+    pairs, pages = prefill_tiles(n_tokens, n_seqs, rows) * nq, -(-reach // 64)
+    best, gained = 1, 0.0
+    for splits, most in _RESIDENT.items():
+        if pairs > most or reach < 512 or 2 * splits > pages:
+            break
+        gain = 0.55 * (pages - -(-pages // splits)) - (2.0 if pairs * splits <= 148 else 4.0)
+        gain -= (0.065 if wide > 64 else 0.1) * -(-min(rows, 128) // splits)
+        if gain > gained:
+            best, gained = splits, gain
+    return best
 
 
 def takes(nq: int, nkv: int, d: int, dv: int) -> bool:
@@ -118,11 +139,13 @@ def try_make(nq: int, nkv: int, d: int, scale: float, window: int, dv: Optional[
             attn_decode_tma(q, k_pool, v_pool, out, ctx.positions, ctx.seq_of_token, table, page_size, T, nq, nkv, d,
                             scale, window, splits, cluster=True, **kw)
             return
-        splits = prefill_splits(T, ctx.n_seqs, nq, min([ctx.max_ctx] + [n + 192 for n in (window, chunk) if n]))
-        if ctx.max_new >= 32 or splits > 1:
-            # 128-query tiles on tcgen05 (S and O in tensor memory); a few tokens per sequence too where their history is long
-            # enough to be shared (10 tokens on 6,000, 32 heads: 25 us against 187)
-            max_tiles = -(-T // 128) if ctx.n_seqs == 1 else T // 128 + ctx.n_seqs
+        max_tiles = prefill_tiles(T, ctx.n_seqs, ctx.max_new)
+        reach = min([ctx.max_ctx] + [n + 192 for n in (window, chunk) if n])
+        if ctx.max_new >= 32 or (reach >= 512 and max_tiles * nq <= _RESIDENT[2]):
+            # 128-query tiles on tcgen05 (S and O in tensor memory); a few tokens per sequence too where a walk over their history
+            # is what takes the time (3 tokens on 520, 32 heads of 128: 10.9 us against 20.6; 16 heads of 64: 9.5 against 12.6; 10
+            # tokens on 6,400, 32 heads of 128: 20 in shares against 194)
+            splits = prefill_splits(T, ctx.n_seqs, nq, reach, ctx.max_new, dv)
             attn_prefill_tc(q, k_pool, v_pool, out, ctx.cu_seqlens, ctx.ctx_lens, ctx.seq_of_token, table, page_size,
                             T, ctx.n_seqs, max_tiles, nq, nkv, d, scale, window, splits=splits, **kw)
         else:
