@@ -919,7 +919,8 @@ __global__ void __launch_bounds__(192) attn_prefill_tc_kernel(
     constexpr int Q_BYTES = HK * QBOX, K_STAGE = HK * KBOX, V_BYTES = HV * KBOX;
     constexpr int TMEM_COLS = 256;
     // The dynamic segment is the only shared memory of this kernel and is asked to start on a 1024-byte
-    // boundary (the swizzled tiles need it) instead of being rounded up in the kernel: two CTAs of 96.25 KB share an SM.
+    // boundary (the swizzled tiles need it) instead of being rounded up in the kernel: two CTAs of 96.25 KB (97.25 where
+    // they share pages: the rows' maxima and sums) share an SM.
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* Qs = smem;
     uint8_t* Ks = Qs + Q_BYTES;                     // two stages
@@ -984,7 +985,8 @@ __global__ void __launch_bounds__(192) attn_prefill_tc_kernel(
     const int pos0 = active ? ctx_lens[b] - n_new + row0 : 0;
     const int lo = attn_first(pos0, window, sh.chunk);
     const int kt_begin = lo / PAGE, kt_last = active ? (pos0 + rows - 1) / PAGE : -1;
-    const int splits = (int)gridDim.z, all_tiles = kt_last - kt_begin + 1, per = (all_tiles + splits - 1) / splits;
+    const int splits = (int)gridDim.z, all_tiles = kt_last - kt_begin + 1;
+    const int per = splits == 1 ? all_tiles : (all_tiles + splits - 1) / splits;
     const int kt_first = kt_begin + (int)blockIdx.z * per;                       // this CTA's share of the pages
     const int ntiles = max(0, min(per, kt_last - kt_first + 1));
     // tensor memory: two score buffers of 64 columns (the scores of page j + 1 are computed while the softmax
@@ -1445,16 +1447,16 @@ static int launch_attn_prefill_tc(const CUtensorMap& tq, const CUtensorMap& tk, 
                                   const int* cu_seqlens, const int* ctx_lens, const int* seq_of_token, const int* page_table,
                                   int max_pages, int n_seqs, int nq, int nkv, float scale_log2, int window, const float* sink,
                                   float out_scale, int n_pages, int* status, const AttnShape& sh, cudaStream_t stream) {
-    // Q, K x 2, V x 2 (boxes of 64 columns: 16 KB of Q, 8 KB of K or V), barriers, the rows' maxima and sums
-    constexpr int smem = (DK / 64) * (16384 + 2 * 8192) + (DV / 64) * 2 * 8192 + 256 + 1024;
-    static_assert(smem - 1280 >= 128 * DV * 4, "the float32 rows that a cluster adds lie where Q, K and V were");
+    // Q, K x 2, V x 2 (boxes of 64 columns: 16 KB of Q, 8 KB of K or V), barriers; with shares the rows' maxima and sums
+    constexpr int smem = (DK / 64) * (16384 + 2 * 8192) + (DV / 64) * 2 * 8192 + 256, smem_shares = smem + 1024;
+    static_assert(smem - 256 >= 128 * DV * 4, "the float32 rows that a cluster adds lie where Q, K and V were");
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<DK, DV, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<DK, DV, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_shares);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    return gg_launch(attn_prefill_tc_kernel<DK, DV, EXACT>, grid, dim3(192), smem, stream, (int)grid.z, tq, tk, tv, (bf16*)out, cu_seqlens,
+    return gg_launch(attn_prefill_tc_kernel<DK, DV, EXACT>, grid, dim3(192), grid.z > 1 ? smem_shares : smem, stream, (int)grid.z, tq, tk, tv, (bf16*)out, cu_seqlens,
                      ctx_lens, seq_of_token, page_table, max_pages, n_seqs, nq, nkv, scale_log2, window, sink, out_scale, n_pages,
                      status, sh);
 }
