@@ -27,6 +27,11 @@ __device__ __forceinline__ void gp_cp16(float* smem, const float* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(gmem) : "memory");
 }
 
+__device__ __forceinline__ void gp_cp4(float* smem, const float* gmem) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(a), "l"(gmem) : "memory");
+}
+
 template <int THREADS>
 __device__ __forceinline__ void group_sync(int g) {
     if (THREADS == 32) __syncwarp();
@@ -34,11 +39,21 @@ __device__ __forceinline__ void group_sync(int g) {
 }
 
 // Rows r0.. of a row-major operand into [R][BK + 4] floats; rows from `rows` on and columns from `k_end` on are zero.
-// ASYNC (float32 on 16-byte boundaries, K a multiple of 4): copies are issued and not waited for.
-template <typename T, int R, int BK, int THREADS>
+// float32 is copied without being waited for: 16 bytes at a time where `chunks` (rows on 16-byte boundaries, K a multiple
+// of 4), an element at a time with ELEMENTS.  (A form of the kernel of its own: with both in one, the tiles of up to 64 rows took 10 %
+// longer for rows in chunks.)  What is left is loaded, four elements in flight, and converted.
+template <typename T, int R, int BK, int THREADS, bool ELEMENTS>
 __device__ __forceinline__ void stage_rows(float* dst, const T* src, long long ld, int r0, int rows, int k0, int k_end, int tid,
-                                           bool async) {
-    if (sizeof(T) == 4 && async) {
+                                           bool chunks) {
+    if (sizeof(T) == 4 && ELEMENTS) {
+#pragma unroll 8
+        for (int c = tid; c < R * BK; c += THREADS) {
+            const int r = c / BK, kk = c % BK;
+            float* d = dst + r * (BK + 4) + kk;
+            if (r0 + r < rows && k0 + kk < k_end) gp_cp4(d, reinterpret_cast<const float*>(src) + (size_t)(r0 + r) * ld + k0 + kk);
+            else *d = 0.f;
+        }
+    } else if (sizeof(T) == 4 && chunks) {
         constexpr int V = BK / 4;
 #pragma unroll
         for (int c = tid; c < R * V; c += THREADS) {
@@ -58,7 +73,7 @@ __device__ __forceinline__ void stage_rows(float* dst, const T* src, long long l
     }
 }
 
-template <typename TX, typename TW, int BM, int BN, int TM, int TN, int G, int BK, int STAGES>
+template <typename TX, typename TW, int BM, int BN, int TM, int TN, int G, int BK, int STAGES, bool ELEMENTS>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
     const TX* x, const TW* __restrict__ w, void* out, int out_bf16, int accumulate, int M, int N, int K, long long ldx,
     long long ldo, const float* __restrict__ bias, int m_tiles, int async_x, int async_w, int early) {
@@ -74,10 +89,10 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
     const int steps = (k_end - k_begin + BK - 1) / BK;
     float* ring = sm + (size_t)g * STAGES * STAGE;
     auto load_w = [&](int it) {
-        if (it < steps) stage_rows<TW, BN, BK, THREADS>(ring + (it % STAGES) * STAGE + BM * (BK + 4), w, K, n0, N, k_begin + it * BK, k_end, tid, async_w);
+        if (it < steps) stage_rows<TW, BN, BK, THREADS, ELEMENTS>(ring + (it % STAGES) * STAGE + BM * (BK + 4), w, K, n0, N, k_begin + it * BK, k_end, tid, async_w);
     };
     auto load_x = [&](int it) {
-        if (it < steps) stage_rows<TX, BM, BK, THREADS>(ring + (it % STAGES) * STAGE, x, ldx, m0, M, k_begin + it * BK, k_end, tid, async_x);
+        if (it < steps) stage_rows<TX, BM, BK, THREADS, ELEMENTS>(ring + (it % STAGES) * STAGE, x, ldx, m0, M, k_begin + it * BK, k_end, tid, async_x);
     };
 #pragma unroll 1
     for (int s = 0; s < STAGES - 1; ++s) load_w(s);     // weights: nothing before this kernel writes them
@@ -164,13 +179,13 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
     }
 }
 
-template <typename TX, typename TW, int BM, int BN, int TM, int TN, int G, int BK, int STAGES>
+template <typename TX, typename TW, int BM, int BN, int TM, int TN, int G, int BK, int STAGES, bool ELEMENTS = false>
 static int launch_tile(const TX* x, const TW* w, void* out, int out_bf16, int accumulate, int M, int N, int K,
                        long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
     constexpr int threads = (BM / TM) * (BN / TN) * G;
     constexpr size_t ring = (size_t)G * STAGES * (BM + BN) * (BK + 4) * sizeof(float);
     static_assert(ring <= 227 * 1024 && ring >= (size_t)(G - 1) * BM * BN * sizeof(float), "shared memory");
-    auto kern = gemm_plain_kernel<TX, TW, BM, BN, TM, TN, G, BK, STAGES>;
+    auto kern = gemm_plain_kernel<TX, TW, BM, BN, TM, TN, G, BK, STAGES, ELEMENTS>;
     static int known[GG_MAX_DEVICES] = {};
     int resident = 0;
     const int rc = gg_resident(kern, threads, ring, known, resident);
@@ -196,22 +211,41 @@ static int launch_tile(const TX* x, const TW* w, void* out, int out_bf16, int ac
 #define WIDE_BN 64
 #define WIDE_BK 16
 
-template <typename T>
-__device__ __forceinline__ float4 gp_load4(const T* p, int left, bool vec) {
-    if (vec) {
-        if (left <= 0) return make_float4(0.f, 0.f, 0.f, 0.f);
-        if (sizeof(T) == 4) return *reinterpret_cast<const float4*>(p);
-        const uint2 u = *reinterpret_cast<const uint2*>(p);
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
-        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
-        return make_float4(a.x, a.y, b.x, b.y);
+// This thread's part of a stage, R rows of WIDE_BK columns, into registers as it lies in memory (a conversion would wait for the load):
+// VEC (rows of four elements aligned): columns 4 (tid % 4) .. + 3 of rows tid / 4 + THREADS / 4 i; else column tid % 16 of rows
+// tid / 16 + THREADS / 16 j, so that a warp's loads are two runs of neighbours.
+template <typename T, int R, int THREADS, bool VEC>
+__device__ __forceinline__ void wide_load(T (&v)[R * WIDE_BK / THREADS], const T* src, long long ld, int r0, int rows, int k0, int k_end,
+                                          int tid) {
+    constexpr int PER = R * WIDE_BK / THREADS;
+    if (VEC) {
+        const int k = k0 + tid % 4 * 4;
+#pragma unroll
+        for (int i = 0; i < PER / 4; ++i) {
+            const int r = r0 + tid / 4 + THREADS / 4 * i;
+            const bool in = r < rows && k < k_end;
+            const T* p = src + (size_t)r * ld + k;
+            if (sizeof(T) == 4) *reinterpret_cast<uint4*>(&v[4 * i]) = in ? *reinterpret_cast<const uint4*>(p) : make_uint4(0u, 0u, 0u, 0u);
+            else *reinterpret_cast<uint2*>(&v[4 * i]) = in ? *reinterpret_cast<const uint2*>(p) : make_uint2(0u, 0u);
+        }
+    } else {
+        const int k = k0 + tid % 16;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const int r = r0 + tid / 16 + THREADS / 16 * j;
+            v[j] = r < rows && k < k_end ? src[(size_t)r * ld + k] : from_f<T>(0.f);
+        }
     }
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (left > 0) v.x = to_f<T>(p[0]);
-    if (left > 1) v.y = to_f<T>(p[1]);
-    if (left > 2) v.z = to_f<T>(p[2]);
-    if (left > 3) v.w = to_f<T>(p[3]);
-    return v;
+}
+// and from there to shared memory as float32, k as the slow index, rows of LD floats
+template <typename T, int R, int THREADS, int LD, bool VEC>
+__device__ __forceinline__ void wide_store(float* dst, const T (&v)[R * WIDE_BK / THREADS], int tid) {
+    constexpr int PER = R * WIDE_BK / THREADS;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        if (VEC) dst[(tid % 4 * 4 + j % 4) * LD + tid / 4 + THREADS / 4 * (j / 4)] = to_f<T>(v[j]);
+        else dst[tid % 16 * LD + tid / 16 + THREADS / 16 * j] = to_f<T>(v[j]);
+    }
 }
 __device__ __forceinline__ unsigned long long gp_pack(float lo, float hi) {
     unsigned long long r;
@@ -224,12 +258,11 @@ __device__ __forceinline__ float2 gp_unpack(unsigned long long v) {
     return r;
 }
 
-template <typename TX, typename TW, int BM>
+template <typename TX, typename TW, int BM, bool VEC>
 __global__ void __launch_bounds__(2 * BM) gemm_plain_wide_kernel(
     const TX* x, const TW* __restrict__ w, void* out, int out_bf16, int accumulate, int M, int N, int K, long long ldx,
-    long long ldo, const float* __restrict__ bias, int m_tiles, int vec_x, int vec_w, int early) {
+    long long ldo, const float* __restrict__ bias, int m_tiles, int early) {
     constexpr int BN = WIDE_BN, BK = WIDE_BK, LX = BM + 4, LW = BN + 4, STAGE = BK * (LX + LW);
-    constexpr int WROWS = BN * 4 / BM;                  // float4s of W a thread loads per stage (of x: 4)
     extern __shared__ __align__(16) float sm[];
     if (early) pdl_launch();
     const int g = threadIdx.x / BM, tid = threadIdx.x % BM;
@@ -239,37 +272,14 @@ __global__ void __launch_bounds__(2 * BM) gemm_plain_wide_kernel(
     const int k_begin = min(K, g * 2 * len), k_end = min(K, (g + 1) * 2 * len);
     const int steps = (k_end - k_begin + BK - 1) / BK, per_slice = len / BK;
     float* ring = sm + (size_t)g * 2 * STAGE;
-    const int lr = tid / 4, lk = (tid % 4) * 4;         // this thread's loads: rows lr + (BM / 4) i, columns lk .. lk + 3 of the stage
-    float4 xr[4], wr[WROWS];
-    auto load_w = [&](int it) {
-        const int k = k_begin + it * BK + lk;
-#pragma unroll
-        for (int i = 0; i < WROWS; ++i) {
-            const int n = n0 + lr + BM / 4 * i;
-            wr[i] = gp_load4<TW>(w + (size_t)(n < N ? n : 0) * K + k, n < N ? k_end - k : 0, vec_w);
-        }
-    };
-    auto load_x = [&](int it) {
-        const int k = k_begin + it * BK + lk;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int m = m0 + lr + BM / 4 * i;
-            xr[i] = gp_load4<TX>(x + (size_t)(m < M ? m : 0) * ldx + k, m < M ? k_end - k : 0, vec_x);
-        }
-    };
+    alignas(16) TX xr[BK];
+    alignas(16) TW wr[BN * BK / BM];
+    auto load_w = [&](int it) { wide_load<TW, BN, BM, VEC>(wr, w, K, n0, N, k_begin + it * BK, k_end, tid); };
+    auto load_x = [&](int it) { wide_load<TX, BM, BM, VEC>(xr, x, ldx, m0, M, k_begin + it * BK, k_end, tid); };
     auto store = [&](int it) {
         float* xs = ring + (it & 1) * STAGE;
-        float* ws = xs + BK * LX;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float* d = xs + lk * LX + lr + BM / 4 * i;
-            d[0] = xr[i].x; d[LX] = xr[i].y; d[2 * LX] = xr[i].z; d[3 * LX] = xr[i].w;
-        }
-#pragma unroll
-        for (int i = 0; i < WROWS; ++i) {
-            float* d = ws + lk * LW + lr + BM / 4 * i;
-            d[0] = wr[i].x; d[LW] = wr[i].y; d[2 * LW] = wr[i].z; d[3 * LW] = wr[i].w;
-        }
+        wide_store<TX, BM, BM, LX, VEC>(xs, xr, tid);
+        wide_store<TW, BN, BM, LW, VEC>(xs + BK * LX, wr, tid);
     };
     unsigned long long acc[8][4], run[8][4];
 #pragma unroll
@@ -362,12 +372,12 @@ __global__ void __launch_bounds__(2 * BM) gemm_plain_wide_kernel(
     }
 }
 
-template <typename TX, typename TW, int BM>
-static int launch_wide(const TX* x, const TW* w, void* out, int out_bf16, int accumulate, int M, int N, int K,
+template <typename TX, typename TW, int BM, bool VEC>
+static int launch_wide_as(const TX* x, const TW* w, void* out, int out_bf16, int accumulate, int M, int N, int K,
                        long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
     constexpr size_t ring = (size_t)4 * WIDE_BK * (BM + WIDE_BN + 8) * sizeof(float);
     static_assert(ring >= (size_t)64 * BM * sizeof(float), "the second group's sums go through the stages");
-    auto kern = gemm_plain_wide_kernel<TX, TW, BM>;
+    auto kern = gemm_plain_wide_kernel<TX, TW, BM, VEC>;
     static int known[GG_MAX_DEVICES] = {};
     int resident = 0;
     const int rc = gg_resident(kern, 2 * BM, ring, known, resident);
@@ -375,10 +385,16 @@ static int launch_wide(const TX* x, const TW* w, void* out, int out_bf16, int ac
     const int m_tiles = (M + BM - 1) / BM;
     const long long tiles = (long long)m_tiles * ((N + WIDE_BN - 1) / WIDE_BN);
     if (tiles > 0x7fffffffLL) return GG_ERR_ARG;
-    const int vec_x = K % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & (sizeof(TX) * 4 - 1)) == 0;
-    const int vec_w = K % 4 == 0 && ((uintptr_t)w & (sizeof(TW) * 4 - 1)) == 0;
     return gg_launch(kern, dim3((unsigned)tiles), dim3(2 * BM), ring, stream, 1, x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo,
-                     bias, m_tiles, vec_x, vec_w, (int)(tiles <= resident));
+                     bias, m_tiles, (int)(tiles <= resident));
+}
+
+template <typename TX, typename TW, int BM>
+static int launch_wide(const TX* x, const TW* w, void* out, int out_bf16, int accumulate, int M, int N, int K,
+                       long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
+    const bool vec = K % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & (sizeof(TX) * 4 - 1)) == 0 && ((uintptr_t)w & (sizeof(TW) * 4 - 1)) == 0;
+    if (vec) return launch_wide_as<TX, TW, BM, true>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream);
+    return launch_wide_as<TX, TW, BM, false>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream);
 }
 
 template <typename TX, typename TW>
@@ -386,7 +402,7 @@ static int launch(const void* xv, const void* wv, void* out, int out_bf16, int a
                   int M, int N, int K, long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
     const TX* x = (const TX*)xv;
     const TW* w = (const TW*)wv;
-#define GP(BM, BN, TM, TN, G, BK, ST) return launch_tile<TX, TW, BM, BN, TM, TN, G, BK, ST>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream)
+#define GP(BM, BN, TM, TN, G, BK, ...) return launch_tile<TX, TW, BM, BN, TM, TN, G, BK, __VA_ARGS__>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream)
     // Up to 16 rows the time is that of reading W, and what counts is how much of it is asked for at a time.  With a CTA an SM
     // or less, deep rings of wide stages; with more tiles, the ring that lets most of them be resident.  Measured, M = 4
     // (us; BK 32 in 6 stages for all | as below): 2,048 x 2,048 10.7 | 6.4, 2,048 x 5,376 25.4 | 13.6, 4,096 x 2,048 11.6 | 9.3,
@@ -413,15 +429,32 @@ static int launch(const void* xv, const void* wv, void* out, int out_bf16, int a
         if (tiles <= 296) GP(16, 16, 4, 2, 4, 64, 3);
         GP(16, 16, 4, 2, 4, 64, 2);
     }
-    // cycles of an SM per column of k, as its multipliers (128 a cycle) and each tile's measured share of them give
-    auto cost = [&](int bm, int bn, double share) {
-        const long long t = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-        return (double)((t + 147) / 148) * bm * bn / (128.0 * share);
-    };
-    const double small = cost(32, 16, 0.5), mid = cost(64, 32, 0.6), tall = cost(64, 64, 0.7), large = cost(128, 64, 0.8);
-    if (small <= mid && small <= large && small <= tall) GP(32, 16, 4, 4, 4, 32, 4);
-    if (mid <= large && mid <= tall) GP(64, 32, 8, 4, 4, 16, 3);
-    if (tall <= large) return launch_wide<TX, TW, 64>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream);
+    // More rows: the quickest of four tiles.  Measured per tile, in microseconds per 1,000 of K: 148 tiles or fewer, and 296 (two an
+    // SM); a grid is as many rounds of 296 and one of what is left.  Three rows of the table: float32 in chunks, float32 by elements, any
+    // bfloat16 operand.  Over 352 products (17 to 2,048 rows, ten matrices) the choice is within 1 % of the best tile on average
+    // and 25 % at worst; one share of the multipliers' rate per tile, whatever the operands, was 12 % and 211 %.
+    static const float round_us[3][4][2] = {{{11, 11}, {30, 35}, {42, 55}, {54, 110}},
+                                            {{12, 21}, {27, 59}, {62, 70}, {60, 120}},
+                                            {{16, 23}, {38, 48}, {57, 76}, {60, 130}}};
+    const bool elements = (sizeof(TX) == 4 && (K % 4 || ldx % 4 || ((uintptr_t)x & 15))) || (sizeof(TW) == 4 && (K % 4 || ((uintptr_t)w & 15)));
+    const float (*us)[2] = round_us[sizeof(TX) == 2 || sizeof(TW) == 2 ? 2 : (int)elements];
+    const int rows[4] = {32, 64, 64, 128}, cols[4] = {16, 32, 64, 64};
+    int best = 0;
+    float least = 0.f;
+    for (int i = 0; i < 4; ++i) {
+        const long long t = (long long)((M + rows[i] - 1) / rows[i]) * ((N + cols[i] - 1) / cols[i]), left = t % 296;
+        const float cost = us[i][1] * (float)(t / 296) + (left == 0 ? 0.f : us[i][left > 148]);
+        if (i == 0 || cost < least) { best = i; least = cost; }
+    }
+    if (best == 0) {
+        if (elements) GP(32, 16, 4, 4, 4, 32, 4, true);
+        GP(32, 16, 4, 4, 4, 32, 4, false);
+    }
+    if (best == 1) {
+        if (elements) GP(64, 32, 8, 4, 4, 16, 3, true);
+        GP(64, 32, 8, 4, 4, 16, 3, false);
+    }
+    if (best == 2) return launch_wide<TX, TW, 64>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream);
     return launch_wide<TX, TW, 128>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream);
 #undef GP
 }

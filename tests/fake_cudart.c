@@ -6,7 +6,7 @@
 enum { DEVICES = 128, KERNELS = 4096, OK = 0, INVALID = 1 };
 static int device_now, last_error;
 static const void* kernels[KERNELS];
-static int n_kernels, allowed[KERNELS][DEVICES];
+static int n_kernels, allowed[KERNELS][DEVICES], early_at[KERNELS];
 static void* handle;
 int fake_launches, fake_last_grid, fake_last_early, fake_attribute_calls;
 
@@ -40,7 +40,7 @@ int cudaLaunchKernelExC(const struct config* c, const void* f, void** args) {
     if (c->smem > (size_t)(most > 48 * 1024 ? most : 48 * 1024)) return last_error = INVALID;
     ++fake_launches;
     fake_last_grid = (int)c->gx;
-    fake_last_early = *(int*)args[14];       /* the plain product's kernels: their last argument */
+    fake_last_early = *(int*)args[early_at[place(f)]];
     return OK;
 }
 int cudaLaunchKernel(const void* f, unsigned gx, unsigned gy, unsigned gz, unsigned bx, unsigned by, unsigned bz, void** a, size_t s, void* st) {
@@ -51,7 +51,8 @@ void** __cudaRegisterFatBinary(void* p) { (void)p; return &handle; }
 void __cudaRegisterFatBinaryEnd(void** h) { (void)h; }
 void __cudaUnregisterFatBinary(void** h) { (void)h; }
 void __cudaRegisterFunction(void** h, const char* host, char* dev, const char* name, int lim, void* a, void* b, void* c, void* d, int* e) {
-    (void)h; (void)host; (void)dev; (void)name; (void)lim; (void)a; (void)b; (void)c; (void)d; (void)e;
+    early_at[place(host)] = strstr(name, "wide") ? 12 : 14;      /* the last argument of the plain product's kernels */
+    (void)h; (void)dev; (void)lim; (void)a; (void)b; (void)c; (void)d; (void)e;
 }
 int __cudaPopCallConfiguration(void* g, void* b, size_t* s, void* st) { (void)g; (void)b; (void)s; (void)st; return INVALID; }
 unsigned __cudaPushCallConfiguration(void) { return 1; }

@@ -77,3 +77,25 @@ def test_attention_head_sizes(d, dv):
         keys, vals = (t[[2, 0, 1], 0].reshape(-1, t.shape[-1])[:pos + 1].double() for t in (kp, vp))
         want = torch.softmax(q[0].double() @ keys.T * d ** -0.5, -1) @ vals
         assert (out[0].double() - want).abs().max() <= tol * vals.abs().max()
+
+
+@pytest.mark.parametrize("dtypes", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("N,K_,off", [(70, 33, 0), (1000, 129, 0), (333, 260, 1), (5000, 67, 0), (2100, 64, 0)])
+def test_rows_by_elements(N, K_, off, dtypes):
+    """Rows off their boundaries and bfloat16 matrices in the tiles of more than 16 rows: element copies, values kept as they lie in
+    memory; outputs in bfloat16 and behind a stride."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(1300, K_ + 7, device="cuda", generator=g).to(dtypes[0])[:, off:off + K_]
+    w = torch.randn(N, K_, device="cuda", generator=g).to(dtypes[1])
+    first = None
+    for M in (1, 31, 63, 64, 65, 128, 300, 610, 1300):
+        wide = torch.full((M, N + 3), -7.0, device="cuda")
+        K().gemm_plain(x[:M], w, wide[:, :N])
+        out = wide[:, :N]
+        want = x[:M].double() @ w.double().T
+        assert (out.double() - want).norm() <= bound(K_) * (x[:M].double().abs() @ w.double().abs().T).norm()
+        first = out[0].clone() if first is None else first
+        assert torch.equal(out[0], first) and (wide[:, N:] == -7.0).all()
+        half = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        K().gemm_plain(x[:M], w, half)
+        assert torch.equal(half, out.to(torch.bfloat16))
