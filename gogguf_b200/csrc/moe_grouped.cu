@@ -144,26 +144,43 @@ __global__ void __launch_bounds__(NUM_THREADS, MINB) moe_grouped_kernel(
     __syncthreads();
     tc5::fence_after();
     if (warp == 0) {                           // running sums of the experts' tile counts
-        int base = 0;
-        for (int e0 = 0; e0 < E; e0 += 32) {
-            const int e = e0 + lane;
-            int v = e < E ? (off[e + 1] - off[e] + BM - 1) / BM * tiles_n : 0;
-            const int mine = v;
+        auto tiles_of = [&](int e) { return (off[e + 1] - off[e] + BM - 1) / BM * tiles_n; };
+        auto scan = [&](int v) {
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, v, o);
                 if (lane >= o) v += y;
             }
-            if (e < E) start[e] = base + v - mine;
-            base += __shfl_sync(0xffffffffu, v, 31);
+            return v;
+        };
+        if (E <= 32) {
+            const int mine = lane < E ? tiles_of(lane) : 0, v = scan(mine);
+            if (lane < E) start[lane] = v - mine;
+            if (lane == 31) start[E] = v;
+        } else {           // a run of neighbouring experts a lane (an odd number: no bank twice)
+            const int per = (E + 31) / 32 | 1, e0 = min(E, lane * per), e1 = min(E, e0 + per);
+            int mine = 0;
+            for (int e = e0; e < e1; ++e) mine += tiles_of(e);
+            int at = scan(mine);
+            if (lane == 31) start[E] = at;
+            at -= mine;
+            for (int e = e0; e < e1; ++e) { start[e] = at; at += tiles_of(e); }
         }
-        if (lane == 0) start[E] = base;
     }
     __syncthreads();
     const uint32_t tmem_base = *tmem_slot;
     const int total = start[E];
-    // the walk's tile t -> expert (e moves on with t), row tile, column tile
+    // the walk's tile t -> expert (the last that starts at or before t), row tile, column tile.  With many experts by halves: a walk
+    // from one to the next took most of the 80 us of a layer with 1,000.
     auto tile_of = [&](int t, int& e, int& row0, int& rows, int& tn) {
+        if (E > 32 && t >= start[e + 1]) {
+            int hi = E;                                // start[++e] <= t < start[hi]
+            ++e;
+            while (hi - e > 1) {
+                const int mid = (e + hi) >> 1;
+                if (start[mid] <= t) e = mid; else hi = mid;
+            }
+        }
         while (t >= start[e + 1]) ++e;
         const int cnt = off[e + 1] - off[e], mt = (cnt + BM - 1) / BM, r = t - start[e];
         const int tm = r % mt;
