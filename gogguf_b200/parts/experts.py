@@ -19,8 +19,8 @@ weight.  `weight_scale` multiplies the weights after the renormalisation (which 
 The experts' matrices are reached through the chosen index with nothing read back: on the CUDA cores pair by pair
 (the 32-bit path, sizes the tensor-core forms do not take), or in bfloat16 with the pairs' rows placed expert by expert
 and one tcgen05 launch per matrix for all experts (decode steps, prompts; beyond 1,024 experts on mma.sync, a CTA per
-expert and 64 output rows).  Steps whose experts have very many rows each sort the pairs, read the ranges back and run one
-tcgen05 product per expert.
+expert and 64 output rows).  Prompts of more than 16,384 pairs sort them, read the ranges back and run one tcgen05 product per
+expert and matrix.
 """
 from __future__ import annotations
 
@@ -36,7 +36,13 @@ from .base import Linear, Runtime, StepContext
 from .registry import FEED_FORWARDS, lookup, register_feed_forward
 
 
-SORTED_FORM_MIN_WORK = 1.5e9      # rows per expert x inner width x width from which prompts take the sorted form
+# The most (token, choice) pairs of the form with one launch per matrix; longer prompts take the sorted form.  Placing the pairs
+# compares each with all others (11 us up to 2,048, 41 with 8,192, 127 with 16,384, 474 with 32,768); sorting reads the experts'
+# ranges back and launches a product per expert and matrix.  us a layer, one launch / sorted: 16 experts of 4,096 x 2,048, 4,096
+# pairs 300 / 712, 16,384 pairs 906 / 1,471; 4 of 4,096 x 14,336, 8,192 pairs 2,309 / 2,946; 128 of 2,048 x 768, 16,384
+# pairs 438 / 3,338; 8 of 1,024 x 512, 16,384 pairs 235 / 300, 32,768 pairs 675 / 441.
+ONE_LAUNCH_MAX_PAIRS = 16384
+SORTED_FORM_MIN_WORK = float("inf")   # rows per expert x inner width x width from which fewer pairs are sorted too (2.4e11 was measured: no)
 
 
 def _softplus(v: float) -> float:
@@ -182,7 +188,7 @@ class RoutedExperts:
             cls = lookup(FEED_FORWARDS, sh.kind, "feed-forward")
             self.shared = cls(sh, {local: weights.pop(sh.prefix + local) for local in cls.tensors(sh)}, rt)
         self._grouped = None
-        # rows on 16-byte boundaries: what the tensor-core forms (mma.sync for few pairs, tcgen05 for many) take
+        # rows on 16-byte boundaries: what the tensor-core forms (tcgen05; mma.sync for more experts than that form keeps ranges for) take
         self._mma = (rt.fast and rt.dtype == torch.bfloat16 and self.w_gu.dtype == torch.bfloat16
                      and self.hidden % 8 == 0 and self.inter % 8 == 0)
         if rt.fast and rt.dtype == torch.bfloat16 and self.w_gu.dtype == torch.bfloat16:
@@ -225,19 +231,18 @@ class RoutedExperts:
                 raise ValueError("routed experts: identity experts take their weight on the output")
             K.moe_identity(h, idx, wts, residual, T, self.top, ctx.seq_of_token)
         P = T * self.top
-        # the sorted form pays one launch per expert and matrix behind a read-back: worth it where an expert's
-        # product is large (measured: 256 rows of 2,048 x 4,096 yes, of 1,024 x 2,048 no)
-        prefer_mma = (self._mma and P <= K.MOE_MMA_MAX_PAIRS
-                      and (P / self.E) * self.inter * self.hidden < SORTED_FORM_MIN_WORK)
-        if self._grouped is not None and self._grouped.takes(ctx) and not prefer_mma:
+        one_launch = self.E <= K.MOE_GROUPED_MAX_EXPERTS
+        most = ONE_LAUNCH_MAX_PAIRS if one_launch else K.MOE_MMA_MAX_PAIRS
+        large = P > most or (P / self.E) * self.inter * self.hidden >= SORTED_FORM_MIN_WORK
+        if self._grouped is not None and large and self._grouped.takes(ctx):
             self._grouped.run(h, idx, wts, residual, ctx)
             return
-        if self._mma and h.dtype == torch.bfloat16 and (P <= K.MOE_MMA_MAX_PAIRS or self._grouped is None):
+        if self._mma and h.dtype == torch.bfloat16 and (P <= most or self._grouped is None):
             xs = ctx.ws.get("moe_rows_in", (P, self.hidden), torch.bfloat16)
             yb = ctx.ws.get("moe_act_rows", (P, self.inter), torch.bfloat16)
             rows = ctx.ws.get("moe_rows_out", (P, self.hidden), torch.float32)
             flat_idx, flat_wts = idx.view(-1), wts.view(-1)
-            if self.E <= K.MOE_GROUPED_MAX_EXPERTS:
+            if one_launch:
                 # every expert's rows side by side, one tcgen05 launch per matrix for all experts
                 offsets = ctx.ws.get("moe_offsets", (self.E + 1,), torch.int32)
                 place = ctx.ws.get("moe_place", (P,), torch.int32)
