@@ -359,9 +359,10 @@ GG_API gg_moe_grouped(const void* x, const void* w, const int* offsets, int P, i
     if (E <= 0 || E > MAX_E || N <= 0 || K <= 0 || (K % 8) || status == nullptr || (((uintptr_t)x | (uintptr_t)w) & 15) ||
         (long long)E * 2 * N > 0x7fffffffLL)
         return GG_ERR_ARG;
-    // Measured (16 experts of 2,048 x 1,024, two a token, gate/up + down): 4,096 pairs 95 us on 256-wide tiles; 994 pairs 53 us
-    // on 128-wide ones, where each expert's weights are read for some sixty rows.  Few pairs: an expert may have all of them (the rows of a
-    // padded batch all go to the first), so P bounds the rows of a tile.
+    // Measured, gate/up + down, us with 128-wide tiles / 256-wide ones by pairs per expert: 16 experts of 4,096 x 2,048: 32 147 / 147, 96 155 / 156,
+    // 128 192 / 183, 160 263 / 214, 256 289 / 255, 512 477 / 420; 16 of 2,048 x 1,024: 32 44 / 48, 96 48 / 53, 128 68 / 68, 256 92 / 88,
+    // 512 133 / 120; 64 of 2,048 x 768: 32 113 / 124, 96 128 / 135, 128 160 / 157.  (8 of 1,024 x 512 keep to the narrow tiles at any number:
+    // 512 27 / 28.)  Few pairs: an expert may have all of them (the rows of a padded batch all go to the first), so P bounds the rows of a tile.
     const bool wide = P >= 128LL * E;
     CUtensorMap tb;
     const int rc = tma::make_map_bf16(&tb, w, (unsigned long long)E * (gated ? 2 : 1) * N, K, K, wide ? 128 : 64);

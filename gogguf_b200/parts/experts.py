@@ -18,8 +18,8 @@ weight.  `weight_scale` multiplies the weights after the renormalisation (which 
 + 1e-20).
 The experts' matrices are reached through the chosen index with nothing read back: on the CUDA cores pair by pair
 (the 32-bit path, sizes the tensor-core forms do not take), or in bfloat16 with the pairs' rows placed expert by expert
-and one tcgen05 launch per matrix for all experts (decode steps, prompts; beyond 1,024 experts on mma.sync, a CTA per
-expert and 64 output rows).  Prompts of more than 16,384 pairs sort them, read the ranges back and run one tcgen05 product per
+and one tcgen05 launch per matrix for all experts (decode steps, prompts; small matrices with few pairs, and more than 1,024
+experts, on mma.sync, a CTA per expert and 64 output rows).  Prompts of more than 16,384 pairs sort them, read the ranges back and run one tcgen05 product per
 expert and matrix.
 """
 from __future__ import annotations
@@ -188,7 +188,7 @@ class RoutedExperts:
             cls = lookup(FEED_FORWARDS, sh.kind, "feed-forward")
             self.shared = cls(sh, {local: weights.pop(sh.prefix + local) for local in cls.tensors(sh)}, rt)
         self._grouped = None
-        # rows on 16-byte boundaries: what the tensor-core forms (tcgen05; mma.sync for more experts than that form keeps ranges for) take
+        # rows on 16-byte boundaries: what the tensor-core forms (tcgen05; mma.sync for small or very many experts) take
         self._mma = (rt.fast and rt.dtype == torch.bfloat16 and self.w_gu.dtype == torch.bfloat16
                      and self.hidden % 8 == 0 and self.inter % 8 == 0)
         if rt.fast and rt.dtype == torch.bfloat16 and self.w_gu.dtype == torch.bfloat16:
@@ -231,7 +231,11 @@ class RoutedExperts:
                 raise ValueError("routed experts: identity experts take their weight on the output")
             K.moe_identity(h, idx, wts, residual, T, self.top, ctx.seq_of_token)
         P = T * self.top
-        one_launch = self.E <= K.MOE_GROUPED_MAX_EXPERTS
+        # (small matrices with few pairs each: the fixed cost of the tcgen05 kernels, 3 us a launch, is more than all of the mma.sync
+        # form.  us a layer, one launch / mma.sync: 4 experts of 64 x 64, 32 pairs 15 / 11, 256 pairs 15 / 16; 32 of 256 x 256, 64 pairs 20 / 16; 128 of
+        # 256 x 128, 128 pairs 21 / 15; of 512 x 256 and larger no case where mma.sync is quicker)
+        small = self.hidden * self.inter <= 1 << 16 and P <= min(32 * self.E, K.MOE_MMA_MAX_PAIRS)
+        one_launch = self.E <= K.MOE_GROUPED_MAX_EXPERTS and not small
         most = ONE_LAUNCH_MAX_PAIRS if one_launch else K.MOE_MMA_MAX_PAIRS
         large = P > most or (P / self.E) * self.inter * self.hidden >= SORTED_FORM_MIN_WORK
         if self._grouped is not None and large and self._grouped.takes(ctx):
@@ -253,7 +257,7 @@ class RoutedExperts:
                 K.moe_grouped(yb, self.w_d, offsets, P, rows, False)
                 K.moe_combine(rows, place, residual, T, self.top, ctx.seq_of_token, idx=idx if self.identity else None)
                 return
-            # more experts than that kernel keeps ranges for: their rows stream through mma.sync (a launch per slice of pairs)
+            # small matrices, or more experts than that kernel keeps ranges for: the rows stream through mma.sync (a launch per slice of pairs)
             K.moe_gather(h, wts, None, xs, P, self.top, self.on_input)
             for p0 in range(0, P, K.MOE_MMA_MAX_PAIRS):
                 p1 = min(P, p0 + K.MOE_MMA_MAX_PAIRS)

@@ -41,3 +41,11 @@ def test_forms_at_the_limits(monkeypatch):
     assert route(monkeypatch, 16, 2048, 1024, 2, 250, decode=True) == "one launch"
     assert route(monkeypatch, 16, 2048, 1024, 2, 10000) == "sorted"
     assert route(monkeypatch, 16, 2048, 1024, 2, 10000, decode=True) == "cores"   # (a step that may not read back)
+
+
+@pytest.mark.parametrize("E,W,F,top,T,mma_us,one_launch_us", [
+    # measured, us a layer
+    (4, 64, 64, 1, 16, 8.8, 14.7), (4, 64, 64, 1, 128, 11.4, 15.0), (8, 128, 128, 2, 16, 10.8, 16.1), (32, 256, 256, 2, 4, 14.6, 17.9),
+    (128, 256, 128, 1, 61, 14.3, 19.3), (1000, 256, 128, 1, 8, 19.2, 22.2), (8, 512, 256, 2, 4, 20.2, 18.4), (128, 1024, 512, 1, 16, 39.9, 24.6), (4, 64, 64, 1, 256, 17.5, 15.7)])
+def test_small_experts(monkeypatch, E, W, F, top, T, mma_us, one_launch_us):
+    assert route(monkeypatch, E, W, F, top, T) == ("mma" if mma_us < one_launch_us else "one launch")
