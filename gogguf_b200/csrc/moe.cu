@@ -14,13 +14,12 @@
 
 // ----------------------------------------------------------------------------- router logits
 // z[t, e] = Wr[e] . h[t] in float32: a CTA has 8 warps, TB tokens' rows in shared memory and EB experts a warp.  A product
-// of so few output columns would be one or two CTAs of the tiled kernels.  A lane takes four neighbouring elements of every
-// 128 (VEC: 8- or 16-byte loads, W a multiple of 4 and aligned rows; shared-memory reads without bank conflicts); the order
-// of the sums depends on neither TB, EB nor VEC.  (The form of the loads is no run-time branch: behind one, a warp's sixteen
+// of so few output columns would be one or two CTAs of the tiled kernels.  W is a multiple of 4; a lane takes four neighbouring
+// elements of every 128 (VEC: 8- or 16-byte loads from aligned rows; shared-memory reads without bank conflicts); the order of
+// the sums depends on neither TB, EB nor VEC.  (The form of the loads is no run-time branch: behind one, a warp's sixteen
 // loads of a row of 2,048 waited for one another, 11 us for 8 tokens.)
 template <typename T, bool VEC>
-__device__ __forceinline__ float4 load4(const T* p, int left) {
-    float v[4];
+__device__ __forceinline__ float4 load4(const T* p) {
     if (VEC) {
         if (sizeof(T) == 4) return *reinterpret_cast<const float4*>(p);
         const uint2 u = *reinterpret_cast<const uint2*>(p);
@@ -28,22 +27,41 @@ __device__ __forceinline__ float4 load4(const T* p, int left) {
         const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
         return make_float4(a.x, a.y, b.x, b.y);
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = j < left ? to_f<T>(p[j]) : 0.f;
-    return make_float4(v[0], v[1], v[2], v[3]);
+    return make_float4(to_f<T>(p[0]), to_f<T>(p[1]), to_f<T>(p[2]), to_f<T>(p[3]));
+}
+
+// W that is no multiple of 4: a warp per (token, expert), an element of every 32 a lane (four one by one took up to twice as long:
+// 20.6 against 10.9 us for 30 tokens, 384 experts and W = 2,050)
+template <typename TX, typename TW>
+__global__ void __launch_bounds__(256) moe_router_logits_odd_kernel(const TX* h, const TW* __restrict__ wr, float* z, int W, int E) {
+    pdl_launch();
+    pdl_wait();
+    extern __shared__ float ro[];
+    const int t = blockIdx.x;
+    const TX* ht = h + (size_t)t * W;
+    for (int i = threadIdx.x; i < W; i += blockDim.x) ro[i] = to_f<TX>(ht[i]);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int e = blockIdx.y * 8 + warp;
+    if (e >= E) return;
+    const TW* w = wr + (size_t)e * W;
+    float s = 0.f;
+    for (int i = lane; i < W; i += 32) s = fmaf(to_f<TW>(w[i]), ro[i], s);
+    s = warp_sum(s);
+    if (lane == 0) z[(size_t)t * E + e] = s;
 }
 
 template <typename TX, typename TW, int TB, int EB, bool VEC>
 __global__ void __launch_bounds__(256) moe_router_logits_kernel(const TX* h, const TW* __restrict__ wr, float* z, int T, int W, int E) {
     pdl_launch();
     pdl_wait();
-    extern __shared__ __align__(16) float rx[];          // [TB][W4], zeros from W on
-    const int t0 = blockIdx.x * TB, W4 = (W + 3) / 4 * 4;
+    extern __shared__ __align__(16) float rx[];          // [TB][W]
+    const int t0 = blockIdx.x * TB;
 #pragma unroll
     for (int u = 0; u < TB; ++u)
-        for (int k = threadIdx.x * 4; k < W4; k += 256 * 4)
-            *reinterpret_cast<float4*>(rx + u * W4 + k) =
-                t0 + u < T ? load4<TX, VEC>(h + (size_t)(t0 + u) * W + k, W - k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = threadIdx.x * 4; k < W; k += 256 * 4)
+            *reinterpret_cast<float4*>(rx + u * W + k) =
+                t0 + u < T ? load4<TX, VEC>(h + (size_t)(t0 + u) * W + k) : make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e0 = (blockIdx.y * 8 + warp) * EB;
@@ -57,10 +75,10 @@ __global__ void __launch_bounds__(256) moe_router_logits_kernel(const TX* h, con
     for (int i = lane * 4; i < W; i += 128) {
         float4 w[EB];
 #pragma unroll
-        for (int v = 0; v < EB; ++v) w[v] = load4<TW, VEC>(wr + (size_t)min(e0 + v, E - 1) * W + i, W - i);
+        for (int v = 0; v < EB; ++v) w[v] = load4<TW, VEC>(wr + (size_t)min(e0 + v, E - 1) * W + i);
 #pragma unroll
         for (int u = 0; u < TB; ++u) {
-            const float4 a = *reinterpret_cast<const float4*>(rx + u * W4 + i);
+            const float4 a = *reinterpret_cast<const float4*>(rx + u * W + i);
 #pragma unroll
             for (int v = 0; v < EB; ++v)
                 s[v][u] = fmaf(w[v].w, a.w, fmaf(w[v].z, a.z, fmaf(w[v].y, a.y, fmaf(w[v].x, a.x, s[v][u]))));
@@ -79,15 +97,20 @@ GG_API gg_moe_router_logits(const void* h, int h_dtype, const void* wr, int w_dt
                             cudaStream_t stream) {
     if (T <= 0) return 0;
     if (W <= 0 || E <= 0 || (size_t)W * 4 > 48 * 1024 || (E + 7) / 8 > 65535) return GG_ERR_ARG;
-    // four tokens and two experts a warp share what is read, once that leaves CTAs enough for the chip
-    const size_t row = (size_t)((W + 3) / 4 * 4) * sizeof(float);
-    const bool many = (long long)T * ((E + 15) / 16) >= 4 * 148 && 4 * row <= 48 * 1024;
+    // four tokens and two experts a warp share what is read, once that leaves CTAs enough for the chip and, with few experts, warps
+    // (592 tokens, 4 experts, W = 2,048: 6.1 us against 2.9 a token and an expert at a time; 900, W = 7,168: 8.3 against 11.6; 592 tokens,
+    // 16 experts: 5.7 against 8.5)
+    const size_t row = (size_t)W * sizeof(float);
+    const long long groups = (T + 3) / 4;
+    const bool many = (long long)T * ((E + 15) / 16) >= 4 * 148 && groups * ((E + 1) / 2) >= 400 && 4 * row <= 48 * 1024;
     const dim3 grid = many ? dim3((T + 3) / 4, (E + 15) / 16) : dim3(T, (E + 7) / 8);
-    const bool vec = W % 4 == 0 && (((uintptr_t)h | (uintptr_t)wr) & 15) == 0;
+    const bool vec = (((uintptr_t)h | (uintptr_t)wr) & 15) == 0;
 #define GG_RL1(TX, TW, TB, EB, VEC) gg_launch(moe_router_logits_kernel<TX, TW, TB, EB, VEC>, grid, dim3(256), TB * row, stream, 1, \
         (const TX*)h, (const TW*)wr, z, T, W, E)
-#define GG_RL(TX, TW) (many ? (vec ? GG_RL1(TX, TW, 4, 2, true) : GG_RL1(TX, TW, 4, 2, false)) \
-                            : (vec ? GG_RL1(TX, TW, 1, 1, true) : GG_RL1(TX, TW, 1, 1, false)))
+#define GG_RL(TX, TW) (W % 4 ? gg_launch(moe_router_logits_odd_kernel<TX, TW>, dim3(T, (E + 7) / 8), dim3(256), row, stream, 1, (const TX*)h, \
+                                         (const TW*)wr, z, W, E) \
+                       : many ? (vec ? GG_RL1(TX, TW, 4, 2, true) : GG_RL1(TX, TW, 4, 2, false)) \
+                              : (vec ? GG_RL1(TX, TW, 1, 1, true) : GG_RL1(TX, TW, 1, 1, false)))
     if (h_dtype == GG_F32 && w_dtype == GG_F32) return GG_RL(float, float);
     if (h_dtype == GG_BF16 && w_dtype == GG_BF16) return GG_RL(bf16, bf16);
     if (h_dtype == GG_BF16 && w_dtype == GG_F32) return GG_RL(bf16, float);
