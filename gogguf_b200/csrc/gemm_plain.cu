@@ -11,11 +11,12 @@
 // is summed with one fused multiply-add after another in ascending k, and the four sums are added as
 // (s0 + s1) + (s2 + s3).  Every tile size below keeps this order, so the same bits come from all of them.
 //
-// A CTA owns a BM x BN tile of the output and has G groups of threads; a group sums 4 / G neighbouring
-// slices of its whole tile, with TM x TN outputs per thread, from a ring of STAGES shared-memory stages of
+// A CTA owns a BM x BN tile of the output and has four groups of threads; a group sums one slice of the
+// whole tile, with TM x TN outputs per thread, from a ring of STAGES shared-memory stages of
 // its own (BK columns of x and W as float32, rows padded by 16 bytes: the float4 reads along k of eight
 // neighbouring rows touch all banks once).  Four slices side by side are what keeps a CTA's loads of
 // W in flight when M is small and the time is that of reading W; at large M the arithmetic bounds.
+// (The tile for many rows, below, has two groups with two slices each.)
 #include "common.cuh"
 
 #define SLICES 4
@@ -73,19 +74,19 @@ __device__ __forceinline__ void stage_rows(float* dst, const T* src, long long l
     }
 }
 
-template <typename TX, typename TW, int BM, int BN, int TM, int TN, int G, int BK, int STAGES, bool ELEMENTS>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
+template <typename TX, typename TW, int BM, int BN, int TM, int TN, int BK, int STAGES, bool ELEMENTS>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN) * SLICES) gemm_plain_kernel(
     const TX* x, const TW* __restrict__ w, void* out, int out_bf16, int accumulate, int M, int N, int K, long long ldx,
     long long ldo, const float* __restrict__ bias, int m_tiles, int async_x, int async_w, int early) {
     constexpr int THN = BN / TN, THM = BM / TM, THREADS = THN * THM;
-    constexpr int STAGE = (BM + BN) * (BK + 4), PER = SLICES / G;
+    constexpr int STAGE = (BM + BN) * (BK + 4);
     extern __shared__ __align__(16) float sm[];
     if (early) pdl_launch();
     const int g = threadIdx.x / THREADS, tid = threadIdx.x % THREADS;
     const int tx = tid % THN, ty = tid / THN;
     const int m0 = (int)(blockIdx.x % m_tiles) * BM, n0 = (int)(blockIdx.x / m_tiles) * BN;
     const int len = slice_len(K);
-    const int k_begin = min(K, g * PER * len), k_end = min(K, (g + 1) * PER * len);
+    const int k_begin = min(K, g * len), k_end = min(K, (g + 1) * len);
     const int steps = (k_end - k_begin + BK - 1) / BK;
     float* ring = sm + (size_t)g * STAGES * STAGE;
     auto load_w = [&](int it) {
@@ -102,12 +103,11 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
         load_x(s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    float acc[TM][TN], run[PER > 1 ? TM : 1][PER > 1 ? TN : 1];
+    float acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-    const int per_slice = len / BK;
 #pragma unroll 1
     for (int it = 0; it < steps; ++it) {
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
@@ -115,12 +115,6 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
         load_w(it + STAGES - 1);
         load_x(it + STAGES - 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (PER > 1 && it == per_slice) {                // the first of the group's two slices is done
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) { run[PER > 1 ? i : 0][PER > 1 ? j : 0] = acc[i][j]; acc[i][j] = 0.f; }
-        }
         const float* xs = ring + (it % STAGES) * STAGE + ty * (BK + 4);
         const float* ws = ring + (it % STAGES) * STAGE + (BM + tx) * (BK + 4);
 #pragma unroll
@@ -142,12 +136,6 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
             }
         }
     }
-    if (PER > 1 && steps > per_slice) {
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = run[PER > 1 ? i : 0][PER > 1 ? j : 0] + acc[i][j];
-    }
     // the groups' sums through shared memory: (s0 + s1) + (s2 + s3)
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -168,7 +156,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
             if (m >= M || n >= N) continue;
             const float* o = sm + (i * TN + j) * THREADS + tid;
             float v = acc[i][j] + o[0];
-            if (G == 4) v += o[TM * TN * THREADS] + o[2 * TM * TN * THREADS];
+            v += o[TM * TN * THREADS] + o[2 * TM * TN * THREADS];
             if (bias != nullptr) v += bias[n];
             if (out_bf16) reinterpret_cast<bf16*>(out)[(size_t)m * ldo + n] = __float2bfloat16_rn(v);
             else {
@@ -179,13 +167,13 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN) * G) gemm_plain_kernel(
     }
 }
 
-template <typename TX, typename TW, int BM, int BN, int TM, int TN, int G, int BK, int STAGES, bool ELEMENTS = false>
+template <typename TX, typename TW, int BM, int BN, int TM, int TN, int BK, int STAGES, bool ELEMENTS = false>
 static int launch_tile(const TX* x, const TW* w, void* out, int out_bf16, int accumulate, int M, int N, int K,
                        long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
-    constexpr int threads = (BM / TM) * (BN / TN) * G;
-    constexpr size_t ring = (size_t)G * STAGES * (BM + BN) * (BK + 4) * sizeof(float);
-    static_assert(ring <= 227 * 1024 && ring >= (size_t)(G - 1) * BM * BN * sizeof(float), "shared memory");
-    auto kern = gemm_plain_kernel<TX, TW, BM, BN, TM, TN, G, BK, STAGES, ELEMENTS>;
+    constexpr int threads = (BM / TM) * (BN / TN) * SLICES;
+    constexpr size_t ring = (size_t)SLICES * STAGES * (BM + BN) * (BK + 4) * sizeof(float);
+    static_assert(ring <= 227 * 1024 && ring >= (size_t)(SLICES - 1) * BM * BN * sizeof(float), "shared memory");
+    auto kern = gemm_plain_kernel<TX, TW, BM, BN, TM, TN, BK, STAGES, ELEMENTS>;
     static int known[GG_MAX_DEVICES] = {};
     int resident = 0;
     const int rc = gg_resident(kern, threads, ring, known, resident);
@@ -206,8 +194,8 @@ static int launch_tile(const TX* x, const TW* w, void* out, int out_bf16, int ac
 // fma.rn.f32x2 74): a thread's sums are pairs of neighbouring columns.  So x and W lie in shared memory with k as the
 // slow index, four columns or rows a 16-byte read, and come there through registers (the next stage's loads are
 // issued before this stage's arithmetic).  Shared-memory reads bound it next: with x stored as pairs, which saves packing each
-// value twice but reads six times 16 bytes a column instead of four, a prompt batch took 6.29 ms instead of 4.97.  Both halves of a packed multiply-add are rounded as fma.rn.f32, so the bits
-// are those of the other tiles.
+// value twice but reads six times 16 bytes a column instead of four, a prompt batch took 6.29 ms instead of 4.97.  Both halves of a
+// packed multiply-add are rounded as fma.rn.f32, so the bits are those of the other tiles.
 #define WIDE_BN 64
 #define WIDE_BK 16
 
@@ -402,32 +390,32 @@ static int launch(const void* xv, const void* wv, void* out, int out_bf16, int a
                   int M, int N, int K, long long ldx, long long ldo, const float* bias, cudaStream_t stream) {
     const TX* x = (const TX*)xv;
     const TW* w = (const TW*)wv;
-#define GP(BM, BN, TM, TN, G, BK, ...) return launch_tile<TX, TW, BM, BN, TM, TN, G, BK, __VA_ARGS__>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream)
+#define GP(BM, BN, TM, TN, BK, ...) return launch_tile<TX, TW, BM, BN, TM, TN, BK, __VA_ARGS__>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream)
     // Up to 16 rows the time is that of reading W, and what counts is how much of it is asked for at a time.  With a CTA an SM
     // or less, deep rings of wide stages; with more tiles, the ring that lets most of them be resident.  Measured, M = 4
     // (us; BK 32 in 6 stages for all | as below): 2,048 x 2,048 10.7 | 6.4, 2,048 x 5,376 25.4 | 13.6, 4,096 x 2,048 11.6 | 9.3,
     // 10,752 x 2,048 25.2 | 22.2, 65,536 x 2,048 106 | 98 (5.5 TB/s).
     const long long tiles = (long long)((N + 15) / 16) * ((M + 15) / 16);
     if (M <= 2) {
-        if (tiles <= 148) GP(2, 16, 1, 1, 4, 128, 4);
-        if (tiles <= 296) GP(2, 16, 1, 1, 4, 64, 4);
-        GP(2, 16, 1, 1, 4, 64, 2);
+        if (tiles <= 148) GP(2, 16, 1, 1, 128, 4);
+        if (tiles <= 296) GP(2, 16, 1, 1, 64, 4);
+        GP(2, 16, 1, 1, 64, 2);
     }
     if (M <= 4) {
-        if (tiles <= 148) GP(4, 16, 2, 1, 4, 128, 4);
-        if (tiles <= 296) GP(4, 16, 2, 1, 4, 64, 4);
-        GP(4, 16, 2, 1, 4, 64, 2);
+        if (tiles <= 148) GP(4, 16, 2, 1, 128, 4);
+        if (tiles <= 296) GP(4, 16, 2, 1, 64, 4);
+        GP(4, 16, 2, 1, 64, 2);
     }
     if (M <= 8) {
-        if (tiles <= 74) GP(8, 8, 2, 1, 4, 128, 3);
-        if (tiles <= 148) GP(8, 16, 2, 2, 4, 64, 6);
-        if (tiles <= 296) GP(8, 16, 2, 2, 4, 64, 4);
-        GP(8, 16, 2, 2, 4, 64, 2);
+        if (tiles <= 74) GP(8, 8, 2, 1, 128, 3);
+        if (tiles <= 148) GP(8, 16, 2, 2, 64, 6);
+        if (tiles <= 296) GP(8, 16, 2, 2, 64, 4);
+        GP(8, 16, 2, 2, 64, 2);
     }
     if (M <= 16) {
-        if (tiles <= 148) GP(16, 8, 2, 2, 4, 64, 3);
-        if (tiles <= 296) GP(16, 16, 4, 2, 4, 64, 3);
-        GP(16, 16, 4, 2, 4, 64, 2);
+        if (tiles <= 148) GP(16, 8, 2, 2, 64, 3);
+        if (tiles <= 296) GP(16, 16, 4, 2, 64, 3);
+        GP(16, 16, 4, 2, 64, 2);
     }
     // More rows: the quickest of four tiles.  Measured per tile, in microseconds per 1,000 of K: 148 tiles or fewer, and 296 (two an
     // SM); a grid is as many rounds of 296 and one of what is left.  Three rows of the table: float32 in chunks, float32 by elements, any
@@ -447,12 +435,12 @@ static int launch(const void* xv, const void* wv, void* out, int out_bf16, int a
         if (i == 0 || cost < least) { best = i; least = cost; }
     }
     if (best == 0) {
-        if (elements) GP(32, 16, 4, 4, 4, 32, 4, true);
-        GP(32, 16, 4, 4, 4, 32, 4, false);
+        if (elements) GP(32, 16, 4, 4, 32, 4, true);
+        GP(32, 16, 4, 4, 32, 4, false);
     }
     if (best == 1) {
-        if (elements) GP(64, 32, 8, 4, 4, 16, 3, true);
-        GP(64, 32, 8, 4, 4, 16, 3, false);
+        if (elements) GP(64, 32, 8, 4, 16, 3, true);
+        GP(64, 32, 8, 4, 16, 3, false);
     }
     if (best == 2) return launch_wide<TX, TW, 64>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream);
     return launch_wide<TX, TW, 128>(x, w, out, out_bf16, accumulate, M, N, K, ldx, ldo, bias, stream);
