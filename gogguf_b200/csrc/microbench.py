@@ -1,4 +1,4 @@
-"""Kernel micro-benchmarks: python -m gogguf_b200.csrc.microbench [gemm|gemm_layer|attn|prefill_attn|sample|latent|retention|recurrence|dinuzen|kulesun|niresun] [--m 1,8,64] [--ctx 2048,8192]
+"""Kernel micro-benchmarks: python -m gogguf_b200.csrc.microbench [gemm|gemm_layer|attn|prefill_attn|sample|latent|retention|recurrence|dinuzen|kulesun|niresun|plain|shares|experts] [--m 1,8,64] [--ctx 2048,8192]
 
 Times single kernels the way a decode step runs them: forty launches captured in a CUDA graph and
 replayed, so that host launch cost is out of the picture and dependent launches overlap as they do
@@ -733,9 +733,119 @@ def mixed_head_runner(H, G, d, dv, g_off, talk, kw, ps, value_heads=None):
     return run
 
 
+def plain() -> None:
+    """The 32-bit path's two kernels (csrc/gemm_plain.cu, csrc/attention_plain.cu): products over numbers of rows and matrices, rows in
+    chunks of 16 bytes and by elements, and attention of decode steps and prompts."""
+    from . import kernels as K
+    dev = "cuda:0"
+    for dx, dw in ((torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16)):
+        for N, k in ((2048, 2048), (10752, 2048), (2048, 5376), (4096, 1001), (300, 2051)):
+            nbuf = max(2, min(24, int(200e6 // (N * k * 4)) + 1))
+            ws = [torch.randn(N, k, device=dev).to(dw) for _ in range(nbuf)]
+            for M in (1, 4, 16, 64, 270, 700, 2048):
+                x, out = torch.randn(M, k, device=dev).to(dx), torch.empty(M, N, device=dev)
+                us = _time_graph(lambda i: K.gemm_plain(x, ws[i % nbuf], out), 10)
+                print(f"gemm_plain {str(dx)[6:]} x {str(dw)[6:]} N={N} K={k} M={M:4d}: {us:8.1f} us {2 * M * N * k / us / 1e6:6.2f} TFLOP/s "
+                      f"{N * k * ws[0].element_size() / us / 1e6:5.2f} TB/s of weights", flush=True)
+            del ws
+    for nq, nkv, d in ((16, 8, 128), (16, 8, 64), (8, 8, 256)):
+        for B, new, history in ((1, 1, 23), (4, 1, 600), (8, 1, 2048), (3, 150, 0), (1, 450, 0)):
+            q, pools, out, ctx, table = _paged_step(B, new, history, nq, nkv, d, torch.float32, 1)
+            us = _time_graph(lambda i: K.attention_plain(q, pools[0][0], pools[0][1], out, ctx["pos"], ctx["sot"], table, 64, B * new, nq, nkv,
+                                                         d, d ** -0.5, 0), 10)
+            print(f"attention_plain float32 nq={nq} nkv={nkv} d={d} B={B} new={new} history={history}: {us:8.1f} us", flush=True)
+
+
+def _paged_step(B, new, history, nq, nkv, d, dtype, nrot):
+    """q, nrot pairs of pools, out, the step's integers and the page table of B sequences of `new` tokens behind `history`."""
+    dev = "cuda:0"
+    c = history + new
+    width = -(-c // 64)
+    pools = [tuple((torch.randn(B * width, nkv, 64, d, device=dev) * 0.5).to(dtype) for _ in range(2)) for _ in range(nrot)]
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)                      # noqa: E731
+    ctx = dict(pos=ints([history + i for _ in range(B) for i in range(new)]), sot=ints([b for b in range(B) for _ in range(new)]),
+               cu=ints([b * new for b in range(B + 1)]), cl=ints([c] * B))
+    q = torch.randn(B * new, nq * d, device=dev).to(dtype)
+    return q, pools, torch.empty_like(q), ctx, ints([[b * width + j for j in range(width)] for b in range(B)])
+
+
+def shares() -> None:
+    """Prefill attention over a history (csrc/attention_fast.cu, bfloat16) with the pages of a query tile in 1, 2, 4 and 8 shares, and the
+    number of shares that the steps take."""
+    from . import fast_attention as FA
+    for nq, nkv, d in ((32, 8, 128), (16, 8, 128), (16, 8, 64), (24, 8, 96)):
+        for B, new in ((1, 3), (1, 128), (1, 333), (1, 640), (3, 64)):
+            for reach in (520, 1024, 2100, 6400):
+                if reach <= new:
+                    continue
+                q, pools, out, ctx, table = _paged_step(B, new, reach - new, nq, nkv, d, torch.bfloat16, 1)
+                tiles = FA.prefill_tiles(B * new, B, new)
+                took = FA.prefill_splits(B * new, B, nq, reach, new, d)
+                us = {s: _time_graph(lambda i: FA.attn_prefill_tc(q, *pools[0], out, ctx["cu"], ctx["cl"], ctx["sot"], table, 64, B * new, B, tiles,
+                                                                  nq, nkv, d, d ** -0.5, 0, splits=s), 10) for s in (1, 2, 4, 8)}
+                print(f"prefill attention nq={nq} d={d} B={B} new={new} positions={reach}: "
+                      + ", ".join(f"{s} shares {t:.1f}" for s, t in us.items()) + f" us; {took} taken", flush=True)
+
+
+def experts() -> None:
+    """The routed experts after routing (csrc/moe_grouped.cu, csrc/moe.cu): one launch per matrix, the form through the index on
+    mma.sync, and the sorted form with its read-back (wall clock), by numbers of pairs."""
+    import time
+    from types import SimpleNamespace
+    from . import kernels as K
+    from ..parts import experts_grouped
+    from ..parts.base import Runtime, Workspace
+    dev = torch.device("cuda:0")
+    for E, W, F, top in ((16, 2048, 1024, 2), (16, 4096, 2048, 2), (64, 2048, 768, 8), (128, 256, 128, 2), (1000, 256, 128, 2)):
+        nrot = max(1, min(4, int(300e6 // (E * 3 * F * W * 2)) + 1))
+        gus = [(torch.randn(E, 2, F, W, device=dev) * 0.02).to(torch.bfloat16) for _ in range(nrot)]
+        dns = [(torch.randn(E, W, F, device=dev) * 0.02).to(torch.bfloat16) for _ in range(nrot)]
+        part = SimpleNamespace(E=E, inter=F, hidden=W, w_gu=gus[0], w_d=dns[0], rt=Runtime(dtype=torch.bfloat16, device=dev), top=top,
+                               on_input=False, limit=7.0, slope=1.0, up_offset=0.0, out_scale=1.0, identity=0)
+        in_order = experts_grouped.try_make(part) if E <= 64 else None
+        for P in (16, 64, 256, 1000, 4096, 8192, 16384):
+            T = P // top
+            P = T * top
+            idx = torch.rand(T, E, device=dev).topk(top, dim=-1).indices.to(torch.int32)
+            flat, wts, h = idx.view(-1), torch.rand(T, top, device=dev), torch.randn(T, W, device=dev).to(torch.bfloat16)
+            xs, y = torch.empty(P, W, device=dev, dtype=torch.bfloat16), torch.empty(P, F, device=dev, dtype=torch.bfloat16)
+            rows, res, row_wts = torch.empty(P, W, device=dev), torch.zeros(T, W, device=dev), torch.empty(P, device=dev)
+            offsets, place = torch.empty(E + 1, dtype=torch.int32, device=dev), torch.empty(P, dtype=torch.int32, device=dev)
+
+            def one(i):
+                K.moe_place_gather(h, wts.view(-1), flat, P, E, top, False, offsets, place, row_wts, xs)
+                K.moe_grouped(xs, gus[i % nrot], offsets, P, y, True, 7.0, 1.0, 1.0, row_wts, up_offset=0.0)
+                K.moe_grouped(y, dns[i % nrot], offsets, P, rows, False)
+                K.moe_combine(rows, place, res, T, top, None)
+
+            def through_index(i):
+                K.moe_gather(h, wts, None, xs, P, top, False)
+                K.moe_expert_mma(xs, gus[i % nrot], flat, P, y, True, 7.0, 1.0, 1.0, wts.view(-1), up_offset=0.0)
+                K.moe_expert_mma(y, dns[i % nrot], flat, P, rows, False)
+                K.moe_combine(rows, None, res, T, top, None)
+
+            line = f"experts E={E} W={W} F={F} top={top} pairs={P:5d}: one launch {_time_graph(one, 10):8.1f} us"
+            if P <= K.MOE_MMA_MAX_PAIRS:
+                line += f", through the index {_time_graph(through_index, 10):8.1f} us"
+            if in_order is not None and P >= 512:
+                ctx = SimpleNamespace(n_tokens=T, ws=Workspace(dev), seq_of_token=torch.zeros(T, dtype=torch.int32, device=dev))
+                for _ in range(3):
+                    in_order.run(h, idx, wts, res, ctx)
+                torch.cuda.synchronize()
+                t0 = time.perf_counter()
+                for _ in range(10):
+                    in_order.run(h, idx, wts, res, ctx)
+                torch.cuda.synchronize()
+                line += f", sorted {(time.perf_counter() - t0) * 1e5:8.1f} us"
+            print(line, flush=True)
+        del gus, dns, part, in_order
+        torch.cuda.empty_cache()
+
+
 def main() -> None:
     ap = argparse.ArgumentParser()
-    ap.add_argument("what", choices=["gemm", "gemm_layer", "attn", "prefill_attn", "sample", "latent", "retention", "recurrence", "dinuzen", "kulesun", "niresun"])
+    ap.add_argument("what", choices=["gemm", "gemm_layer", "attn", "prefill_attn", "sample", "latent", "retention", "recurrence", "dinuzen", "kulesun", "niresun",
+                                     "plain", "shares", "experts"])
     ap.add_argument("--m", default="1,8,64", help="token counts (gemm), batch sizes (attn) or prompt lengths (prefill_attn)")
     ap.add_argument("--ctx", default="2048", help="attn: cached positions per sequence (comma separated)")
     ap.add_argument("--scratch", action="store_true", help="attn: splits merged by a second kernel instead of inside clusters")
@@ -750,8 +860,9 @@ def main() -> None:
     if a.what == "recurrence":
         recurrence()
         return
-    if a.what in ("dinuzen", "kulesun", "niresun"):
-        {"dinuzen": dinuzen, "kulesun": kulesun, "niresun": niresun}[a.what]()
+    alone = {"dinuzen": dinuzen, "kulesun": kulesun, "niresun": niresun, "plain": plain, "shares": shares, "experts": experts}
+    if a.what in alone:
+        alone[a.what]()
         return
     if a.what == "attn":
         for c in a.ctx.split(","):
