@@ -6,7 +6,9 @@ tensor that is not on a CUDA device, or a missing compiler, raises.
 """
 from __future__ import annotations
 
-from typing import Optional
+import struct
+from operator import index
+from typing import List, Optional, Sequence
 
 import torch
 
@@ -1322,6 +1324,33 @@ def sample_topk(logits: torch.Tensor, temp: float, top_k: int, top_p: float, min
         buf = _topk_scratch[logits.device] = torch.empty(max(words, 1 << 16), dtype=torch.int64, device=logits.device)
     kernel("sampling", "gg_sample_topk")(_p(logits), logits.stride(0), float(temp), int(top_k), float(top_p),
                                           float(min_p), _p(uniforms), _p(out), R, V, _p(buf), buf.numel(), _stream())
+
+
+def _words64(numbers: Sequence[int]) -> bytes:
+    """Whole numbers as 64-bit words, modulo 2^64 (an array of ctypes takes seven times as long)."""
+    try:
+        return struct.pack(f"{len(numbers)}q", *numbers)
+    except struct.error:
+        return struct.pack(f"{len(numbers)}Q", *(index(n) & ((1 << 64) - 1) for n in numbers))
+
+
+def sample_topk_ids(logits: torch.Tensor, temp: float, top_k: int, top_p: float, min_p: float, seed: int, streams: Sequence[int],
+                    steps: Sequence[int], ids: torch.Tensor) -> List[int]:
+    """`sample_topk` for a caller that waits for the ids: row r draws with the uniform number of (seed, streams[r], steps[r]), computed
+    on the way; `ids` is page-locked host memory (int32) that the kernel writes to."""
+    _need(logits, torch.float32, "logits")
+    R, V = len(streams), logits.shape[1]
+    if R > logits.shape[0] or len(steps) < R:
+        raise KernelError(f"sample: {R} streams for {logits.shape[0]} rows and {len(steps)} step counts")
+    if ids.dtype != torch.int32 or not ids.is_pinned() or ids.numel() < R:
+        raise KernelError("sample: the ids go to page-locked int32 host memory, one for each row")
+    words = -(-V // 8192) * min(int(top_k), V) * min(R, 256)
+    buf = _topk_scratch.get(logits.device)
+    if buf is None or buf.numel() < words:
+        buf = _topk_scratch[logits.device] = torch.empty(max(words, 1 << 16), dtype=torch.int64, device=logits.device)
+    kernel("sampling", "gg_sample_topk_ids")(_p(logits), logits.stride(0), float(temp), int(top_k), float(top_p), float(min_p), int(seed),
+                                             _words64(streams), _words64(steps[:R]), ids.data_ptr(), R, V, _p(buf), buf.numel(), _stream())
+    return ids[:R].tolist()
 
 
 _nucleus_scratch = {}

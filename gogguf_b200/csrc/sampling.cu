@@ -453,18 +453,16 @@ __device__ unsigned long long block_kth_largest(int n_mine, KeyOf key_of, int k,
 // What bounds it is instructions: a pass over the digits is some 300 a thread with four keys, several times that with 32.  So a
 // threshold on the value comes first: the keys form groups, and at least k keys reach the k-th largest of the groups'
 // largest (one per group), so the k best are among the keys that reach it.  In a row without order those are k to
-// 1.4 k of the 8,192.  For k up to 64: 128 groups of 64 (two threads each), the k-th found by counting, and the survivors ranked by
-// counting too.  Up to SAMP_SIEVE_K: 1,024 groups of eight, the k-th and then the survivors' k-th by digits, at most four keys
-// a thread.  Where more than SAMP_SIEVE_ROOM pass (large logits side by side) the digits of all keys are walked, as for larger k,
-// where the sieve would let most through.  64 rows of 151,936, k = 20: all keys by digits 187 us, the larger sieve alone
-// 121, as it is 19.
+// 1.4 k of the 8,192.  For k up to 64 a kernel of its own (below).  Up to SAMP_SIEVE_K: 1,024 groups of eight, the k-th and
+// then the survivors' k-th by digits, at most four keys a thread.  Where more than SAMP_SIEVE_ROOM pass (large logits side by
+// side) the digits of all keys are walked, as for larger k, where the sieve would let most through.
 #define SAMP_SLICE_THREADS 256
 #define SAMP_SLICE_PER (SAMP_SLICE / SAMP_SLICE_THREADS)
 #define SAMP_SIEVE_K 512
-#define SAMP_COUNT_K 64
+#define SAMP_FEW_K 64
 #define SAMP_SIEVE_ROOM 1024
 
-// SIEVE: k up to SAMP_SIEVE_K (a kernel of its own, so that the walk over all keys, which it takes only where its sieve fails,
+// SIEVE: k of SAMP_FEW_K + 1 to SAMP_SIEVE_K (a kernel of its own, so that the walk over all keys, which it takes only where its sieve fails,
 // need not keep them in registers).
 template <bool SIEVE>
 __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const float* logits, long long ld, int V, float temp,
@@ -473,10 +471,8 @@ __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const fl
     pdl_wait();
     __shared__ unsigned long long tot[3][4];
     __shared__ unsigned long long room[SAMP_SIEVE_ROOM];
-    __shared__ __align__(16) uint32_t tops[SAMP_SLICE_THREADS / 2];
     __shared__ int n_out, n_room;
-    __shared__ uint32_t at_least;
-    const int row = blockIdx.y, slice = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int row = blockIdx.y, slice = blockIdx.x, tid = threadIdx.x;
     const float* x = logits + (size_t)row * ld;
     const bool scale = temp > 0.f && temp != 1.f;
     const double inv_temp = scale ? 1.0 / (double)temp : 1.0;
@@ -495,39 +491,15 @@ __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const fl
         const int id = id0 + u * SAMP_SLICE_THREADS;
         return id < V ? ((unsigned long long)val[u] << 32) | (unsigned long long)(0xffffffffu - (uint32_t)id) : 0ull;
     };
-    if (tid == 0) { n_out = 0; n_room = 0; at_least = 0xffffffffu; }
+    if (tid == 0) { n_out = 0; n_room = 0; }
     unsigned long long* dst = cand + ((size_t)row * gridDim.x + slice) * k;
     bool sieved = false;
     if (SIEVE) {
-        uint32_t sieve;
-        if (k <= SAMP_COUNT_K) {
-            uint32_t top = 0u;
+        uint32_t best[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-            for (int u = 0; u < SAMP_SLICE_PER; ++u) top = max(top, val[u]);
-            top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
-            if ((lane & 1) == 0) tops[tid >> 1] = top;
-            __syncthreads();
-            if (tid < SAMP_SLICE_THREADS / 2) {
-                const uint32_t mine = tops[tid];
-                int above = 0;
-#pragma unroll 8
-                for (int j = 0; j < SAMP_SLICE_THREADS / 2; j += 4) {
-                    const uint4 t = *reinterpret_cast<const uint4*>(tops + j);
-                    above += (t.x > mine) + (t.y > mine) + (t.z > mine) + (t.w > mine);
-                }
-                // (the smallest value that fewer than k others exceed is the k-th largest)
-                const uint32_t least = __reduce_min_sync(0xffffffffu, above < k ? mine : 0xffffffffu);
-                if (lane == 0) atomicMin(&at_least, least);
-            }
-            __syncthreads();
-            sieve = at_least;
-        } else {
-            uint32_t best[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-            for (int u = 0; u < SAMP_SLICE_PER; ++u) best[u & 3] = max(best[u & 3], val[u]);
-            // (equal values are fine here: only the threshold is asked for; 0: fewer than k groups, every key passes)
-            sieve = (uint32_t)(block_kth_largest<4>(4, [&](int j) { return best[j] != 0u ? ((unsigned long long)best[j] << 32) | 1ull : 0ull; }, k, tot) >> 32);
-        }
+        for (int u = 0; u < SAMP_SLICE_PER; ++u) best[u & 3] = max(best[u & 3], val[u]);
+        // (equal values are fine here: only the threshold is asked for; 0: fewer than k groups, every key passes)
+        const uint32_t sieve = (uint32_t)(block_kth_largest<4>(4, [&](int j) { return best[j] != 0u ? ((unsigned long long)best[j] << 32) | 1ull : 0ull; }, k, tot) >> 32);
 #pragma unroll
         for (int u = 0; u < SAMP_SLICE_PER; ++u) {
             if (val[u] >= sieve && id0 + u * SAMP_SLICE_THREADS < V) {
@@ -571,6 +543,154 @@ __global__ void __launch_bounds__(SAMP_SLICE_THREADS) topk_slice_kernel(const fl
         if (key_of(u) != 0ull && key_of(u) >= thr) dst[atomicAdd(&n_out, 1)] = key_of(u);
 }
 
+// ---- k up to SAMP_FEW_K: what is sieved lies in shared memory and is ranked by counting
+// The k-th largest of GROUPS values (a power of two, 64 or 128, for 0 < k <= GROUPS; ties: the value at the k-th place), by
+// counting: thread g < GROUPS has group g's value, `tops` is a copy that the block has written and synchronised.  *at_least starts
+// as 0xffffffff; the answer is there after the caller's next barrier.
+__device__ __forceinline__ void few_threshold(const uint32_t* tops, int groups, int k, uint32_t* at_least) {
+    const int tid = threadIdx.x;
+    if (tid >= groups) return;
+    const uint32_t mine = tops[tid];
+    int above = 0;
+#pragma unroll 8
+    for (int j = 0; j < groups; j += 4) {
+        const uint4 t = *reinterpret_cast<const uint4*>(tops + j);
+        above += (t.x > mine) + (t.y > mine) + (t.z > mine) + (t.w > mine);
+    }
+    // (the smallest value that fewer than k others exceed is the k-th largest)
+    const uint32_t least = __reduce_min_sync(0xffffffffu, above < k ? mine : 0xffffffffu);
+    if ((tid & 31) == 0) atomicMin(at_least, least);
+}
+// How many groups: n values without order pass a threshold at the k-th of G group maxima with some G ln(G / (G - k)) of them,
+// 24 of 64 groups and 22 of 128 for k = 20, and the counting costs G^2.
+__device__ __forceinline__ int few_groups(int k) { return k <= 24 ? 64 : 128; }
+
+// Stage one for k up to SAMP_FEW_K.  The sieve runs on the logits as they lie in memory, and only what passes is divided by the
+// temperature: in 64 bits for all 32 values of a thread that was a third of the kernel (two conversions and a product each).
+// Dividing by a temperature keeps the order but may make neighbours equal, and among equals the lower id wins, so the sieve lets
+// values a few steps below its threshold pass too; where those are not seen to fall below it after the division (overflow,
+// numbers next to zero) or a NaN is among the logits, everything passes and the digits decide.
+// 512 threads with 16 logits, four blocks an SM: 256 with 32 held 80 registers and three blocks (the code of what passes stood there
+// 32 times).  64 rows of 151,936, k = 20, temperature 0.6, nothing in L2: 16 us, the copy of it would take 6; 19 with 256 threads
+// (what bounds it is the way from one barrier to the next in 2.1 rounds of blocks).
+#define SAMP_FEW_SLICE_THREADS 512
+#define SAMP_FEW_SLICE_PER (SAMP_SLICE / SAMP_FEW_SLICE_THREADS)
+template <bool VEC>
+__global__ void __launch_bounds__(SAMP_FEW_SLICE_THREADS, 4) topk_slice_few_kernel(const float* logits, long long ld, int V, float temp,
+                                                                                   int k, unsigned long long* __restrict__ cand) {
+    pdl_launch();
+    __shared__ unsigned long long tot[3][4];
+    __shared__ unsigned long long room[SAMP_SIEVE_ROOM];
+    __shared__ __align__(16) uint32_t tops[128];
+    __shared__ int n_out, n_room;
+    __shared__ uint32_t at_least;
+    const int row = blockIdx.y, slice = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const float* x = logits + (size_t)row * ld;
+    const bool scale = temp > 0.f && temp != 1.f;
+    const double inv_temp = scale ? 1.0 / (double)temp : 1.0;
+    const int base = slice * SAMP_SLICE + 4 * tid;           // this thread's logits: base + 2,048 u + {0..3}
+    if (tid == 0) { n_out = 0; n_room = 0; at_least = 0xffffffffu; }
+    pdl_wait();
+    uint32_t val[SAMP_FEW_SLICE_PER];                        // ordered values before the division; 0 beyond the row
+#pragma unroll
+    for (int u = 0; u < SAMP_FEW_SLICE_PER / 4; ++u) {
+        const int id = base + 4 * SAMP_FEW_SLICE_THREADS * u;
+        if (VEC) {
+            uint4 t = make_uint4(0u, 0u, 0u, 0u);
+            if (id < V) t = *reinterpret_cast<const uint4*>(x + id);        // V is a multiple of four
+            val[4 * u] = t.x; val[4 * u + 1] = t.y; val[4 * u + 2] = t.z; val[4 * u + 3] = t.w;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) val[4 * u + c] = id + c < V ? __float_as_uint(x[id + c]) : 0u;
+        }
+    }
+    uint32_t top = 0u, low = 0xffffffffu;
+#pragma unroll
+    for (int u = 0; u < SAMP_FEW_SLICE_PER; ++u) {
+        const bool in = base + 4 * SAMP_FEW_SLICE_THREADS * (u >> 2) + (VEC ? 0 : (u & 3)) < V;
+        const uint32_t key = order_key(__uint_as_float(val[u]));
+        low = min(low, in ? key : 0xffffffffu);
+        val[u] = in ? key : 0u;
+        top = max(top, val[u]);
+    }
+    const bool nan = top > 0xff800000u || low < 0x007fffffu;             // beyond either infinity
+    const int groups = few_groups(k);
+    const int share = SAMP_FEW_SLICE_THREADS / groups;
+    for (int o = 1; o < share; o <<= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (lane % share == 0) tops[tid / share] = top;
+    const bool any_nan = __syncthreads_or(nan && scale);
+    few_threshold(tops, groups, k, &at_least);
+    __syncthreads();
+    uint32_t sieve = at_least;
+    if (scale) {
+        const uint32_t below = sieve > 8u ? sieve - 9u : 0u;
+        const bool apart = (float)((double)key_value(below) * inv_temp) < (float)((double)key_value(sieve) * inv_temp);
+        sieve = below != 0u && apart && !any_nan ? below + 1u : 0u;
+    }
+    auto key_of = [&](uint32_t v, int id) -> unsigned long long {        // of an ordered value before the division
+        if (scale) v = order_key((float)((double)key_value(v) * inv_temp));
+        return ((unsigned long long)v << 32) | (unsigned long long)(0xffffffffu - (uint32_t)id);
+    };
+    uint32_t passed = 0u;                                    // a bit a value: few pass, and their code stands here once
+#pragma unroll
+    for (int u = 0; u < SAMP_FEW_SLICE_PER; ++u)
+        if (val[u] >= sieve && base + 4 * SAMP_FEW_SLICE_THREADS * (u >> 2) + (u & 3) < V) passed |= 1u << u;
+    for (; passed != 0u; passed &= passed - 1u) {
+        const int u = __ffs(passed) - 1, id = base + 4 * SAMP_FEW_SLICE_THREADS * (u >> 2) + (u & 3);
+        const int at = atomicAdd(&n_room, 1);
+        if (at < SAMP_SIEVE_ROOM) room[at] = key_of(order_key(x[id]), id);
+    }
+    __syncthreads();
+    unsigned long long* dst = cand + ((size_t)row * gridDim.x + slice) * k;
+    const int n = n_room;
+    if (n <= SAMP_FEW_SLICE_THREADS) {                       // ranks by counting: no two keys are equal
+        if (tid < n) {
+            const unsigned long long mine = room[tid];
+            int above = 0;
+            for (int j = 0; j < n; ++j) above += room[j] > mine;
+            if (above < k) dst[above] = mine;
+        }
+        for (int j = n + tid; j < k; j += SAMP_FEW_SLICE_THREADS) dst[j] = 0ull;
+        return;
+    }
+    // too many for that (equal or large logits side by side): the digits, of what passed or, beyond the room, of all
+    const bool fits = n <= SAMP_SIEVE_ROOM;
+    const int mine = fits ? (n - tid + SAMP_FEW_SLICE_THREADS - 1) / SAMP_FEW_SLICE_THREADS : SAMP_FEW_SLICE_PER;
+    auto any_key = [&](int j) -> unsigned long long {
+        const int at = tid + j * SAMP_FEW_SLICE_THREADS;
+        if (fits) return room[at];
+        const int id = slice * SAMP_SLICE + at;
+        return id < V ? key_of(order_key(x[id]), id) : 0ull;
+    };
+    const unsigned long long thr = block_kth_largest(mine, any_key, k, tot);
+    for (int j = tid; j < k; j += SAMP_FEW_SLICE_THREADS) dst[j] = 0ull;
+    __syncthreads();
+    for (int j = 0; j < mine; ++j) {
+        const unsigned long long key = any_key(j);
+        if (key != 0ull && key >= thr) dst[atomicAdd(&n_out, 1)] = key;
+    }
+}
+
+static int launch_topk_slices(const float* logits, long long ld, int V, float temp, int k, unsigned long long* cand, int R,
+                              cudaStream_t stream) {
+    const dim3 grid((V + SAMP_SLICE - 1) / SAMP_SLICE, R), block(k > SAMP_FEW_K ? SAMP_SLICE_THREADS : SAMP_FEW_SLICE_THREADS);
+    const bool vec = V % 4 == 0 && ld % 4 == 0 && ((uintptr_t)logits & 15) == 0;
+    auto kern = k > SAMP_SIEVE_K ? topk_slice_kernel<false> : k > SAMP_FEW_K ? topk_slice_kernel<true> : vec ? topk_slice_few_kernel<true>
+                                                                                                           : topk_slice_few_kernel<false>;
+    return gg_launch(kern, grid, block, 0, stream, 1, logits, ld, V, temp, k, cand);
+}
+
+// The rows' uniform numbers: in device memory, or in the launch's own arguments where the host has them (no copy ahead of the kernel).
+#define SAMP_DRAWS 256           // rows of a launch that carries its numbers
+struct DrawsAt {
+    const double* p;
+    __device__ __forceinline__ double of(int row) const { return p[row]; }
+};
+struct DrawsIn {
+    double u[SAMP_DRAWS];
+    __device__ __forceinline__ double of(int row) const { return u[row]; }
+};
+
 // Inclusive prefix sums of one double per thread over the block, in thread order; *total gets the block's sum.
 __device__ __forceinline__ double block_scan_f64(double v, double* warp_tot /* 33 */, double* total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -604,9 +724,10 @@ __device__ __forceinline__ double block_scan_f64(double v, double* warp_tot /* 3
 // of exp(x - max) is the sum of zs[row * z_slices ..], and flags[row] is set when the candidates do not hold
 // the whole answer (min-p keeps even the last candidate, or the running sum never reaches top-p): the caller
 // then takes that row through the host chain.
+template <typename Draws>
 __global__ void __launch_bounds__(SAMP_THREADS) sample_topk_kernel(
     const unsigned long long* cand, int n_cand_keys, int top_k, float top_p, float min_p,
-    const double* __restrict__ uniforms, int* __restrict__ out, const double* zs, int z_slices, int* __restrict__ flags,
+    const __grid_constant__ Draws uniforms, int* __restrict__ out, const double* zs, int z_slices, int* __restrict__ flags,
     int V) {
     pdl_launch();
     pdl_wait();
@@ -701,7 +822,7 @@ __global__ void __launch_bounds__(SAMP_THREADS) sample_topk_kernel(
         const double p = kept ? cand_e[a] / Z : 0.0;
         double total;
         const double run = block_scan_f64(p, wtot, &total);
-        const double target = uniforms[row] * total;
+        const double target = uniforms.of(row) * total;
         if (kept) {
             atomicMax(&last_r, tid);
             if (target - run <= 0.0) atomicMin(&pick_r, tid);
@@ -717,6 +838,140 @@ __global__ void __launch_bounds__(SAMP_THREADS) sample_topk_kernel(
     }
 }
 
+// Stage two for a top-k of up to SAMP_FEW_K: one block of 256 threads per row.  What is left of the candidates (a few hundred) behind a
+// threshold as in stage one is ranked by counting, and the chain on the k survivors is one warp's, two of them a lane: sums
+// by shuffles in the order of block_scan_f64, so the numbers are those of the kernel above.  There 1,024 threads walked the digits,
+// scanned three times and met at some 40 barriers for k = 20.
+// 64 rows of 151,936, k = 20, temperature 0.6, top-p 0.95: 4.6 us beyond the kernel before it, 21.7 with sample_topk_kernel.
+#define SAMP_FEW_THREADS 256
+__device__ __forceinline__ double warp_scan_f64(double v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+    }
+    return v;
+}
+// Inclusive prefix sums of 64 numbers, number lane in a and number lane + 32 in b; returns their sum.
+__device__ __forceinline__ double warp_scan2_f64(double& a, double& b, int lane) {
+    a = warp_scan_f64(a, lane);
+    b = warp_scan_f64(b, lane);
+    const double ta = __shfl_sync(0xffffffffu, a, 31), tb = __shfl_sync(0xffffffffu, b, 31);
+    b += ta;
+    return tb + ta;
+}
+
+template <typename Draws>
+__global__ void __launch_bounds__(SAMP_FEW_THREADS) sample_few_kernel(const unsigned long long* cand, int n_cand, int k, float top_p,
+                                                                      float min_p, const __grid_constant__ Draws uniforms,
+                                                                      int* __restrict__ out) {
+    pdl_launch();
+    extern __shared__ unsigned long long ckeys[];
+    __shared__ unsigned long long tot[3][4];
+    __shared__ unsigned long long room[SAMP_FEW_THREADS], best[SAMP_FEW_K];
+    __shared__ __align__(16) uint32_t tops[128];
+    __shared__ double v_e[SAMP_FEW_K], i_e[SAMP_FEW_K];      // exponentials by rank of the value, and by rank of the id
+    __shared__ int v_ri[SAMP_FEW_K], i_id[SAMP_FEW_K];
+    __shared__ unsigned char v_keep[SAMP_FEW_K], i_keep[SAMP_FEW_K];
+    __shared__ int n_room;
+    __shared__ uint32_t at_least;
+    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) { n_room = 0; at_least = 0xffffffffu; }
+    pdl_wait();
+    const unsigned long long* src = cand + (size_t)row * n_cand;
+    const int groups = few_groups(k), share = SAMP_FEW_THREADS / groups;
+    uint32_t top = 0u;
+    for (int j = tid; j < n_cand; j += SAMP_FEW_THREADS) {
+        const unsigned long long key = src[j];
+        ckeys[j] = key;
+        top = max(top, (uint32_t)(key >> 32));
+    }
+    top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    if (groups == 64) top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
+    if (lane % share == 0) tops[tid / share] = top;
+    __syncthreads();
+    few_threshold(tops, groups, k, &at_least);
+    __syncthreads();
+    const uint32_t sieve = at_least;
+    for (int j = tid; j < n_cand; j += SAMP_FEW_THREADS) {
+        const unsigned long long key = ckeys[j];
+        if (key != 0ull && (uint32_t)(key >> 32) >= sieve) {
+            const int at = atomicAdd(&n_room, 1);
+            if (at < SAMP_FEW_THREADS) room[at] = key;
+        }
+    }
+    __syncthreads();
+    if (n_room > SAMP_FEW_THREADS) {                         // many equal values: the digits, ids among them, leave k
+        const int mine = (n_cand - tid + SAMP_FEW_THREADS - 1) / SAMP_FEW_THREADS;
+        const unsigned long long thr = block_kth_largest(mine, [&](int j) { return ckeys[tid + j * SAMP_FEW_THREADS]; }, k, tot);
+        __syncthreads();
+        if (tid == 0) n_room = 0;
+        __syncthreads();
+        for (int j = tid; j < n_cand; j += SAMP_FEW_THREADS)
+            if (ckeys[j] != 0ull && ckeys[j] >= thr) room[atomicAdd(&n_room, 1)] = ckeys[j];
+        __syncthreads();
+    }
+    const int passed = n_room, n = min(k, passed);
+    if (tid < passed) {
+        const unsigned long long mine = room[tid];
+        int above = 0;
+        for (int j = 0; j < passed; ++j) above += room[j] > mine;
+        if (above < k) best[above] = mine;
+    }
+    __syncthreads();
+    // ---- min-p, the exponentials, and both orders: by value (ties, and zeros of either sign, to the lower id) and by id
+    if (tid < n) {
+        const unsigned long long key = best[tid];
+        const float x = key_value((uint32_t)(key >> 32)), xmax = key_value((uint32_t)(best[0] >> 32));
+        const uint32_t ix = order_key(x + 0.0f), low = (uint32_t)key;
+        int rv = 0, ri = 0;
+        for (int j = 0; j < n; ++j) {
+            const uint32_t jl = (uint32_t)best[j], jx = order_key(key_value((uint32_t)(best[j] >> 32)) + 0.0f);
+            rv += jx > ix || (jx == ix && jl > low);
+            ri += jl > low;
+        }
+        const double e = exp((double)(x - xmax));
+        const bool ok = !(min_p > 0.f && e < (double)min_p);     // p < min_p * p_max with p_max = e(0) / Z
+        v_e[rv] = i_e[ri] = ok ? e : 0.0;
+        v_keep[rv] = i_keep[ri] = ok ? 1 : 0;
+        v_ri[rv] = ri;
+        i_id[ri] = (int)(0xffffffffu - low);
+    }
+    __syncthreads();
+    if (tid >= 32) return;
+    const int second = lane + 32;
+    double Z;
+    {
+        double a = lane < n ? i_e[lane] : 0.0, b = second < n ? i_e[second] : 0.0;
+        Z = warp_scan2_f64(a, b, lane);
+    }
+    // ---- top-p: in descending order keep until the running sum reaches p - 1e-6, the crossing element included
+    if (top_p > 0.f && top_p < 1.f) {
+        const double thr_p = (double)top_p - 1e-6;
+        const bool ka = lane < n && v_keep[lane], kb = second < n && v_keep[second];
+        const double pa = ka ? v_e[lane] / Z : 0.0, pb = kb ? v_e[second] / Z : 0.0;
+        double a = pa, b = pb;
+        warp_scan2_f64(a, b, lane);
+        if (ka && a - pa >= thr_p) i_keep[v_ri[lane]] = 0;
+        if (kb && b - pb >= thr_p) i_keep[v_ri[second]] = 0;
+        __syncwarp();
+    }
+    // ---- the draw in id order
+    const bool ka = lane < n && i_keep[lane], kb = second < n && i_keep[second];
+    double a = ka ? i_e[lane] / Z : 0.0, b = kb ? i_e[second] / Z : 0.0;
+    const double total = warp_scan2_f64(a, b, lane), target = uniforms.of(row) * total;
+    const uint32_t hit_a = __ballot_sync(0xffffffffu, ka && target - a <= 0.0), hit_b = __ballot_sync(0xffffffffu, kb && target - b <= 0.0);
+    const uint32_t in_a = __ballot_sync(0xffffffffu, ka), in_b = __ballot_sync(0xffffffffu, kb);
+    if (lane == 0) {
+        int pick = (int)(0xffffffffu - (uint32_t)best[0]);   // (sums that are no numbers, or zero: the largest)
+        if (total > 0.0) {
+            const int r = hit_a != 0u ? __ffs(hit_a) - 1 : hit_b != 0u ? 31 + __ffs(hit_b) : in_b != 0u ? 63 - __clz(in_b) : 31 - __clz(in_a);
+            pick = i_id[r];
+        }
+        out[row] = pick;
+    }
+}
+
 // Scratch that gg_sample_topk needs for R rows of V logits with this top-k, in 64-bit words.
 GG_API gg_sample_topk_scratch_words(int R, int V, int top_k, long long* words) {
     if (R <= 0 || V <= 0 || top_k < 1 || words == nullptr) return GG_ERR_ARG;
@@ -726,13 +981,9 @@ GG_API gg_sample_topk_scratch_words(int R, int V, int top_k, long long* words) {
     return 0;
 }
 
-// out[r] = the reference's sampling chain on row r with a top-k (1 <= min(top_k, V) <= 1024).  temp <= 0 or
-// == 1: no scaling; top_p outside (0, 1) and min_p <= 0: off.  uniforms[r] in [0, 1).  scratch: what
-// gg_sample_topk_scratch_words says.
-GG_API gg_sample_topk(const float* logits, long long ld, float temp, int top_k, float top_p, float min_p,
-                      const double* uniforms, int* out, int R, int V, void* scratch, long long scratch_words,
-                      cudaStream_t stream) {
-    if (R <= 0) return 0;
+template <typename Draws>
+static int launch_topk_chain(const float* logits, long long ld, float temp, int top_k, float top_p, float min_p, const Draws& uniforms,
+                             int* out, int R, int V, void* scratch, long long scratch_words, cudaStream_t stream) {
     if (V <= 0 || ld < V || top_k < 1 || R > 65535) return GG_ERR_ARG;
     const int k = top_k < V ? top_k : V;
     const int slices = (V + SAMP_SLICE - 1) / SAMP_SLICE;
@@ -740,18 +991,57 @@ GG_API gg_sample_topk(const float* logits, long long ld, float temp, int top_k, 
     if (k > SAMP_TOPK_MAX || scratch == nullptr || scratch_words < per_row * R) return GG_ERR_ARG;
     const size_t smem = (size_t)per_row * sizeof(unsigned long long);
     if (smem > 160 * 1024) return GG_ERR_ARG;          // 1,024 best of 20 slices still fit
-    static size_t configured = 0;
-    if (smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(sample_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = smem;
-    }
-    int rc = gg_launch(k <= SAMP_SIEVE_K ? topk_slice_kernel<true> : topk_slice_kernel<false>, dim3(slices, R), dim3(SAMP_SLICE_THREADS), 0, stream, 1, logits, ld, V, temp, k,
-                       (unsigned long long*)scratch);
+    unsigned long long* cand = (unsigned long long*)scratch;
+    int rc = launch_topk_slices(logits, ld, V, temp, k, cand, R, stream);
     if (rc != 0) return rc;
-    return gg_launch(sample_topk_kernel, dim3(R), dim3(SAMP_THREADS), smem, stream, 1,
-                     (const unsigned long long*)scratch, (int)per_row, k, top_p, min_p, uniforms, out,
-                     (const double*)nullptr, 0, (int*)nullptr, V);
+    if (k <= SAMP_FEW_K && smem <= 32 * 1024)          // (64 best of 64 slices: rows of 524,288)
+        return gg_launch(sample_few_kernel<Draws>, dim3(R), dim3(SAMP_FEW_THREADS), smem, stream, 1, (const unsigned long long*)cand,
+                         (int)per_row, k, top_p, min_p, uniforms, out);
+    static int known[GG_MAX_DEVICES] = {};
+    int resident = 0;
+    if ((rc = gg_resident(sample_topk_kernel<Draws>, SAMP_THREADS, 160 * 1024, known, resident)) != 0) return rc;
+    return gg_launch(sample_topk_kernel<Draws>, dim3(R), dim3(SAMP_THREADS), smem, stream, 1, (const unsigned long long*)cand,
+                     (int)per_row, k, top_p, min_p, uniforms, out, (const double*)nullptr, 0, (int*)nullptr, V);
+}
+
+// out[r] = the reference's sampling chain on row r with a top-k (1 <= min(top_k, V) <= 1024).  temp <= 0 or
+// == 1: no scaling; top_p outside (0, 1) and min_p <= 0: off.  uniforms[r] in [0, 1).  scratch: what
+// gg_sample_topk_scratch_words says.
+GG_API gg_sample_topk(const float* logits, long long ld, float temp, int top_k, float top_p, float min_p,
+                      const double* uniforms, int* out, int R, int V, void* scratch, long long scratch_words,
+                      cudaStream_t stream) {
+    if (R <= 0) return 0;
+    return launch_topk_chain(logits, ld, temp, top_k, top_p, min_p, DrawsAt{uniforms}, out, R, V, scratch, scratch_words, stream);
+}
+
+static inline uint64_t samp_mix64(uint64_t z) {
+    z += 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+
+// The same for a caller that waits for the ids: row r draws with the uniform number of (seed, streams[r], steps[r])
+// (sampler.py: uniform01; the three arrays are the host's), `ids` is page-locked host memory, and the ids are in it when this returns.
+// The numbers travel as the kernels' arguments and the ids leave through the kernel's own stores, so no copy stands before or
+// behind the two kernels.  scratch: what gg_sample_topk_scratch_words says for R or 256 rows, whichever is less.
+GG_API gg_sample_topk_ids(const float* logits, long long ld, float temp, int top_k, float top_p, float min_p, uint64_t seed,
+                          const uint64_t* streams, const uint64_t* steps, int* ids, int R, int V, void* scratch,
+                          long long scratch_words, cudaStream_t stream) {
+    if (R <= 0) return 0;
+    if (streams == nullptr || steps == nullptr || ids == nullptr) return GG_ERR_ARG;
+    const uint64_t from = samp_mix64(seed);
+    DrawsIn draws;
+    for (int r0 = 0; r0 < R; r0 += SAMP_DRAWS) {
+        const int n = R - r0 < SAMP_DRAWS ? R - r0 : SAMP_DRAWS;
+        for (int r = 0; r < n; ++r)
+            draws.u[r] = (double)(samp_mix64(samp_mix64(from ^ streams[r0 + r]) ^ steps[r0 + r]) >> 11) / 9007199254740992.0;
+        for (int r = n; r < SAMP_DRAWS; ++r) draws.u[r] = 0.0;
+        const int rc = launch_topk_chain(logits + (size_t)r0 * ld, ld, temp, top_k, top_p, min_p, draws, ids + r0, n, V, scratch,
+                                         scratch_words, stream);
+        if (rc != 0) return rc;
+    }
+    return (int)cudaStreamSynchronize(stream);
 }
 
 // Top-p and / or min-p without a top-k (temp > 0): the 1,024 largest logits of each row are the candidates, the
@@ -770,25 +1060,22 @@ GG_API gg_sample_nucleus(const float* logits, long long ld, float temp, float to
     if (scratch_bytes < need) return GG_ERR_ARG;
     const size_t smem = (size_t)per_row * sizeof(unsigned long long);
     if (smem > 160 * 1024) return GG_ERR_ARG;
-    static size_t configured = 0;
-    if (smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(sample_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = smem;
-    }
+    static int known[GG_MAX_DEVICES] = {};
+    int resident = 0, rc = gg_resident(sample_topk_kernel<DrawsAt>, SAMP_THREADS, 160 * 1024, known, resident);
+    if (rc != 0) return rc;
     int* best = out;                                   // the row maxima's ids, overwritten by the samples at the end
     double* zs = reinterpret_cast<double*>(reinterpret_cast<int*>(scratch) + (size_t)R * 128);
     unsigned long long* cand = reinterpret_cast<unsigned long long*>(zs + (size_t)R * slices);
-    int rc = gg_argmax(logits, ld, best, R, V, scratch, (long long)R * 128, stream);
+    rc = gg_argmax(logits, ld, best, R, V, scratch, (long long)R * 128, stream);
     if (rc != 0) return rc;
     // every row at this temperature: the slice sums take one temperature per row
     rc = gg_launch(sample_slice_sum_uniform_kernel, dim3(slices, R), dim3(SAMP_THREADS), 0, stream, 1, logits, ld, temp,
                    (const int*)best, zs, V);
     if (rc != 0) return rc;
-    rc = gg_launch(k <= SAMP_SIEVE_K ? topk_slice_kernel<true> : topk_slice_kernel<false>, dim3(slices, R), dim3(SAMP_SLICE_THREADS), 0, stream, 1, logits, ld, V, temp, k, cand);
+    rc = launch_topk_slices(logits, ld, V, temp, k, cand, R, stream);
     if (rc != 0) return rc;
-    return gg_launch(sample_topk_kernel, dim3(R), dim3(SAMP_THREADS), smem, stream, 1, (const unsigned long long*)cand,
-                     (int)per_row, k, top_p, min_p, uniforms, out, (const double*)zs, slices, flags, V);
+    return gg_launch(sample_topk_kernel<DrawsAt>, dim3(R), dim3(SAMP_THREADS), smem, stream, 1, (const unsigned long long*)cand,
+                     (int)per_row, k, top_p, min_p, DrawsAt{uniforms}, out, (const double*)zs, slices, flags, V);
 }
 
 

@@ -180,6 +180,7 @@ class Sampler:
         self.repeat_penalty = float(repeat_penalty)
         self.repeat_last_n = int(repeat_last_n) if repeat_last_n else 64   # 0 means 64 (session.go:87-91)
         self._out: Optional[torch.Tensor] = None
+        self._ids: Optional[torch.Tensor] = None       # page-locked, where a waited-for sample leaves its ids
         self._outs = None
         self._turn = 0
         self._rings = None        # device rings of the sequences' last ids (repeat penalty on the device)
@@ -261,6 +262,12 @@ class Sampler:
         """`streams[r]`: request index of row r; `steps[r]`: tokens it has generated so far;
         `histories[r]`: prompt + generated ids (only read when a repeat penalty is set)."""
         rows = len(streams)
+        if rows and logits.is_cuda and self.on_device and self.device_chain and not self.cfg.greedy and not self.penalised:
+            from ..csrc import kernels as K
+            if self._ids is None or self._ids.numel() < rows:
+                self._ids = torch.empty(max(rows, 64), dtype=torch.int32, pin_memory=True)
+            return K.sample_topk_ids(logits, self.cfg.temp, self.cfg.top_k, self.cfg.top_p, self.cfg.min_p, self.cfg.seed, streams, steps,
+                                     self._ids)
         us = _uniforms(self.cfg.seed, streams, steps)
         if logits.is_cuda and self.on_device and not self.penalised:
             from ..csrc import kernels as K
@@ -271,11 +278,8 @@ class Sampler:
                 K.argmax(logits, out, rows)
             else:
                 uni = torch.tensor(us, dtype=torch.float64).to(logits.device, non_blocking=True)
-                if self.device_chain:
-                    K.sample_topk(logits, self.cfg.temp, self.cfg.top_k, self.cfg.top_p, self.cfg.min_p, uni, out, rows)
-                else:
-                    temps = torch.full((rows,), float(self.cfg.temp), dtype=torch.float32).to(logits.device, non_blocking=True)
-                    K.sample(logits, temps, uni, out, rows)
+                temps = torch.full((rows,), float(self.cfg.temp), dtype=torch.float32).to(logits.device, non_blocking=True)
+                K.sample(logits, temps, uni, out, rows)
             return out.cpu().tolist()
         if (logits.is_cuda and not self.penalised and self.cfg.temp > 0 and self.cfg.top_k <= 0
                 and logits.dtype == torch.float32 and logits.shape[1] >= 2048):

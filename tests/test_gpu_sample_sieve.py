@@ -30,3 +30,26 @@ def test_rows_through_the_sieve(V, top_k):
         got = Sampler(cfg).sample(logits.cuda(), list(range(len(rows))), [step] * len(rows))
         want = [sample_host(r.numpy().astype(np.float32), cfg, uniform01(5, i, step)) for i, r in enumerate(rows)]
         assert got == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V", [64, 8191, 16388])
+@pytest.mark.parametrize("temp,top_k", [(0.75, 20), (1.0, 20), (0.875, 24), (1.75, 25), (2.0 ** 20, 20), (2.0 ** -20, 7), (0.625, 64)])
+def test_sieve_before_the_division(V, temp, top_k):
+    """The sieve runs on undivided logits: values a step apart that the division makes equal (the lower id wins), quotients that
+    vanish, many zeros, infinities (temperatures that
+    32 bits hold, as the host's 64 do; no top-p: the host orders equal probabilities by id); more rows than one launch carries numbers for."""
+    from gogguf_b200.sampling.sampler import Sampler, SamplerConfig, sample_host, uniform01
+    g = torch.Generator().manual_seed(V + top_k)
+    steps_apart = torch.tensor(5.0).view(torch.int32) + torch.randint(0, 12, (V,), generator=g, dtype=torch.int32)
+    normal = torch.randn(V, generator=g)
+    ids = torch.arange(V)
+    rows = [normal, steps_apart.view(torch.float32), -steps_apart.view(torch.float32), normal.abs() * 1e-38,
+            torch.where(ids % 2 == 0, torch.tensor(0.0), normal), torch.where(ids < V - top_k // 2, -normal.abs(), normal.abs()),
+            torch.where(ids % 5 == 0, normal, torch.tensor(-float("inf")))]
+    cfg = SamplerConfig(temp=temp, top_k=top_k, seed=-3)
+    logits = torch.stack(rows * 40)
+    n = len(logits)
+    got = Sampler(cfg).sample(logits.cuda(), [-5 + i for i in range(n)], [3] * n)
+    want = [sample_host(logits[i].numpy(), cfg, uniform01(-3, i - 5, 3)) for i in range(n)]
+    assert n > 256 and got == want
