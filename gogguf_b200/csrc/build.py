@@ -71,6 +71,7 @@ MODULES: Dict[str, str] = {
     "mixed_head_decode": "mixed_head_decode.cu",
     "sampling": "sampling.cu",
     "gemm_tcgen05": "gemm_tcgen05.cu",
+    "gemm_f32_parts": "gemm_f32_parts.cu",
     "attention_fast": "attention_fast.cu",
     "gemm_tcgen05_static": "gemm_tcgen05_static.cu",
     "diagnostics": "diagnostics.cu",
@@ -82,6 +83,7 @@ _INCLUDES: Dict[str, List[str]] = {
     "attention_fast.cu": ["tma_util.cuh"],
     "mixed_head_prompt.cu": ["tma_util.cuh"],
     "gemm_tcgen05.cu": ["tma_util.cuh"],
+    "gemm_f32_parts.cu": ["tma_util.cuh"],
     "moe_grouped.cu": ["tma_util.cuh"],
     "gemm_tcgen05_static.cu": ["gemm_tcgen05.cu", "gemm_tcgen05_static.h", "tma_util.cuh"],
     "diagnostics.cu": ["tma_util.cuh"],

@@ -6,13 +6,14 @@ tensor that is not on a CUDA device, or a missing compiler, raises.
 """
 from __future__ import annotations
 
+import ctypes
 import struct
 from operator import index
 from typing import List, Optional, Sequence
 
 import torch
 
-from .build import KernelError, kernel, need_rows, stream_ptr
+from .build import KernelError, kernel, module, need_rows, stream_ptr
 
 F32, BF16 = 0, 1
 
@@ -418,6 +419,41 @@ def gemm_plain(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: 
     kernel("gemm_plain", "gg_gemm_plain")(_p(x), dtype_code(x.dtype), _p(w), dtype_code(w.dtype), _p(out),
                                            dtype_code(out.dtype), int(accumulate), M, N, K,
                                            x.stride(0), out.stride(0), _p(bias), _stream())
+
+
+F32_PARTS_ROWS = 17           # rows from which the 32-bit path's products are made in parts on the tensor cores (see gemm_f32_parts.cu)
+
+
+def f32_parts_scratch(M: int, N: int, K: int, tile: int = -1, shares: int = 0) -> int:
+    """Bytes of scratch for `gemm_f32_parts` (tile, shares: see there)."""
+    n = ctypes.c_longlong(0)
+    rc = module("gemm_f32_parts").lib.gg_gemm_f32_parts_scratch(int(M), int(N), int(K), int(tile), int(shares), ctypes.byref(n))
+    if rc != 0:
+        raise KernelError(f"gemm_f32_parts: no product of {M} x {N} x {K}")
+    return n.value
+
+
+def gemm_f32_parts(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, scratch: torch.Tensor, accumulate: bool = False,
+                   m: Optional[int] = None, bias: Optional[torch.Tensor] = None, tile: int = -1, shares: int = 0) -> None:
+    """out[M, N] (+)= x[M, K] @ w[N, K]^T (+ bias [N]), all float32, on the tensor cores: each operand as the sum of three bfloat16 numbers
+    (csrc/gemm_f32_parts.cu).  K is a multiple of 4 and w lies on a 16-byte boundary.  scratch: `f32_parts_scratch` bytes (uint8); tile
+    (0 to 5: 32, 64, 96, 128, 160, 192 rows of x) and shares of K other than the plan's are for measurements and tests."""
+    N, K = w.shape
+    M = x.shape[0] if m is None else m
+    if x.shape[-1] != K or out.shape[-1] != N:
+        raise KernelError(f"gemm: x{tuple(x.shape)} w{tuple(w.shape)} out{tuple(out.shape)} disagree")
+    if not (x.dtype == w.dtype == out.dtype == torch.float32):
+        raise KernelError("gemm_f32_parts: operands and output are float32")
+    if x.stride(-1) != 1 or out.stride(-1) != 1 or not w.is_contiguous():
+        raise KernelError("gemm: operands must be row-major")
+    need_rows(out, M, N, "gemm")
+    if bias is not None:
+        _need(bias, torch.float32, "bias")
+        if bias.numel() != N:
+            raise KernelError("gemm: the bias has one number per output column")
+    from .tcgen05_gemm import status_word
+    kernel("gemm_f32_parts", "gg_gemm_f32_parts")(_p(x), _p(w), _p(out), int(accumulate), M, N, K, x.stride(0), out.stride(0), _p(bias),
+                                                  _p(scratch), scratch.numel(), int(tile), int(shares), _p(status_word(x.device)), _stream())
 
 
 # ------------------------------------------------------------------------------- attention

@@ -15,7 +15,8 @@ from ..csrc import kernels as K
 class Runtime:
     """How a model is run: compute dtype, device, and whether the tensor-core kernels are used.
 
-    dtype float32: everything is true 32-bit on the CUDA cores (no reduced-precision matrix mode).
+    dtype float32: everything is true 32-bit (no reduced-precision matrix mode): on the CUDA cores, and products of
+    many rows on the tensor cores with every operand as an exact sum of three bfloat16 numbers.
     dtype bfloat16: activations and the cache are bfloat16; the residual stream, norms, softmax,
     rotary angles and logits stay float32.  `fast=False` keeps bfloat16 storage but runs the plain
     kernels (the twins the fast kernels are checked against).
@@ -143,7 +144,8 @@ class Linear:
     [N] is kept in float32 and added to the float32 sums inside the product.
 
     The bfloat16 path uses the tcgen05 tensor-core kernel when the sizes allow it and the plain CUDA
-    core kernel otherwise (and always in the 32-bit path and for a matrix stored in 32-bit).
+    core kernel otherwise (and for a matrix stored in 32-bit).  The 32-bit path uses the plain kernel for few rows and
+    the product in parts for many (`K.gemm_f32_parts`).
 
     `fold_input_norm` turns the projection into one that reads `RowStats` instead of normalised rows;
     `emit=stats` asks an accumulating product to write the statistics of the rows it updates, or (`NormedRows`) those
@@ -161,6 +163,9 @@ class Linear:
         if rt.fast and rt.dtype == torch.bfloat16 and self.weight.dtype == torch.bfloat16:
             from ..csrc import tcgen05_gemm
             self._fast = tcgen05_gemm.make_linear(self.weight, swiglu=swiglu, glu_act=glu_act)
+        # the 32-bit path's products of many rows: on the tensor cores in parts (rows of W on 16-byte boundaries, which TMA asks for)
+        self._parts = rt.fast and rt.dtype == torch.float32 and self.in_features % 4 == 0 and self.weight.data_ptr() % 16 == 0
+        self._parts_room: Dict[int, int] = {}        # rows -> bytes of scratch
         self.bias = rt.vector(bias) if bias is not None else None
         if self.bias is not None and (swiglu or self.bias.numel() != self.out_features):
             raise ValueError("Linear: a bias has one number per output and does not go with the fused SwiGLU form")
@@ -228,5 +233,12 @@ class Linear:
             if self.bias is not None:
                 kw.update(bias=self.bias)
             self._fast(x, out, accumulate, m, ws, **kw)
+            return
+        rows = x.shape[0] if m is None else m
+        if self._parts and ws is not None and rows >= K.F32_PARTS_ROWS and x.dtype == out.dtype == torch.float32:
+            room = self._parts_room.get(rows)
+            if room is None:
+                room = self._parts_room[rows] = K.f32_parts_scratch(rows, self.out_features, self.in_features)
+            K.gemm_f32_parts(x, self.weight, out, ws.get("product_parts", (room,), torch.uint8), accumulate, m, bias=self.bias)
         else:
             K.gemm_plain(x, self.weight, out, accumulate, m, bias=self.bias)

@@ -1,0 +1,86 @@
+"""The 32-bit product on the tensor cores (csrc/gemm_f32_parts.cu): every tile and edge of it, shares of K, rows off 16-byte
+boundaries, infinities and NaN, and an error against 64 bits no larger than that of the multiply-adds of the plain product."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+TILES = (32, 64, 96, 128, 160, 192)
+
+
+def K():
+    from gogguf_b200.csrc import kernels
+    return kernels
+
+
+def parts(x, w, out, tile=-1, shares=0, **kw):
+    M = kw.get("m") or x.shape[0]
+    scratch = torch.full((K().f32_parts_scratch(M, w.shape[0], w.shape[1], tile, shares),), 255, dtype=torch.uint8, device="cuda")
+    K().gemm_f32_parts(x, w, out, scratch, tile=tile, shares=shares, **kw)
+    return out
+
+
+def off(out, want):
+    return float((out.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("tile", range(6))
+@pytest.mark.parametrize("N,K_,shares", [(1, 4, 1), (127, 60, 1), (128, 64, 1), (130, 196, 2), (300, 1800, 3), (2048, 520, 1)])
+def test_tiles_and_shares(tile, N, K_, shares):
+    g = torch.Generator(device="cuda").manual_seed(N + K_)
+    wide = torch.randn(400, K_ + 8, device="cuda", generator=g)
+    w = torch.randn(N, K_, device="cuda", generator=g)
+    bias = torch.randn(N, device="cuda", generator=g)
+    for o, M in ((0, 1), (1, TILES[tile] - 1), (0, TILES[tile]), (1, TILES[tile] + 1), (0, 390)):
+        x = wide[:, o:o + K_]
+        room = torch.full((M + 1, N + 3), -7.0, device="cuda")
+        parts(x, w, room[:M, :N], tile, shares, m=M)
+        out = room[:M, :N]
+        want = x[:M].double() @ w.double().T
+        # (the parts left out are 2^-23 of a product, a sum of 32 columns is cut off twice at 2^-23, the sums of those are rounded)
+        bound = (3 + (K_ / 32) ** 0.5 / 2) * 2.0 ** -23
+        assert (out.double() - want).norm() <= bound * (x[:M].double().abs() @ w.double().abs().T).norm()
+        assert (room[:, N:] == -7.0).all() and (room[M:] == -7.0).all()
+        again = parts(x, w, torch.empty(M, N, device="cuda"), tile, shares, m=M)
+        assert torch.equal(again, out)
+        res = torch.randn(M, N, device="cuda", generator=g)
+        acc = parts(x, w, res.clone(), tile, shares, m=M, accumulate=True, bias=bias)
+        assert torch.equal(acc, res + (out + bias))
+
+
+@pytest.mark.parametrize("M,N,K_", [(17, 2048, 2048), (64, 4096, 1024), (150, 1800, 1800), (450, 2048, 5376), (600, 1024, 3072), (333, 700, 12288)])
+def test_error_is_no_larger_than_the_multiply_adds(M, N, K_):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    for spread in (0.0, 3.0):                      # rows and columns of like size, and over some powers of ten
+        x = torch.randn(M, K_, device="cuda", generator=g) * torch.exp(spread * torch.randn(K_, device="cuda", generator=g))
+        w = torch.randn(N, K_, device="cuda", generator=g) * 0.02
+        want = x.double() @ w.double().T
+        plain = torch.empty(M, N, device="cuda")
+        K().gemm_plain(x, w, plain)
+        assert off(parts(x, w, torch.empty(M, N, device="cuda")), want) <= off(plain, want)
+
+
+@pytest.mark.parametrize("shares", [1, 3])
+def test_infinities_and_nan(shares):
+    g = torch.Generator(device="cuda").manual_seed(2)
+    M, N, K_ = 70, 200, 260
+    x, w = torch.randn(M, K_, device="cuda", generator=g), torch.randn(N, K_, device="cuda", generator=g)
+    inf = float("inf")
+    x[3, 5], x[4, 7], x[5, 0], x[6, :] = inf, -inf, float("nan"), 0.0
+    x[7, 9] = torch.tensor(0x7f800001, dtype=torch.int32).view(torch.float32).item()       # a NaN whose upper half is an infinity
+    x[8, 11], x[9, 12] = 3.4e38, 2e38
+    w[10, 12], w[11, 5], w[12, 130], w[13, 5] = 3.0, 0.0, inf, inf
+    out, plain = parts(x, w, torch.empty(M, N, device="cuda"), shares=shares), torch.empty(M, N, device="cuda")
+    K().gemm_plain(x, w, plain)
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isinf(), plain.isinf())
+    assert torch.equal(out[out.isinf()], plain[plain.isinf()])
+    fin = plain.isfinite()
+    assert torch.allclose(out[fin], plain[fin], rtol=1e-4, atol=1e-4)
+
+
+def test_refusals():
+    x, w, out = torch.zeros(4, 8, device="cuda"), torch.zeros(16, 8, device="cuda"), torch.zeros(4, 16, device="cuda")
+    from gogguf_b200.csrc.build import KernelError
+    s = torch.empty(1 << 16, dtype=torch.uint8, device="cuda")
+    for args in ((x[:, :6], torch.zeros(16, 6, device="cuda"), out, s), (x, w, out, s[:64]), (x.bfloat16(), w, out, s), (x, w, out[:3], s)):
+        with pytest.raises(KernelError):
+            K().gemm_f32_parts(*args)
