@@ -461,11 +461,17 @@ def attention_plain(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                     positions: torch.Tensor, seq_of_token: torch.Tensor, page_table: torch.Tensor,
                     page_size: int, n_tokens: int, nq: int, nkv: int, d: int, scale: float, window: int,
                     dv: Optional[int] = None, sink: Optional[torch.Tensor] = None, out_scale: float = 1.0,
-                    chunk: int = 0, gate: Optional[torch.Tensor] = None) -> None:
+                    chunk: int = 0, gate: Optional[torch.Tensor] = None, cu_seqlens: Optional[torch.Tensor] = None,
+                    n_seqs: int = 0) -> None:
     """Attention over the paged cache on the CUDA cores; `dv` is the values' head size (default d), `sink` one
     float32 per query head that joins the softmax's denominator, `out_scale` a factor on the result; chunk > 0: a
     position sees its own chunk of that many positions only; gate (rows of nq * dv logits): the result is multiplied by
-    their sigmoid."""
+    their sigmoid.  cu_seqlens ([n_seqs + 1], prefix sums of the sequences' tokens, each at consecutive positions): steps of many
+    tokens a sequence may then share the keys' reads between them."""
+    if cu_seqlens is not None:
+        _need(cu_seqlens, torch.int32, "cu_seqlens")
+        if n_seqs < 1 or cu_seqlens.numel() < n_seqs + 1:
+            raise KernelError("attention: cu_seqlens holds n_seqs + 1 numbers")
     if not (q.dtype == k_pool.dtype == v_pool.dtype == out.dtype):
         raise KernelError("attention: q, cache and out must share one dtype")
     dv = d if dv is None else int(dv)
@@ -480,7 +486,7 @@ def attention_plain(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
         _p(q), _p(k_pool), _p(v_pool), _p(out), dtype_code(q.dtype), _p(positions), _p(seq_of_token),
         _p(page_table), page_table.shape[-1], page_size, k_pool.shape[0], n_tokens, nq, nkv, d, dv, float(scale),
         int(window), int(chunk), _p(sink), float(out_scale), _p(gate), gate.stride(0) if gate is not None else 0,
-        _p(status_word(q.device)), _stream())
+        _p(cu_seqlens), int(n_seqs), _p(status_word(q.device)), _stream())
 
 
 def diff_qk_prep(qkv: torch.Tensor, q_out: torch.Tensor, q_weight: torch.Tensor, k_weight: Optional[torch.Tensor],

@@ -230,5 +230,5 @@ class AttentionMixer:
         else:
             K.attention_plain(q, cache.k, cache.v, o, ctx.positions, ctx.seq_of_token, table,
                               cache.page_size, T, nq, nkv, d, self.scale, self.window, dv=dv, sink=self.sink,
-                              out_scale=self.out_scale, chunk=self.chunk, gate=gate)
+                              out_scale=self.out_scale, chunk=self.chunk, gate=gate, cu_seqlens=ctx.cu_seqlens, n_seqs=ctx.n_seqs)
         self.o(o, residual, accumulate=not ctx.shared.get("output_empty", False), ws=ctx.ws, emit=ctx.shared.get("row_stats"))
