@@ -312,12 +312,13 @@ __device__ __forceinline__ void store_row_chunk16(const uint32_t* r, int gi, int
 // OUT_SWIGLU: the weight rows were interleaved in blocks of 64 gate rows and 64 up rows, so columns
 // [0,64) and [128,192) of the tile are gates and the 64 columns after each are their ups; the output
 // row has N / 2 columns.
+// Columns c_begin .. c_end of the tile, multiples of 128.
 __device__ __forceinline__ void epilogue_row_256(uint32_t taddr, int gi, int tn, int M, int N, void* __restrict__ out,
-                                                 int out_mode, long long ldo, const NormIO& nio, float sc) {
+                                                 int out_mode, long long ldo, const NormIO& nio, float sc, int c_begin, int c_end) {
     constexpr int BN = 256;
     if (out_mode == OUT_SWIGLU) {
 #pragma unroll 1
-        for (int cb = 0; cb < 2; ++cb) {
+        for (int cb = c_begin / 128; cb < c_end / 128; ++cb) {
 #pragma unroll 1
             for (int c0 = 0; c0 < 64; c0 += 16) {
                 const int gcol = tn * BN + cb * 128 + c0;          // gate column in the interleaved product
@@ -355,26 +356,26 @@ __device__ __forceinline__ void epilogue_row_256(uint32_t taddr, int gi, int tn,
         (ldo & 3) == 0 && (N & 7) == 0) {
         // Adding into the residual reads what is there: one thread's 16 columns at a time, every group would
         // wait a whole trip to L2 for its 64 bytes (about 20 us per tile, in the open after a product's last
-        // tile).  So the old values of 64 columns are asked for at once, before the accumulator is read.
+        // tile).  So the old values of 32 columns are asked for at once, before the accumulator is read.
         const bool stats = nio.out_xhat != nullptr;
         const bool scaled = nio.in_ssq != nullptr;
         const bool live = gi < M;
         float* orow = (float*)out + (size_t)(live ? gi : 0) * ldo + tn * BN;
         bf16* xrow = stats ? nio.out_xhat + (size_t)(live ? gi : 0) * N + tn * BN : nullptr;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 64) {
-            float4 old[16];
+        for (int c0 = c_begin; c0 < c_end; c0 += 32) {
+            float4 old[8];
             if (live) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) old[j] = reinterpret_cast<const float4*>(orow + c0)[j];
+                for (int j = 0; j < 8; ++j) old[j] = reinterpret_cast<const float4*>(orow + c0)[j];
             }
-            uint32_t r[64];
+            uint32_t r[32];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) tmem_ld16(taddr + (uint32_t)(c0 + 16 * q), r + 16 * q);
-            if (nio.bias != nullptr && live) {           // the same 64 numbers for every row: from L1
+            for (int q = 0; q < 2; ++q) tmem_ld16(taddr + (uint32_t)(c0 + 16 * q), r + 16 * q);
+            if (nio.bias != nullptr && live) {           // the same 32 numbers for every row: from L1
                 const float4* bp = reinterpret_cast<const float4*>(nio.bias + tn * BN + c0);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
+                for (int j = 0; j < 8; ++j) {
                     const float4 b = __ldg(bp + j);
                     old[j].x += b.x; old[j].y += b.y; old[j].z += b.z; old[j].w += b.w;
                 }
@@ -382,7 +383,7 @@ __device__ __forceinline__ void epilogue_row_256(uint32_t taddr, int gi, int tn,
             tmem_ld_wait();
             if (!live) continue;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < 2; ++q) {
                 uint32_t pk[8];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -406,7 +407,7 @@ __device__ __forceinline__ void epilogue_row_256(uint32_t taddr, int gi, int tn,
                     reinterpret_cast<uint4*>(xrow + c0 + 16 * q)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
                 }
             }
-            if (stats && (c0 & 64)) {            // a part of 128 columns is complete
+            if (stats && (c0 & 96) == 96) {          // a part of 128 columns is complete
                 if (nio.out_ssq != nullptr) nio.out_ssq[(size_t)gi * ((N + 127) / 128) + ((tn * BN + c0) >> 7)] = ss;
                 ss = 0.f;
             }
@@ -414,7 +415,7 @@ __device__ __forceinline__ void epilogue_row_256(uint32_t taddr, int gi, int tn,
         return;
     }
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 16) {
+    for (int c0 = c_begin; c0 < c_end; c0 += 16) {
         if (tn * BN + c0 >= N) break;
         uint32_t r[16];
         tmem_ld16(taddr + (uint32_t)c0, r);
@@ -434,8 +435,8 @@ __device__ __forceinline__ void epilogue_row_256(uint32_t taddr, int gi, int tn,
 // RMSNorm is a sum over the thread's own columns and the rotation's pairs (i, i + 64) need no exchange.  q
 // goes to its buffer, k (normed, rotated) and v (raw) into the paged cache at the token's position, as in the
 // decode form (QkvIO).  Every thread of the warp reads tensor memory; rows beyond M and tokens of padding
-// write nothing.
-__device__ __forceinline__ void epilogue_row_qkv(uint32_t taddr, int gi, int tn, int M, const QkvIO& qio, float sc) {
+// write nothing.  `hh`: which of the two heads.
+__device__ __forceinline__ void epilogue_row_qkv(uint32_t taddr, int gi, int tn, int hh, int M, const QkvIO& qio, float sc) {
     const bool live = gi < M;
     const int nheads = qio.nq + 2 * qio.nkv;
     int b = -1, pos = 0, page = 0;
@@ -450,91 +451,88 @@ __device__ __forceinline__ void epilogue_row_qkv(uint32_t taddr, int gi, int tn,
     }
     const float* cs = qio.cosv + (size_t)(live ? gi : 0) * 64;
     const float* sn = qio.sinv + (size_t)(live ? gi : 0) * 64;
-#pragma unroll 1
-    for (int hh = 0; hh < 2; ++hh) {
-        const int h = tn * 2 + hh;
-        if (h >= nheads) break;
-        const bool is_q = h < qio.nq, is_k = !is_q && h < qio.nq + qio.nkv;
-        const uint32_t tcol = taddr + (uint32_t)(hh * 128);
-        bf16* dst = nullptr;
-        if (live) {
-            if (is_q) {
-                dst = qio.q_out + ((size_t)gi * qio.nq + h) * 128;
-            } else if (qio.k_pool != nullptr && b >= 0) {
-                const int kvh = is_k ? h - qio.nq : h - qio.nq - qio.nkv;
-                dst = (is_k ? qio.k_pool : qio.v_pool) +
-                      (((size_t)page * qio.nkv + kvh) * qio.page_size + (pos % qio.page_size)) * 128;
-            }
+    const int h = tn * 2 + hh;
+    if (h >= nheads) return;
+    const bool is_q = h < qio.nq, is_k = !is_q && h < qio.nq + qio.nkv;
+    const uint32_t tcol = taddr + (uint32_t)(hh * 128);
+    bf16* dst = nullptr;
+    if (live) {
+        if (is_q) {
+            dst = qio.q_out + ((size_t)gi * qio.nq + h) * 128;
+        } else if (qio.k_pool != nullptr && b >= 0) {
+            const int kvh = is_k ? h - qio.nq : h - qio.nq - qio.nkv;
+            dst = (is_k ? qio.k_pool : qio.v_pool) +
+                  (((size_t)page * qio.nkv + kvh) * qio.page_size + (pos % qio.page_size)) * 128;
         }
-        if (!is_q && !is_k) {                      // value head: the sums as they are
+    }
+    if (!is_q && !is_k) {                      // value head: the sums as they are
 #pragma unroll 1
-            for (int c = 0; c < 128; c += 16) {
-                uint32_t r[16];
-                tmem_ld16(tcol + (uint32_t)c, r);
-                tmem_ld_wait();
-                if (dst == nullptr) continue;
-                uint32_t pk[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(r[2 * j]) * sc, __uint_as_float(r[2 * j + 1]) * sc);
-                    pk[j] = *reinterpret_cast<uint32_t*>(&h2);
-                }
-                reinterpret_cast<uint4*>(dst + c)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                reinterpret_cast<uint4*>(dst + c)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-            }
-            continue;
-        }
-        const float* w = is_q ? qio.qw : qio.kw;
-        float scale = sc;
-        if (w != nullptr) {
-            float ss = 0.f;
-#pragma unroll 1
-            for (int c = 0; c < 128; c += 16) {
-                uint32_t r[16];
-                tmem_ld16(tcol + (uint32_t)c, r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 16; ++j) { const float v = __uint_as_float(r[j]) * sc; ss = fmaf(v, v, ss); }
-            }
-            scale = sc * (1.0f / sqrtf(ss * (1.0f / 128.0f) + qio.eps));
-        }
-#pragma unroll 1
-        for (int c = 0; c < 64; c += 16) {
-            uint32_t lo[16], hi[16];
-            tmem_ld16(tcol + (uint32_t)c, lo);
-            tmem_ld16(tcol + (uint32_t)(64 + c), hi);
+        for (int c = 0; c < 128; c += 16) {
+            uint32_t r[16];
+            tmem_ld16(tcol + (uint32_t)c, r);
             tmem_ld_wait();
             if (dst == nullptr) continue;
-            uint32_t pl[8], ph[8];
+            uint32_t pk[8];
 #pragma unroll
-            for (int j4 = 0; j4 < 4; ++j4) {
-                const float4 c4 = *reinterpret_cast<const float4*>(cs + c + 4 * j4);
-                const float4 s4 = *reinterpret_cast<const float4*>(sn + c + 4 * j4);
-                float4 wl = make_float4(1.f, 1.f, 1.f, 1.f), wh = wl;
-                if (w != nullptr) {
-                    wl = *reinterpret_cast<const float4*>(w + c + 4 * j4);
-                    wh = *reinterpret_cast<const float4*>(w + 64 + c + 4 * j4);
-                }
-                const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, sv[4] = {s4.x, s4.y, s4.z, s4.w};
-                const float wlv[4] = {wl.x, wl.y, wl.z, wl.w}, whv[4] = {wh.x, wh.y, wh.z, wh.w};
-                float ol[4], oh[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const float x0 = __uint_as_float(lo[4 * j4 + t]) * scale * wlv[t];
-                    const float x1 = __uint_as_float(hi[4 * j4 + t]) * scale * whv[t];
-                    ol[t] = x0 * cc[t] - x1 * sv[t];
-                    oh[t] = x1 * cc[t] + x0 * sv[t];
-                }
-                __nv_bfloat162 a = __floats2bfloat162_rn(ol[0], ol[1]), bb = __floats2bfloat162_rn(ol[2], ol[3]);
-                pl[2 * j4] = *reinterpret_cast<uint32_t*>(&a); pl[2 * j4 + 1] = *reinterpret_cast<uint32_t*>(&bb);
-                a = __floats2bfloat162_rn(oh[0], oh[1]); bb = __floats2bfloat162_rn(oh[2], oh[3]);
-                ph[2 * j4] = *reinterpret_cast<uint32_t*>(&a); ph[2 * j4 + 1] = *reinterpret_cast<uint32_t*>(&bb);
+            for (int j = 0; j < 8; ++j) {
+                __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(r[2 * j]) * sc, __uint_as_float(r[2 * j + 1]) * sc);
+                pk[j] = *reinterpret_cast<uint32_t*>(&h2);
             }
-            reinterpret_cast<uint4*>(dst + c)[0] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
-            reinterpret_cast<uint4*>(dst + c)[1] = make_uint4(pl[4], pl[5], pl[6], pl[7]);
-            reinterpret_cast<uint4*>(dst + 64 + c)[0] = make_uint4(ph[0], ph[1], ph[2], ph[3]);
-            reinterpret_cast<uint4*>(dst + 64 + c)[1] = make_uint4(ph[4], ph[5], ph[6], ph[7]);
+            reinterpret_cast<uint4*>(dst + c)[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            reinterpret_cast<uint4*>(dst + c)[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
         }
+        return;
+    }
+    const float* w = is_q ? qio.qw : qio.kw;
+    float scale = sc;
+    if (w != nullptr) {
+        float ss = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < 128; c += 16) {
+            uint32_t r[16];
+            tmem_ld16(tcol + (uint32_t)c, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) { const float v = __uint_as_float(r[j]) * sc; ss = fmaf(v, v, ss); }
+        }
+        scale = sc * (1.0f / sqrtf(ss * (1.0f / 128.0f) + qio.eps));
+    }
+#pragma unroll 1
+    for (int c = 0; c < 64; c += 16) {
+        uint32_t lo[16], hi[16];
+        tmem_ld16(tcol + (uint32_t)c, lo);
+        tmem_ld16(tcol + (uint32_t)(64 + c), hi);
+        tmem_ld_wait();
+        if (dst == nullptr) continue;
+        uint32_t pl[8], ph[8];
+#pragma unroll
+        for (int j4 = 0; j4 < 4; ++j4) {
+            const float4 c4 = *reinterpret_cast<const float4*>(cs + c + 4 * j4);
+            const float4 s4 = *reinterpret_cast<const float4*>(sn + c + 4 * j4);
+            float4 wl = make_float4(1.f, 1.f, 1.f, 1.f), wh = wl;
+            if (w != nullptr) {
+                wl = *reinterpret_cast<const float4*>(w + c + 4 * j4);
+                wh = *reinterpret_cast<const float4*>(w + 64 + c + 4 * j4);
+            }
+            const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, sv[4] = {s4.x, s4.y, s4.z, s4.w};
+            const float wlv[4] = {wl.x, wl.y, wl.z, wl.w}, whv[4] = {wh.x, wh.y, wh.z, wh.w};
+            float ol[4], oh[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float x0 = __uint_as_float(lo[4 * j4 + t]) * scale * wlv[t];
+                const float x1 = __uint_as_float(hi[4 * j4 + t]) * scale * whv[t];
+                ol[t] = x0 * cc[t] - x1 * sv[t];
+                oh[t] = x1 * cc[t] + x0 * sv[t];
+            }
+            __nv_bfloat162 a = __floats2bfloat162_rn(ol[0], ol[1]), bb = __floats2bfloat162_rn(ol[2], ol[3]);
+            pl[2 * j4] = *reinterpret_cast<uint32_t*>(&a); pl[2 * j4 + 1] = *reinterpret_cast<uint32_t*>(&bb);
+            a = __floats2bfloat162_rn(oh[0], oh[1]); bb = __floats2bfloat162_rn(oh[2], oh[3]);
+            ph[2 * j4] = *reinterpret_cast<uint32_t*>(&a); ph[2 * j4 + 1] = *reinterpret_cast<uint32_t*>(&bb);
+        }
+        reinterpret_cast<uint4*>(dst + c)[0] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+        reinterpret_cast<uint4*>(dst + c)[1] = make_uint4(pl[4], pl[5], pl[6], pl[7]);
+        reinterpret_cast<uint4*>(dst + 64 + c)[0] = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+        reinterpret_cast<uint4*>(dst + 64 + c)[1] = make_uint4(ph[4], ph[5], ph[6], ph[7]);
     }
 }
 
@@ -548,13 +546,13 @@ __device__ __forceinline__ void epilogue_row_qkv(uint32_t taddr, int gi, int tn,
 constexpr int ROWBUF_BYTES = 32 * 128;
 
 // (not inlined: inside the kernel its registers spilled)
-__device__ __noinline__ void store_partial_rows(uint32_t taddr, int gi0, int tn, int M, int NS, float* out, uint4* buf, int lane) {
+__device__ __noinline__ void store_partial_rows(uint32_t taddr, int gi0, int tn, int c_begin, int M, int NS, float* out, uint4* buf, int lane) {
     constexpr int BN = 256;
     if (gi0 >= M) return;
     const int rr = lane >> 3, ch = lane & 7;                 // round i of 8 below: row 4 i + rr, chunk ch
     const bool chunks = (NS & 3) == 0 && (((uintptr_t)out) & 15) == 0;
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN && tn * BN + c0 < NS; c0 += 32) {
+    for (int c0 = c_begin; c0 < c_begin + 128 && tn * BN + c0 < NS; c0 += 32) {
         const int oc = tn * BN + c0;
         uint32_t r[32];
         tc5::ld32(taddr + (uint32_t)c0, r);
@@ -1233,7 +1231,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_persistent_kernel(
             const float sc = gi < M ? norm_factor(nio, gi) : 1.0f;      // while the tile is still being multiplied
             if (!mbar_wait(&acc_full[buf], aph, abort_flag, status, 3)) break;
             tc_fence_after();
-            epilogue_row_256(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN), gi, tn, M, N, out, out_mode, ldo, nio, sc);
+            epilogue_row_256(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN), gi, tn, M, N, out, out_mode, ldo, nio, sc, 0, BN);
             tc_fence_before();
             mbar_arrive(&acc_empty[buf]);        // 128 arrivals free the accumulator for tile i + 2
         }
@@ -1283,7 +1281,7 @@ int launch_persistent(const CUtensorMap& ta, const CUtensorMap& tb, void* out, i
 // Barriers live at the same shared-memory offsets in both CTAs.  full[s]: in the leader; it expects
 // the bytes of both CTAs' copies (the peer's TMA signals the leader's barrier).  empty[s] and
 // acc_full[b]: in both; the leader's tcgen05.commit arrives on both at once.  acc_empty[b]: in the
-// leader; the 128 epilogue threads of each CTA arrive on it, the peer's through the cluster.
+// leader; the 256 epilogue threads of each CTA arrive on it, the peer's through the cluster.
 constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;
 
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
@@ -1308,8 +1306,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t rank
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
 }
 
+// Eight epilogue warps, two for each quarter of a CTA's rows: 128 of the tile's 256 columns each (one head, one gate-up block, one
+// part of a row's sums of squares).  A product of a few hundred tokens is one or two tiles a pair, and its last epilogue stands
+// in the open.
+constexpr int PAIR_THREADS = 64 + 8 * 32;
 template <int STAGES>
-__global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_pair_kernel(
+__global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_tc_pair_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     void* __restrict__ out, int out_mode, long long ldo, int M, int N, int K, int* __restrict__ status,
     const NormIO nio, int splits, int whole, int kb_per_split, float* __restrict__ partial, const QkvIO qio) {
@@ -1351,7 +1353,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_pair_kernel(
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 256); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 512); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmA) : "memory");
@@ -1438,7 +1440,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_pair_kernel(
             }
         }
     } else {
-        const int q = warp & 3;
+        const int q = warp & 3, half = (warp - 2) >> 2;
         const int row = q * 32 + lane;
         pdl_wait();
         int i = 0;
@@ -1455,14 +1457,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_tc_pair_kernel(
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
             if (parted) {
-                uint4* lines = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + 256 + q * ROWBUF_BYTES);
-                store_partial_rows(taddr, gi - lane, tn - tn_split, M, NS, partial + (size_t)split * M * NS, lines, lane);
+                uint4* lines = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + 256 + (warp - 2) * ROWBUF_BYTES);
+                store_partial_rows(taddr, gi - lane, tn - tn_split, 128 * half, M, NS, partial + (size_t)split * M * NS, lines, lane);
             } else if (out_mode == OUT_QKV)
-                epilogue_row_qkv(taddr, gi, tn, M, qio, sc);
+                epilogue_row_qkv(taddr, gi, tn, half, M, qio, sc);
             else
-                epilogue_row_256(taddr, gi, tn, M, N, out, out_mode, ldo, nio, sc);
+                epilogue_row_256(taddr, gi, tn, M, N, out, out_mode, ldo, nio, sc, 128 * half, 128 * half + 128);
             tc_fence_before();
-            mbar_arrive_cluster(&acc_empty[buf], 0);     // 256 arrivals in the leader free the accumulator pair
+            mbar_arrive_cluster(&acc_empty[buf], 0);     // 512 arrivals in the leader free the accumulator pair
         }
     }
 
@@ -1582,7 +1584,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out
     // the warps' buffers for partial tiles only where there are any: the other epilogues read a thread's row 16 bytes at a
     // time through what shared memory leaves of the L1, and with 16 KB less of it the product that adds 2,048 tokens of
     // 4,096 columns into the residual took 65 us instead of 62.5
-    constexpr int smem_whole = STAGES * (A_BYTES + 128 * BK * 2) + 1024 + 256, smem_split = smem_whole + 4 * ROWBUF_BYTES;
+    constexpr int smem_whole = STAGES * (A_BYTES + 128 * BK * 2) + 1024 + 256, smem_split = smem_whole + 8 * ROWBUF_BYTES;
     static int sms = 0;
     auto kern = gemm_tc_pair_kernel<STAGES>;
     if (sms == 0) {
@@ -1602,7 +1604,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out
     const int total = whole + (tiles - whole) * used;
     int pairs = sms / 2;
     if (pairs > total) pairs = total;
-    int rc = gg_launch2(kern, dim3(2 * pairs), dim3(NUM_THREADS), used > 1 ? smem_split : smem_whole, stream, ta, tb, out, out_mode, ldo, M, N, K, status, nio,
+    int rc = gg_launch2(kern, dim3(2 * pairs), dim3(PAIR_THREADS), used > 1 ? smem_split : smem_whole, stream, ta, tb, out, out_mode, ldo, M, N, K, status, nio,
                         used, whole, per, partial, qio);
     if (rc != 0 || used == 1) return rc;
     const int col0 = (whole / tiles_m) * 256, NS = N - col0;
