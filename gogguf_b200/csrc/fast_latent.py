@@ -31,11 +31,12 @@ def latent_attention_mma(qcat: torch.Tensor, pool: torch.Tensor, out: torch.Tens
                          page_size: int, n_seqs: int, n_tokens: int, heads: int, R: int, r: int, scale: float,
                          window: int, splits: int = 1, part_o: Optional[torch.Tensor] = None,
                          part_ml: Optional[torch.Tensor] = None, max_new: Optional[int] = None,
-                         sink: Optional[torch.Tensor] = None) -> None:
+                         sink: Optional[torch.Tensor] = None, merge: bool = True) -> None:
     """splits > 1 cuts every CTA's range of cached positions into that many shares (steps with few CTAs); part_o
     float32 [n_tokens * heads, splits, R] and part_ml [n_tokens * heads, splits, 2] take the partial results.
     max_new: the most new tokens any sequence brings (default: all could be one sequence's); a step of few rows
-    per sequence keeps less shared memory for its queries."""
+    per sequence keeps less shared memory for its queries.  merge=False leaves the shares in part_o and part_ml for
+    `expand_shares`; `out` then only gets the zero rows of padding."""
     for t in (qcat, pool, out):
         if t.dtype != torch.bfloat16:
             raise KernelError("latent_attention_mma takes bfloat16 queries, cache and output")
@@ -46,8 +47,24 @@ def latent_attention_mma(qcat: torch.Tensor, pool: torch.Tensor, out: torch.Tens
         int(n_seqs), int(n_tokens), heads, R, r, float(scale), int(window), int(splits),
         part_o.data_ptr() if part_o is not None else 0, part_ml.data_ptr() if part_ml is not None else 0,
         int(max_new) if max_new is not None else int(n_tokens), sink.data_ptr() if sink is not None else 0,
-        status_word(qcat.device).data_ptr(),
-        stream_ptr())
+        int(merge), status_word(qcat.device).data_ptr(), stream_ptr())
+
+
+def expand_shares(part_o: torch.Tensor, part_ml: torch.Tensor, seq_of_token: torch.Tensor, uv: torch.Tensor, out: torch.Tensor, m: int,
+                  alpha: float = 1.0, gate: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None) -> None:
+    """out[t, h, :] = alpha * uv[h] @ (the merged shares of token t, head h): the shares that `latent_attention_mma` has left with
+    merge=False, for up to 16 tokens and a latent of up to 256."""
+    H, N, R = uv.shape
+    if uv.dtype != torch.bfloat16 or not uv.is_contiguous() or part_o.dtype != torch.float32 or not part_o.is_contiguous() \
+            or part_o.shape[-1] != R or part_o.numel() < m * H * part_o.shape[1] * R or part_ml.numel() < m * H * part_o.shape[1] * 2:
+        raise KernelError("expand_shares: uv is bfloat16 [H, N, R], part_o float32 [rows, splits, R]")
+    if gate is not None and (gate.dtype != out.dtype or gate.stride(-1) != 1 or gate.shape[-1] != H * N):
+        raise KernelError("expand_shares: the gate has rows of H * N logits in the output's dtype")
+    from .kernels import dtype_code
+    kernel("latent_attention", "gg_latent_expand_shares")(
+        part_o.data_ptr(), part_ml.data_ptr(), part_o.shape[1], seq_of_token.data_ptr(), sink.data_ptr() if sink is not None else 0,
+        uv.data_ptr(), out.data_ptr(), dtype_code(out.dtype), H * N, N, int(m), N, R, H, float(alpha),
+        gate.data_ptr() if gate is not None else 0, gate.stride(0) if gate is not None else 0, stream_ptr())
 
 
 def mma_splits(n_seqs: int, n_tokens: int, heads: int, R: int, r: int, window: int, max_ctx: int) -> int:
@@ -85,6 +102,9 @@ def mma_takes(R: int, r: int) -> bool:
     return bool(module("latent_attention").lib.gg_latent_attention_mma_takes(int(R), int(r)))
 
 
+FEW_TOKENS, FEW_LATENT = 16, 256          # what the kernel of few tokens takes (HF_M, HF_K)
+
+
 class _Fast:
     def __init__(self, heads: int, R: int, r: int, scale: float, window: int, sink: Optional[torch.Tensor] = None):
         self.H, self.R, self.r, self.scale, self.window = heads, R, r, scale, window
@@ -95,7 +115,8 @@ class _Fast:
         D = self.R + self.r
         headwise_gemm_mma(qd, ldx, hx, uk_t, qcat, self.H * D, D, m)
 
-    def attention(self, qcat, pool, out, ctx, table, page_size: int) -> None:
+    def attention(self, qcat, pool, out, ctx, table, page_size: int):
+        """Latent outputs into `out`, or, for a step of few tokens that is cut into shares of the keys, the shares (for `expand`)."""
         T, H, R = ctx.n_tokens, self.H, self.R
         # ctx.max_ctx is the longest sequence of the step (an upper bound under a captured graph)
         splits = mma_splits(ctx.n_seqs, T, H, R, self.r, self.window, max(int(ctx.max_ctx), 1))
@@ -103,14 +124,20 @@ class _Fast:
         if splits > 1:
             part_o = ctx.ws.get("lat_part_o", (T * H, splits, R), torch.float32)
             part_ml = ctx.ws.get("lat_part_ml", (T * H, splits, 2), torch.float32)
+        merge = splits == 1 or T > FEW_TOKENS or R > FEW_LATENT
         latent_attention_mma(qcat, pool, out, ctx.cu_seqlens, ctx.positions, ctx.seq_of_token, table, page_size,
                              ctx.n_seqs, T, H, R, self.r, self.scale, self.window, splits, part_o, part_ml,
-                             max_new=max(int(ctx.max_new), 1), sink=self.sink)
+                             max_new=max(int(ctx.max_new), 1), sink=self.sink, merge=merge)
+        return None if merge else (part_o, part_ml, ctx.seq_of_token)
 
     def expand(self, olat: torch.Tensor, uv: torch.Tensor, av: torch.Tensor, m: int, alpha: float,
-               gate: Optional[torch.Tensor] = None) -> None:
-        """av[t, h, :] = alpha * Wuv_h olat[t, h] (times the gate's sigmoid)."""
+               gate: Optional[torch.Tensor] = None, shares=None) -> None:
+        """av[t, h, :] = alpha * Wuv_h olat[t, h] (times the gate's sigmoid); shares: what `attention` has returned."""
         dv = uv.shape[1]
+        if shares is not None:
+            part_o, part_ml, seq_of_token = shares
+            expand_shares(part_o, part_ml, seq_of_token, uv, av, m, alpha, gate, self.sink)
+            return
         headwise_gemm_mma(olat, self.H * self.R, self.R, uv, av, self.H * dv, dv, m, alpha, gate)
 
 

@@ -405,6 +405,118 @@ __global__ void __launch_bounds__(128) headwise_mma_kernel(const bf16* x, long l
     }
 }
 
+// The same for up to 16 tokens and k up to 256, the per-head products of decode steps, whose time is that of their loads one after
+// another: all of w's tile is asked for before the wait for the kernel before this one, all of x behind it at once, and four warps
+// take 16 of the tile's 64 outputs each.  With MERGE the rows of x are made here from the attention's shares of the keys
+// (part_o [row][splits][k], part_ml [row][splits][2], row = token * H + head; see latent_combine_kernel, which then does not
+// run): weights by a warp a token, the sum over the shares in their order, rounded to bfloat16 as that kernel's output is.
+#define HF_M 16
+#define HF_K 256
+#define HF_LD (HF_K + 8)
+#define HF_SPLITS 32
+struct Shares {
+    const float* part_o;
+    const float* part_ml;
+    int splits;
+    const int* seq_of_token;
+    const float* sink;
+};
+template <typename TO, bool MERGE>
+__global__ void __launch_bounds__(128) headwise_few_kernel(const bf16* x, long long ldx, long long hx, const Shares sh,
+                                                           const bf16* __restrict__ w, TO* out, long long ldo, long long ho, int M, int N,
+                                                           int K, int H, float alpha, const TO* gate, long long ldg) {
+    pdl_launch();
+    __shared__ __align__(16) bf16 xs[HF_M * HF_LD];
+    __shared__ __align__(16) bf16 ws[64 * HF_LD];
+    const int h = blockIdx.y, n0 = blockIdx.x * 64;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bf16* wh = w + (size_t)h * N * K;
+    const int kpad = (K + 15) / 16 * 2;                      // 16-byte pieces of a row, with the zeros that fill 16 columns
+    for (int c = tid; c < 64 * kpad; c += 128) {
+        const int row = c / kpad, k = (c % kpad) * 8;
+        bf16* d = ws + row * HF_LD + k;
+        if (n0 + row < N && k < K) cp_async16(d, wh + (size_t)(n0 + row) * K + k); else zero16(d);
+    }
+    pdl_wait();
+    if (!MERGE) {
+        const bf16* xh = x + (size_t)h * hx;
+        for (int c = tid; c < HF_M * kpad; c += 128) {
+            const int row = c / kpad, k = (c % kpad) * 8;
+            bf16* d = xs + row * HF_LD + k;
+            if (row < M && k < K) cp_async16(d, xh + (size_t)row * ldx + k); else zero16(d);
+        }
+    } else {
+        for (int m = warp; m < HF_M; m += 4) {
+            bf16* d = xs + m * HF_LD;
+            if (m >= M || sh.seq_of_token[m] < 0) {
+                for (int c = lane; c < kpad; c += 32) zero16(d + 8 * c);
+                continue;
+            }
+            const size_t row = (size_t)m * H + h;
+            float ms = -INFINITY, ls = 0.f;
+            if (lane < sh.splits) { const float2 t = *reinterpret_cast<const float2*>(sh.part_ml + (row * sh.splits + lane) * 2); ms = t.x; ls = t.y; }
+            const float sk = sh.sink != nullptr ? sh.sink[h] * 1.4426950408889634f : -INFINITY;
+            const float mx = fmaxf(warp_max(ms), sk);
+            float f = ms == -INFINITY ? 0.f : exp2f(ms - mx);
+            const float L = warp_sum(f * ls) + (sh.sink != nullptr ? exp2f(sk - mx) : 0.f);
+            f *= 1.0f / L;
+            const int c = 8 * lane;
+            const bool in = c < K;
+            const float* po = sh.part_o + row * sh.splits * K + (in ? c : 0);
+            float acc[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+            // (a share without a key has weight zero and sums of zero)
+#pragma unroll 8
+            for (int s = 0; s < sh.splits; ++s) {
+                const float fs = __shfl_sync(0xffffffffu, f, s);
+                const float4 a = *reinterpret_cast<const float4*>(po + (size_t)s * K), b = *reinterpret_cast<const float4*>(po + (size_t)s * K + 4);
+                acc[0] = fmaf(fs, a.x, acc[0]); acc[1] = fmaf(fs, a.y, acc[1]); acc[2] = fmaf(fs, a.z, acc[2]); acc[3] = fmaf(fs, a.w, acc[3]);
+                acc[4] = fmaf(fs, b.x, acc[4]); acc[5] = fmaf(fs, b.y, acc[5]); acc[6] = fmaf(fs, b.z, acc[6]); acc[7] = fmaf(fs, b.w, acc[7]);
+            }
+            if (in) *reinterpret_cast<uint4*>(d + c) = make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]),
+                                                                  pack_bf16(acc[4], acc[5]), pack_bf16(acc[6], acc[7]));
+            else if (c < kpad * 8) zero16(d + c);
+        }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    float acc[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    const int steps = (K + 15) / 16;
+#pragma unroll 4
+    for (int ks = 0; ks < steps; ++ks) {
+        uint32_t a[4], b[4];
+        ldsm_x4(a, xs + (lane & 15) * HF_LD + ks * 16 + (lane >> 4) * 8);
+        ldsm_x4(b, ws + (warp * 16 + (lane & 7) + (lane >> 4) * 8) * HF_LD + ks * 16 + ((lane >> 3) & 1) * 8);
+        mma16816(acc[0], a, b[0], b[1]);
+        mma16816(acc[1], a, b[2], b[3]);
+    }
+    const int g = lane >> 2, q4 = lane & 3;
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+        const int n = n0 + warp * 16 + nt * 8 + 2 * q4;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int m = g + half * 8;
+            if (m >= M) continue;
+            TO* o = out + (size_t)m * ldo + (size_t)h * ho + n;
+            float v0 = acc[nt][2 * half] * alpha, v1 = acc[nt][2 * half + 1] * alpha;
+            if (gate != nullptr) {
+                const size_t at = (size_t)m * ldg + (size_t)h * N + n;
+                if (n < N) v0 *= gate_factor(gate, at);
+                if (n + 1 < N) v1 *= gate_factor(gate, at + 1);
+            }
+            if (n < N) o[0] = from_f<TO>(v0);
+            if (n + 1 < N) o[1] = from_f<TO>(v1);
+        }
+    }
+}
+
 GG_API gg_headwise_gemm_mma(const void* x, long long ldx, long long hx, const void* w, void* out, int out_dtype,
                             long long ldo, long long ho, int M, int N, int K, int H, float alpha, const void* gate,
                                 long long ldg, cudaStream_t stream) {
@@ -412,11 +524,31 @@ GG_API gg_headwise_gemm_mma(const void* x, long long ldx, long long hx, const vo
     if (K <= 0 || (K % 8) || (ldx % 8) || (hx % 8) || (((uintptr_t)x) & 15) || (((uintptr_t)w) & 15) || H > 65535 ||
         (M + 63) / 64 > 65535)
         return GG_ERR_ARG;
+    if (M <= HF_M && K <= HF_K) {
+        GG_DISPATCH_DTYPE(out_dtype, TO,
+            return gg_launch(headwise_few_kernel<TO, false>, dim3((N + 63) / 64, H), dim3(128), 0, stream, 1, (const bf16*)x, ldx, hx,
+                             Shares{}, (const bf16*)w, (TO*)out, ldo, ho, M, N, K, H, alpha, (const TO*)gate, ldg));
+    }
     dim3 grid((N + 63) / 64, (M + 63) / 64, H);
     GG_DISPATCH_DTYPE(out_dtype, TO,
         gg_launch(headwise_mma_kernel<TO>, dim3(grid), dim3(128), 0, stream, 1, (const bf16*)x, ldx, hx,
                   (const bf16*)w, (TO*)out, ldo, ho, M, N, K, alpha, (const TO*)gate, ldg));
     return gg_last_error();
+}
+
+// out[t, h, :] = alpha * w[h] (the merged shares of row t * H + h), for up to 16 tokens and R up to 256 (a multiple of 8): what
+// latent_combine_kernel and gg_headwise_gemm_mma do together.  splits: at most 32.
+GG_API gg_latent_expand_shares(const float* part_o, const float* part_ml, int splits, const int* seq_of_token, const float* sink,
+                               const void* w, void* out, int out_dtype, long long ldo, long long ho, int M, int N, int R, int H,
+                               float alpha, const void* gate, long long ldg, cudaStream_t stream) {
+    if (M <= 0 || N <= 0 || H <= 0) return 0;
+    if (M > HF_M || R <= 0 || R > HF_K || (R % 8) || splits < 1 || splits > HF_SPLITS || H > 65535 || part_o == nullptr || part_ml == nullptr ||
+        ((((uintptr_t)w) | (uintptr_t)part_o) & 15) || (((uintptr_t)part_ml) & 7))
+        return GG_ERR_ARG;
+    const Shares sh = {part_o, part_ml, splits, seq_of_token, sink};
+    GG_DISPATCH_DTYPE(out_dtype, TO,
+        return gg_launch(headwise_few_kernel<TO, true>, dim3((N + 63) / 64, H), dim3(128), 0, stream, 1, (const bf16*)nullptr, 0LL, 0LL, sh,
+                         (const bf16*)w, (TO*)out, ldo, ho, M, N, R, H, alpha, (const TO*)gate, ldg));
 }
 
 // ----------------------------------------------------------------------------- attention on mma.sync
@@ -688,13 +820,25 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const float* part_o
     M = fmaxf(M, sk);
     float L = sink != nullptr ? exp2f(sk - M) : 0.f;
     for (int s = 0; s < splits; ++s) L += ml[2 * s] == -INFINITY ? 0.f : exp2f(ml[2 * s] - M) * ml[2 * s + 1];
+    // (the weights once, not once a column: the loads of the shares' sums are then in flight together)
+    __shared__ float f[128];
     const float inv = 1.0f / L;
-    for (int c = threadIdx.x; c < R; c += blockDim.x) {
-        float acc = 0.f;
-        for (int s = 0; s < splits; ++s) {
-            const float m = ml[2 * s];
-            if (m != -INFINITY) acc = fmaf(exp2f(m - M), part_o[(row * splits + s) * R + c], acc);
+    auto weight = [&](int s) { return ml[2 * s] == -INFINITY ? 0.f : exp2f(ml[2 * s] - M); };
+    if (splits > 128) {
+        for (int c = threadIdx.x; c < R; c += blockDim.x) {
+            float acc = 0.f;
+            for (int s = 0; s < splits; ++s) acc = fmaf(weight(s), part_o[(row * splits + s) * R + c], acc);
+            out[row * R + c] = __float2bfloat16_rn(acc * inv);
         }
+        return;
+    }
+    if ((int)threadIdx.x < splits) f[threadIdx.x] = weight(threadIdx.x);
+    __syncthreads();
+    for (int c = threadIdx.x; c < R; c += blockDim.x) {
+        const float* po = part_o + row * splits * R + c;
+        float acc = 0.f;
+#pragma unroll 8
+        for (int s = 0; s < splits; ++s) acc = fmaf(f[s], po[(size_t)s * R], acc);
         out[row * R + c] = __float2bfloat16_rn(acc * inv);
     }
 }
@@ -730,12 +874,12 @@ GG_API gg_latent_attention_mma_takes(int R, int r) {
 
 // qcat [T, H, R + r], pool [page][page_size][pool_row], out [T, H, R], all bfloat16; cu_seqlens [n_seqs + 1].
 // splits > 1: part_o [T * H, splits, R] and part_ml [T * H, splits, 2] (float32) take the shares' partial results
-// and a second kernel merges them.  max_new: the most new tokens any sequence of the step brings.
+// and a second kernel merges them (merge 0: it does not run, the caller reads the shares).  max_new: the most new tokens any sequence of the step brings.
 GG_API gg_latent_attention_mma(const void* qcat, const void* pool, int pool_row, void* out, const int* cu_seqlens,
                                const int* positions, const int* seq_of_token, const int* page_table, int max_pages,
                                int page_size, int n_pages, int n_seqs, int ntok, int H, int R, int r, float scale,
                                int window, int splits, float* part_o, float* part_ml, int max_new, const float* sink,
-                               int* status, cudaStream_t stream) {
+                               int merge, int* status, cudaStream_t stream) {
     if (ntok <= 0 || n_seqs <= 0) return 0;
     if (!gg_latent_attention_mma_takes(R, r) || H <= 0 || (pool_row % 8) || pool_row < R + r || page_size <= 0 ||
         (page_size % 64) || (((uintptr_t)qcat | (uintptr_t)pool | (uintptr_t)out) & 15))
@@ -753,7 +897,7 @@ GG_API gg_latent_attention_mma(const void* qcat, const void* pool, int pool_row,
     else if (R <= 128) rc = wide ? GG_LM(64, 128) : GG_LM(32, 128);
     else rc = wide ? GG_LM(64, 256) : GG_LM(32, 256);
 #undef GG_LM
-    if (rc != 0 || splits == 1) return rc;
+    if (rc != 0 || splits == 1 || !merge) return rc;
     return gg_launch(latent_combine_kernel, dim3((unsigned)(ntok * H)), dim3(128), 0, stream, 1, (const float*)part_o,
                      (const float*)part_ml, (bf16*)out, seq_of_token, H, R, splits, sink);
 }

@@ -210,13 +210,14 @@ class LatentAttentionMixer:
         else:
             K.headwise_gemm(qd, width, d + r, self.uk_t, qcat, H * (R + r), R + r, T)
         olat = ctx.ws.get("lat_out", (T, H, R), mid)
+        shares = None
         if self._fast is not None:
-            self._fast.attention(qcat, cache.pool, olat, ctx, table, cache.page_size)
+            shares = self._fast.attention(qcat, cache.pool, olat, ctx, table, cache.page_size)
         else:
             K.latent_attention_plain(qcat, cache.pool, olat, ctx.positions, ctx.seq_of_token, table,
                                      cache.page_size, T, H, R, r, self.scale, self.window, self.sink)
         if self._fast is not None:
-            self._fast.expand(olat, self.uv, av, T, self.out_scale, gate)
+            self._fast.expand(olat, self.uv, av, T, self.out_scale, gate, shares)
         else:
             K.headwise_gemm(olat, H * R, R, self.uv, av, H * dv, dv, T, alpha=self.out_scale, gate=gate)
         self.o(av, residual, accumulate=True, ws=ctx.ws)
