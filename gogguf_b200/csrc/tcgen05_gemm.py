@@ -211,6 +211,29 @@ def gemm_tc_qkv_rope(x: torch.Tensor, w: torch.Tensor, m: int, q_out: torch.Tens
         st.data_ptr(), stream_ptr())
 
 
+def gemm_tc_xielu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ap: float, aq: float, out_scale: float = 1.0,
+                  m: Optional[int] = None, in_ssq: Optional[torch.Tensor] = None, eps: float = 0.0,
+                  scratch: Optional[torch.Tensor] = None) -> None:
+    """out (bfloat16) = out_scale * xIELU(x @ w^T) with the activation in the product's epilogue (csrc/gemm_tcgen05.cu, gg_gemm_tc_xielu);
+    in_ssq, eps and scratch as in `gemm_tc_norm`."""
+    N, K = w.shape
+    M = x.shape[0] if m is None else m
+    if not (x.dtype == w.dtype == out.dtype == torch.bfloat16):
+        raise KernelError("gemm_tc_xielu takes bfloat16 operands and output")
+    if x.stride(-1) != 1 or out.stride(-1) != 1 or not w.is_contiguous():
+        raise KernelError("gemm_tc_xielu: operands must be row-major")
+    need_rows(out, M, N, "gemm_tc_xielu")
+    in_parts = (K + 127) // 128 if in_ssq is not None else 0
+    if in_ssq is not None and (in_ssq.dtype != torch.float32 or not in_ssq.is_contiguous() or in_ssq.shape[-1] != in_parts
+                               or in_ssq.numel() < M * in_parts):
+        raise KernelError("gemm_tc_xielu: in_ssq must be float32 [M, ceil(K / 128)]")
+    kernel("gemm_tcgen05", "gg_gemm_tc_xielu")(
+        x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), out.stride(0),
+        in_ssq.data_ptr() if in_ssq is not None else 0, in_parts, float(eps), float(ap), float(aq), float(out_scale),
+        scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
+        status_word(x.device).data_ptr(), stream_ptr())
+
+
 def make_linear(weight: torch.Tensor, swiglu: bool = False, glu_act: int = 0) -> Optional[Callable]:
     """A callable f(x, out, accumulate, m, ws, in_ssq=None, eps=0.0, out_ssq=None, out_xhat=None, bias=None, out_norm=None) for this
     weight, or None if its sizes are not taken (K must be a multiple of 8 so that rows start on 16-byte

@@ -206,6 +206,22 @@ class Linear:
             x = x.xhat
         tcgen05_gemm.gemm_tc_qkv_rope(x, self.weight, m, **outputs)
 
+    def xielu(self, x, out: torch.Tensor, ap: float, aq: float, out_scale: float, ws: Workspace) -> bool:
+        """out = out_scale * xIELU(y) in the product's epilogue; False (and nothing done) where this product has no such form."""
+        from ..csrc import tcgen05_gemm
+        kw = {}
+        if self.folded_eps is not None and isinstance(x, RowStats):
+            kw.update(in_ssq=x.ssq, eps=self.folded_eps)
+            x = x.xhat
+        N, width = self.weight.shape
+        if (self._fast is None or self.swiglu or self.bias is not None or not isinstance(x, torch.Tensor) or (self.folded_eps is not None) != bool(kw)
+                or x.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or x.stride(0) % 8 or x.data_ptr() % 16 or N <= 128):
+            return False
+        need = tcgen05_gemm.pair_scratch_elems(x.shape[0], N, width) if x.shape[0] > 128 else 0
+        scratch = ws.get("gemm_partial_tiles", (need,), torch.float32) if need else None
+        tcgen05_gemm.gemm_tc_xielu(x, self.weight, out, ap, aq, out_scale, scratch=scratch, **kw)
+        return True
+
     def __call__(self, x, out: torch.Tensor, accumulate: bool = False, m: Optional[int] = None,
                  ws: Optional[Workspace] = None, emit=None) -> None:
         kw = {}
