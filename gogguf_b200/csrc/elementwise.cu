@@ -1030,6 +1030,81 @@ __global__ void __launch_bounds__(1024) rmsnorm_add_vec_kernel(float* x, float* 
 // zeroed (the buffer the next part of the block adds its output into, without a fill of its own).  gate (float32
 // [rows, H], may be null) with gate_bias ([H], may be null): y is first multiplied by sigmoid(gate + gate_bias),
 // element by element, and the norm is taken of the product.
+// The same and the norm that comes next, in one pass: x += y / rms(y) * w, out = x / rms(x) * w2 of the updated rows, which are in
+// registers then.  One block a row, VPT groups of four columns a thread.  As two kernels a decode step paid a launch and a read of
+// the row more.
+template <typename TO, int VPT>
+__global__ void __launch_bounds__(VPT <= 2 ? 1024 : 256) rmsnorm_add_norm_kernel(float* x, float* y, const float* __restrict__ w, int H, float eps, int zero_y,
+                                                                const float* __restrict__ w2, float eps2, TO* __restrict__ out) {
+    pdl_launch();
+    __shared__ float red[33];
+    const size_t r = blockIdx.x;
+    const int n4 = H >> 2;
+    float4 a[VPT], c[VPT];
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        c[j] = i < n4 ? reinterpret_cast<const float4*>(w)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    pdl_wait();
+    float4* yr = reinterpret_cast<float4*>(y + r * H);
+    float4* xr = reinterpret_cast<float4*>(x + r * H);
+    float4 v[VPT];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        v[j] = i < n4 ? yr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        a[j] = i < n4 ? xr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+        ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss); ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+    }
+    ss = block_sum(ss, red);
+    const float f = 1.0f / sqrtf(ss / (float)H + eps);
+    float s2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        a[j].x += v[j].x * f * c[j].x; a[j].y += v[j].y * f * c[j].y; a[j].z += v[j].z * f * c[j].z; a[j].w += v[j].w * f * c[j].w;
+        if (i < n4) {
+            xr[i] = a[j];
+            if (zero_y) yr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            c[j] = reinterpret_cast<const float4*>(w2)[i];
+        }
+        s2 = fmaf(a[j].x, a[j].x, s2); s2 = fmaf(a[j].y, a[j].y, s2); s2 = fmaf(a[j].z, a[j].z, s2); s2 = fmaf(a[j].w, a[j].w, s2);
+    }
+    s2 = block_sum(s2, red);
+    const float f2 = 1.0f / sqrtf(s2 / (float)H + eps2);
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i >= n4) continue;
+        const float o[4] = {a[j].x * f2 * c[j].x, a[j].y * f2 * c[j].y, a[j].z * f2 * c[j].z, a[j].w * f2 * c[j].w};
+        store_row_v<TO, 4>(out + r * H + 4 * i, o);
+    }
+}
+
+// H a multiple of 4 up to 8,192, all rows and vectors on 16-byte boundaries (GG_ERR_ARG otherwise: the caller has the two kernels).
+GG_API gg_rmsnorm_add_norm(float* x, float* y, const float* w, int rows, int H, float eps, int zero_y, const float* w2, float eps2, void* out,
+                           int out_dtype, cudaStream_t stream) {
+    if (rows <= 0) return 0;
+    if (H <= 0 || (H & 3) != 0 || H > 8192 || (((uintptr_t)x | (uintptr_t)y | (uintptr_t)w | (uintptr_t)w2 | (uintptr_t)out) & 15) != 0) return GG_ERR_ARG;
+    // few rows (decode steps): a thread for four columns, up to 1,024; many: 256, so that several blocks share an SM
+    const int n4 = H >> 2;
+    int threads = (n4 + 31) / 32 * 32;
+    if (threads > 1024) threads = 1024;
+    if (threads > 256 && (rows >= 512 || n4 > 2048)) threads = 256;
+    const int vpt = (n4 + threads - 1) / threads;
+    GG_DISPATCH_DTYPE(out_dtype, TO, {
+        if (vpt <= 1) return gg_launch(rmsnorm_add_norm_kernel<TO, 1>, dim3(rows), dim3(threads), 0, stream, 1, x, y, w, H, eps, zero_y, w2, eps2, (TO*)out);
+        if (vpt <= 2) return gg_launch(rmsnorm_add_norm_kernel<TO, 2>, dim3(rows), dim3(threads), 0, stream, 1, x, y, w, H, eps, zero_y, w2, eps2, (TO*)out);
+        if (vpt <= 4) return gg_launch(rmsnorm_add_norm_kernel<TO, 4>, dim3(rows), dim3(threads), 0, stream, 1, x, y, w, H, eps, zero_y, w2, eps2, (TO*)out);
+        return gg_launch(rmsnorm_add_norm_kernel<TO, 8>, dim3(rows), dim3(threads), 0, stream, 1, x, y, w, H, eps, zero_y, w2, eps2, (TO*)out);
+    });
+}
+
 GG_API gg_rmsnorm_add(float* x, float* y, const float* w, int rows, int H, float eps, void* xhat, float* ssq,
                       int zero_y, const float* gate, const float* gate_bias, cudaStream_t stream) {
     if (rows <= 0) return 0;

@@ -198,6 +198,27 @@ def qkv_prep(qkv: torch.Tensor, q_out: torch.Tensor, q_weight: Optional[torch.Te
         float(coef), float(every), _p(status_word(qkv.device)), _stream())
 
 
+def rmsnorm_add_norm_takes(x: torch.Tensor, y: torch.Tensor, out: torch.Tensor) -> bool:
+    """Does `rmsnorm_add_norm` take these rows?"""
+    H = x.shape[-1]
+    return (H % 4 == 0 and H <= 8192 and x.is_contiguous() and y.is_contiguous() and out.is_contiguous()
+            and (x.data_ptr() | y.data_ptr() | out.data_ptr()) % 16 == 0)
+
+
+def rmsnorm_add_norm(x: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: float, next_weight: torch.Tensor, next_eps: float,
+                     out: torch.Tensor, zero_y: bool = False) -> None:
+    """x[r] += y[r] / sqrt(mean(y[r]^2) + eps) * weight, and out[r] = x[r] / sqrt(mean(x[r]^2) + next_eps) * next_weight of the updated
+    rows; x, y and the weights float32, out float32 or bfloat16.  zero_y: y is left zeroed."""
+    for t, what in ((x, "x"), (y, "y"), (weight, "norm weight"), (next_weight, "next norm's weight")):
+        _need(t, torch.float32, what)
+    H = x.shape[-1]
+    if y.shape != x.shape or weight.numel() != H or next_weight.numel() != H or out.shape[-1] != H or out.numel() < x.numel() \
+            or not out.is_contiguous():
+        raise KernelError("rmsnorm_add_norm: shapes disagree")
+    kernel("elementwise", "gg_rmsnorm_add_norm")(_p(x), _p(y), _p(weight), x.numel() // H, H, float(eps), int(zero_y), _p(next_weight),
+                                                  float(next_eps), _p(out), dtype_code(out.dtype), _stream())
+
+
 def rmsnorm_add(x: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: float,
                 xhat: Optional[torch.Tensor] = None, ssq: Optional[torch.Tensor] = None, zero_y: bool = False,
                 gate: Optional[torch.Tensor] = None, gate_bias: Optional[torch.Tensor] = None, groups: int = 1) -> None:

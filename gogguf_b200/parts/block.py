@@ -1,7 +1,7 @@
 """Block arrangements: how a mixer, a feed-forward and their norms are wired around the residual."""
 from __future__ import annotations
 
-from typing import Dict
+from typing import Dict, Optional
 
 import torch
 
@@ -170,11 +170,18 @@ class SandwichNormBlock:
         self.ff_folded = (self.feed_forward is not None and self.ff_gate is None
                           and _offer_norm(self.feed_forward, self.ff_norm, rt))
         self.any_folded = self.mixer_folded or self.ff_folded
+        # the feed-forward's norm, where it stays a norm of its own: the kernel that ends the mixer's part applies it too
+        self.ff_ahead = self.ff_norm if (self.feed_forward is not None and not self.ff_folded and rt.fast
+                                         and getattr(self.ff_norm, "foldable", False)) else None
 
     def _part(self, x: torch.Tensor, ctx: StepContext, pre, post, call, folded: bool, stats, emit: bool,
-              gate=None) -> None:
+              gate=None, ready: Optional[torch.Tensor] = None, ahead=None) -> Optional[torch.Tensor]:
+        """`ready`: the rows behind `pre`, made already.  `ahead`: a norm that reads the stream next; where the kernel after the part can
+        apply it too, its rows are returned."""
         if folded:
             h = stats.ensure(x)
+        elif ready is not None:
+            h = ready
         else:
             h = ctx.ws.get("block_normed", tuple(x.shape), self.rt.dtype)
             pre.forward(x, h)
@@ -190,10 +197,17 @@ class SandwichNormBlock:
             K.rmsnorm_add(x, y, post.weight, post.eps, xhat=stats.xhat, ssq=stats.ssq, zero_y=True, gate=g, gate_bias=gb)
             stats.fresh = True
         else:
-            K.rmsnorm_add(x, y, post.weight, post.eps, zero_y=True, gate=g, gate_bias=gb)
             if stats is not None:
                 stats.fresh = False
+            if ahead is not None and g is None:
+                rows = ctx.ws.get("block_normed", tuple(x.shape), self.rt.dtype)
+                if K.rmsnorm_add_norm_takes(x, y, rows):
+                    K.rmsnorm_add_norm(x, y, post.weight, post.eps, ahead.weight, ahead.eps, rows, zero_y=True)
+                    ctx.shared[self.ZEROED] = y.data_ptr()
+                    return rows
+            K.rmsnorm_add(x, y, post.weight, post.eps, zero_y=True, gate=g, gate_bias=gb)
         ctx.shared[self.ZEROED] = y.data_ptr()
+        return None
 
     def forward(self, x: torch.Tensor, ctx: StepContext, cache, writes_cache: bool) -> None:
         # The statistics live under a key of this arrangement's own: a part's last product writes into the part's
@@ -206,12 +220,12 @@ class SandwichNormBlock:
                 ctx.ws.get("residual_ssq", (T, (H + 127) // 128), torch.float32))
         # the norm-and-add after a part leaves the statistics where the part that comes next in this block reads them
         # folded; across blocks it always does (the next block may be of another make: it re-makes what is stale)
-        self._part(x, ctx, self.mixer_norm, self.mixer_post,
-                   lambda h, y: self.mixer.forward(h, y, ctx, cache, writes_cache), self.mixer_folded, stats,
-                   emit=self.feed_forward is None or self.ff_folded, gate=self.mixer_gate)
+        ready = self._part(x, ctx, self.mixer_norm, self.mixer_post,
+                           lambda h, y: self.mixer.forward(h, y, ctx, cache, writes_cache), self.mixer_folded, stats,
+                           emit=self.feed_forward is None or self.ff_folded, gate=self.mixer_gate, ahead=self.ff_ahead)
         if self.feed_forward is not None:
             self._part(x, ctx, self.ff_norm, self.ff_post, lambda h, y: self.feed_forward.forward(h, y, ctx),
-                       self.ff_folded, stats, emit=True, gate=self.ff_gate)
+                       self.ff_folded, stats, emit=True, gate=self.ff_gate, ready=ready)
 
 
 @register_arrangement("post_norm")
