@@ -108,9 +108,11 @@ struct NormIO {
     float x_p, x_q, x_scale;
 };
 
-// x_scale (x_p v^2 + v / 2) for v > 0, x_scale (x_q (e^v - 1 - v) + v / 2) otherwise
-__device__ __forceinline__ float xielu_value(const NormIO& nio, float v) {
-    return (v > 0.f ? fmaf(nio.x_p * v, v, 0.5f * v) : fmaf(nio.x_q, expm1f(v) - v, 0.5f * v)) * nio.x_scale;
+// scale (p v^2 + v / 2) for v > 0, scale (q (e^v - 1 - v) + v / 2) otherwise.  A call: as code in every epilogue it lengthened the small
+// products of a decode step (a chain of 30 kernels 127.4 -> 129.6 us).
+__device__ __noinline__ float4 xielu_value(float4 v, float p, float q, float scale) {
+    auto one = [&](float t) { return (t > 0.f ? fmaf(p * t, t, 0.5f * t) : fmaf(q, expm1f(t) - t, 0.5f * t)) * scale; };
+    return make_float4(one(v.x), one(v.y), one(v.z), one(v.w));
 }
 
 // tanh(x) in float32: 1 - 2 / (e^2x + 1), its Taylor polynomial where that would cancel (|x| < 1/8: an error below 3e-8)
@@ -435,7 +437,11 @@ __device__ __forceinline__ void epilogue_row_256(uint32_t taddr, int gi, int tn,
         if (nio.bias != nullptr) add_bias<16>(reinterpret_cast<float*>(r), nio.bias, tn * BN + c0, N);
         if (nio.xielu) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(xielu_value(nio, __uint_as_float(r[j])));
+            for (int j = 0; j < 16; j += 4) {
+                const float4 v = xielu_value(make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3])),
+                                             nio.x_p, nio.x_q, nio.x_scale);
+                r[j] = __float_as_uint(v.x); r[j + 1] = __float_as_uint(v.y); r[j + 2] = __float_as_uint(v.z); r[j + 3] = __float_as_uint(v.w);
+            }
         }
         store_row_chunk16(r, gi, tn * BN + c0, N, out, out_mode, ldo, nio, ss);
     }
@@ -605,6 +611,7 @@ __device__ __forceinline__ bool residual_prefetch(int gj, int tile_a, int lane, 
     old = *reinterpret_cast<const float4*>(op);
     return true;
 }
+template <bool XIELU = false>
 __device__ __forceinline__ void finish_token_block(float4 acc, int gj, int tile_a, int lane, void* __restrict__ out,
                                                    int out_mode, long long ldo, int N, const NormIO& nio,
                                                    bool have_old = false, float4 old_pre = make_float4(0.f, 0.f, 0.f, 0.f)) {
@@ -635,9 +642,9 @@ __device__ __forceinline__ void finish_token_block(float4 acc, int gj, int tile_
         if (nio.bias != nullptr) add_bias<4>(f, nio.bias, gi0, N);
         if (out_mode == OUT_BF16) {
             bf16* op = (bf16*)out + o;
-            if (nio.xielu) {
-#pragma unroll
-                for (int t = 0; t < 4; ++t) f[t] = xielu_value(nio, f[t]);
+            if (XIELU && nio.xielu) {
+                const float4 v = xielu_value(make_float4(f[0], f[1], f[2], f[3]), nio.x_p, nio.x_q, nio.x_scale);
+                f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
             }
             if (whole && (((uintptr_t)op) & 7) == 0) {
                 __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
@@ -716,8 +723,12 @@ constexpr int RECV16_SLOTS = 22;
 template <int BN, bool SWAP> constexpr int recv_bytes() { return (SWAP && BN == 16) ? RECV16_SLOTS * BM * 4 : 0; }
 
 // cluster_reduce != 0: the grid was launched with clusters of gridDim.z CTAs along z (the K splits).
-template <int BN, int STAGES, bool SWAP, int MINB>
-__global__ void __launch_bounds__(NUM_THREADS, MINB) gemm_tc_kernel(
+// From 64 tokens on two more warps share an owner's tokens (each round of tokens is a trip through the cluster).
+template <int BN, bool SWAP> constexpr int decode_threads() { return SWAP && BN >= 64 ? 256 : NUM_THREADS; }
+// XIELU: the output may be an activation's (NormIO::xielu).  A form of its own: the test alone lengthened a decode step of small
+// products (a chain of 30 kernels) by 1.5 %.
+template <int BN, int STAGES, bool SWAP, int MINB, bool XIELU>
+__global__ void __launch_bounds__((decode_threads<BN, SWAP>()), MINB) gemm_tc_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     void* __restrict__ out, int out_mode, long long ldo, int M, int N, int K, int kb_per_split,
     float* __restrict__ partial, int cluster_reduce, int* __restrict__ status, const NormIO nio, const QkvIO qio) {
@@ -733,7 +744,7 @@ __global__ void __launch_bounds__(NUM_THREADS, MINB) gemm_tc_kernel(
     // activation, and (decode form) whenever a norm is folded into this product or a bias goes with it
     // (only the decode form splits K or fuses the activation; the launcher sees to that)
     const bool staged = SWAP && (cluster_reduce || out_mode == OUT_SWIGLU || out_mode == OUT_QKV ||
-                                 (partial == nullptr && (nio.in_ssq != nullptr || nio.out_xhat != nullptr || nio.bias != nullptr || nio.xielu)));
+                                 (partial == nullptr && (nio.in_ssq != nullptr || nio.out_xhat != nullptr || nio.bias != nullptr || XIELU)));
     uint32_t* tmem_slot = (uint32_t*)(recv_bar + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     // decode form with a folded norm: the factor of every token of the tile, computed by the epilogue warps while
@@ -849,6 +860,8 @@ __global__ void __launch_bounds__(NUM_THREADS, MINB) gemm_tc_kernel(
             mbar_wait(accum, 0, abort_flag, status, 2);
             cluster_arrive();
         }
+    } else if (warp >= 6) {
+        pdl_wait();                              // (the tile lies in shared memory before these have anything to do)
     } else {
         // epilogue: warp w reads tensor-memory lanes 32*(w%4) .. +31 (row i of D is lane i)
         const int q = warp & 3;
@@ -935,7 +948,7 @@ __global__ void __launch_bounds__(NUM_THREADS, MINB) gemm_tc_kernel(
         const int S = cluster_reduce ? (int)gridDim.z : 1;
         const int cols = min(BN, M - tile_b * BN);
         const uint32_t stage = smem_u32(smem);
-        constexpr int WARPS = NUM_THREADS / 32;
+        constexpr int WARPS = decode_threads<BN, SWAP>() / 32;
         const bool push = push2 || push3;
         const int LJ = (cols + S - 1) / S;                           // tokens an owner handles at most
         // where the pushed rows land, [source rank][owner's token][128] float32: beside the stages (16 tokens) or
@@ -1005,7 +1018,7 @@ __global__ void __launch_bounds__(NUM_THREADS, MINB) gemm_tc_kernel(
                     float4 old4 = r == 0 ? old_r[0] : (r == 1 ? old_r[1] : old_r[2]);
                     bool have_old = r < RPRE && (r == 0 ? have_r[0] : (r == 1 ? have_r[1] : have_r[2]));
                     if (r >= RPRE) have_old = residual_prefetch(gj, tile_a, lane, out, out_mode, ldo, N, nio, old4);
-                    finish_token_block(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio, have_old, old4);
+                    finish_token_block<XIELU>(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio, have_old, old4);
                 }
             }
         };
@@ -1059,7 +1072,7 @@ __global__ void __launch_bounds__(NUM_THREADS, MINB) gemm_tc_kernel(
                     qkv_token_finish(acc, gj, tile_a, lane, qio, qt);
                     continue;
                 }
-                finish_token_block(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio, have_old, old4);
+                finish_token_block<XIELU>(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio, have_old, old4);
             }
         }
         if (cluster_reduce && !push) {
@@ -1533,7 +1546,7 @@ __global__ void __launch_bounds__(256) gemm_splitk_finish_kernel(const float* pa
         qkv_token_finish(acc, gj, tile_a, lane, qio, qt);
         return;
     }
-    finish_token_block(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio);
+    finish_token_block<true>(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio);
 }
 
 // Work items of the CTA-pair form for a product whose tiles do not fill the 74 pairs well.  `splits` > 1: the K range
@@ -1627,7 +1640,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out
                      (const float*)partial, used, out, out_mode, ldo, M, N, col0, NS, nio, qio);
 }
 
-template <int BN, int STAGES, bool SWAP, int MINB>
+template <int BN, int STAGES, bool SWAP, int MINB, bool XIELU = false>
 int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out_mode, long long ldo, int M, int N, int K,
            int splits, int kb_per_split, float* partial, bool cluster, int* status, const NormIO& nio,
            const QkvIO& qio, cudaStream_t stream) {
@@ -1636,7 +1649,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out_mode
     static_assert(!SWAP || BN != 32 || STAGES * (A_BYTES + BN * BK * 2) >= (2 * BN + MAX_CLUSTER - 1) * BM * 4,
                   "at 32 tokens the stages must also hold what the other ranks push");
     static bool configured = false;
-    auto kern = gemm_tc_kernel<BN, STAGES, SWAP, MINB>;
+    auto kern = gemm_tc_kernel<BN, STAGES, SWAP, MINB, XIELU>;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
@@ -1647,11 +1660,19 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out_mode
     float* part = (splits > 1 && !cluster) ? partial : nullptr;
     const int cl = (splits > 1 && cluster) ? 1 : 0;
     if (!SWAP && (cl || out_mode == OUT_SWIGLU || out_mode == OUT_QKV)) return GG_ERR_ARG;      // forms the normal orientation does not have
-    return gg_launch(kern, grid, dim3(NUM_THREADS), smem, stream, cl ? splits : 1, ta, tb, out, out_mode, ldo, M, N, K,
+    return gg_launch(kern, grid, dim3(decode_threads<BN, SWAP>()), smem, stream, cl ? splits : 1, ta, tb, out, out_mode, ldo, M, N, K,
                      kb_per_split, part, cl, status, nio, qio);
 }
 
 }  // namespace
+
+// GOGGUF_B200_GEMM_DEEP=0: three CTAs an SM for every decode product
+static bool gemm_deep() {
+    static int on = -1;
+    if (on < 0) { const char* e = getenv("GOGGUF_B200_GEMM_DEEP"); on = (e != nullptr && e[0] == '0') ? 0 : 1; }
+    return on == 1;
+}
+static bool three_per_sm_at_64(long long tiles) { return tiles > 148 && tiles <= 222; }
 
 // Number of K splits the launcher uses for a product of this shape (0: the shape is not taken).
 // use_cluster != 0: the splits of a tile form a thread-block cluster (at most 8) and no scratch is
@@ -1665,6 +1686,17 @@ GG_API gg_gemm_tc_splits(int M, int N, int K, int use_cluster) {
     int splits = (148 * per_sm + tiles / 2) / tiles;
     if (splits > num_kb / 2) splits = num_kb / 2;  // at least two 64-wide slabs per CTA
     const int most = use_cluster ? MAX_CLUSTER : 16;
+    // 33 to 64 tokens, splits in clusters: two CTAs share an SM with a deeper ring, and K is cut for 256 of the 296 places (or two CTAs a tile
+    // where that many fit), fewer cuts than three an SM would give: every cut sends a float32 row for each token through the cluster.
+    // Measured, 61 tokens (us, three an SM | as it is): 4,096 x 2,048 9.6 | 8.5, 2,048 x 2,048 7.9 | 7.1, 10,752 x 2,048 20.8 | 13.1,
+    // 2,048 x 5,376 11.2 | 9.9, 6,144 x 4,096 15.0 | 13.5, 4,096 x 12,288 24.7 | 22.4, 65,536 x 2,048 53.5 | 49.1; with 149 to 222 tiles
+    // three an SM and two cuts are quicker (24,576 x 4,096: 37.3, 41.4 uncut).
+    if (use_cluster && M > 32 && M <= 64 && gemm_deep() && !three_per_sm_at_64(tiles)) {
+        const int cut = 256 / tiles;
+        splits = cut >= 1 ? cut : 1;
+        if (tiles <= 148 && splits < 2) splits = 2;
+        if (splits > num_kb / 2) splits = num_kb / 2;
+    }
     if (splits > most) splits = most;
     if (splits < 1) splits = 1;
     // no empty split: the last one must own at least one slab
@@ -1714,16 +1746,17 @@ static int gemm_tc_impl(const void* x, const void* w, void* out, int out_mode, i
         if ((rc = make_map(&tb, x, M, K, ldx, bn)) != 0) return rc;
         // A grid that fits two CTAs per SM (296 places) gets the deeper ring; a larger one needs three per SM
         // to run as one wave.  GOGGUF_B200_GEMM_DEEP=0 always takes the three-per-SM forms.
-        static int deep_ok = -1;
-        if (deep_ok < 0) { const char* e = getenv("GOGGUF_B200_GEMM_DEEP"); deep_ok = (e != nullptr && e[0] == '0') ? 0 : 1; }
         const long long ctas = (long long)((N + BM - 1) / BM) * ((M + bn - 1) / bn) * splits;
-        const bool deep = deep_ok && ctas <= 296 && bn <= 32;    // measured in whole steps: a gain up to 32 tokens only
-#define GG_DECODE(BN_, ST_, MINB_) launch<BN_, ST_, true, MINB_>(ta, tb, out, out_mode, ldo, M, N, K, splits, per, scratch, \
-                                                                 cluster, status, nio, qio, stream)
+        // (33 to 64 tokens: see gg_gemm_tc_splits; above, three per SM always)
+        const bool deep = gemm_deep() && (bn <= 32 ? ctas <= 296 : bn == 64 && cluster && !three_per_sm_at_64((N + BM - 1) / BM));
+#define GG_DECODE_AS(BN_, ST_, MINB_, X_) launch<BN_, ST_, true, MINB_, X_>(ta, tb, out, out_mode, ldo, M, N, K, splits, per, scratch, \
+                                                                          cluster, status, nio, qio, stream)
+#define GG_DECODE(BN_, ST_, MINB_) (nio.xielu ? GG_DECODE_AS(BN_, ST_, MINB_, true) : GG_DECODE_AS(BN_, ST_, MINB_, false))
         if (bn == 16) rc = deep ? GG_DECODE(16, 5, 2) : GG_DECODE(16, 3, 3);     // stages + the receive area fill the SM
         else if (bn == 32) rc = deep ? GG_DECODE(32, 5, 2) : GG_DECODE(32, 3, 3);
         else if (bn == 64) rc = deep ? GG_DECODE(64, 4, 2) : GG_DECODE(64, 3, 3);
-        else rc = deep ? GG_DECODE(128, 3, 2) : GG_DECODE(128, 2, 3);
+        else rc = GG_DECODE(128, 2, 3);
+#undef GG_DECODE_AS
 #undef GG_DECODE
     } else {
         const int bn = N > 128 ? 256 : 128;
