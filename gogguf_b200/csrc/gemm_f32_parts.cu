@@ -14,8 +14,7 @@
 // 10,752 x 2,048 547 | 118, 2,048 x 5,376 288 | 61; 17 rows: 23 | 15, 69 | 40, 58 | 26.
 //
 // A CTA owns 128 rows of W (the instruction's M) and BN rows of x, over the whole of K or a share of it, and has
-//   warp 0      TMA: W as float32 (128 x 32 a stage), the three parts of x (BN x 32 each; split_rows_kernel makes them).  Stages of 64
-//               columns, of which two fit beside 160 rows, left the copies' latency in the open (1.78 us for 64 columns);
+//   warp 0      TMA: W as float32 (two boxes of 128 x 32 a stage), the three parts of x (BN x 64 each; split_rows_kernel makes them);
 //   warp 1      the products: parts of W from tensor memory, parts of x from shared memory;
 //   warps 2-5   W's parts: a row a thread, 32 columns at a time from shared memory to tensor memory.  W is split here, once for every
 //               tile of x, because its parts would be half as much again to keep and to read;
@@ -32,10 +31,11 @@
 namespace {
 
 constexpr int ROWS = 128;                 // of W in a tile
-constexpr int STEP = 32;                  // columns of K in a stage, and that are summed in tensor memory
+constexpr int STEP = 64;                  // columns of K in a stage
+constexpr int CHUNK = 32;                 // columns of K that are summed in tensor memory
 constexpr int W_BYTES = ROWS * STEP * 4;
 constexpr int THREADS = 448;
-constexpr int PART_COLS = STEP / 2;       // 32-bit columns of tensor memory that hold a part of 32 columns of K
+constexpr int PART_COLS = CHUNK / 2;      // 32-bit columns of tensor memory that hold a part of 32 columns of K
 constexpr int A_COLS = 3 * PART_COLS;
 
 struct Shape {
@@ -43,11 +43,6 @@ struct Shape {
     int m_tiles, n_tiles, shares, steps;  // steps: stages in a share of K (the last share may have fewer)
     int items;
 };
-
-// Shared-memory descriptor of a K-major operand with rows of 64 bytes, 64-byte swizzle: 8-row groups are 512 bytes apart.
-__device__ __forceinline__ uint64_t half_desc(uint32_t saddr) {
-    return (uint64_t)((saddr & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
-}
 
 // The sum that a not-finite one is replaced by.
 __device__ __noinline__ float plain_dot(const float* x, const float* w, int k0, int k1) {
@@ -138,6 +133,7 @@ __global__ void __launch_bounds__(THREADS, 1) parts_kernel(const __grid_constant
             auto load_w = [&](int s, int step) {
                 tma::mbar_expect_tx(&full_w[s], W_BYTES);
                 tma::load_2d(smem + s * STAGE_BYTES, &map_w, &full_w[s], step * STEP, n0);
+                tma::load_2d(smem + s * STAGE_BYTES + W_BYTES / 2, &map_w, &full_w[s], step * STEP + 32, n0);
             };
             auto load_x = [&](int s, int step) {
                 tma::mbar_expect_tx(&full_x[s], 3 * X_PART);
@@ -167,62 +163,67 @@ __global__ void __launch_bounds__(THREADS, 1) parts_kernel(const __grid_constant
     } else if (warp == 1) {
         if (lane == 0) {
             const uint32_t idesc = tc5::idesc_bf16(ROWS, BN, 0);
-            int it = 0;
+            int it = 0, c = 0;
             bool ok = true;
             for (int item = blockIdx.x; item < sh.items && ok; item += gridDim.x) {
                 place(item, m0, n0, step0, n_steps, share);
                 for (int i = 0; i < n_steps && ok; ++i, ++it) {
-                    const int s = it % STAGES, pb = it % PARTS, ab = it & 1;
-                    ok = tma::mbar_wait(&full_x[s], (it / STAGES) & 1, abort_flag, status, 2)
-                         && tma::mbar_wait(&acc_empty[ab], ((it >> 1) & 1) ^ 1, abort_flag, status, 4)
-                         && tma::mbar_wait(&a_full[pb], (it / PARTS) & 1, abort_flag, status, 2);
-                    if (!ok) break;
-                    tc5::fence_after();
-                    const uint32_t acc = tmem + (uint32_t)(ab * BN), a = tmem + (uint32_t)(2 * BN + pb * A_COLS);
-                    const uint64_t xd = half_desc(tma::smem_u32(smem + s * STAGE_BYTES + W_BYTES));
-                    // the small products first: what the tensor core cuts off is a part of the larger addend
-                    constexpr int PW[6] = {0, 1, 2, 0, 1, 0}, PX[6] = {2, 1, 0, 1, 0, 0};
+                    const int s = it % STAGES;
+                    ok = tma::mbar_wait(&full_x[s], (it / STAGES) & 1, abort_flag, status, 2);
+                    for (int h = 0; h < 2 && ok; ++h, ++c) {
+                        const int pb = c % PARTS, ab = c & 1;
+                        ok = tma::mbar_wait(&a_full[pb], (c / PARTS) & 1, abort_flag, status, 2)
+                             && tma::mbar_wait(&acc_empty[ab], ((c >> 1) & 1) ^ 1, abort_flag, status, 4);
+                        if (!ok) break;
+                        tc5::fence_after();
+                        const uint32_t acc = tmem + (uint32_t)(ab * BN), a = tmem + (uint32_t)(2 * BN + pb * A_COLS);
+                        const uint32_t xs = tma::smem_u32(smem + s * STAGE_BYTES + W_BYTES) + (uint32_t)(h * 64);
+                        // the small products first: what the tensor core cuts off is a part of the larger addend
+                        constexpr int PW[6] = {0, 1, 2, 0, 1, 0}, PX[6] = {2, 1, 0, 1, 0, 0};
 #pragma unroll
-                    for (int q = 0; q < 6; ++q)
+                        for (int q = 0; q < 6; ++q)
 #pragma unroll
-                        for (int k = 0; k < 2; ++k)
-                            tc5::mma_a_tmem(acc, a + (uint32_t)(PW[q] * PART_COLS + 8 * k), xd + (uint64_t)((PX[q] * X_PART + 32 * k) >> 4), idesc,
-                                            q + k > 0 ? 1u : 0u);
-                    tc5::commit(&a_empty[pb]);
-                    tc5::commit(&empty[s]);
-                    tc5::commit(&acc_full[ab]);
+                            for (int k = 0; k < 2; ++k)
+                                tc5::mma_a_tmem(acc, a + (uint32_t)(PW[q] * PART_COLS + 8 * k),
+                                                tc5::smem_desc(xs + (uint32_t)(PX[q] * X_PART + 32 * k), 16, 1024), idesc, q + k > 0 ? 1u : 0u);
+                        tc5::commit(&a_empty[pb]);
+                        tc5::commit(&acc_full[ab]);
+                    }
+                    if (ok) tc5::commit(&empty[s]);
                 }
             }
         }
     } else if (warp < 6) {
         const int row = (warp & 3) * 32 + lane;
-        int it = 0;
+        int it = 0, c = 0;
         bool ok = true;
         for (int item = blockIdx.x; item < sh.items && ok; item += gridDim.x) {
             place(item, m0, n0, step0, n_steps, share);
-            for (int i = 0; i < n_steps; ++i, ++it) {
-                const int s = it % STAGES, pb = it % PARTS;
+            for (int i = 0; i < n_steps && ok; ++i, ++it) {
+                const int s = it % STAGES;
                 // (a warp's waits may end apart when one runs out; what follows is the whole warp's)
                 ok = __all_sync(0xffffffffu, tma::mbar_wait(&full_w[s], (it / STAGES) & 1, abort_flag, status, 3));
-                if (!ok) break;
-                const uint8_t* src = smem + s * STAGE_BYTES + row * 128;
-                uint32_t p[3][PART_COLS];
+                for (int h = 0; h < 2 && ok; ++h, ++c) {
+                    const uint8_t* src = smem + s * STAGE_BYTES + h * (W_BYTES / 2) + row * 128;
+                    uint32_t p[3][PART_COLS];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {                         // 16-byte pieces, where the 128-byte swizzle has put them
-                    const float4 v = *reinterpret_cast<const float4*>(src + ((j ^ (row & 7)) << 4));
-                    split_pair(v.x, v.y, p[0][2 * j], p[1][2 * j], p[2][2 * j]);
-                    split_pair(v.z, v.w, p[0][2 * j + 1], p[1][2 * j + 1], p[2][2 * j + 1]);
+                    for (int j = 0; j < 8; ++j) {                     // 16-byte pieces, where the 128-byte swizzle has put them
+                        const float4 v = *reinterpret_cast<const float4*>(src + ((j ^ (row & 7)) << 4));
+                        split_pair(v.x, v.y, p[0][2 * j], p[1][2 * j], p[2][2 * j]);
+                        split_pair(v.z, v.w, p[0][2 * j + 1], p[1][2 * j + 1], p[2][2 * j + 1]);
+                    }
+                    const int pb = c % PARTS;
+                    ok = __all_sync(0xffffffffu, tma::mbar_wait(&a_empty[pb], ((c / PARTS) & 1) ^ 1, abort_flag, status, 3));
+                    if (!ok) break;
+                    tc5::fence_after();
+                    const uint32_t dst = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(2 * BN + pb * A_COLS);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) tc5::st16(dst + (uint32_t)(q * PART_COLS), p[q]);
+                    tc5::wait_st();
+                    tc5::fence_before();
+                    tma::mbar_arrive(&a_full[pb]);
+                    if (h == 1) tma::mbar_arrive(&empty[s]);
                 }
-                tma::mbar_arrive(&empty[s]);
-                ok = __all_sync(0xffffffffu, tma::mbar_wait(&a_empty[pb], ((it / PARTS) & 1) ^ 1, abort_flag, status, 3));
-                if (!ok) break;
-                tc5::fence_after();
-                const uint32_t dst = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(2 * BN + pb * A_COLS);
-#pragma unroll
-                for (int q = 0; q < 3; ++q) tc5::st16(dst + (uint32_t)(q * PART_COLS), p[q]);
-                tc5::wait_st();
-                tc5::fence_before();
-                tma::mbar_arrive(&a_full[pb]);
             }
         }
     } else {
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(THREADS, 1) parts_kernel(const __grid_constant
             float acc[HALF];
 #pragma unroll
             for (int j = 0; j < HALF; ++j) acc[j] = 0.f;
-            for (int i = 0; i < n_steps; ++i, ++c) {
+            for (int i = 0; i < 2 * n_steps; ++i, ++c) {
                 const int ab = c & 1;
                 ok = __all_sync(0xffffffffu, tma::mbar_wait(&acc_full[ab], (c >> 1) & 1, abort_flag, status, 5));
                 if (!ok) break;
@@ -332,7 +333,7 @@ struct Plan {
 // The tile and the shares of K with the least modelled time: rounds of 148 items, each its stages at the tile's measured rate and 2.5 us
 // beside, and for shares the second kernel with its traffic.  (Measured, us a stage: 1.45 to 1.8 whatever the tile up to 160 rows.)
 Plan plan_for(int M, int N, int K, int force_tile, int force_shares) {
-    static const float step_us[TILES] = {0.5f, 0.5f, 0.5f, 0.55f, 0.6f, 0.72f};
+    static const float step_us[TILES] = {1.44f, 1.5f, 1.5f, 1.6f, 1.7f, 1.95f};
     const int all = (K + STEP - 1) / STEP;
     const long long n_tiles = (N + ROWS - 1) / ROWS;
     Plan best = {0, 1, all};
@@ -346,7 +347,7 @@ Plan plan_for(int M, int N, int K, int force_tile, int force_shares) {
             const int steps = (all + s - 1) / s;
             if ((all + steps - 1) / steps != s) continue;            // (a share would be empty)
             const long long rounds = (m_tiles * n_tiles * s + 147) / 148;
-            float us = (float)rounds * ((float)steps * step_us[t] + 2.0f);
+            float us = (float)rounds * ((float)steps * step_us[t] + 2.5f);
             if (s > 1) us += 3.0f + (float)(s + 1) * (float)M * (float)N * (4e-6f / 4.0f);
             if (!any || us < least) { best = {t, s, steps}; least = us; any = true; }
         }
@@ -377,12 +378,7 @@ int launch_tile(const float* x, long long ldx, const float* w, float* out, long 
     if (fn(&map_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return GG_ERR_TMAP;
-    cuuint64_t dims_x[2] = {(cuuint64_t)sh.K, (cuuint64_t)sh.M * 3};
-    cuuint64_t strides_x[1] = {(cuuint64_t)ldp * 2};
-    cuuint32_t box_x[2] = {(cuuint32_t)STEP, (cuuint32_t)BN};
-    if (fn(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(parts), dims_x, strides_x, box_x, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return GG_ERR_TMAP;
+    if ((rc = tma::make_map_bf16(&map_x, parts, 3ull * sh.M, sh.K, ldp, BN)) != 0) return rc;
     const int grid = sh.items < resident ? sh.items : resident;
     return gg_launch(kern, dim3(grid), dim3(THREADS), smem, stream, 1, map_w, map_x, x, ldx, w, out, ldo, accumulate, bias, partial, sh, status);
 }
@@ -424,12 +420,12 @@ GG_API gg_gemm_f32_parts(const float* x, const float* w, float* out, int accumul
     Shape sh = {M, N, K, 0, (N + ROWS - 1) / ROWS, plan.shares, plan.steps, 0};
 #define GT(BN, ST, PA) rc = launch_tile<BN, ST, PA>(x, ldx, w, out, ldo, accumulate, bias, partial, parts, ld, sh, status, stream)
     switch (plan.tile) {
-        case 0: GT(32, 8, 4); break;
-        case 1: GT(64, 7, 4); break;
-        case 2: GT(96, 6, 4); break;
-        case 3: GT(128, 5, 4); break;
-        case 4: GT(160, 4, 4); break;
-        default: GT(192, 4, 2); break;
+        case 0: GT(32, 4, 4); break;
+        case 1: GT(64, 3, 4); break;
+        case 2: GT(96, 3, 4); break;
+        case 3: GT(128, 2, 4); break;
+        case 4: GT(160, 2, 4); break;
+        default: GT(192, 2, 2); break;
     }
 #undef GT
     if (rc != 0 || plan.shares == 1) return rc;
