@@ -1209,6 +1209,27 @@ def moe_route(z: torch.Tensor, top: int, idx: torch.Tensor, wts: torch.Tensor, s
                                    _stream())
 
 
+def moe_logits_route_takes(h: torch.Tensor, wr: torch.Tensor, n_tokens: int) -> bool:
+    """Does `moe_logits_route` take this many tokens of h and this router?"""
+    E, W = wr.shape
+    return n_tokens <= 148 and E <= 32 and W % 4 == 0 and W <= 12000 and (h.data_ptr() | wr.data_ptr()) % 16 == 0
+
+
+def moe_logits_route(h: torch.Tensor, wr: torch.Tensor, z: torch.Tensor, top: int, idx: torch.Tensor, wts: torch.Tensor,
+                     seq_of_token: Optional[torch.Tensor], n_tokens: int, softmax: bool = False, renormalize: bool = False, n_real: int = 0,
+                     scale: float = 1.0) -> None:
+    """`moe_router_logits` and `moe_route` (without a correction or groups) in one kernel, for few tokens and experts."""
+    _need(z, torch.float32, "router logits")
+    _need(idx, torch.int32, "idx")
+    _need(wts, torch.float32, "wts")
+    E, W = wr.shape
+    if h.shape[-1] != W or z.shape[-1] != E or not h.is_contiguous() or not wr.is_contiguous():
+        raise KernelError("moe_logits_route: shapes disagree")
+    kernel("moe", "gg_moe_logits_route")(_p(h), dtype_code(h.dtype), _p(wr), dtype_code(wr.dtype), _p(z), int(n_tokens), W, E, int(top),
+                                         int(softmax), int(renormalize), int(n_real), float(scale), _p(idx), _p(wts), _p(seq_of_token),
+                                         _stream())
+
+
 def moe_gate_up(h: torch.Tensor, w_gu: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, y: torch.Tensor,
                 n_tokens: int, top: int, weight_on_input: bool, limit: float, slope: float, out_scale: float,
                 up_offset: float = 1.0) -> None:

@@ -122,17 +122,9 @@ GG_API gg_moe_router_logits(const void* h, int h_dtype, const void* wr, int w_dt
 
 // ----------------------------------------------------------------------------- route
 // One warp per token.  z [T, E] float32 logits.  softmax != 0: scores are softmax(z), else sigmoid(z).
-__global__ void __launch_bounds__(32) moe_route_kernel(const float* z, int E, int top, int softmax, int renorm,
-                                                       int n_real, float scale,
-                                                       int* idx, float* wts, const int* __restrict__ seq_of_token) {
-    pdl_launch();
-    pdl_wait();
-    const int t = blockIdx.x, lane = threadIdx.x;
-    const float* zt = z + (size_t)t * E;
-    if (seq_of_token != nullptr && seq_of_token[t] < 0) {      // padding: expert 0 with weight 0
-        for (int k = lane; k < top; k += 32) { idx[(size_t)t * top + k] = 0; wts[(size_t)t * top + k] = 0.f; }
-        return;
-    }
+// The token's choice and weights from its logits zt [E], one warp.
+__device__ __forceinline__ void route_token(const float* zt, int E, int top, int softmax, int renorm, int n_real, float scale, int* idx,
+                                            float* wts, int t, int lane) {
     float mx = -INFINITY, den = 1.f;
     if (softmax) {
         for (int e = lane; e < E; e += 32) mx = fmaxf(mx, zt[e]);
@@ -170,6 +162,78 @@ __global__ void __launch_bounds__(32) moe_route_kernel(const float* z, int E, in
         const float f = renorm ? scale / (total + 1e-20f) : scale;
         for (int k = lane; k < top; k += 32) wts[(size_t)t * top + k] *= f;
     }
+}
+
+__global__ void __launch_bounds__(32) moe_route_kernel(const float* z, int E, int top, int softmax, int renorm,
+                                                       int n_real, float scale,
+                                                       int* idx, float* wts, const int* __restrict__ seq_of_token) {
+    pdl_launch();
+    pdl_wait();
+    const int t = blockIdx.x, lane = threadIdx.x;
+    if (seq_of_token != nullptr && seq_of_token[t] < 0) {      // padding: expert 0 with weight 0
+        for (int k = lane; k < top; k += 32) { idx[(size_t)t * top + k] = 0; wts[(size_t)t * top + k] = 0.f; }
+        return;
+    }
+    route_token(z + (size_t)t * E, E, top, softmax, renorm, n_real, scale, idx, wts, t, lane);
+}
+
+// Logits and choice in one kernel for few tokens and up to 32 experts (decode steps): a block a token, a warp an expert, the sums those of
+// moe_router_logits_kernel; the first warp then chooses.  The router's first columns are asked for before the wait.
+#define ROUTE_AHEAD 8
+template <typename TX, typename TW>
+__global__ void __launch_bounds__(1024) moe_logits_route_kernel(const TX* h, const TW* __restrict__ wr, float* z, int W, int E, int top, int softmax,
+                                                                int renorm, int n_real, float scale, int* idx, float* wts,
+                                                                const int* __restrict__ seq_of_token) {
+    pdl_launch();
+    extern __shared__ __align__(16) float rx[];          // [W]
+    __shared__ float logits[32];
+    const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const TW* w = wr + (size_t)warp * W;
+    float4 ahead[ROUTE_AHEAD];
+#pragma unroll
+    for (int j = 0; j < ROUTE_AHEAD; ++j)
+        ahead[j] = lane * 4 + 128 * j < W ? load4<TW, true>(w + lane * 4 + 128 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait();
+    for (int k = threadIdx.x * 4; k < W; k += blockDim.x * 4) *reinterpret_cast<float4*>(rx + k) = load4<TX, true>(h + (size_t)t * W + k);
+    __syncthreads();
+    float s = 0.f;
+    auto add = [&](const float4& c, int i) {
+        const float4 a = *reinterpret_cast<const float4*>(rx + i);
+        s = fmaf(c.w, a.w, fmaf(c.z, a.z, fmaf(c.y, a.y, fmaf(c.x, a.x, s))));
+    };
+#pragma unroll
+    for (int j = 0; j < ROUTE_AHEAD; ++j)
+        if (lane * 4 + 128 * j < W) add(ahead[j], lane * 4 + 128 * j);
+#pragma unroll 4
+    for (int i = lane * 4 + 128 * ROUTE_AHEAD; i < W; i += 128) add(load4<TW, true>(w + i), i);
+    s = warp_sum(s);
+    if (lane == 0) { logits[warp] = s; z[(size_t)t * E + warp] = s; }
+    __syncthreads();
+    if (warp > 0) return;
+    if (seq_of_token != nullptr && seq_of_token[t] < 0) {      // padding: expert 0 with weight 0
+        for (int k = lane; k < top; k += 32) { idx[(size_t)t * top + k] = 0; wts[(size_t)t * top + k] = 0.f; }
+        return;
+    }
+    route_token(logits, E, top, softmax, renorm, n_real, scale, idx, wts, t, lane);
+}
+
+// z[t] = wr h[t], then the token's `top` experts and their weights as gg_moe_route without a correction or groups.  Up to 148 tokens and 32
+// experts, W a multiple of 4 up to 12,000, rows on 16-byte boundaries; GG_ERR_ARG otherwise (the caller has the two kernels).
+GG_API gg_moe_logits_route(const void* h, int h_dtype, const void* wr, int w_dtype, float* z, int T, int W, int E, int top, int softmax, int renorm,
+                           int n_real, float scale, int* idx, float* wts, const int* seq_of_token, cudaStream_t stream) {
+    if (T <= 0) return 0;
+    if (T > 148 || W <= 0 || (W % 4) != 0 || W > 12000 || E <= 0 || E > 32 || top <= 0 || top > E || n_real < 0 || n_real > E ||
+        (((uintptr_t)h | (uintptr_t)wr) & 15) != 0)
+        return GG_ERR_ARG;
+    if (n_real == 0) n_real = E;
+#define GG_LR(TX, TW) return gg_launch(moe_logits_route_kernel<TX, TW>, dim3(T), dim3(32 * E), (size_t)W * sizeof(float), stream, 1, (const TX*)h, \
+                                       (const TW*)wr, z, W, E, top, softmax, renorm, n_real, scale, idx, wts, seq_of_token)
+    if (h_dtype == GG_F32 && w_dtype == GG_F32) GG_LR(float, float);
+    if (h_dtype == GG_BF16 && w_dtype == GG_BF16) GG_LR(bf16, bf16);
+    if (h_dtype == GG_BF16 && w_dtype == GG_F32) GG_LR(bf16, float);
+    if (h_dtype == GG_F32 && w_dtype == GG_BF16) GG_LR(float, bf16);
+    return GG_ERR_DTYPE;
+#undef GG_LR
 }
 
 // The same choice with a correction and groups: scores s = sigmoid(z) (or softmax); the choice scores are

@@ -207,9 +207,13 @@ class RoutedExperts:
     def route(self, h: torch.Tensor, ctx: StepContext):
         T = ctx.n_tokens
         z = ctx.ws.get("moe_logits", (T, self.R), torch.float32)
-        K.moe_router_logits(h, self.router_w, z, T)      # CUDA cores, float32 sums: the router is never reduced
         idx = ctx.ws.get("moe_idx", (T, self.top), torch.int32)
         wts = ctx.ws.get("moe_wts", (T, self.top), torch.float32)
+        if self.correction is None and self.groups <= 1 and K.moe_logits_route_takes(h, self.router_w, T):
+            K.moe_logits_route(h, self.router_w, z, self.top, idx, wts, ctx.seq_of_token, T, softmax=self.softmax, renormalize=self.renorm,
+                               n_real=self.E if self.identity else 0, scale=self.weight_scale)
+            return idx, wts
+        K.moe_router_logits(h, self.router_w, z, T)      # CUDA cores, float32 sums: the router is never reduced
         K.moe_route(z, self.top, idx, wts, ctx.seq_of_token, softmax=self.softmax, renormalize=self.renorm, rows=T,
                     correction=self.correction, groups=self.groups, keep=self.keep,
                     n_real=self.E if self.identity else 0, scale=self.weight_scale)
