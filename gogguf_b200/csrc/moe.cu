@@ -562,36 +562,38 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* rows, con
                                                           int top, const int* __restrict__ seq_of_token, const int* idx) {
     pdl_launch();
     pdl_wait();
+    // (a block takes one round of the columns: a decode step's few tokens walked over theirs with a trip to memory a round)
     const int t = blockIdx.x;
     if (seq_of_token != nullptr && seq_of_token[t] < 0) return;
     constexpr int V = VEC ? 4 : 1;
-    for (int i = threadIdx.x * V; i < W; i += blockDim.x * V) {
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int k = 0; k < top; ++k) {
-            const size_t p = (size_t)t * top + k;
-            if (idx != nullptr && idx[p] < 0) continue;      // a choice without an expert left no row
-            const float* r = rows + (place != nullptr ? (size_t)place[p] : p) * W + i;
-            if (VEC) {
-                const float4 v = *reinterpret_cast<const float4*>(r);
-                s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w;
-            } else s[0] += *r;
-        }
-        float* o = residual + (size_t)t * W + i;
+    const int i = (blockIdx.y * blockDim.x + threadIdx.x) * V;
+    if (i >= W) return;
+    float* o = residual + (size_t)t * W + i;
+    float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (VEC) old = *reinterpret_cast<const float4*>(o);
+    else old.x = *o;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int k = 0; k < top; ++k) {
+        const size_t p = (size_t)t * top + k;
+        if (idx != nullptr && idx[p] < 0) continue;          // a choice without an expert left no row
+        const float* r = rows + (place != nullptr ? (size_t)place[p] : p) * W + i;
         if (VEC) {
-            float4 v = *reinterpret_cast<const float4*>(o);
-            v.x += s[0]; v.y += s[1]; v.z += s[2]; v.w += s[3];
-            *reinterpret_cast<float4*>(o) = v;
-        } else *o += s[0];
+            const float4 v = *reinterpret_cast<const float4*>(r);
+            s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w;
+        } else s[0] += *r;
     }
+    if (VEC) *reinterpret_cast<float4*>(o) = make_float4(old.x + s[0], old.y + s[1], old.z + s[2], old.w + s[3]);
+    else *o = old.x + s[0];
 }
 
 // idx (may be null): the pairs' expert indices; pairs whose index is negative are left out.
 GG_API gg_moe_combine(const float* rows, const int* place, float* residual, int T, int W, int top,
                       const int* seq_of_token, const int* idx, cudaStream_t stream) {
-    if (T <= 0) return 0;
+    if (T <= 0 || W <= 0) return 0;
     if (W % 4 == 0 && (((uintptr_t)rows | (uintptr_t)residual) & 15) == 0)
-        return gg_launch(moe_combine_kernel<true>, dim3(T), dim3(256), 0, stream, 1, rows, place, residual, W, top, seq_of_token, idx);
-    return gg_launch(moe_combine_kernel<false>, dim3(T), dim3(256), 0, stream, 1, rows, place, residual, W, top, seq_of_token, idx);
+        return gg_launch(moe_combine_kernel<true>, dim3(T, (W / 4 + 255) / 256), dim3(256), 0, stream, 1, rows, place, residual, W, top, seq_of_token, idx);
+    return gg_launch(moe_combine_kernel<false>, dim3(T, (W + 255) / 256), dim3(256), 0, stream, 1, rows, place, residual, W, top, seq_of_token, idx);
 }
 
 // ----------------------------------------------------------------------------- identity experts
