@@ -147,8 +147,7 @@ __device__ __forceinline__ void add_bias(float* v, const float* __restrict__ bia
 // one head per 128-row weight tile of the decode form, two per tile of the CTA-pair form): per-head RMSNorm of q and k with one shared weight
 // each, rotation of pairs (i, i + 64) by the step's cos/sin tables, q to its buffer, k (normed, rotated)
 // and v (raw) into the paged cache at the token's position.  Padding tokens (seq_of_token < 0) write
-// nothing to the cache; k_pool == null writes no cache at all.  Heads of 64 (decode form only): two per weight tile, half a warp each,
-// pairs (i, i + 32); sizes of 128 below are then 64, and 64 are 32.
+// nothing to the cache; k_pool == null writes no cache at all.
 struct QkvIO {
     bf16* q_out;                 // [M, nq * 128]
     const float* qw;             // [128] or null: no norm
@@ -165,7 +164,6 @@ struct QkvIO {
     bf16* v_pool;
     int nq;
     int nkv;
-    int head_dim;                // 128, or 64
     int n_pages;                 // pages in the pools (the debug build checks every page id against it)
     int* status;                 // where the debug build records a page id or table index out of range (code 48)
 };
@@ -177,10 +175,7 @@ struct QkvTok {
     int b, pos, page;
     float4 c4, s4, w4;
 };
-// D = 64: the lane's head is one of the tile's two, `h` counts tiles.
-template <int D>
 __device__ __forceinline__ QkvTok qkv_token_data(const QkvIO& qio, int gj, int h, int lane) {
-    if (D == 64) h = 2 * h + (lane >> 4);
     QkvTok t;
     t.b = -1; t.pos = 0; t.page = 0;
     t.c4 = make_float4(1.f, 1.f, 1.f, 1.f); t.s4 = make_float4(0.f, 0.f, 0.f, 0.f); t.w4 = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -193,54 +188,44 @@ __device__ __forceinline__ QkvTok qkv_token_data(const QkvIO& qio, int gj, int h
     }
     if (is_q || is_k) {
         const float* w = is_q ? qio.qw : qio.kw;
-        if (w != nullptr) t.w4 = *reinterpret_cast<const float4*>(w + 4 * (lane & (D / 4 - 1)));
-        const int i0 = 4 * (lane & (D / 8 - 1));
-        t.c4 = *reinterpret_cast<const float4*>(qio.cosv + (size_t)gj * (D / 2) + i0);
-        t.s4 = *reinterpret_cast<const float4*>(qio.sinv + (size_t)gj * (D / 2) + i0);
+        if (w != nullptr) t.w4 = *reinterpret_cast<const float4*>(w + 4 * lane);
+        const int i0 = 4 * (lane & 15);
+        t.c4 = *reinterpret_cast<const float4*>(qio.cosv + (size_t)gj * 64 + i0);
+        t.s4 = *reinterpret_cast<const float4*>(qio.sinv + (size_t)gj * 64 + i0);
     }
     return t;
 }
-// acc: features 4 lane .. 4 lane + 3 of head h (D = 64: of tile h) of token gj, already multiplied by the folded norm's factor.
+// acc: features 4 lane .. 4 lane + 3 of head h of token gj, already multiplied by the folded norm's factor.
 // Per-head RMSNorm and rotation for q and k; q to its buffer, k and v into the paged cache.  All 32 lanes call it.
-template <int D>
 __device__ __forceinline__ void qkv_token_finish(float4 acc, int gj, int h, int lane, const QkvIO& qio, const QkvTok& t) {
-    if (D == 64) h = 2 * h + (lane >> 4);
     const bool is_q = h < qio.nq, is_k = !is_q && h < qio.nq + qio.nkv;
-    if (D == 128 && !is_q && (qio.k_pool == nullptr || t.b < 0)) return;
+    if (!is_q && (qio.k_pool == nullptr || t.b < 0)) return;
     float f[4] = {acc.x, acc.y, acc.z, acc.w};
-    // (a tile's two heads of 64 may be of two kinds: the exchanges below are the whole warp's, what does not apply is dropped)
-    if (D == 64 || is_q || is_k) {
-        if (D == 64 || (is_q ? qio.qw : qio.kw) != nullptr) {
+    if (is_q || is_k) {
+        if ((is_q ? qio.qw : qio.kw) != nullptr) {
             float ss = fmaf(f[0], f[0], fmaf(f[1], f[1], fmaf(f[2], f[2], f[3] * f[3])));
-            if (D == 128) ss = warp_sum(ss);
-            else {
-#pragma unroll
-                for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            }
-            if (D == 128 || ((is_q || is_k) && (is_q ? qio.qw : qio.kw) != nullptr)) {
-                const float scale = 1.0f / sqrtf(ss * (1.0f / (float)D) + qio.eps);
-                f[0] *= scale * t.w4.x; f[1] *= scale * t.w4.y; f[2] *= scale * t.w4.z; f[3] *= scale * t.w4.w;
-            }
+            ss = warp_sum(ss);
+            const float scale = 1.0f / sqrtf(ss * (1.0f / 128.0f) + qio.eps);
+            f[0] *= scale * t.w4.x; f[1] *= scale * t.w4.y; f[2] *= scale * t.w4.z; f[3] *= scale * t.w4.w;
         }
         const float cs[4] = {t.c4.x, t.c4.y, t.c4.z, t.c4.w}, sn[4] = {t.s4.x, t.s4.y, t.s4.z, t.s4.w};
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const float p = __shfl_xor_sync(0xffffffffu, f[u], D / 8);   // the other half of the pair 
-            if (D == 128 || is_q || is_k) f[u] = (lane & (D / 8)) == 0 ? f[u] * cs[u] - p * sn[u] : p * sn[u] + f[u] * cs[u];
+            const float p = __shfl_xor_sync(0xffffffffu, f[u], 16);      // the other half of the pair
+            f[u] = lane < 16 ? f[u] * cs[u] - p * sn[u] : p * sn[u] + f[u] * cs[u];
         }
     }
     bf16* dst;
     if (is_q) {
-        dst = qio.q_out + ((size_t)gj * qio.nq + h) * D;
+        dst = qio.q_out + ((size_t)gj * qio.nq + h) * 128;
     } else {
-        if (D == 64 && (h >= qio.nq + 2 * qio.nkv || qio.k_pool == nullptr || t.b < 0)) return;
         if (t.page < 0) return;      // (debug build) outside the pools: nothing is written
         const int kvh = is_k ? h - qio.nq : h - qio.nq - qio.nkv;
         dst = (is_k ? qio.k_pool : qio.v_pool) +
-              (((size_t)t.page * qio.nkv + kvh) * qio.page_size + (t.pos % qio.page_size)) * D;
+              (((size_t)t.page * qio.nkv + kvh) * qio.page_size + (t.pos % qio.page_size)) * 128;
     }
     __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), bb = __floats2bfloat162_rn(f[2], f[3]);
-    *reinterpret_cast<uint2*>(dst + 4 * (lane & (D / 4 - 1))) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&bb));
+    *reinterpret_cast<uint2*>(dst + 4 * lane) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&bb));
 }
 
 // One thread computes its token's factor (four running sums keep the loads independent).
@@ -740,9 +725,9 @@ template <int BN, bool SWAP> constexpr int recv_bytes() { return (SWAP && BN == 
 // cluster_reduce != 0: the grid was launched with clusters of gridDim.z CTAs along z (the K splits).
 // From 64 tokens on two more warps share an owner's tokens (each round of tokens is a trip through the cluster).
 template <int BN, bool SWAP> constexpr int decode_threads() { return SWAP && BN >= 64 ? 256 : NUM_THREADS; }
-// FORM: 0; 1 the output may be an activation's (NormIO::xielu); 2 q/k/v with heads of 64.  Forms of their own: the first's test alone
-// lengthened a decode step of small products (a chain of 30 kernels) by 1.5 %.
-template <int BN, int STAGES, bool SWAP, int MINB, int FORM>
+// XIELU: the output may be an activation's (NormIO::xielu).  A form of its own: the test alone lengthened a decode step of small
+// products (a chain of 30 kernels) by 1.5 %.
+template <int BN, int STAGES, bool SWAP, int MINB, bool XIELU>
 __global__ void __launch_bounds__((decode_threads<BN, SWAP>()), MINB) gemm_tc_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     void* __restrict__ out, int out_mode, long long ldo, int M, int N, int K, int kb_per_split,
@@ -759,7 +744,7 @@ __global__ void __launch_bounds__((decode_threads<BN, SWAP>()), MINB) gemm_tc_ke
     // activation, and (decode form) whenever a norm is folded into this product or a bias goes with it
     // (only the decode form splits K or fuses the activation; the launcher sees to that)
     const bool staged = SWAP && (cluster_reduce || out_mode == OUT_SWIGLU || out_mode == OUT_QKV ||
-                                 (partial == nullptr && (nio.in_ssq != nullptr || nio.out_xhat != nullptr || nio.bias != nullptr || FORM == 1)));
+                                 (partial == nullptr && (nio.in_ssq != nullptr || nio.out_xhat != nullptr || nio.bias != nullptr || XIELU)));
     uint32_t* tmem_slot = (uint32_t*)(recv_bar + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     // decode form with a folded norm: the factor of every token of the tile, computed by the epilogue warps while
@@ -1033,7 +1018,7 @@ __global__ void __launch_bounds__((decode_threads<BN, SWAP>()), MINB) gemm_tc_ke
                     float4 old4 = r == 0 ? old_r[0] : (r == 1 ? old_r[1] : old_r[2]);
                     bool have_old = r < RPRE && (r == 0 ? have_r[0] : (r == 1 ? have_r[1] : have_r[2]));
                     if (r >= RPRE) have_old = residual_prefetch(gj, tile_a, lane, out, out_mode, ldo, N, nio, old4);
-                    finish_token_block<FORM == 1>(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio, have_old, old4);
+                    finish_token_block<XIELU>(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio, have_old, old4);
                 }
             }
         };
@@ -1060,7 +1045,7 @@ __global__ void __launch_bounds__((decode_threads<BN, SWAP>()), MINB) gemm_tc_ke
                 if (!have_old && out_mode != OUT_QKV && (push || round >= RPRE))
                     have_old = residual_prefetch(gj, tile_a, lane, out, out_mode, ldo, N, nio, old4);
                 QkvTok qt;
-                if (out_mode == OUT_QKV) qt = qkv_token_data<FORM == 2 ? 64 : 128>(qio, gj, tile_a, lane);       // this tile is head `tile_a`
+                if (out_mode == OUT_QKV) qt = qkv_token_data(qio, gj, tile_a, lane);       // this tile is head `tile_a`
                 if (!received) {
                     if (!mbar_wait(recv_bar, 0, abort_flag, status, 5)) break;
                     received = true;
@@ -1084,10 +1069,10 @@ __global__ void __launch_bounds__((decode_threads<BN, SWAP>()), MINB) gemm_tc_ke
                 if (!left && j + S * WARPS >= cols) { cluster_arrive(); left = true; }
                 if (nio.in_ssq != nullptr) { acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc; }
                 if (out_mode == OUT_QKV) {
-                    qkv_token_finish<FORM == 2 ? 64 : 128>(acc, gj, tile_a, lane, qio, qt);
+                    qkv_token_finish(acc, gj, tile_a, lane, qio, qt);
                     continue;
                 }
-                finish_token_block<FORM == 1>(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio, have_old, old4);
+                finish_token_block<XIELU>(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio, have_old, old4);
             }
         }
         if (cluster_reduce && !push) {
@@ -1695,7 +1680,7 @@ __global__ void __launch_bounds__(256) gemm_splitk_finish_kernel(const float* pa
     if (gj >= M) return;
     const int c0 = tile_a * 128 + 4 * lane;
     QkvTok qt;
-    if (out_mode == OUT_QKV) qt = qkv_token_data<128>(qio, gj, tile_a, lane);       // a block of 128 columns is one head
+    if (out_mode == OUT_QKV) qt = qkv_token_data(qio, gj, tile_a, lane);       // a block of 128 columns is one head
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c0 + 4 <= N && (NS & 3) == 0) {
         for (int s = 0; s < splits; ++s) {
@@ -1714,7 +1699,7 @@ __global__ void __launch_bounds__(256) gemm_splitk_finish_kernel(const float* pa
         acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
     }
     if (out_mode == OUT_QKV) {
-        qkv_token_finish<128>(acc, gj, tile_a, lane, qio, qt);
+        qkv_token_finish(acc, gj, tile_a, lane, qio, qt);
         return;
     }
     finish_token_block<true>(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio);
@@ -1845,7 +1830,7 @@ int launch_pair_tokens(const void* x, const void* w, long long ldx, void* out, i
                      out_mode, ldo, M, N, 0, N, nio, qio);
 }
 
-template <int BN, int STAGES, bool SWAP, int MINB, int FORM = 0>
+template <int BN, int STAGES, bool SWAP, int MINB, bool XIELU = false>
 int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out_mode, long long ldo, int M, int N, int K,
            int splits, int kb_per_split, float* partial, bool cluster, int* status, const NormIO& nio,
            const QkvIO& qio, cudaStream_t stream) {
@@ -1854,7 +1839,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out_mode
     static_assert(!SWAP || BN != 32 || STAGES * (A_BYTES + BN * BK * 2) >= (2 * BN + MAX_CLUSTER - 1) * BM * 4,
                   "at 32 tokens the stages must also hold what the other ranks push");
     static bool configured = false;
-    auto kern = gemm_tc_kernel<BN, STAGES, SWAP, MINB, FORM>;
+    auto kern = gemm_tc_kernel<BN, STAGES, SWAP, MINB, XIELU>;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
@@ -1922,9 +1907,8 @@ static int gemm_tc_impl(const void* x, const void* w, void* out, int out_mode, i
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || (K % 8) != 0 || (ldx % 8) != 0 || ldx < K || out_mode < 0 || out_mode > 4) return GG_ERR_ARG;
     if (out_mode == OUT_QKV) {
-        // one 128-wide head (two of 64) per weight tile in the decode form, two of 128 per tile in the CTA-pair form; `out` is not used
-        if (qio.nq <= 0 || qio.nkv <= 0 || (qio.head_dim != 128 && (qio.head_dim != 64 || M > 128)) ||
-            N != (qio.nq + 2 * qio.nkv) * qio.head_dim || qio.q_out == nullptr ||
+        // one 128-wide head per weight tile (decode form) or two per tile (CTA-pair form); `out` is not used
+        if (qio.nq <= 0 || qio.nkv <= 0 || N != (qio.nq + 2 * qio.nkv) * 128 || qio.q_out == nullptr ||
             qio.cosv == nullptr || qio.sinv == nullptr || qio.positions == nullptr || qio.seq_of_token == nullptr ||
             (qio.k_pool != nullptr && (qio.v_pool == nullptr || qio.page_table == nullptr || qio.page_size <= 0)))
             return GG_ERR_ARG;
@@ -1957,8 +1941,7 @@ static int gemm_tc_impl(const void* x, const void* w, void* out, int out_mode, i
         const bool deep = gemm_deep() && (bn <= 32 ? ctas <= 296 : bn == 64 && cluster && !three_per_sm_at_64((N + BM - 1) / BM));
 #define GG_DECODE_AS(BN_, ST_, MINB_, X_) launch<BN_, ST_, true, MINB_, X_>(ta, tb, out, out_mode, ldo, M, N, K, splits, per, scratch, \
                                                                           cluster, status, nio, qio, stream)
-#define GG_DECODE(BN_, ST_, MINB_) (nio.xielu ? GG_DECODE_AS(BN_, ST_, MINB_, 1) : out_mode == OUT_QKV && qio.head_dim == 64 ? \
-                                    GG_DECODE_AS(BN_, ST_, MINB_, 2) : GG_DECODE_AS(BN_, ST_, MINB_, 0))
+#define GG_DECODE(BN_, ST_, MINB_) (nio.xielu ? GG_DECODE_AS(BN_, ST_, MINB_, true) : GG_DECODE_AS(BN_, ST_, MINB_, false))
         if (bn == 16) rc = deep ? GG_DECODE(16, 5, 2) : GG_DECODE(16, 3, 3);     // stages + the receive area fill the SM
         else if (bn == 32) rc = deep ? GG_DECODE(32, 5, 2) : GG_DECODE(32, 3, 3);
         else if (bn == 64) rc = deep ? GG_DECODE(64, 4, 2) : GG_DECODE(64, 3, 3);
@@ -2055,19 +2038,19 @@ GG_API gg_gemm_tc_pair_scratch_elems(int M, int N, int K, long long* elems) {
     return 0;
 }
 
-// The q/k/v projection of a step (head size 128; up to 128 tokens also 64; more than 128 tokens in the CTA-pair form) with the per-head q/k RMSNorm,
-// the rotation and the cache write in its epilogue: x[M, K] * w[(nq + 2 nkv) * head_dim, K]^T, rows of w being
+// The q/k/v projection of a step (head size 128; more than 128 tokens in the CTA-pair form) with the per-head q/k RMSNorm,
+// the rotation and the cache write in its epilogue: x[M, K] * w[(nq + 2 nkv) * 128, K]^T, rows of w being
 // all q heads, then all k heads, then all v heads.  See QkvIO for the outputs; in_ssq / in_parts / in_eps
 // as in gg_gemm_tc_norm (null: x is already normalised).  qw / kw null: no q/k norm.
 GG_API gg_gemm_tc_qkv_rope(const void* x, const void* w, int M, int K, long long ldx, const float* in_ssq, int in_parts,
                            float in_eps, void* q_out, const float* qw, const float* kw, float eps, const float* cosv,
                            const float* sinv, const int* positions, const int* seq_of_token, const int* page_table,
-                           int max_pages, int page_size, int n_pages, void* k_pool, void* v_pool, int nq, int nkv, int head_dim,
+                           int max_pages, int page_size, int n_pages, void* k_pool, void* v_pool, int nq, int nkv,
                            float* scratch, long long scratch_elems, int* status, cudaStream_t stream) {
     if (in_ssq != nullptr && (in_parts != (K + 127) / 128 || !(in_eps > 0.f))) return GG_ERR_ARG;
     const NormIO nio = {in_ssq, in_parts, K > 0 ? 1.0f / (float)K : 0.f, in_eps, nullptr, nullptr, nullptr, nullptr, nullptr, 0.f, 0};
     const QkvIO qio = {(bf16*)q_out, qw, kw, eps, cosv, sinv, positions, seq_of_token, page_table, max_pages, page_size,
-                       (bf16*)k_pool, (bf16*)v_pool, nq, nkv, head_dim, n_pages, status};
-    const int N = (nq + 2 * nkv) * head_dim;
+                       (bf16*)k_pool, (bf16*)v_pool, nq, nkv, n_pages, status};
+    const int N = (nq + 2 * nkv) * 128;
     return gemm_tc_impl(x, w, q_out, OUT_QKV, M, N, K, ldx, N, scratch, scratch_elems, 1, status, nio, qio, stream);
 }

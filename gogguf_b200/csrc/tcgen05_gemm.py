@@ -59,12 +59,10 @@ def pair_scratch_elems(M: int, N: int, K: int) -> int:
     return int(n.value)
 
 
-def qkv_rope_takes(m: int, head_dim: int = 128) -> bool:
-    """Does `gemm_tc_qkv_rope` take m tokens?  Up to 128 always (decode form, heads of 128 or 64); more, with heads of 128, in the
-    CTA-pair form, which GOGGUF_B200_GEMM_PAIR=0 switches off."""
+def qkv_rope_takes(m: int) -> bool:
+    """Does `gemm_tc_qkv_rope` take m tokens?  Up to 128 always (decode form); more in the CTA-pair form, which
+    GOGGUF_B200_GEMM_PAIR=0 switches off."""
     import os
-    if head_dim != 128:
-        return head_dim == 64 and m <= 128
     return m <= 128 or os.environ.get("GOGGUF_B200_GEMM_PAIR", "1") != "0"
 
 
@@ -179,27 +177,26 @@ def gemm_tc_qkv_rope(x: torch.Tensor, w: torch.Tensor, m: int, q_out: torch.Tens
                      positions: torch.Tensor, seq_of_token: torch.Tensor, page_table: torch.Tensor, page_size: int,
                      k_pool: Optional[torch.Tensor], v_pool: Optional[torch.Tensor], nq: int, nkv: int,
                      in_ssq: Optional[torch.Tensor] = None, in_eps: float = 0.0,
-                     scratch: Optional[torch.Tensor] = None, head_dim: int = 128) -> None:
-    """The q/k/v projection of a step (head sizes and m: see `qkv_rope_takes`) with the per-head q/k RMSNorm,
+                     scratch: Optional[torch.Tensor] = None) -> None:
+    """The q/k/v projection of a step (head size 128; any m, see `qkv_rope_takes`) with the per-head q/k RMSNorm,
     the rotation and the cache write in the product's epilogue (csrc/gemm_tcgen05.cu, gg_gemm_tc_qkv_rope).
     scratch: room for the partial tiles of a K split at more than 128 tokens (`pair_scratch_elems`); the kernel that
     adds them then does the per-head work."""
     N, K = w.shape
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or q_out.dtype != torch.bfloat16:
         raise KernelError("gemm_tc_qkv_rope takes bfloat16 operands")
-    d = int(head_dim)
-    if N != (nq + 2 * nkv) * d or not qkv_rope_takes(m, d) or q_out.numel() < m * nq * d or not q_out.is_contiguous():
-        raise KernelError("gemm_tc_qkv_rope: head size 128 or 64, q_out [m, nq * head size]; more than 128 tokens only in the "
-                          "CTA-pair form, with heads of 128")
-    if cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.shape[-1] != d // 2 or sin.shape[-1] != d // 2 \
+    if N != (nq + 2 * nkv) * 128 or not qkv_rope_takes(m) or q_out.numel() < m * nq * 128 or not q_out.is_contiguous():
+        raise KernelError("gemm_tc_qkv_rope: head size 128, q_out [m, nq * 128]; more than 128 tokens only in the "
+                          "CTA-pair form")
+    if cos.dtype != torch.float32 or sin.dtype != torch.float32 or cos.shape[-1] != 64 or sin.shape[-1] != 64 \
             or not cos.is_contiguous() or not sin.is_contiguous():
-        raise KernelError("gemm_tc_qkv_rope: cos and sin are float32 [m, head size / 2]")
+        raise KernelError("gemm_tc_qkv_rope: cos and sin are float32 [m, 64]")
     for t in (positions, seq_of_token, page_table):
         if t.dtype != torch.int32 or not t.is_contiguous():
             raise KernelError("gemm_tc_qkv_rope: integer inputs are contiguous int32")
     for t in (qw, kw):
-        if t is not None and (t.dtype != torch.float32 or t.numel() != d):
-            raise KernelError("gemm_tc_qkv_rope: norm weights are float32 [head size]")
+        if t is not None and (t.dtype != torch.float32 or t.numel() != 128):
+            raise KernelError("gemm_tc_qkv_rope: norm weights are float32 [128]")
     if k_pool is not None and (k_pool.dtype != torch.bfloat16 or v_pool is None or v_pool.dtype != torch.bfloat16):
         raise KernelError("gemm_tc_qkv_rope: the cache pools are bfloat16")
     in_parts = (K + 127) // 128 if in_ssq is not None else 0
@@ -210,7 +207,7 @@ def gemm_tc_qkv_rope(x: torch.Tensor, w: torch.Tensor, m: int, q_out: torch.Tens
         float(eps), cos.data_ptr(), sin.data_ptr(), positions.data_ptr(), seq_of_token.data_ptr(),
         page_table.data_ptr(), page_table.shape[-1], int(page_size), k_pool.shape[0] if k_pool is not None else 0,
         k_pool.data_ptr() if k_pool is not None else 0, v_pool.data_ptr() if v_pool is not None else 0,
-        nq, nkv, d, scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
+        nq, nkv, scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
         st.data_ptr(), stream_ptr())
 
 

@@ -165,9 +165,9 @@ class AttentionMixer:
         if rt.fast and rt.dtype == torch.bfloat16:
             from ..csrc import fast_attention
             self._fast = fast_attention.try_make(self.nq, self.nkv, self.d, self.scale, self.window, dv=self.dv, chunk=self.chunk)
-        # head sizes 128 and 64 with a full rotation by cos/sin tables: the decode form of the q/k/v product can do
-        # the per-head work itself (one head, or two, per 128-row weight tile)
-        self._fused_rope = (self.qkv.tensor_core and self.d in (64, 128) and self.rot == self.d and not self._general
+        # head size 128 with a full rotation by cos/sin tables: the decode form of the q/k/v product can do
+        # the per-head work itself (one head per 128-row weight tile)
+        self._fused_rope = (self.qkv.tensor_core and self.d == 128 and self.rot == self.d and not self._general
                             and os.environ.get("GOGGUF_B200_FUSE_QKV_ROPE", "1") != "0")
 
     def can_absorb_norm(self, norm) -> bool:
@@ -202,12 +202,12 @@ class AttentionMixer:
         cos, sin = self.position.tables(ctx) if self.position is not None else (None, None)
         table = ctx.page_tables[cache.group]
         gate = None
-        if self._fused_rope and tcgen05_gemm.qkv_rope_takes(T, d):
+        if self._fused_rope and tcgen05_gemm.qkv_rope_takes(T):
             # norm, rotation and cache write happen in the projection's epilogue
             self.qkv.qkv_rope(h, T, ws=ctx.ws, q_out=q, qw=self.q_norm, kw=self.k_norm, eps=self.eps, cos=cos, sin=sin,
                               positions=ctx.positions, seq_of_token=ctx.seq_of_token, page_table=table,
                               page_size=cache.page_size, k_pool=cache.k if writes_cache else None,
-                              v_pool=cache.v if writes_cache else None, nq=nq, nkv=nkv, head_dim=d)
+                              v_pool=cache.v if writes_cache else None, nq=nq, nkv=nkv)
         elif self._general:
             row = ctx.ws.get("attn_qkv", (T, self.qkv.out_features), dt)
             self.qkv(h, row, ws=ctx.ws)
