@@ -1510,162 +1510,6 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_tc_pair_kernel(
     }
 }
 
-// The same pairs with the operands the other way round, for 129 to 768 tokens: the weights are the instruction's 256 rows and the tokens its
-// columns, nt of them (a multiple of 32 up to 256) in each of the fewest equal tiles, so that 333 tokens are multiplied as 384 and not as
-// 512.  Everything leaves as raw sums, [splits][M][N]: a lane has a weight row, so a warp's store is a line of 32 neighbouring outputs of a
-// token; gemm_splitk_finish_kernel adds the splits and applies the output mode.  333 tokens (us, both kernels, tokens as rows | as columns):
-// @@
-template <int STAGES>
-__global__ void __launch_bounds__(PAIR_THREADS, 1) gemm_tc_pair_tokens_kernel(
-    const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, float* __restrict__ partial, int M, int N, int K, int nt,
-    int splits, int kb_per_split, int* __restrict__ status) {
-    constexpr int STAGE_BYTES = A_BYTES + 128 * BK * 2;      // at most nt / 2 = 128 tokens a CTA
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = (uint64_t*)(smem + STAGES * STAGE_BYTES);
-    uint64_t* empty = full + STAGES;
-    uint64_t* acc_full = empty + STAGES;
-    uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
-    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-
-    pdl_launch();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t rank;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    const bool leader = rank == 0;
-    const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-    const int num_kb = (K + BK - 1) / BK;
-    const int tiles_m = (M + nt - 1) / nt;
-    const int total = tiles_m * ((N + 255) / 256) * splits;
-    const uint32_t stage_tx = 2u * (uint32_t)(A_BYTES + nt / 2 * BK * 2);
-    // item -> token tile (fastest: the pairs that run together share weights in L2), split of K, weight tile
-    auto item_of = [&](int t, int& tm, int& tn, int& split, int& kb0, int& kb1) {
-        tm = t % tiles_m;
-        const int r = t / tiles_m;
-        split = r % splits;
-        tn = r / splits;
-        kb0 = split * kb_per_split;
-        kb1 = min(num_kb, kb0 + kb_per_split);
-    };
-    int tm, tn, split, kb0, kb1;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 512); }
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmW) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmX) : "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();          // the peer's barriers exist before anything is signalled across the pair
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            int it = 0;
-            bool first = true, ok = true;
-            for (int t = pair; t < total && ok; t += num_pairs) {
-                item_of(t, tm, tn, split, kb0, kb1);
-                const int wrow = tn * 256 + (int)rank * 128, xrow = tm * nt + (int)rank * (nt / 2);
-                int kb = kb0;
-                if (first) {
-                    const int pre = kb1 - kb0 < STAGES ? kb1 - kb0 : STAGES;
-                    for (int i = 0; i < pre; ++i) {
-                        if (leader) mbar_expect_tx(&full[i], stage_tx);
-                        tma_load_2d_pair(smem + i * STAGE_BYTES, &tmW, &full[i], (kb0 + i) * BK, wrow);
-                    }
-                    pdl_wait();
-                    for (int i = 0; i < pre; ++i) tma_load_2d_pair(smem + i * STAGE_BYTES + A_BYTES, &tmX, &full[i], (kb0 + i) * BK, xrow);
-                    kb = kb0 + pre;
-                    it = pre;
-                    first = false;
-                }
-                for (; kb < kb1; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(&empty[s], ((uint32_t)(it / STAGES) & 1u) ^ 1u, abort_flag, status, 1)) { ok = false; break; }
-                    if (leader) mbar_expect_tx(&full[s], stage_tx);
-                    tma_load_2d_pair(smem + s * STAGE_BYTES, &tmW, &full[s], kb * BK, wrow);
-                    tma_load_2d_pair(smem + s * STAGE_BYTES + A_BYTES, &tmX, &full[s], kb * BK, xrow);
-                }
-            }
-            if (first) pdl_wait();
-        }
-    } else if (warp == 1) {
-        if (lane == 0 && leader) {
-            const uint32_t idesc = make_idesc(256, nt);
-            int it = 0, i = 0;
-            bool ok = true;
-            for (int t = pair; t < total && ok; t += num_pairs, ++i) {
-                const int buf = i & 1;
-                ok = mbar_wait(&acc_empty[buf], ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, status, 4);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t tacc = tmem_base + (uint32_t)(buf * 256);
-                item_of(t, tm, tn, split, kb0, kb1);
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    ok = mbar_wait(&full[s], (uint32_t)(it / STAGES) & 1u, abort_flag, status, 2);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
-                    const uint64_t adesc = make_smem_desc(sa), bdesc = make_smem_desc(sa + A_BYTES);
-#pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k)
-                        umma_pair(tacc, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-                    umma_commit_pair(&empty[s]);
-                }
-                if (ok) umma_commit_pair(&acc_full[buf]);
-            }
-        }
-    } else {
-        const int q = warp & 3, half = (warp - 2) >> 2;
-        pdl_wait();
-        int i = 0;
-        for (int t = pair; t < total; t += num_pairs, ++i) {
-            item_of(t, tm, tn, split, kb0, kb1);
-            const int buf = i & 1, n = tn * 256 + (int)rank * 128 + q * 32 + lane, m0 = tm * nt;
-            if (!mbar_wait(&acc_full[buf], (uint32_t)(i >> 1) & 1u, abort_flag, status, 3)) break;
-            tc_fence_after();
-            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 256);
-            float* dst = partial + (size_t)split * M * N + n;
-#pragma unroll 2
-            for (int c0 = 16 * half; c0 < nt && m0 + c0 < M; c0 += 32) {
-                uint32_t r[16];
-                tmem_ld16(taddr + (uint32_t)c0, r);
-                tmem_ld_wait();
-                if (n < N) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (m0 + c0 + j < M) dst[(size_t)(m0 + c0 + j) * N] = __uint_as_float(r[j]);
-                }
-            }
-            tc_fence_before();
-            mbar_arrive_cluster(&acc_empty[buf], 0);     // 512 arrivals in the leader free the accumulator pair
-        }
-    }
-
-    tc_fence_before();
-    __syncthreads();
-    if (*abort_flag) {
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000LL) { }
-        __syncthreads();
-    }
-    cluster_sync_all();          // neither CTA leaves while the other may still signal its barriers
-    if (warp == 1) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
-    }
-}
-
 // out (mode) = sum over splits of partial[s], scaled by the folded norm's factor: a warp per (token, block of 128
 // columns), the epilogue of the decode form.  The partial tiles cover the columns from `col0` on (the tile columns
 // that were split), NS of them per row.
@@ -1711,13 +1555,10 @@ __global__ void __launch_bounds__(256) gemm_splitk_finish_kernel(const float* pa
 // hundred tokens), or the full waves whole and only the tiles of a last wave that is less than half full split.  Every split
 // keeps eight 64-wide slabs, and the float32 partial tiles (written and read once, then a second kernel) must cost
 // less than the idle pairs.  {1, tiles}: no split.
-// nt > 0: tokens as columns, nt a tile, all tiles in `splits` (gemm_tc_pair_tokens_kernel).
 struct PairPlan {
     int splits;
     int whole;
-    int nt = 0;
     long long scratch_elems(int M, int N) const {
-        if (nt > 0) return (long long)splits * M * N;
         if (splits <= 1) return 0;
         const int tiles_m = (M + 255) / 256;
         return (long long)splits * M * (N - (whole / tiles_m) * 256);
@@ -1738,17 +1579,6 @@ PairPlan pair_plan(int M, int N, int K, bool uneven_ok) {
         const int waves = (items + pairs - 1) / pairs;
         const double cost = waves * tile_s / s + (s > 1 ? 2.0 * s * M * (double)N * 4 / 6e12 : 0.0);
         if (cost < best_cost * 0.97) { best_cost = cost; best = PairPlan{s, s > 1 ? 0 : tiles}; }
-    }
-    // Tokens as columns, where rows in tiles of 256 would be multiplied for nothing; the sums leave unfinished even when K is not
-    // split.
-    if (tiles_m <= 3) {
-        const int nt = ((M + tiles_m - 1) / tiles_m + 31) / 32 * 32;
-        for (int s = 1; s <= 8; ++s) {
-            if (s > 1 && num_kb / s < 8) break;
-            const int waves = (tiles * s + pairs - 1) / pairs;
-            const double cost = waves * tile_s * nt / 256.0 / s + 2.0 * s * M * (double)N * 4 / 6e12 + (best.splits == 1 ? 3e-6 : 0.0);
-            if (cost < best_cost * 0.95) { best_cost = cost; best = PairPlan{s, 0, nt}; }
-        }
     }
     // The second shape, for products in the compute-bound range (more than 768 tokens; measured: the gate-up product
     // of 256 tokens, which streams its weights at the memory's rate, gains nothing from it).  The pairs walk the
@@ -1808,26 +1638,6 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out
     const int col0 = (whole / tiles_m) * 256, NS = N - col0;
     return gg_launch(gemm_splitk_finish_kernel, dim3((NS + 127) / 128, (M + 7) / 8), dim3(256), 0, stream, 1,
                      (const float*)partial, used, out, out_mode, ldo, M, N, col0, NS, nio, qio);
-}
-
-int launch_pair_tokens(const void* x, const void* w, long long ldx, void* out, int out_mode, long long ldo, int M, int N, int K, int* status,
-                       const NormIO& nio, const QkvIO& qio, PairPlan plan, float* partial, cudaStream_t stream) {
-    constexpr int STAGES = 6, smem = STAGES * (A_BYTES + 128 * BK * 2) + 1024 + 256;
-    auto kern = gemm_tc_pair_tokens_kernel<STAGES>;
-    static int known[GG_MAX_DEVICES] = {};
-    int resident = 0;
-    int rc = gg_resident(kern, PAIR_THREADS, smem, known, resident);
-    if (rc != 0) return rc;
-    CUtensorMap tw, tx;
-    if ((rc = make_map(&tw, w, N, K, K, 128)) != 0) return rc;
-    if ((rc = make_map(&tx, x, M, K, ldx, plan.nt / 2)) != 0) return rc;
-    const int num_kb = (K + BK - 1) / BK, per = (num_kb + plan.splits - 1) / plan.splits, used = (num_kb + per - 1) / per;
-    const int total = (M + plan.nt - 1) / plan.nt * ((N + 255) / 256) * used;
-    const int pairs = total < resident / 2 ? total : resident / 2;
-    rc = gg_launch2(kern, dim3(2 * pairs), dim3(PAIR_THREADS), smem, stream, tw, tx, partial, M, N, K, plan.nt, used, per, status);
-    if (rc != 0) return rc;
-    return gg_launch(gemm_splitk_finish_kernel, dim3((N + 127) / 128, (M + 7) / 8), dim3(256), 0, stream, 1, (const float*)partial, used, out,
-                     out_mode, ldo, M, N, 0, N, nio, qio);
 }
 
 template <int BN, int STAGES, bool SWAP, int MINB, bool XIELU = false>
@@ -1959,10 +1769,9 @@ static int gemm_tc_impl(const void* x, const void* w, void* out, int out_mode, i
             if ((rc = make_map(&tb, w, N, K, K, 128)) != 0) return rc;
             // (a split q/k/v product leaves the per-head epilogue to the kernel that adds the partial tiles)
             PairPlan plan = pair_plan(M, N, K, true);
-            if (plan.scratch_elems(M, N) > 0 && (scratch == nullptr || scratch_elems < plan.scratch_elems(M, N)))
+            if (plan.splits > 1 && (scratch == nullptr || scratch_elems < plan.scratch_elems(M, N)))
                 plan = PairPlan{1, 0};                                                   // no room for partial tiles
-            if (plan.nt > 0) rc = launch_pair_tokens(x, w, ldx, out, out_mode, ldo, M, N, K, status, nio, qio, plan, scratch, stream);
-            else rc = launch_pair(ta, tb, out, out_mode, ldo, M, N, K, status, nio, qio, plan, scratch, stream);
+            rc = launch_pair(ta, tb, out, out_mode, ldo, M, N, K, status, nio, qio, plan, scratch, stream);
         } else if (out_mode == OUT_QKV) rc = GG_ERR_ARG;       // only the CTA-pair form has the q/k/v epilogue
         else if (bn == 256) rc = launch_persistent(ta, tb, out, out_mode, ldo, M, N, K, status, nio, stream);
         else rc = launch<128, 6, false, 1>(ta, tb, out, out_mode, ldo, M, N, K, 1, per, scratch, false, status, nio, qio, stream);
