@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const float* partial, int s
 }
 
 constexpr int TILES = 6;
+constexpr float PAYS_BESIDE = 12.0f;      // us: two launches more on the host, where a step of few rows is bound
 const int TILE_BN[TILES] = {32, 64, 96, 128, 160, 192};
 
 struct Plan {
@@ -332,7 +333,7 @@ struct Plan {
 
 // The tile and the shares of K with the least modelled time: rounds of 148 items, each its stages at the tile's measured rate and 2.5 us
 // beside, and for shares the second kernel with its traffic.  (Measured, us a stage: 1.45 to 1.8 whatever the tile up to 160 rows.)
-Plan plan_for(int M, int N, int K, int force_tile, int force_shares) {
+Plan plan_for(int M, int N, int K, int force_tile, int force_shares, float* modelled = nullptr) {
     static const float step_us[TILES] = {1.44f, 1.5f, 1.5f, 1.6f, 1.7f, 1.95f};
     const int all = (K + STEP - 1) / STEP;
     const long long n_tiles = (N + ROWS - 1) / ROWS;
@@ -352,6 +353,7 @@ Plan plan_for(int M, int N, int K, int force_tile, int force_shares) {
             if (!any || us < least) { best = {t, s, steps}; least = us; any = true; }
         }
     }
+    if (modelled != nullptr) *modelled = least;
     return best;
 }
 
@@ -392,6 +394,30 @@ GG_API gg_gemm_f32_parts_scratch(int M, int N, int K, int force_tile, int force_
     if (M <= 0 || N <= 0 || K <= 0 || bytes == nullptr) return GG_ERR_ARG;
     const Plan p = plan_for(M, N, K, force_tile, force_shares);
     *bytes = ((3LL * M * parts_ld(K) * 2 + 255) / 256) * 256 + (p.shares > 1 ? (long long)p.shares * M * N * 4 : 0);
+    return 0;
+}
+
+// Is a product of this size quicker in parts than on the CUDA cores?  On the GPU alone it is from 17 rows and K = 1,024 on (us, CUDA cores |
+// parts: 17 rows by 1,024 x 1,024 8.9 | 8.3, 2,048 x 2,048 20.8 | 13.5; 100 rows 13.2 | 12.1, 46.3 | 17.2; by 512 x 512 5.2 | 7.4), but it is
+// two or three launches instead of one, and a prompt of few rows is bound by the host's launches: 20 tokens, two layers of a
+// 1,024-wide model 297 -> 376 us with every product in parts.  So the CUDA cores' time, modelled, has to be PAYS_BESIDE longer.  Below
+// K = 256 the sums are no more exact than theirs either (K = 128: 1.1e-7 both).
+GG_API gg_gemm_f32_parts_pays(int M, int N, int K, int* pays) {
+    if (M <= 0 || N <= 0 || K <= 0 || pays == nullptr) return GG_ERR_ARG;
+    *pays = 0;
+    if (M < 17 || K < 256 || K % 4 != 0) return 0;
+    // the CUDA cores' tiles as gemm_plain.cu chooses among them: rounds of 296, us per 1,000 of K
+    static const float round_us[4][2] = {{11, 11}, {30, 35}, {42, 55}, {54, 110}};
+    static const int rows[4] = {32, 64, 64, 128}, cols[4] = {16, 32, 64, 64};
+    float plain = 0.f;
+    for (int i = 0; i < 4; ++i) {
+        const long long t = (long long)((M + rows[i] - 1) / rows[i]) * ((N + cols[i] - 1) / cols[i]), left = t % 296;
+        const float us = (round_us[i][1] * (float)(t / 296) + (left == 0 ? 0.f : round_us[i][left > 148])) * (float)K * 1e-3f;
+        if (i == 0 || us < plain) plain = us;
+    }
+    float parts = 0.f;
+    plan_for(M, N, K, -1, 0, &parts);
+    *pays = parts + PAYS_BESIDE < plain;
     return 0;
 }
 

@@ -442,7 +442,11 @@ def gemm_plain(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: 
                                            x.stride(0), out.stride(0), _p(bias), _stream())
 
 
-F32_PARTS_ROWS = 17           # rows from which the 32-bit path's products are made in parts on the tensor cores (see gemm_f32_parts.cu)
+def f32_parts_pays(M: int, N: int, K: int) -> bool:
+    """Is a product of M rows with a float32 [N, K] quicker in parts on the tensor cores (`gemm_f32_parts`) than with `gemm_plain`?"""
+    yes = ctypes.c_int(0)
+    module("gemm_f32_parts").lib.gg_gemm_f32_parts_pays(int(M), int(N), int(K), ctypes.byref(yes))
+    return bool(yes.value)
 
 
 def f32_parts_scratch(M: int, N: int, K: int, tile: int = -1, shares: int = 0) -> int:

@@ -165,7 +165,7 @@ class Linear:
             self._fast = tcgen05_gemm.make_linear(self.weight, swiglu=swiglu, glu_act=glu_act)
         # the 32-bit path's products of many rows: on the tensor cores in parts (rows of W on 16-byte boundaries, which TMA asks for)
         self._parts = rt.fast and rt.dtype == torch.float32 and self.in_features % 4 == 0 and self.weight.data_ptr() % 16 == 0
-        self._parts_room: Dict[int, int] = {}        # rows -> bytes of scratch
+        self._parts_room: Dict[int, int] = {}        # rows -> bytes of scratch, 0 where the CUDA cores are quicker
         self.bias = rt.vector(bias) if bias is not None else None
         if self.bias is not None and (swiglu or self.bias.numel() != self.out_features):
             raise ValueError("Linear: a bias has one number per output and does not go with the fused SwiGLU form")
@@ -218,6 +218,8 @@ class Linear:
                 or x.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or x.stride(0) % 8 or x.data_ptr() % 16 or N <= 128):
             return False
         need = tcgen05_gemm.pair_scratch_elems(x.shape[0], N, width) if x.shape[0] > 128 else 0
+        if x.shape[0] > 128 and need == 0:
+            return False                 # (an unsplit product of many rows has its last epilogue in the open: the activation is longer there)
         scratch = ws.get("gemm_partial_tiles", (need,), torch.float32) if need else None
         tcgen05_gemm.gemm_tc_xielu(x, self.weight, out, ap, aq, out_scale, scratch=scratch, **kw)
         return True
@@ -251,10 +253,13 @@ class Linear:
             self._fast(x, out, accumulate, m, ws, **kw)
             return
         rows = x.shape[0] if m is None else m
-        if self._parts and ws is not None and rows >= K.F32_PARTS_ROWS and x.dtype == out.dtype == torch.float32:
+        room = 0
+        if self._parts and ws is not None and rows > 16 and x.dtype == out.dtype == torch.float32:
             room = self._parts_room.get(rows)
             if room is None:
-                room = self._parts_room[rows] = K.f32_parts_scratch(rows, self.out_features, self.in_features)
+                size = (rows, self.out_features, self.in_features)
+                room = self._parts_room[rows] = K.f32_parts_scratch(*size) if K.f32_parts_pays(*size) else 0
+        if room:
             K.gemm_f32_parts(x, self.weight, out, ws.get("product_parts", (room,), torch.uint8), accumulate, m, bias=self.bias)
         else:
             K.gemm_plain(x, self.weight, out, accumulate, m, bias=self.bias)
