@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const float* partial, int s
 }
 
 constexpr int TILES = 6;
-constexpr float PAYS_BESIDE = 12.0f;      // us: two launches more on the host, where a step of few rows is bound
+constexpr float PAYS_BESIDE = 8.0f, PAYS_FROM_FEW = 40.0f, PAYS_FROM_MANY = 24.0f;      // us: see gg_gemm_f32_parts_pays
 const int TILE_BN[TILES] = {32, 64, 96, 128, 160, 192};
 
 struct Plan {
@@ -399,9 +399,11 @@ GG_API gg_gemm_f32_parts_scratch(int M, int N, int K, int force_tile, int force_
 
 // Is a product of this size quicker in parts than on the CUDA cores?  On the GPU alone it is from 17 rows and K = 1,024 on (us, CUDA cores |
 // parts: 17 rows by 1,024 x 1,024 8.9 | 8.3, 2,048 x 2,048 20.8 | 13.5; 100 rows 13.2 | 12.1, 46.3 | 17.2; by 512 x 512 5.2 | 7.4), but it is
-// two or three launches instead of one, and a prompt of few rows is bound by the host's launches: 20 tokens, two layers of a
-// 1,024-wide model 297 -> 376 us with every product in parts.  So the CUDA cores' time, modelled, has to be PAYS_BESIDE longer.  Below
-// K = 256 the sums are no more exact than theirs either (K = 128: 1.1e-7 both).
+// two or three launches instead of one, and a step whose products are all short is bound by the host's launches: prompts of 18 and
+// 40 tokens through two layers 1,024 wide took 322 and 339 us instead of 297 with every product in parts.  So the CUDA cores'
+// time, modelled, has to be PAYS_BESIDE longer, and PAYS_FROM_FEW at least up to 99 rows (from 100 on the four products of a layer together
+// outlast its launches, so PAYS_FROM_MANY).  Below K = 256 the sums are no more exact than theirs
+// either (K = 128: 1.1e-7 both).
 GG_API gg_gemm_f32_parts_pays(int M, int N, int K, int* pays) {
     if (M <= 0 || N <= 0 || K <= 0 || pays == nullptr) return GG_ERR_ARG;
     *pays = 0;
@@ -417,7 +419,7 @@ GG_API gg_gemm_f32_parts_pays(int M, int N, int K, int* pays) {
     }
     float parts = 0.f;
     plan_for(M, N, K, -1, 0, &parts);
-    *pays = parts + PAYS_BESIDE < plain;
+    *pays = plain >= (M >= 100 ? PAYS_FROM_MANY : PAYS_FROM_FEW) && parts + PAYS_BESIDE < plain;
     return 0;
 }
 
