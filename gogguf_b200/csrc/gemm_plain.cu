@@ -1,7 +1,7 @@
 // Plain matrix product on the CUDA cores: out[M,N] (+)= x[M,K] * W[N,K]^T, float32 accumulate.
 //
-// This is the true 32-bit path of every projection (no tensor cores, no reduced
-// precision mode) and the plain twin the tensor-core kernels are checked against.
+// This is the 32-bit path of projections of few rows and of sizes that gemm_f32_parts.cu does not take or is not quicker for (no reduced
+// precision mode in either), and the plain twin the tensor-core kernels are checked against.
 // It also serves mixed operands (bfloat16 activations with a matrix that is stored
 // in 32-bit and stays so).  The reference's counterpart is the one-thread-per-row matmul_vec PTX
 // kernel (pkg/gpu/cuda/ptx.go:67-129) and ops.MatMulVecInto (pkg/ops/ops.go:30-53).
