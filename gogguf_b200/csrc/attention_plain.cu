@@ -18,14 +18,16 @@
 // exponential is known.  So a warp takes eight neighbouring keys at a time (eight rows in flight, eight reductions side
 // by side, one running maximum and one rescaling for the eight), and eight warps share a token's keys: a decode step has
 // few (token, head) pairs.  Where even so most SMs would have nothing to do, up to eight blocks share a token's keys: they form a
-// cluster, and each leaves its sums in the shared memory of the first, which adds them in the order of the shares.  Keys are given
-// out by position and the number of shares alone, and that number follows from the step's (token, head) pairs and the table's width.
+// cluster, and each leaves its sums in the shared memory of the first, which adds them in the order of the shares.  A token's keys are
+// cut by its position and the most shares of the step, which follow from the heads and the number of tokens rounded up to a power of two: a
+// captured step's padding rows and wider tables change nothing.
 #include <type_traits>
 #include "common.cuh"
 
 #define ATT_WARPS 8
 #define ATT_KEYS 8
 #define ATT_MAXD 256
+#define ATT_SHARE_KEYS 128
 #define ATT_SHARES 8                     // at most (the warps' factors and the shares' are kept in one array)
 
 template <typename T> __device__ __forceinline__ float4 att_load4(const T* p);
@@ -48,7 +50,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_plain_kernel(
     const int* __restrict__ positions, const int* __restrict__ seq_of_token,
     const int* __restrict__ page_table, int max_pages, int page_size,
     int nq, int nkv, int d, int dv, float scale, int window, int chunk, const float* __restrict__ sink, float out_scale,
-    const T* gate, long long ldg, const PageBounds pb) {
+    const T* gate, long long ldg, int most_shares, const PageBounds pb) {
     pdl_launch();
     pdl_wait();
     extern __shared__ __align__(16) float sm[];
@@ -56,7 +58,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_plain_kernel(
     float* accs = sm + d;                 // [ATT_WARPS][dv]
     float* ml = accs + ATT_WARPS * dv;    // [ATT_WARPS][2]
     float* got = ml + 2 * ATT_WARPS;      // SHARED: the shares' sums, maxima and weights, [shares][dv + 2], in the first block
-    const int share = SHARED ? (int)blockIdx.z : 0, shares = SHARED ? (int)gridDim.z : 1;
+    const int share = SHARED ? (int)blockIdx.z : 0, launched = SHARED ? (int)gridDim.z : 1;
     const int t = blockIdx.x, h = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     T* o = out + ((size_t)t * nq + h) * dv;
@@ -92,7 +94,9 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_plain_kernel(
             q4[c] = in_k[c] ? *reinterpret_cast<const float4*>(qs + 128 * c + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
-    for (int j0 = lo + (share * ATT_WARPS + warp) * ATT_KEYS; j0 <= pos; j0 += shares * ATT_WARPS * ATT_KEYS) {
+    // (a share of at least ATT_SHARE_KEYS keys; the blocks beyond a token's shares have none)
+    const int shares = SHARED ? min(most_shares, 1 + (pos - lo) / ATT_SHARE_KEYS) : 1;
+    for (int j0 = share < shares ? lo + (share * ATT_WARPS + warp) * ATT_KEYS : pos + 1; j0 <= pos; j0 += shares * ATT_WARPS * ATT_KEYS) {
         size_t base[ATT_KEYS];
         float dot[ATT_KEYS];
 #pragma unroll
@@ -204,9 +208,9 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_plain_kernel(
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (share > 0) return;
         M = sink != nullptr ? sink[h] : -INFINITY;
-        for (int r = 0; r < shares; ++r) M = fmaxf(M, got[r * (dv + 2) + dv]);
+        for (int r = 0; r < launched; ++r) M = fmaxf(M, got[r * (dv + 2) + dv]);
         L = sink != nullptr ? expf(sink[h] - M) : 0.f;
-        for (int r = 0; r < shares; ++r) {
+        for (int r = 0; r < launched; ++r) {
             const float mr = got[r * (dv + 2) + dv];
             f[r] = mr == -INFINITY ? 0.f : expf(mr - M);
             L += got[r * (dv + 2) + dv + 1] * f[r];
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_plain_kernel(
         const float inv = out_scale / L;
         for (int i = threadIdx.x; i < dv; i += blockDim.x) {
             float s = 0.f;
-            for (int r = 0; r < shares; ++r) s += got[r * (dv + 2) + i] * f[r];
+            for (int r = 0; r < launched; ++r) s += got[r * (dv + 2) + i] * f[r];
             s *= inv;
             if (gate != nullptr) s /= 1.0f + expf(-to_f<T>(gate[(size_t)t * ldg + (size_t)h * dv + i]));
             o[i] = from_f<T>(s);
@@ -468,11 +472,13 @@ GG_API gg_attention_plain(const void* q, const void* k_pool, const void* v_pool,
                          (const float*)k_pool, (const float*)v_pool, (float*)out, positions, seq_of_token, cu_seqlens, n_seqs, page_table, max_pages,
                          page_size, nq, nkv, d, dv, scale, window, chunk, sink, out_scale, (const float*)gate, ldg, PageBounds{n_pages, status});
     }
-    // Shares of a token's keys: as many as keep the grid within three blocks an SM, of no fewer than 64 keys of the widest context that
-    // the tables have room for.
-    const long long pairs = (long long)ntok * nq, widest = (long long)max_pages * page_size;
-    int shares = 1;
-    while (shares < ATT_SHARES && pairs * shares * 2 <= 148 * 3 && widest >= 128LL * shares) shares *= 2;
+    // The most shares of a token's keys: as many as keep the grid within three blocks an SM; launched are no more than a token of the widest
+    // context that the tables have room for would take.
+    long long tokens = 1;
+    while (tokens < ntok) tokens *= 2;
+    int most = 1, shares = 1;
+    while (most < ATT_SHARES && tokens * nq * most * 2 <= 148 * 3) most *= 2;
+    while (shares < most && 1 + ((long long)max_pages * page_size - 1) / ATT_SHARE_KEYS > shares) shares *= 2;
     size_t smem = ((size_t)d + (size_t)ATT_WARPS * dv + 2 * ATT_WARPS) * sizeof(float);
     if (shares > 1) smem += (size_t)shares * (dv + 2) * sizeof(float);
     dim3 grid(ntok, nq, shares);
@@ -481,7 +487,7 @@ GG_API gg_attention_plain(const void* q, const void* k_pool, const void* v_pool,
     const int nv = (d % 4 == 0 && dv % 4 == 0 && wide <= 256 && (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0) ? (wide + 127) / 128 : 0;
 #define GG_ATT_AS(NV, SH) return gg_launch(attention_plain_kernel<T, NV, SH>, grid, dim3(ATT_WARPS * 32), smem, stream, shares, \
             (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, positions, seq_of_token, page_table, \
-            max_pages, page_size, nq, nkv, d, dv, scale, window, chunk, sink, out_scale, (const T*)gate, ldg, PageBounds{n_pages, status})
+            max_pages, page_size, nq, nkv, d, dv, scale, window, chunk, sink, out_scale, (const T*)gate, ldg, most, PageBounds{n_pages, status})
 #define GG_ATT(NV) { if (shares > 1) GG_ATT_AS(NV, true); GG_ATT_AS(NV, false); }
     GG_DISPATCH_DTYPE(dtype, T,
         if (nv == 1) GG_ATT(1)
