@@ -261,8 +261,8 @@ __global__ void __launch_bounds__(128) attention_plain_tile_kernel(
     const float* q, const float* k_pool, const float* v_pool, float* __restrict__ out, const int* __restrict__ positions,
     const int* __restrict__ seq_of_token, const int* __restrict__ cu_seqlens, int n_seqs, const int* __restrict__ page_table, int max_pages,
     int page_size, int nq, int nkv, int d, int dv, float scale, int window, int chunk, const float* __restrict__ sink, float out_scale,
-    const float* gate, long long ldg, const PageBounds pb) {
-    pdl_launch();
+    const float* gate, long long ldg, int early_release, const PageBounds pb) {
+    if (early_release) pdl_launch();              // (the grid is resident as a whole; the note on dependent launches in common.cuh)
     extern __shared__ __align__(16) float sm[];
     const int LD = d + 4, LV = dv + 4, G = nq / nkv, g = blockIdx.y;
     float* qs = sm;                               // [32][LD]
@@ -470,7 +470,8 @@ GG_API gg_attention_plain(const void* q, const void* k_pool, const void* v_pool,
         if (tiles > 0x7fffffffLL) return GG_ERR_ARG;
         return gg_launch(attention_plain_tile_kernel, dim3((unsigned)tiles, nkv), dim3(128), tile_smem, stream, 1, (const float*)q,
                          (const float*)k_pool, (const float*)v_pool, (float*)out, positions, seq_of_token, cu_seqlens, n_seqs, page_table, max_pages,
-                         page_size, nq, nkv, d, dv, scale, window, chunk, sink, out_scale, (const float*)gate, ldg, PageBounds{n_pages, status});
+                         page_size, nq, nkv, d, dv, scale, window, chunk, sink, out_scale, (const float*)gate, ldg,
+                         tiles * nkv <= resident ? 1 : 0, PageBounds{n_pages, status});
     }
     // The most shares of a token's keys: as many as keep the grid within three blocks an SM; launched are no more than a token of the widest
     // context that the tables have room for would take.
