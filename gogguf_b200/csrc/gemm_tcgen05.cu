@@ -435,14 +435,6 @@ __device__ __forceinline__ void epilogue_row_256(uint32_t taddr, int gi, int tn,
             for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * sc);
         }
         if (nio.bias != nullptr) add_bias<16>(reinterpret_cast<float*>(r), nio.bias, tn * BN + c0, N);
-        if (nio.xielu) {
-#pragma unroll
-            for (int j = 0; j < 16; j += 4) {
-                const float4 v = xielu_value(make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3])),
-                                             nio.x_p, nio.x_q, nio.x_scale);
-                r[j] = __float_as_uint(v.x); r[j + 1] = __float_as_uint(v.y); r[j + 2] = __float_as_uint(v.z); r[j + 3] = __float_as_uint(v.w);
-            }
-        }
         store_row_chunk16(r, gi, tn * BN + c0, N, out, out_mode, ldo, nio, ss);
     }
 }
@@ -1546,7 +1538,7 @@ __global__ void __launch_bounds__(256) gemm_splitk_finish_kernel(const float* pa
         qkv_token_finish(acc, gj, tile_a, lane, qio, qt);
         return;
     }
-    finish_token_block<true>(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio);
+    finish_token_block(acc, gj, tile_a, lane, out, out_mode, ldo, N, nio);
 }
 
 // Work items of the CTA-pair form for a product whose tiles do not fill the 74 pairs well.  `splits` > 1: the K range
@@ -1823,13 +1815,14 @@ GG_API gg_gemm_tc_norm(const void* x, const void* w, void* out, int out_mode, in
 }
 
 // out[M, N] (bfloat16) = out_scale * xIELU(x w^T) with the activation's two parameters, taken of the float32 sums; the input side as in
-// gg_gemm_tc_norm.  (As a kernel of its own the activation reads and writes the rows once more: decode steps of a 2,048-wide
-// model with 8,192 inner columns 3 us a layer, prompts of 1,400 tokens 15.)
+// gg_gemm_tc_norm.  Up to 128 tokens (as a kernel of its own the activation is 3 us a layer more in decode steps of a 2,048-wide model
+// with 8,192 inner columns); a product of more tokens has its last epilogue in the open, where the exponentials are longer than the
+// kernel of their own (prompts of 333 to 700 tokens through four layers 1 to 4 % slower).
 GG_API gg_gemm_tc_xielu(const void* x, const void* w, void* out, int M, int N, int K, long long ldx, long long ldo, const float* in_ssq,
                         int in_parts, float eps, float ap, float aq, float out_scale, float* scratch, long long scratch_elems, int* status,
                         cudaStream_t stream) {
     if (in_ssq != nullptr && (in_parts != (K + 127) / 128 || !(eps > 0.f))) return GG_ERR_ARG;
-    if (M > 128 && N <= 128) return GG_ERR_ARG;          // (the form of few outputs has no such epilogue)
+    if (M > 128) return GG_ERR_ARG;                      // (see above)
     NormIO nio = {};
     nio.in_ssq = in_ssq; nio.in_parts = in_parts; nio.in_inv_k = K > 0 ? 1.0f / (float)K : 0.f; nio.eps = eps;
     nio.xielu = 1; nio.x_p = ap; nio.x_q = aq; nio.x_scale = out_scale;

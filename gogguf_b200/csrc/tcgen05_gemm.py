@@ -212,10 +212,9 @@ def gemm_tc_qkv_rope(x: torch.Tensor, w: torch.Tensor, m: int, q_out: torch.Tens
 
 
 def gemm_tc_xielu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ap: float, aq: float, out_scale: float = 1.0,
-                  m: Optional[int] = None, in_ssq: Optional[torch.Tensor] = None, eps: float = 0.0,
-                  scratch: Optional[torch.Tensor] = None) -> None:
+                  m: Optional[int] = None, in_ssq: Optional[torch.Tensor] = None, eps: float = 0.0) -> None:
     """out (bfloat16) = out_scale * xIELU(x @ w^T) with the activation in the product's epilogue (csrc/gemm_tcgen05.cu, gg_gemm_tc_xielu);
-    in_ssq, eps and scratch as in `gemm_tc_norm`."""
+    up to 128 rows.  in_ssq and eps as in `gemm_tc_norm`."""
     N, K = w.shape
     M = x.shape[0] if m is None else m
     if not (x.dtype == w.dtype == out.dtype == torch.bfloat16):
@@ -230,7 +229,7 @@ def gemm_tc_xielu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ap: float
     kernel("gemm_tcgen05", "gg_gemm_tc_xielu")(
         x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), out.stride(0),
         in_ssq.data_ptr() if in_ssq is not None else 0, in_parts, float(eps), float(ap), float(aq), float(out_scale),
-        scratch.data_ptr() if scratch is not None else 0, scratch.numel() if scratch is not None else 0,
+        0, 0,
         status_word(x.device).data_ptr(), stream_ptr())
 
 

@@ -165,7 +165,6 @@ class Linear:
             self._fast = tcgen05_gemm.make_linear(self.weight, swiglu=swiglu, glu_act=glu_act)
         # the 32-bit path's products of many rows: on the tensor cores in parts (rows of W on 16-byte boundaries, which TMA asks for)
         self._parts = rt.fast and rt.dtype == torch.float32 and self.in_features % 4 == 0 and self.weight.data_ptr() % 16 == 0
-        self._xielu_room: Dict[int, int] = {}        # rows -> floats of scratch of the product with an activation behind it
         self._parts_room: Dict[int, int] = {}        # rows -> bytes of scratch, 0 where the CUDA cores are quicker
         self.bias = rt.vector(bias) if bias is not None else None
         if self.bias is not None and (swiglu or self.bias.numel() != self.out_features):
@@ -207,26 +206,17 @@ class Linear:
             x = x.xhat
         tcgen05_gemm.gemm_tc_qkv_rope(x, self.weight, m, **outputs)
 
-    def xielu(self, x, out: torch.Tensor, ap: float, aq: float, out_scale: float, ws: Workspace) -> bool:
+    def xielu(self, x, out: torch.Tensor, ap: float, aq: float, out_scale: float) -> bool:
         """out = out_scale * xIELU(y) in the product's epilogue; False (and nothing done) where this product has no such form."""
         kw = {}
         if self.folded_eps is not None and isinstance(x, RowStats):
             kw.update(in_ssq=x.ssq, eps=self.folded_eps)
             x = x.xhat
-        N, width = self.weight.shape
         if (self._fast is None or self.swiglu or self.bias is not None or not isinstance(x, torch.Tensor) or (self.folded_eps is not None) != bool(kw)
-                or x.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or x.stride(0) % 8 or x.data_ptr() % 16 or N <= 128):
+                or x.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or x.stride(0) % 8 or x.data_ptr() % 16 or x.shape[0] > 128):
             return False
         from ..csrc import tcgen05_gemm
-        rows, need = x.shape[0], 0
-        if rows > 128:
-            need = self._xielu_room.get(rows)
-            if need is None:
-                need = self._xielu_room[rows] = tcgen05_gemm.pair_scratch_elems(rows, N, width)
-            if need == 0:
-                return False             # (an unsplit product of many rows has its last epilogue in the open: the activation is longer there)
-        scratch = ws.get("gemm_partial_tiles", (need,), torch.float32) if need else None
-        tcgen05_gemm.gemm_tc_xielu(x, self.weight, out, ap, aq, out_scale, scratch=scratch, **kw)
+        tcgen05_gemm.gemm_tc_xielu(x, self.weight, out, ap, aq, out_scale, **kw)
         return True
 
     def __call__(self, x, out: torch.Tensor, accumulate: bool = False, m: Optional[int] = None,

@@ -82,7 +82,7 @@ class XieluMLP:
     def forward(self, h: torch.Tensor, residual: torch.Tensor, ctx: StepContext) -> None:
         T = ctx.n_tokens
         z = ctx.ws.get("ffn_act", (T, self.inter), self.rt.dtype)
-        if not self.up.xielu(h, z, self.ap, self.aq, self.out_scale, ctx.ws):
+        if not self.up.xielu(h, z, self.ap, self.aq, self.out_scale):
             self.up(h, z, ws=ctx.ws)
             K.xielu(z, z, self.ap, self.aq, self.out_scale)
         self.down(z, residual, accumulate=True, ws=ctx.ws)
