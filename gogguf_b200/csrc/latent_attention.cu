@@ -410,6 +410,7 @@ __global__ void __launch_bounds__(128) headwise_mma_kernel(const bf16* x, long l
 // take 16 of the tile's 64 outputs each.  With MERGE the rows of x are made here from the attention's shares of the keys
 // (part_o [row][splits][k], part_ml [row][splits][2], row = token * H + head; see latent_combine_kernel, which then does not
 // run): weights by a warp a token, the sum over the shares in their order, rounded to bfloat16 as that kernel's output is.
+// 16 heads, 64 columns to 256 outputs: 4 tokens 2.5 us in headwise_mma_kernel's tiles, 1.7 here; 16 tokens 2.7 | 1.8.
 #define HF_M 16
 #define HF_K 256
 #define HF_LD (HF_K + 8)

@@ -178,7 +178,8 @@ __global__ void __launch_bounds__(32) moe_route_kernel(const float* z, int E, in
 }
 
 // Logits and choice in one kernel for few tokens and up to 32 experts (decode steps): a block a token, a warp an expert, the sums those of
-// moe_router_logits_kernel; the first warp then chooses.  The router's first columns are asked for before the wait.
+// moe_router_logits_kernel; the first warp then chooses.  The router's first columns are asked for before the wait.  The two
+// kernels | this, 16 experts, rows of 2,048: 8 tokens 4.6 | 3.6 us, 64 4.8 | 3.9, 148 (a block an SM) 6.7 | 3.9.
 #define ROUTE_AHEAD 8
 template <typename TX, typename TW>
 __global__ void __launch_bounds__(1024) moe_logits_route_kernel(const TX* h, const TW* __restrict__ wr, float* z, int W, int E, int top, int softmax,
