@@ -213,7 +213,8 @@ class Linear:
             kw.update(in_ssq=x.ssq, eps=self.folded_eps)
             x = x.xhat
         if (self._fast is None or self.swiglu or self.bias is not None or not isinstance(x, torch.Tensor) or (self.folded_eps is not None) != bool(kw)
-                or x.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or x.stride(0) % 8 or x.data_ptr() % 16 or x.shape[0] > 128):
+                or x.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or x.stride(0) % 8 or x.data_ptr() % 16
+                or x.shape[0] > 128 or self.weight.shape[0] <= 128):
             return False
         from ..csrc import tcgen05_gemm
         tcgen05_gemm.gemm_tc_xielu(x, self.weight, out, ap, aq, out_scale, **kw)

@@ -6,7 +6,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M", [1, 16, 17, 61, 128])
-@pytest.mark.parametrize("N,K_", [(100, 72), (136, 72), (200, 264), (2048, 1024), (8192, 2048)])
+@pytest.mark.parametrize("N,K_", [(136, 72), (200, 264), (2048, 1024), (8192, 2048)])
 @pytest.mark.parametrize("folded", [False, True])
 def test_activation_of_the_sums(M, N, K_, folded):
     from gogguf_b200.csrc import tcgen05_gemm as G
