@@ -198,11 +198,11 @@ def qkv_prep(qkv: torch.Tensor, q_out: torch.Tensor, q_weight: Optional[torch.Te
         float(coef), float(every), _p(status_word(qkv.device)), _stream())
 
 
-def rmsnorm_add_norm_takes(x: torch.Tensor, y: torch.Tensor, out: torch.Tensor) -> bool:
-    """Does `rmsnorm_add_norm` take these rows?"""
+def rmsnorm_add_norm_takes(x: torch.Tensor, y: torch.Tensor, out: torch.Tensor, *weights: torch.Tensor) -> bool:
+    """Does `rmsnorm_add_norm` take these rows and the norms' weights?  (A weight may be a view anywhere in a packed tensor.)"""
     H = x.shape[-1]
     return (H % 4 == 0 and H <= 8192 and x.is_contiguous() and y.is_contiguous() and out.is_contiguous()
-            and (x.data_ptr() | y.data_ptr() | out.data_ptr()) % 16 == 0)
+            and all(t.data_ptr() % 16 == 0 for t in (x, y, out) + weights))
 
 
 def rmsnorm_add_norm(x: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: float, next_weight: torch.Tensor, next_eps: float,

@@ -201,7 +201,7 @@ class SandwichNormBlock:
                 stats.fresh = False
             if ahead is not None and g is None:
                 rows = ctx.ws.get("block_normed", tuple(x.shape), self.rt.dtype)
-                if K.rmsnorm_add_norm_takes(x, y, rows):
+                if K.rmsnorm_add_norm_takes(x, y, rows, post.weight, ahead.weight):
                     K.rmsnorm_add_norm(x, y, post.weight, post.eps, ahead.weight, ahead.eps, rows, zero_y=True)
                     ctx.shared[self.ZEROED] = y.data_ptr()
                     return rows
