@@ -1,17 +1,22 @@
 // 32-bit matrix product of many rows on the tensor cores: out[M,N] (+)= x[M,K] * W[N,K]^T (+ bias), all float32.
 //
-// A float32 number is the sum of three bfloat16 numbers without a rest: its upper 16 bits (8 of the 24 of its significand), the upper
-// 16 bits of what that leaves, and what is left then.  So a product of two is nine products of parts, of which the six down to
-// 2^-16 of the first are taken (the three left out are below 2^-23 of it together, under a rounding of the 32-bit product), each exact in
-// the tensor core's multiplier.  What the tensor core does not do is round: it cuts off what an addition shifts out, and over a long
-// contraction that drift would be larger than the rounding of the CUDA cores' sums (2.1e-6 against 0.8e-6 at K = 2,048).  So the
-// accumulator in tensor memory holds 32 columns of K at a time, the small products first and the two large ones (16 columns an
-// instruction) last, and every 32 columns' sum is added in registers, rounded to nearest.  Relative error against 64 bits, normal
-// operands: 1.3e-7 to 2.0e-7 at K of 1,800 to 5,376, where gemm_plain.cu has 3.8e-7 to 6.6e-7.
+// A float32 number is the sum of three bfloat16 numbers without a rest: the nearest one, the one nearest to what that leaves, and
+// what is left then (its 24 bits are 8, 8 and 8 with a sign each).  So a product of two is nine products of parts, of which the six down
+// to 2^-16 of the first are taken.  The second part is at most 2^-8 of a number and the third at most 2^-17, so the three left out
+// are below 2^-24 of the product together, the rounding of a 32-bit product, and have no sign of their own (4 million products of
+// normal numbers: 0.87 x 2^-24 at most, 0.10 in the mean square, where a rounding has 0.42).  Each product taken is exact in the
+// tensor core's multiplier.  (Parts by rounding, and sums kept outside the tensor core: Henry, Tang and Heinecke 2019, Ootomo and
+// Yokota 2022.)  What the tensor core does not do is round: it cuts off what an addition shifts out, and over a long contraction
+// that drift would be larger than the rounding of the CUDA cores' sums (2.1e-6 against 0.8e-6 at K = 2,048).  So the accumulator
+// in tensor memory holds 32 columns of K at a time, the small products first and the two large ones (16 columns an instruction)
+// last, and every 32 columns' sum is added in registers, rounded to nearest.
+// Relative error against 64 bits, gemm_plain.cu | here (1e-7), K = 256, 2,048, 5,376: normal operands 1.5 | 0.75, 4.0 | 1.0, 6.5 | 1.1; of one
+// sign 0.72 | 0.67, 1.8 | 0.84, 2.6 | 0.78; one channel a hundred times the others 1.7 | 0.70, 4.6 | 1.2, 7.2 | 1.2.  A row with one term alone
+// is what the CUDA cores round once and the tensor core cuts off: 0.25 | 0.45, at most 2.3 x 2^-24 of the term.
 //
 // Bounds: six products at the dense bfloat16 rate are 280 TFLOP/s of 32-bit products, where packed multiply-adds on the CUDA cores
-// have 74 (and reach 41, bound by reads of shared memory).  Measured, 450 rows (us, gemm_plain.cu | this): 4,096 x 2,048 227 | 57,
-// 10,752 x 2,048 547 | 118, 2,048 x 5,376 288 | 61; 17 rows: 23 | 15, 69 | 40, 58 | 26.
+// have 74 (and reach 41, bound by reads of shared memory).  Measured, 450 rows (us, gemm_plain.cu | this): 4,096 x 2,048 226 | 51,
+// 10,752 x 2,048 547 | 113, 2,048 x 5,376 287 | 59; 17 rows: 23 | 19, 68 | 40, 52 | 24.
 //
 // A CTA owns 128 rows of W (the instruction's M) and BN rows of x, over the whole of K or a share of it, and has
 //   warp 0      TMA: W as float32 (two boxes of 128 x 32 a stage), the three parts of x (BN x 64 each; split_rows_kernel makes them);
@@ -23,8 +28,9 @@
 // and finish_kernel adds them in the order of K.
 //
 // Infinities and NaN: parts of an infinity are an infinity and NaN, and a zero part times an infinity is NaN, so a product of parts is
-// not finite wherever the 32-bit product is not; every sum that is not finite is made again from the operands, by multiply-adds in the
-// order of k, and is what those give.  Parts below 2^-133 are cut off, an absolute error of that size per operand.
+// not finite wherever the 32-bit product is not; nor is it where an operand is so large that its first part rounds to an
+// infinity.  Every sum that is not finite is made again from the operands, by multiply-adds in the order of k, and is what
+// those give.  Parts below 2^-133 are cut off, an absolute error of that size per operand.
 #include "common.cuh"
 #include "tma_util.cuh"
 
@@ -51,13 +57,20 @@ __device__ __noinline__ float plain_dot(const float* x, const float* w, int k0, 
     return s;
 }
 
-// a, b -> their three parts, two neighbours along k in a word
+// a, b -> their three parts, two neighbours along k in a word.  The third part is what is left: its 8 bits stand in the upper half of a
+// float32 already.
+__device__ __forceinline__ uint32_t nearest_pair(float a, float b) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&t);
+}
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-    p0 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
-    const float ra = a - __uint_as_float(__float_as_uint(a) & 0xffff0000u), rb = b - __uint_as_float(__float_as_uint(b) & 0xffff0000u);
-    p1 = __byte_perm(__float_as_uint(ra), __float_as_uint(rb), 0x7632);
-    const float sa = ra - __uint_as_float(__float_as_uint(ra) & 0xffff0000u), sb = rb - __uint_as_float(__float_as_uint(rb) & 0xffff0000u);
-    p2 = __byte_perm(__float_as_uint(sa), __float_as_uint(sb), 0x7632);
+    p0 = nearest_pair(a, b);
+    a -= __uint_as_float(p0 << 16);
+    b -= __uint_as_float(p0 & 0xffff0000u);
+    p1 = nearest_pair(a, b);
+    a -= __uint_as_float(p1 << 16);
+    b -= __uint_as_float(p1 & 0xffff0000u);
+    p2 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
 // parts[p][m][k], rows of ld elements (K rounded up to 8; what lies between is not read).  Four columns a thread.

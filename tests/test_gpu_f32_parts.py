@@ -36,7 +36,7 @@ def test_tiles_and_shares(tile, N, K_, shares):
         parts(x, w, room[:M, :N], tile, shares, m=M)
         out = room[:M, :N]
         want = x[:M].double() @ w.double().T
-        # (the parts left out are 2^-23 of a product, a sum of 32 columns is cut off twice at 2^-23, the sums of those are rounded)
+        # (the parts left out are 2^-24 of a product, a sum of 32 columns is cut off twice at 2^-23, the sums of those are rounded)
         bound = (3 + (K_ / 32) ** 0.5 / 2) * 2.0 ** -23
         assert (out.double() - want).norm() <= bound * (x[:M].double().abs() @ w.double().abs().T).norm()
         assert (room[:, N:] == -7.0).all() and (room[M:] == -7.0).all()
@@ -57,6 +57,40 @@ def test_error_is_no_larger_than_the_multiply_adds(M, N, K_):
         plain = torch.empty(M, N, device="cuda")
         K().gemm_plain(x, w, plain)
         assert off(parts(x, w, torch.empty(M, N, device="cuda")), want) <= off(plain, want)
+
+
+def low_bits(g, *shape):
+    """Numbers whose significands lie just below 1 + 2^-7, of either sign and over some powers of two: cut off to 8 bits they would leave
+    2^-7 of themselves, and that 2^-8 of itself."""
+    n = 1 + 2.0 ** -7 - 2.0 ** -23 * torch.randint(1, 64, shape, device="cuda", generator=g)
+    return n * torch.exp2(torch.randint(-9, 9, shape, device="cuda", generator=g).float()) * (1 - 2 * torch.randint(0, 2, shape, device="cuda", generator=g))
+
+
+@pytest.mark.parametrize("tile,shares", [(0, 1), (2, 3), (5, 1)])
+@pytest.mark.parametrize("draw", ["low bits", "any"])
+def test_a_term_alone_keeps_its_bits(draw, tile, shares):
+    """A row of x with one number in it: the output is that number's product."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    M, N, K_ = 200, 260, 448
+    some = (lambda *s: low_bits(g, *s)) if draw == "low bits" else (lambda *s: torch.randn(*s, device="cuda", generator=g))
+    at = torch.randint(0, K_, (M, 1), device="cuda", generator=g)
+    x, w = torch.zeros(M, K_, device="cuda").scatter_(1, at, some(M, 1)), some(N, K_)
+    want = x.double() @ w.double().T
+    out = parts(x, w, torch.empty(M, N, device="cuda"), tile, shares)
+    # what is left out of a product is 2^-24 of it, the two sums with the large parts are cut off at 2^-23 of it at most, of which one adds
+    # nothing; the sums before them are 2^-7 of it and are cut off ten times
+    assert ((out.double() - want).abs() <= (1 + 2 + 10 * 2.0 ** -6) * 2.0 ** -24 * want.abs()).all()
+
+
+@pytest.mark.parametrize("K_", [512, 2048])
+def test_terms_of_one_sign(K_):
+    """Equal terms, whose losses add up if they have a sign."""
+    c = 1 + 2.0 ** -7 - 2.0 ** -23
+    x, w = torch.full((96, K_), c, device="cuda"), torch.full((384, K_), c, device="cuda")
+    want = x.double() @ w.double().T
+    e = (parts(x, w, torch.empty(96, 384, device="cuda")).double() - want).abs() / want
+    # 2^-24 left out, a sum of 32 columns cut off twice at 2^-23 of it, and the rounding of K / 32 partial sums, none above 2^-24 of the last
+    assert float(e.max()) <= (1 + 4) * 2.0 ** -24 + K_ / 64 * 2.0 ** -24
 
 
 @pytest.mark.parametrize("shares", [1, 3])
