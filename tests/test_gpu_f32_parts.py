@@ -111,6 +111,28 @@ def test_infinities_and_nan(shares):
     assert torch.allclose(out[fin], plain[fin], rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("o", [0, 1])
+@pytest.mark.parametrize("tile", range(6))
+def test_rows_that_are_not_finite(tile, o):
+    """Whole rows of them, and operands beyond the largest bfloat16 number whose products are finite; rows of x on and off 16-byte boundaries."""
+    g = torch.Generator(device="cuda").manual_seed(tile)
+    M, N, K_ = 230, 140, 260
+    x, w = torch.randn(M, K_ + 4, device="cuda", generator=g)[:, o:o + K_], torch.randn(N, K_, device="cuda", generator=g) * 0.01
+    x[:, 100] = 3.4e38                                                     # rounds to an infinity in 8 bits
+    w[:, 100] = torch.randn(N, device="cuda", generator=g) * 1e-38
+    x[5:90:3, 7], x[6:200:7, 9] = float("nan"), float("inf")
+    w[17, 9], w[18, 9], res = 0.0, -1.0, torch.randn(M, N, device="cuda", generator=g)
+    bias = torch.randn(N, device="cuda", generator=g)
+    out, plain = parts(x, w, res.clone(), tile, accumulate=True, bias=bias), res.clone()
+    K().gemm_plain(x, w, plain, accumulate=True, bias=bias)
+    assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out.isinf(), plain.isinf())
+    assert torch.equal(out[out.isinf()], plain[plain.isinf()])
+    fin = plain.isfinite()
+    want = (x.double() @ w.double().T + bias + res)[fin]
+    mag = (x.double().abs() @ w.double().abs().T + bias.abs() + res.abs())[fin]
+    assert fin.any() and ((out[fin].double() - want).abs() <= (K_ + 2) * 2.0 ** -24 * mag).all()     # (a chain of K multiply-adds)
+
+
 def test_refusals():
     x, w, out = torch.zeros(4, 8, device="cuda"), torch.zeros(16, 8, device="cuda"), torch.zeros(4, 16, device="cuda")
     from gogguf_b200.csrc.build import KernelError
