@@ -31,6 +31,9 @@
 // not finite wherever the 32-bit product is not; nor is it where an operand is so large that its first part rounds to an
 // infinity.  Every sum that is not finite is made again from the operands, by multiply-adds, and is what those give (plain_sums).  Parts
 // below 2^-133 are cut off, an absolute error of that size per operand.
+//
+// Rows of x are taken in slabs, so that their parts fill 256 MB of scratch at most.
+#include <initializer_list>
 #include "common.cuh"
 #include "tma_util.cuh"
 
@@ -473,11 +476,26 @@ int launch_tile(const float* x, long long ldx, const float* w, float* out, long 
 
 static int parts_ld(int K) { return (K + 7) / 8 * 8; }
 
-// Bytes of scratch that gg_gemm_f32_parts needs: the rows' parts, then the shares' sums.
+// Rows of x that are multiplied at a time: their parts are one and a half times x, so what they take is bounded by about 256 MB
+// (a multiple of every tile's rows, 1,920 of them at least: 21 columns of tiles and more).
+static int slab_rows(int K) {
+    const long long rows = (256LL << 20) / (6LL * parts_ld(K)) / 1920 * 1920;
+    return rows < 1920 ? 1920 : rows > 0x3fffffff ? 0x3fffffff / 1920 * 1920 : (int)rows;
+}
+
+static long long parts_bytes(int M, int K) { return (3LL * M * parts_ld(K) * 2 + 255) / 256 * 256; }
+
+// Bytes of scratch that gg_gemm_f32_parts needs: the parts of a slab's rows, then the shares' sums.
 GG_API gg_gemm_f32_parts_scratch(int M, int N, int K, int force_tile, int force_shares, long long* bytes) {
     if (M <= 0 || N <= 0 || K <= 0 || bytes == nullptr) return GG_ERR_ARG;
-    const Plan p = plan_for(M, N, K, force_tile, force_shares);
-    *bytes = ((3LL * M * parts_ld(K) * 2 + 255) / 256) * 256 + (p.shares > 1 ? (long long)p.shares * M * N * 4 : 0);
+    const int slab = slab_rows(K);
+    *bytes = 0;
+    for (int m : {M < slab ? M : slab, M % slab}) {                  // (the last slab may be cut into shares where the others are not)
+        if (m == 0) continue;
+        const Plan p = plan_for(m, N, K, force_tile, force_shares);
+        const long long need = parts_bytes(m, K) + (p.shares > 1 ? (long long)p.shares * m * N * 4 : 0);
+        if (need > *bytes) *bytes = need;
+    }
     return 0;
 }
 
@@ -516,33 +534,39 @@ GG_API gg_gemm_f32_parts(const float* x, const float* w, float* out, int accumul
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 4 != 0 || ldx < K || ldo < N || ((uintptr_t)w & 15) != 0 || scratch == nullptr || ((uintptr_t)scratch & 255) != 0)
         return GG_ERR_ARG;
-    if (force_tile >= TILES || (long long)M * 3 > 0x7fffffffLL) return GG_ERR_ARG;
+    if (force_tile >= TILES) return GG_ERR_ARG;
     long long need = 0;
     gg_gemm_f32_parts_scratch(M, N, K, force_tile, force_shares, &need);
     if (scratch_bytes < need) return GG_ERR_ARG;
-    const Plan plan = plan_for(M, N, K, force_tile, force_shares);
-    const int ld = parts_ld(K);
+    const int ld = parts_ld(K), slab = slab_rows(K);
     bf16* parts = (bf16*)scratch;
-    float* partial = (float*)((char*)scratch + ((3LL * M * ld * 2 + 255) / 256) * 256);
-    const long long quads = (long long)M * (K / 4);
-    const int blocks = (int)((quads + 255) / 256 < 148 * 8 ? (quads + 255) / 256 : 148 * 8);
-    int rc = gg_launch(split_rows_kernel, dim3(blocks), dim3(256), 0, stream, 1, x, ldx, parts, M, K, ld,
-                       (int)(ldx % 4 == 0 && ((uintptr_t)x & 15) == 0));
-    if (rc != 0) return rc;
-    Shape sh = {M, N, K, 0, (N + ROWS - 1) / ROWS, plan.shares, plan.steps, 0};
+    for (long long first = 0; first < M; first += slab, x += (size_t)slab * ldx, out += (size_t)slab * ldo) {
+        const int m = (int)(M - first < slab ? M - first : slab);
+        const Plan plan = plan_for(m, N, K, force_tile, force_shares);
+        float* partial = (float*)((char*)scratch + parts_bytes(m, K));
+        const long long quads = (long long)m * (K / 4);
+        const int blocks = (int)((quads + 255) / 256 < 148 * 8 ? (quads + 255) / 256 : 148 * 8);
+        int rc = gg_launch(split_rows_kernel, dim3(blocks), dim3(256), 0, stream, 1, x, ldx, parts, m, K, ld,
+                           (int)(ldx % 4 == 0 && ((uintptr_t)x & 15) == 0));
+        if (rc != 0) return rc;
+        Shape sh = {m, N, K, 0, (N + ROWS - 1) / ROWS, plan.shares, plan.steps, 0};
 #define GT(BN, ST, PA) rc = launch_tile<BN, ST, PA>(x, ldx, w, out, ldo, accumulate, bias, partial, parts, ld, sh, status, stream)
-    switch (plan.tile) {
-        case 0: GT(32, 4, 4); break;
-        case 1: GT(64, 3, 4); break;
-        case 2: GT(96, 3, 4); break;
-        case 3: GT(128, 2, 4); break;
-        case 4: GT(160, 2, 4); break;
-        default: GT(192, 2, 2); break;
-    }
+        switch (plan.tile) {
+            case 0: GT(32, 4, 4); break;
+            case 1: GT(64, 3, 4); break;
+            case 2: GT(96, 3, 4); break;
+            case 3: GT(128, 2, 4); break;
+            case 4: GT(160, 2, 4); break;
+            default: GT(192, 2, 2); break;
+        }
 #undef GT
-    if (rc != 0 || plan.shares == 1) return rc;
-    const int vec = N % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)out & 15) == 0;
-    const long long n = (long long)M * (vec ? N / 4 : N);
-    const int fb = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
-    return gg_launch(finish_kernel, dim3(fb), dim3(256), 0, stream, 1, (const float*)partial, plan.shares, out, ldo, accumulate, bias, M, N, vec);
+        if (rc != 0) return rc;
+        if (plan.shares == 1) continue;
+        const int vec = N % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)out & 15) == 0;
+        const long long n = (long long)m * (vec ? N / 4 : N);
+        const int fb = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
+        if ((rc = gg_launch(finish_kernel, dim3(fb), dim3(256), 0, stream, 1, (const float*)partial, plan.shares, out, ldo, accumulate, bias, m, N, vec)) != 0)
+            return rc;
+    }
+    return 0;
 }
