@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const float* partial, int s
 }
 
 constexpr int TILES = 6;
-constexpr float PAYS_BESIDE = 8.0f, PAYS_FROM_FEW = 40.0f, PAYS_FROM_MANY = 24.0f;      // us: see gg_gemm_f32_parts_pays
+constexpr float PAYS_BESIDE = 8.0f, PAYS_FROM = 28.0f;      // us: see gg_gemm_f32_parts_pays
 const int TILE_BN[TILES] = {32, 64, 96, 128, 160, 192};
 
 struct Plan {
@@ -500,28 +500,28 @@ GG_API gg_gemm_f32_parts_scratch(int M, int N, int K, int force_tile, int force_
 }
 
 // Is a product of this size quicker in parts than on the CUDA cores?  On the GPU alone it is from 17 rows and K = 1,024 on (us, CUDA cores |
-// parts: 17 rows by 1,024 x 1,024 8.9 | 8.3, 2,048 x 2,048 20.8 | 13.5; 100 rows 13.2 | 12.1, 46.3 | 17.2; by 512 x 512 5.2 | 7.4), but it is
-// two or three launches instead of one, and a step whose products are all short is bound by the host's launches: prompts of 18 and
-// 40 tokens through two layers 1,024 wide took 322 and 339 us instead of 297 with every product in parts.  So the CUDA cores'
-// time, modelled, has to be PAYS_BESIDE longer, and PAYS_FROM_FEW at least up to 99 rows (from 100 on the four products of a layer together
-// outlast its launches, so PAYS_FROM_MANY).  Below K = 256 the sums are no more exact than theirs
-// either (K = 128: 1.1e-7 both).
+// parts: 17 rows by 2,048 x 2,048 21.9 | 13.8, 4,096 x 2,048 23.5 | 19.5; 64 rows 24.3 | 14.8, 46.4 | 20.2; 100 rows by 1,024 x 1,024 13.5 | 11.3,
+// 512 x 512 7.3 | 8.1), but it is two or three launches instead of one, 4.5 us of the host's time each, and the host takes some
+// 28 us for a product and what lies between it and the next (115 us a layer): a step of shorter products waits for the host whatever
+// they are.  So the CUDA cores' time, modelled, has to be PAYS_FROM at least and PAYS_BESIDE longer than the parts'.  (Prompts through
+// four layers, us, nothing in parts | as it is | everything: 1,024 wide, 17 tokens 490 | 478 | 523, 40 573 | 540 | 556, 100 796 | 555 | 594;
+// 2,048 wide, 17 tokens 923 | 651 | 660, 100 1,983 | 717 | 847.)  Below K = 256 the sums are no more exact than theirs (K = 128: 1.1e-7 both).
 GG_API gg_gemm_f32_parts_pays(int M, int N, int K, int* pays) {
     if (M <= 0 || N <= 0 || K <= 0 || pays == nullptr) return GG_ERR_ARG;
     *pays = 0;
     if (M < 17 || K < 256 || K % 4 != 0) return 0;
-    // the CUDA cores' tiles as gemm_plain.cu chooses among them: rounds of 296, us per 1,000 of K
-    static const float round_us[4][2] = {{11, 11}, {30, 35}, {42, 55}, {54, 110}};
+    // the CUDA cores' tiles as gemm_plain.cu chooses among them: rounds of 296, us per 1,000 of K, for up to 74, 148 and 296 tiles left
+    static const float round_us[4][3] = {{7.5f, 10.5f, 11.4f}, {30, 30, 35}, {42, 42, 55}, {54, 54, 110}};
     static const int rows[4] = {32, 64, 64, 128}, cols[4] = {16, 32, 64, 64};
     float plain = 0.f;
     for (int i = 0; i < 4; ++i) {
         const long long t = (long long)((M + rows[i] - 1) / rows[i]) * ((N + cols[i] - 1) / cols[i]), left = t % 296;
-        const float us = (round_us[i][1] * (float)(t / 296) + (left == 0 ? 0.f : round_us[i][left > 148])) * (float)K * 1e-3f;
+        const float us = (round_us[i][2] * (float)(t / 296) + (left == 0 ? 0.f : round_us[i][left > 148 ? 2 : left > 74])) * (float)K * 1e-3f;
         if (i == 0 || us < plain) plain = us;
     }
     float parts = 0.f;
     plan_for(M, N, K, -1, 0, &parts);
-    *pays = plain >= (M >= 100 ? PAYS_FROM_MANY : PAYS_FROM_FEW) && parts + PAYS_BESIDE < plain;
+    *pays = plain >= PAYS_FROM && parts + PAYS_BESIDE < plain;
     return 0;
 }
 
