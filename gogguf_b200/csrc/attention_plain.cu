@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_plain_kernel(
 // with keys tx, tx + 8, .. and, of the same rows, the output's columns 4 tx .. + 3 of every 32; a row's maximum and sum are its
 // eight threads' (neighbouring lanes).  Rows of shared memory are padded by four floats: a read of eight rows touches every bank once.
 // Multiply-adds bound it (a score and a value product each, 16 bytes of shared memory to some five of them).  One prompt of 450 tokens, 16
-// heads of 128 over 8 kv heads: 215 us a row at a time, 141 in tiles.
+// heads of 128 over 8 kv heads: 215 us a row at a time, 141 in tiles; 16 tokens behind 4,000 keys, eight tiles of 126 steps each: 191 and 934.
 #define APT_ROWS 32
 #define APT_KEYS 32
 #define APT_P (APT_KEYS + 4)
@@ -452,7 +452,8 @@ __global__ void __launch_bounds__(128) attention_plain_tile_kernel(
 // `dtype`, n_pages of them.  sink: null or one float per query head.
 // gate: null or logits in `dtype`, rows ldg apart.  chunk 0: none.
 // cu_seqlens (may be null): [n_seqs + 1] prefix sums of the step's tokens by sequence, a sequence's tokens at consecutive positions; with
-// it, steps of 16 or more tokens a sequence on average take the tiled kernel where the sizes allow it.
+// it, steps of 16 or more tokens a sequence on average take the tiled kernel where the sizes allow it: callers pass it where the tiles are
+// quicker (kernels.py, attention_tiles_pay).
 // status (may be null): where the debug build records a page id or table index out of range (code 41).
 GG_API gg_attention_plain(const void* q, const void* k_pool, const void* v_pool, void* out, int dtype,
                           const int* positions, const int* seq_of_token, const int* page_table,
@@ -461,7 +462,7 @@ GG_API gg_attention_plain(const void* q, const void* k_pool, const void* v_pool,
                           long long ldg, const int* cu_seqlens, int n_seqs, int* status, cudaStream_t stream) {
     if (ntok <= 0) return 0;
     if (d <= 0 || dv <= 0 || dv > ATT_MAXD || d > 4096 || nq <= 0 || nkv <= 0 || nq % nkv || nq > 65535 || page_size <= 0) return GG_ERR_ARG;
-    // Tiles of 32 rows where most have 32 (the plain kernel reads a key for every row).
+    // Tiles of 32 rows where most have 32 and the caller asks for them.
     if (cu_seqlens != nullptr && n_seqs > 0 && ntok >= 16LL * n_seqs && dtype == GG_F32 && d % 4 == 0 && dv % 4 == 0 && d <= 128 && dv <= 128 &&
         nkv <= 65535 && (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15) == 0) {
         const size_t tile_smem = (size_t)(APT_ROWS * (d + 4) + 2 * APT_KEYS * (d + 4 + dv + 4) + APT_ROWS * APT_P) * sizeof(float);

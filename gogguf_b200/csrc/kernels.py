@@ -9,7 +9,7 @@ from __future__ import annotations
 import ctypes
 import struct
 from operator import index
-from typing import List, Optional, Sequence
+from typing import List, Optional, Sequence, Tuple
 
 import torch
 
@@ -482,6 +482,37 @@ def gemm_f32_parts(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, scratch:
 
 
 # ------------------------------------------------------------------------------- attention
+def attention_tiles_pay(lengths: Sequence[Tuple[int, int]], nq: int, nkv: int, d: int, dv: int, window: int = 0, chunk: int = 0) -> bool:
+    """Is 32-bit attention of these sequences (cached positions, new tokens) quicker in tiles of 32 rows than a row at a time?
+
+    Tiles read a key once for 32 rows, but a tile walks over its keys alone: 7.4 us for 32 keys of 128, so a few tokens behind a long
+    history are few blocks with a long chain each, where the other kernel gives every (token, head) eight warps.  Both are modelled
+    (us; 16 heads over 8, of 128 | of 64, rows and tiles measured: 16 tokens behind 4,000 191 and 934 | 192 and 629, 64 behind 900
+    115 and 234 | 116 and 158, 128 behind 900 225 and 264 | 225 and 185, three times 64 behind 900 319 and 269 | 318 and 177, 333
+    behind none 131 and 106 | 129 and 70, behind 900 621 and 378 | 620 and 254)."""
+    tokens = sum(n for _, n in lengths)
+    if tokens < 16 * len(lengths) or tokens == 0:
+        return False
+    group = nq // nkv
+    reads, longest, blocks, walks = 0.0, 1, 0, 0
+    for cached, n in lengths:
+        end = cached + n
+        seen = n * cached + n * (n + 1) / 2                    # keys that the tokens see
+        reach = end
+        for bound in (window, chunk):
+            if 0 < bound < end:
+                seen = min(seen, n * bound if bound == window else n * (bound + 1) / 2)
+                reach = min(reach, bound + 32 // group + 1)    # a tile's keys: those of any of its tokens
+        tiles, steps = -(-n * group // 32), (reach - 1) // 32 + 1
+        reads += seen
+        longest, blocks, walks = max(longest, steps), blocks + tiles * nkv, walks + tiles * nkv * (steps if cached >= n else (steps + 1) / 2)
+    size = (d + dv) / 2
+    alone, beside = 2.6 + 0.038 * size, 2.1 + 0.0215 * size    # 32 keys of a block that has an SM, and a block's share of a full SM
+    tiles_us = 5.0 + max(longest * max(alone, min(-(-blocks // 148), 2) * beside), walks / 148 * beside)
+    rows_us = 3.0 + 109e-6 * reads * nq + 5.3e-3 * tokens * nq
+    return 1.05 * tiles_us < rows_us
+
+
 def attention_plain(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor,
                     positions: torch.Tensor, seq_of_token: torch.Tensor, page_table: torch.Tensor,
                     page_size: int, n_tokens: int, nq: int, nkv: int, d: int, scale: float, window: int,
@@ -491,8 +522,8 @@ def attention_plain(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
     """Attention over the paged cache on the CUDA cores; `dv` is the values' head size (default d), `sink` one
     float32 per query head that joins the softmax's denominator, `out_scale` a factor on the result; chunk > 0: a
     position sees its own chunk of that many positions only; gate (rows of nq * dv logits): the result is multiplied by
-    their sigmoid.  cu_seqlens ([n_seqs + 1], prefix sums of the sequences' tokens, each at consecutive positions): steps of many
-    tokens a sequence may then share the keys' reads between them."""
+    their sigmoid.  cu_seqlens ([n_seqs + 1], prefix sums of the sequences' tokens, each at consecutive positions): steps of 16 and
+    more tokens a sequence then share the keys' reads between them, which a caller asks for where `attention_tiles_pay`."""
     if cu_seqlens is not None:
         _need(cu_seqlens, torch.int32, "cu_seqlens")
         if n_seqs < 1 or cu_seqlens.numel() < n_seqs + 1:

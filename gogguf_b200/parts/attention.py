@@ -228,7 +228,12 @@ class AttentionMixer:
         if self._fast is not None:
             self._fast(q, cache.k, cache.v, o, ctx, table, cache.page_size, sink=self.sink, out_scale=self.out_scale, gate=gate)
         else:
+            # (tiles share the keys' reads; asked once a step for layers of one size)
+            asked = ("attention_tiles", nq, nkv, d, dv, self.window, self.chunk)
+            if asked not in ctx.shared:
+                ctx.shared[asked] = dt == torch.float32 and K.attention_tiles_pay(ctx.lengths, nq, nkv, d, dv, self.window, self.chunk)
+            tiles = ctx.shared[asked]
             K.attention_plain(q, cache.k, cache.v, o, ctx.positions, ctx.seq_of_token, table,
                               cache.page_size, T, nq, nkv, d, self.scale, self.window, dv=dv, sink=self.sink,
-                              out_scale=self.out_scale, chunk=self.chunk, gate=gate, cu_seqlens=ctx.cu_seqlens, n_seqs=ctx.n_seqs)
+                              out_scale=self.out_scale, chunk=self.chunk, gate=gate, cu_seqlens=ctx.cu_seqlens if tiles else None, n_seqs=ctx.n_seqs)
         self.o(o, residual, accumulate=not ctx.shared.get("output_empty", False), ws=ctx.ws, emit=ctx.shared.get("row_stats"))

@@ -4,7 +4,7 @@ linear projection that every part with a matrix uses.
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from typing import Any, Dict, Optional, Tuple
+from typing import Any, Dict, Optional, Sequence, Tuple
 
 import torch
 
@@ -99,6 +99,7 @@ class StepContext:
     shared: Dict[Any, Any] = field(default_factory=dict)   # per-step values parts share (rotary tables)
     fresh: bool = False           # every sequence of the step starts at position 0 (whole prompts): what a token
     #                               reads is among the step's own tokens
+    lengths: Sequence[Tuple[int, int]] = ()   # (cached positions, new tokens) of each sequence (host); empty: not known
 
 
 class RowStats:
