@@ -385,8 +385,9 @@ __global__ void __launch_bounds__(128) attention_plain_tile_kernel(
                 for (int e = 0; e < 4; ++e) acc[i][c][e] *= corr;
         }
         __syncwarp();                                                    // a row's weights are its own warp's
-        // Keys that one row sees and another does not lie in tiles on an edge: there a value with weight zero is not
-        // multiplied (it may be an infinity).
+        // Keys that one row sees and another does not lie in tiles on an edge: there a value that a row does not see is not
+        // multiplied (it may be an infinity, and its weight is zero).
+        const int from = lo + it * APT_KEYS;
         auto values = [&](auto edge) {
 #pragma unroll 2
             for (int k0 = 0; k0 < APT_KEYS; k0 += 4) {
@@ -404,7 +405,8 @@ __global__ void __launch_bounds__(128) attention_plain_tile_kernel(
                             const float4 v = *reinterpret_cast<const float4*>(vt + (k0 + kk) * LV + 4 * tx + 32 * c);
 #pragma unroll
                             for (int i = 0; i < 2; ++i) {
-                                const bool in = !decltype(edge)::value || p[i][kk] != 0.f;
+                                const int at = from + k0 + kk;
+                                const bool in = !decltype(edge)::value || (at <= pos[i] && at >= low[i]);
                                 acc[i][c][0] = fmaf(p[i][kk], in ? v.x : 0.f, acc[i][c][0]);
                                 acc[i][c][1] = fmaf(p[i][kk], in ? v.y : 0.f, acc[i][c][1]);
                                 acc[i][c][2] = fmaf(p[i][kk], in ? v.z : 0.f, acc[i][c][2]);
@@ -414,7 +416,6 @@ __global__ void __launch_bounds__(128) attention_plain_tile_kernel(
                     }
             }
         };
-        const int from = lo + it * APT_KEYS;
         if (from + APT_KEYS - 1 > pos0 || from < first_key(last)) values(std::true_type{});
         else values(std::false_type{});
         __syncthreads();

@@ -81,3 +81,21 @@ def test_an_infinity_behind_a_token_stays_there():
                       torch.zeros(1, 1, device="cuda", dtype=torch.int32), 64, 40, 2, 1, 32, 1.0, 0,
                       cu_seqlens=torch.tensor([0, 40], device="cuda", dtype=torch.int32), n_seqs=1)
     assert out[:20].isfinite().all() and not out[20:].isfinite().any()
+
+
+def test_an_infinity_with_a_weight_of_zero():
+    """A value that a row sees counts also where its weight is too small for a float32, in tiles on an edge and inside, as a row at a time."""
+    from gogguf_b200.csrc import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(4)
+    T, ints = 100, dict(device="cuda", dtype=torch.int32)
+    q, kp, vp = torch.ones(T, 2, 32, device="cuda"), torch.zeros(2, 1, 64, 32, device="cuda"), torch.randn(2, 1, 64, 32, device="cuda", generator=g)
+    for at in (5, 90):                                     # scores 200 below the others
+        kp[at // 64, 0, at % 64] = -200.0 / 32
+        vp[at // 64, 0, at % 64] = float("inf")
+    outs = []
+    for cu in (None, torch.tensor([0, T], **ints)):
+        outs.append(torch.empty(T, 2, 32, device="cuda"))
+        K.attention_plain(q, kp, vp, outs[-1], torch.arange(T, **ints), torch.zeros(T, **ints), torch.tensor([[0, 1]], **ints), 64, T, 2, 1, 32,
+                          1.0, 0, cu_seqlens=cu, n_seqs=1)
+    assert torch.equal(outs[0].isfinite(), outs[1].isfinite())
+    assert outs[0][:5].isfinite().all() and not outs[0][5:].isfinite().any()
