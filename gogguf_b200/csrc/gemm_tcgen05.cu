@@ -1664,7 +1664,19 @@ static bool gemm_deep() {
     if (on < 0) { const char* e = getenv("GOGGUF_B200_GEMM_DEEP"); on = (e != nullptr && e[0] == '0') ? 0 : 1; }
     return on == 1;
 }
-static bool three_per_sm_at_64(long long tiles) { return tiles > 148 && tiles <= 222; }
+// 33 to 64 tokens, splits in clusters: do two CTAs an SM with a deeper ring (296 places) beat three (444)?  Up to 148 tiles, where K is
+// cut, they do (see gg_gemm_tc_splits).  149 to 222 tiles, which three an SM hold twice, do better uncut up to about K = 3,000 and in two cuts
+// beyond (64 tokens, us, three an SM in two cuts | two uncut: 160 tiles by 1,024 13.0 | 10.6, 2,048 19.9 | 17.8, 4,096 31.8 | 31.8, 5,120
+// 38.0 | 38.5; 205 tiles 14.4 | 11.8, 23.7 | 20.8, 38.0 | 38.2, 45.6 | 45.8; 33 tokens, 4,096 30.0 | 31.0 and 35.9 | 37.3).  More tiles stay
+// uncut, and it is a matter of rounds: places of three an SM stream a little more in all, so 15 % fewer place-rounds are asked for.
+// Measured, 64 tokens, K = 4,096 | 1,024 (us, three, two): 230 tiles 56, 42 | 23, 12; 300 54, 67 | 17, 21; 440 73, 79 | 23, 26; 445
+// 94, 80 | 29, 26; 592 106, 101 | 33, 31; 600 105, 115 | 34, 35; 1,000 171, 172 | 54, 53; 1,187 (151,936 columns) 194, 208 | 59, 59;
+// 1,340 228, 224 | 67, 67; 2,000 321, 331 | 96, 96.
+static bool two_per_sm_at_64(long long tiles, int K) {
+    if (tiles > 148 && tiles <= 222) return K <= 3072;
+    const long long two = (tiles + 295) / 296, three = (tiles + 443) / 444;
+    return 115 * 296 * two < 100 * 444 * three;
+}
 
 // Number of K splits the launcher uses for a product of this shape (0: the shape is not taken).
 // use_cluster != 0: the splits of a tile form a thread-block cluster (at most 8) and no scratch is
@@ -1678,15 +1690,16 @@ GG_API gg_gemm_tc_splits(int M, int N, int K, int use_cluster) {
     int splits = (148 * per_sm + tiles / 2) / tiles;
     if (splits > num_kb / 2) splits = num_kb / 2;  // at least two 64-wide slabs per CTA
     const int most = use_cluster ? MAX_CLUSTER : 16;
-    // 33 to 64 tokens, splits in clusters: two CTAs share an SM with a deeper ring, and K is cut for 256 of the 296 places (or two CTAs a tile
+    // 33 to 64 tokens, splits in clusters: where two CTAs share an SM with a deeper ring, K is cut for 256 of the 296 places (or two CTAs a tile
     // where that many fit), fewer cuts than three an SM would give: every cut sends a float32 row for each token through the cluster.
     // Measured, 61 tokens (us, three an SM | as it is): 4,096 x 2,048 9.6 | 8.5, 2,048 x 2,048 7.9 | 7.1, 10,752 x 2,048 20.8 | 13.1,
-    // 2,048 x 5,376 11.2 | 9.9, 6,144 x 4,096 15.0 | 13.5, 4,096 x 12,288 24.7 | 22.4, 65,536 x 2,048 53.5 | 49.1; with 149 to 222 tiles
-    // three an SM and two cuts are quicker (24,576 x 4,096: 37.3, 41.4 uncut).
-    if (use_cluster && M > 32 && M <= 64 && gemm_deep() && !three_per_sm_at_64(tiles)) {
-        const int cut = 256 / tiles;
-        splits = cut >= 1 ? cut : 1;
-        if (tiles <= 148 && splits < 2) splits = 2;
+    // 2,048 x 5,376 11.2 | 9.9, 6,144 x 4,096 15.0 | 13.5, 4,096 x 12,288 24.7 | 22.4, 65,536 x 2,048 53.5 | 49.1.
+    if (use_cluster && M > 32 && M <= 64 && gemm_deep()) {
+        if (two_per_sm_at_64(tiles, K)) {
+            const int cut = 256 / tiles;
+            splits = cut >= 1 ? cut : 1;
+            if (tiles <= 148 && splits < 2) splits = 2;
+        } else if (tiles <= 222) splits = 2;         // what three an SM hold at once (a third cut would not fit them)
         if (splits > num_kb / 2) splits = num_kb / 2;
     }
     if (splits > most) splits = most;
@@ -1740,7 +1753,7 @@ static int gemm_tc_impl(const void* x, const void* w, void* out, int out_mode, i
         // to run as one wave.  GOGGUF_B200_GEMM_DEEP=0 always takes the three-per-SM forms.
         const long long ctas = (long long)((N + BM - 1) / BM) * ((M + bn - 1) / bn) * splits;
         // (33 to 64 tokens: see gg_gemm_tc_splits; above, three per SM always)
-        const bool deep = gemm_deep() && (bn <= 32 ? ctas <= 296 : bn == 64 && cluster && !three_per_sm_at_64((N + BM - 1) / BM));
+        const bool deep = gemm_deep() && (bn <= 32 ? ctas <= 296 : bn == 64 && cluster && two_per_sm_at_64((N + BM - 1) / BM, K));
 #define GG_DECODE_AS(BN_, ST_, MINB_, X_) launch<BN_, ST_, true, MINB_, X_>(ta, tb, out, out_mode, ldo, M, N, K, splits, per, scratch, \
                                                                           cluster, status, nio, qio, stream)
 #define GG_DECODE(BN_, ST_, MINB_) (nio.xielu ? GG_DECODE_AS(BN_, ST_, MINB_, true) : GG_DECODE_AS(BN_, ST_, MINB_, false))
