@@ -510,7 +510,7 @@ def attention_tiles_pay(lengths: Sequence[Tuple[int, int]], nq: int, nkv: int, d
     alone, beside = 2.6 + 0.038 * size, 2.1 + 0.0215 * size    # 32 keys of a block that has an SM, and a block's share of a full SM
     tiles_us = 5.0 + max(longest * max(alone, min(-(-blocks // 148), 2) * beside), walks / 148 * beside)
     rows_us = 3.0 + 109e-6 * reads * nq + 5.3e-3 * tokens * nq
-    return 1.05 * tiles_us < rows_us
+    return 1.09 * tiles_us < rows_us
 
 
 def attention_plain(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor,
