@@ -1026,11 +1026,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_add_vec_kernel(float* x, float* 
     }
 }
 
-// xhat (bfloat16 [rows, H]) and ssq (float32 [rows, ceil(H / 128)]) may both be null.  zero_y != 0: y is left
-// zeroed (the buffer the next part of the block adds its output into, without a fill of its own).  gate (float32
-// [rows, H], may be null) with gate_bias ([H], may be null): y is first multiplied by sigmoid(gate + gate_bias),
-// element by element, and the norm is taken of the product.
-// The same and the norm that comes next, in one pass: x += y / rms(y) * w, out = x / rms(x) * w2 of the updated rows, which are in
+// A norm and add (rmsnorm_add above) and the norm that comes next, in one pass: x += y / rms(y) * w, out = x / rms(x) * w2 of the updated rows, which are in
 // registers then.  One block a row, VPT groups of four columns a thread.  As two kernels a decode step paid a launch and a read of
 // the row more: rows of 2,048, 8 tokens 4.4 us, as one 2.3; 64 tokens 4.7 | 2.5; 1,024 tokens 8.4 | 6.5.
 template <typename TO, int VPT>
@@ -1095,7 +1091,7 @@ GG_API gg_rmsnorm_add_norm(float* x, float* y, const float* w, int rows, int H, 
     const int n4 = H >> 2;
     int threads = (n4 + 31) / 32 * 32;
     if (threads > 1024) threads = 1024;
-    if (threads > 256 && (rows >= 512 || n4 > 2048)) threads = 256;
+    if (threads > 256 && rows >= 512) threads = 256;
     const int vpt = (n4 + threads - 1) / threads;
     GG_DISPATCH_DTYPE(out_dtype, TO, {
         if (vpt <= 1) return gg_launch(rmsnorm_add_norm_kernel<TO, 1>, dim3(rows), dim3(threads), 0, stream, 1, x, y, w, H, eps, zero_y, w2, eps2, (TO*)out);
@@ -1105,6 +1101,10 @@ GG_API gg_rmsnorm_add_norm(float* x, float* y, const float* w, int rows, int H, 
     });
 }
 
+// xhat (bfloat16 [rows, H]) and ssq (float32 [rows, ceil(H / 128)]) may both be null.  zero_y != 0: y is left
+// zeroed (the buffer the next part of the block adds its output into, without a fill of its own).  gate (float32
+// [rows, H], may be null) with gate_bias ([H], may be null): y is first multiplied by sigmoid(gate + gate_bias),
+// element by element, and the norm is taken of the product.
 GG_API gg_rmsnorm_add(float* x, float* y, const float* w, int rows, int H, float eps, void* xhat, float* ssq,
                       int zero_y, const float* gate, const float* gate_bias, cudaStream_t stream) {
     if (rows <= 0) return 0;
