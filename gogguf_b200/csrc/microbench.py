@@ -1,4 +1,4 @@
-"""Kernel micro-benchmarks: python -m gogguf_b200.csrc.microbench [gemm|gemm_layer|attn|prefill_attn|sample|latent|retention|recurrence|dinuzen|kulesun|niresun|plain|shares|experts] [--m 1,8,64] [--ctx 2048,8192]
+"""Kernel micro-benchmarks: python -m gogguf_b200.csrc.microbench [gemm|gemm_layer|attn|prefill_attn|sample|latent|retention|recurrence|dinuzen|kulesun|niresun|plain|shares|experts|f32_parts] [--m 1,8,64] [--ctx 2048,8192]
 
 Times single kernels the way a decode step runs them: forty launches captured in a CUDA graph and
 replayed, so that host launch cost is out of the picture and dependent launches overlap as they do
@@ -748,12 +748,72 @@ def plain() -> None:
                 print(f"gemm_plain {str(dx)[6:]} x {str(dw)[6:]} N={N} K={k} M={M:4d}: {us:8.1f} us {2 * M * N * k / us / 1e6:6.2f} TFLOP/s "
                       f"{N * k * ws[0].element_size() / us / 1e6:5.2f} TB/s of weights", flush=True)
             del ws
-    for nq, nkv, d in ((16, 8, 128), (16, 8, 64), (8, 8, 256)):
-        for B, new, history in ((1, 1, 23), (4, 1, 600), (8, 1, 2048), (3, 150, 0), (1, 450, 0)):
+    for nq, nkv, d in ((16, 8, 128), (16, 8, 64), (15, 5, 120), (8, 8, 256)):
+        for B, new, history in ((1, 1, 23), (4, 1, 600), (8, 1, 2048), (3, 150, 0), (1, 450, 0), *((B, new, h) for B, new in
+                                ((1, 16), (1, 32), (1, 64), (1, 128), (1, 333), (2, 16), (4, 16), (8, 16), (3, 64), (8, 64)) for h in (0, 200, 900, 2000, 4000, 6100)
+                                if B * (new + h) <= 16000)):
             q, pools, out, ctx, table = _paged_step(B, new, history, nq, nkv, d, torch.float32, 1)
-            us = _time_graph(lambda i: K.attention_plain(q, pools[0][0], pools[0][1], out, ctx["pos"], ctx["sot"], table, 64, B * new, nq, nkv,
-                                                         d, d ** -0.5, 0), 10)
-            print(f"attention_plain float32 nq={nq} nkv={nkv} d={d} B={B} new={new} history={history}: {us:8.1f} us", flush=True)
+            line = f"attention_plain float32 nq={nq} nkv={nkv} d={d} B={B} new={new} history={history}:"
+            for name, kw in (("a row at a time", {}), ("in tiles", dict(cu_seqlens=ctx["cu"], n_seqs=B))):
+                if kw and (new < 16 or d > 128):
+                    continue
+                us = _time_graph(lambda i: K.attention_plain(q, pools[0][0], pools[0][1], out, ctx["pos"], ctx["sot"], table, 64, B * new, nq, nkv,
+                                                             d, d ** -0.5, 0, **kw), 10)
+                line += f" {name} {us:.1f} us"
+            print(line + (", tiles taken" if K.attention_tiles_pay([(history, new)] * B, nq, nkv, d, d) else ""), flush=True)
+
+
+F32_SHAPES = ((512, 128), (512, 256), (512, 512), (1024, 1024), (2048, 1024), (6144, 1024), (1024, 3072), (1800, 1800), (3000, 1800), (1800, 4744), (9488, 1800),
+              (2048, 2048), (4096, 2048), (10752, 2048), (2048, 5376))
+
+
+def f32_parts() -> None:
+    """32-bit products on the CUDA cores and in parts on the tensor cores (csrc/gemm_plain.cu, csrc/gemm_f32_parts.cu): times with
+    the plan's tile and shares, the time of a stage of every tile, relative errors against float64 of the two for several kinds of
+    operands, and rows that are not finite."""
+    from . import kernels as K
+    dev = "cuda:0"
+
+    def run(x, w, out, tile=-1, shares=0):
+        key = (x.shape[0], tuple(w.shape), tile, shares)
+        if key not in room:
+            room[key] = torch.empty(K.f32_parts_scratch(x.shape[0], *w.shape, tile, shares), dtype=torch.uint8, device=dev)
+        K.gemm_f32_parts(x, w, out, room[key], tile=tile, shares=shares)
+
+    for N, k in F32_SHAPES:
+        nbuf = max(2, min(12, int(260e6 // (N * k * 4)) + 1))
+        ws = [torch.randn(N, k, device=dev) for _ in range(nbuf)]
+        for M in (17, 24, 32, 48, 64, 100, 150, 300, 450, 600):
+            room = {}
+            x, out = torch.randn(M, k, device=dev), torch.empty(M, N, device=dev)
+            t = [_time_graph(lambda i: f(x, ws[i % nbuf], out), 12) for f in (K.gemm_plain, run)]
+            print(f"f32 product N={N} K={k} M={M}: CUDA cores {t[0]:.1f} us, parts {t[1]:.1f} us{', taken' if K.f32_parts_pays(M, N, k) else ''}", flush=True)
+        del ws
+    for tile, bn in enumerate((32, 64, 96, 128, 160, 192)):            # 148 items of many stages: one round
+        room, stage = {}, []
+        x, w = torch.randn(bn, 8192, device=dev), torch.randn(148 * 128, 8192, device=dev)
+        out = torch.empty(bn, w.shape[0], device=dev)
+        for k in (2048, 8192):
+            v, wk = x[:, :k].contiguous(), w[:, :k].contiguous()
+            stage.append(_time_graph(lambda i: run(v, wk, out, tile, 1), 6))
+        print(f"f32 parts, {bn} rows: {(stage[1] - stage[0]) / 96:.2f} us a stage, {stage[0] - (stage[1] - stage[0]) / 3:.1f} us beside", flush=True)
+    g = torch.Generator(device=dev).manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, device=dev, generator=g)                             # noqa: E731
+    for k in (256, 512, 1024, 2048, 5376):
+        for kind, x, w in (("normal", rnd(96, k), rnd(384, k)), ("one sign", rnd(96, k).abs(), rnd(384, k).abs()),
+                           ("a channel a hundred times the others", rnd(96, k) * torch.where(torch.arange(k, device=dev) == k // 3, 100.0, 1.0), rnd(384, k)),
+                           ("one term a row", rnd(96, k) * (torch.arange(k, device=dev) == k // 3), rnd(384, k))):
+            room, want, off = {}, x.double() @ w.double().T, []
+            for f in (K.gemm_plain, run):
+                out = torch.empty(96, 384, device=dev)
+                f(x, w, out)
+                off.append(float((out.double() - want).norm() / want.norm()))
+            print(f"f32 error K={k} {kind}: CUDA cores {off[0]:.2e}, parts {off[1]:.2e}", flush=True)
+    for M, N, k in ((450, 10752, 2048), (96, 2048, 2048)):
+        room, w, out = {}, rnd(N, k), torch.empty(M, N, device=dev)
+        for x in (rnd(M, k), torch.full((M, k), float("nan"), device=dev)):
+            t = [_time_graph(lambda i: f(x, w, out), 6) for f in (K.gemm_plain, run)]
+            print(f"f32 product N={N} K={k} M={M}{', nothing but NaN' if x.isnan().any() else ''}: CUDA cores {t[0]:.1f} us, parts {t[1]:.1f} us", flush=True)
 
 
 def _paged_step(B, new, history, nq, nkv, d, dtype, nrot):
@@ -845,7 +905,7 @@ def experts() -> None:
 def main() -> None:
     ap = argparse.ArgumentParser()
     ap.add_argument("what", choices=["gemm", "gemm_layer", "attn", "prefill_attn", "sample", "latent", "retention", "recurrence", "dinuzen", "kulesun", "niresun",
-                                     "plain", "shares", "experts"])
+                                     "plain", "shares", "experts", "f32_parts"])
     ap.add_argument("--m", default="1,8,64", help="token counts (gemm), batch sizes (attn) or prompt lengths (prefill_attn)")
     ap.add_argument("--ctx", default="2048", help="attn: cached positions per sequence (comma separated)")
     ap.add_argument("--scratch", action="store_true", help="attn: splits merged by a second kernel instead of inside clusters")
@@ -860,7 +920,7 @@ def main() -> None:
     if a.what == "recurrence":
         recurrence()
         return
-    alone = {"dinuzen": dinuzen, "kulesun": kulesun, "niresun": niresun, "plain": plain, "shares": shares, "experts": experts}
+    alone = {"dinuzen": dinuzen, "kulesun": kulesun, "niresun": niresun, "plain": plain, "shares": shares, "experts": experts, "f32_parts": f32_parts}
     if a.what in alone:
         alone[a.what]()
         return
