@@ -825,7 +825,7 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const float* part_o
     __shared__ float f[128];
     const float inv = 1.0f / L;
     auto weight = [&](int s) { return ml[2 * s] == -INFINITY ? 0.f : exp2f(ml[2 * s] - M); };
-    if (splits > 128) {
+    if (splits > 128) {                      // (the planner cuts into 32 at most; a caller of the launcher may cut finer)
         for (int c = threadIdx.x; c < R; c += blockDim.x) {
             float acc = 0.f;
             for (int s = 0; s < splits; ++s) acc = fmaf(weight(s), part_o[(row * splits + s) * R + c], acc);
