@@ -54,8 +54,9 @@ struct Shape {
 };
 
 // The sums of four rows of x with four rows of w by multiply-adds, a warp's lanes along k; a lane gets the four of w's row lane % 4.
-// (450 rows of nothing but NaN by 10,752 x 2,048: 3.1 ms; 44.7 with a thread's walk over K for each of its sums, 0.55 in gemm_plain.cu.)
-__device__ __noinline__ float4 plain_sums(const float* x, long long ldx, int x_rows, int vec, const float* w, int ldw, int w_rows, int k0, int k1) {
+// (450 rows with an infinity each by 10,752 x 2,048: 3.1 ms; 44.7 with a thread's walk over K for each of its sums, 0.55 in gemm_plain.cu.
+// With a NaN each: 0.29, rows_with_nan.)
+__device__ __forceinline__ float4 plain_sums(const float* x, long long ldx, int x_rows, int vec, const float* w, int ldw, int w_rows, int k0, int k1) {
     const int lane = threadIdx.x & 31;
     const float* xr[4];
     const float* wr[4];
@@ -91,6 +92,22 @@ __device__ __noinline__ float4 plain_sums(const float* x, long long ldx, int x_r
     return mine;
 }
 
+// Which of four rows of x have a NaN among their columns k0 .. k1: their sums are NaN whatever w holds.
+__device__ __forceinline__ uint32_t rows_with_nan(const float* x, long long ldx, int x_rows, int vec, int k0, int k1) {
+    uint32_t found = 0u;
+#pragma unroll 4
+    for (int k = k0 + 4 * (int)(threadIdx.x & 31); k < k1; k += 128)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float* r = x + (size_t)min(i, x_rows - 1) * ldx + k;
+            float4 v;
+            if (vec) v = *reinterpret_cast<const float4*>(r);
+            else v = make_float4(r[0], r[1], r[2], r[3]);
+            if (v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w) found |= 1u << i;
+        }
+    return __reduce_or_sync(0xffffffffu, found);
+}
+
 // Where a warp's sums of 32 columns (outputs of rows m .. of x with rows n .. + 31 of w) are made again.
 struct Again {
     const float* x;
@@ -100,11 +117,16 @@ struct Again {
     int M, N, K, k0, k1, accumulate;
     float bias;               // the lane's
 };
-// The warp's outputs whose bits are set in its lanes' words.  (Not inlined: its registers would be the kernel's.)
-__device__ __noinline__ void make_again(uint32_t bits, int m, int n, const Again a) {
+// The warp's outputs whose bits are set in its lanes' words.  (Not inlined, and its numbers by reference: the registers would be the kernel's.)
+__device__ __noinline__ void make_again(uint32_t bits, int m, int n, const Again& a) {
     const int lane = threadIdx.x & 31, vec = a.ldx % 4 == 0 && ((uintptr_t)a.x & 15) == 0;
     for (int j = 0; j < 32; j += 4) {
-        const uint32_t mine = bits >> j & 15u;
+        uint32_t mine = bits >> j & 15u;
+        if (!__any_sync(0xffffffffu, mine != 0u)) continue;
+        const uint32_t nan = rows_with_nan(a.x + (size_t)(m + j) * a.ldx, a.ldx, a.M - m - j, vec, a.k0, a.k1);
+        for (uint32_t left = mine & nan; left != 0u; left &= left - 1u)
+            a.out[(size_t)(m + j + __ffs(left) - 1) * a.ldo + n + lane] = __int_as_float(0x7fffffff);
+        mine &= ~nan;
         uint32_t rows = __ballot_sync(0xffffffffu, mine != 0u);
         while (rows != 0u) {                                         // four neighbouring rows of w at a time
             const int r = (__ffs(rows) - 1) & ~3;
@@ -419,7 +441,7 @@ struct Plan {
 };
 
 // The tile and the shares of K with the least modelled time: rounds of 148 items, each its stages at the tile's measured rate and 2.5 us
-// beside, and for shares the second kernel with its traffic.  (Measured, us a stage: 1.45 to 1.8 whatever the tile up to 160 rows.)
+// beside, and for shares the second kernel with its traffic.  (Measured, us a stage: 1.43 to 1.84 up to 160 rows, 2.0 at 192.)
 Plan plan_for(int M, int N, int K, int force_tile, int force_shares, float* modelled = nullptr) {
     static const float step_us[TILES] = {1.44f, 1.5f, 1.5f, 1.6f, 1.7f, 1.95f};
     const int all = (K + STEP - 1) / STEP;

@@ -811,9 +811,12 @@ def f32_parts() -> None:
             print(f"f32 error K={k} {kind}: CUDA cores {off[0]:.2e}, parts {off[1]:.2e}", flush=True)
     for M, N, k in ((450, 10752, 2048), (96, 2048, 2048)):
         room, w, out = {}, rnd(N, k), torch.empty(M, N, device=dev)
-        for x in (rnd(M, k), torch.full((M, k), float("nan"), device=dev)):
+        for kind in ("finite", "NaN", "an infinity a row"):
+            x = rnd(M, k)
+            if kind != "finite":
+                x[:, 5] = float("nan" if kind == "NaN" else "inf")
             t = [_time_graph(lambda i: f(x, w, out), 6) for f in (K.gemm_plain, run)]
-            print(f"f32 product N={N} K={k} M={M}{', nothing but NaN' if x.isnan().any() else ''}: CUDA cores {t[0]:.1f} us, parts {t[1]:.1f} us", flush=True)
+            print(f"f32 product N={N} K={k} M={M}{'' if kind == 'finite' else ', ' + kind}: CUDA cores {t[0]:.1f} us, parts {t[1]:.1f} us", flush=True)
 
 
 def _paged_step(B, new, history, nq, nkv, d, dtype, nrot):

@@ -121,6 +121,7 @@ def test_rows_that_are_not_finite(tile, o):
     x[:, 100] = 3.4e38                                                     # rounds to an infinity in 8 bits
     w[:, 100] = torch.randn(N, device="cuda", generator=g) * 1e-38
     x[5:90:3, 7], x[6:200:7, 9] = float("nan"), float("inf")
+    x[64:72, 255:] = float("nan")                                          # (the last columns, and whole groups of rows)
     w[17, 9], w[18, 9], res = 0.0, -1.0, torch.randn(M, N, device="cuda", generator=g)
     bias = torch.randn(N, device="cuda", generator=g)
     out, plain = parts(x, w, res.clone(), tile, accumulate=True, bias=bias), res.clone()
