@@ -21,6 +21,7 @@ every scheduled block, as the reference's debug hooks do for its last token
 from __future__ import annotations
 
 from dataclasses import dataclass, field
+from operator import add
 from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -173,6 +174,8 @@ class Stepper:
         cache = self.cache
         slots = [e.slot for e in entries]
         counts = [len(e.tokens) for e in entries]
+        starts = [cache.lengths[s] for s in slots]
+        decode = all(n == 1 for n in counts)
         B = max(len(entries), pad_seqs)
         n_pad = B - len(entries)
         T = sum(counts) + n_pad
@@ -197,7 +200,7 @@ class Stepper:
         rows[:] = -1
         for b, e in enumerate(entries):
             n = counts[b]
-            start = cache.lengths[e.slot]
+            start = starts[b]
             tok[r:r + n] = np.asarray(e.tokens, dtype=np.int32)
             pos[r:r + n] = np.arange(start, start + n, dtype=np.int32)
             sot[r:r + n] = b
@@ -233,10 +236,10 @@ class Stepper:
             slots=lay.view(dev, "slots"), ctx_lens=lay.view(dev, "ctx_lens"),
             page_tables={g: lay.view(dev, f"pages{g}").view(B, width) for g in range(len(cache.groups))},
             max_new=max(counts) if counts else 1,
-            max_ctx=max((cache.lengths[s] + n for s, n in zip(slots, counts)), default=1),
-            decode=all(n == 1 for n in counts),
-            fresh=bool(entries) and all(cache.lengths[e.slot] == 0 for e in entries),
-            lengths=[(cache.lengths[s], n) for s, n in zip(slots, counts)],
+            max_ctx=max(map(add, starts, counts), default=1),
+            decode=decode,
+            fresh=bool(entries) and not any(starts),
+            lengths=() if decode else list(zip(starts, counts)),
         )
         return ctx, lay, lay.view(dev, "logit_rows")
 

@@ -99,7 +99,8 @@ class StepContext:
     shared: Dict[Any, Any] = field(default_factory=dict)   # per-step values parts share (rotary tables)
     fresh: bool = False           # every sequence of the step starts at position 0 (whole prompts): what a token
     #                               reads is among the step's own tokens
-    lengths: Sequence[Tuple[int, int]] = ()   # (cached positions, new tokens) of each sequence (host); empty: not known
+    lengths: Sequence[Tuple[int, int]] = ()   # (cached positions, new tokens) of each sequence (host); empty in decode steps
+    #                               and where they are not known
 
 
 class RowStats:
