@@ -715,13 +715,14 @@ constexpr int RECV16_SLOTS = 22;
 template <int BN, bool SWAP> constexpr int recv_bytes() { return (SWAP && BN == 16) ? RECV16_SLOTS * BM * 4 : 0; }
 
 // cluster_reduce != 0: the grid was launched with clusters of gridDim.z CTAs along z (the K splits).
-// 33 to 64 tokens, two CTAs an SM: up to two more warps share an owner's tokens (each round of tokens is a trip through the cluster).  With three
-// an SM they would leave a thread 80 registers (65 to 128 tokens, K in eight: 6,144 x 4,096 15.3 to 18.9 us, with eight warps 16.0 to 19.4).
-template <int BN, bool SWAP, int MINB> constexpr int decode_threads() { return SWAP && BN == 64 && MINB == 2 ? 256 : NUM_THREADS; }
+// 33 to 64 tokens: up to two more warps share an owner's tokens (each round of tokens is a trip through the cluster).  Beyond, with three CTAs
+// an SM, they would leave a thread 80 registers for 128 columns (65 to 128 tokens, K in eight: 6,144 x 4,096 15.3 to 18.9 us, with eight
+// warps 16.0 to 19.4).
+template <int BN, bool SWAP> constexpr int decode_threads() { return SWAP && BN == 64 ? 256 : NUM_THREADS; }
 // XIELU: the output may be an activation's (NormIO::xielu).  A form of its own: the test alone lengthened a decode step of small
 // products (a chain of 30 kernels) by 1.5 %.
 template <int BN, int STAGES, bool SWAP, int MINB, bool XIELU>
-__global__ void __launch_bounds__((decode_threads<BN, SWAP, MINB>()), MINB) gemm_tc_kernel(
+__global__ void __launch_bounds__((decode_threads<BN, SWAP>()), MINB) gemm_tc_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     void* __restrict__ out, int out_mode, long long ldo, int M, int N, int K, int kb_per_split,
     float* __restrict__ partial, int cluster_reduce, int* __restrict__ status, const NormIO nio, const QkvIO qio) {
@@ -941,7 +942,7 @@ __global__ void __launch_bounds__((decode_threads<BN, SWAP, MINB>()), MINB) gemm
         const int S = cluster_reduce ? (int)gridDim.z : 1;
         const int cols = min(BN, M - tile_b * BN);
         const uint32_t stage = smem_u32(smem);
-        const int WARPS = decode_threads<BN, SWAP, MINB>() == NUM_THREADS ? NUM_THREADS / 32 : (int)(blockDim.x >> 5);
+        const int WARPS = decode_threads<BN, SWAP>() == NUM_THREADS ? NUM_THREADS / 32 : (int)(blockDim.x >> 5);
         const bool push = push2 || push3;
         const int LJ = (cols + S - 1) / S;                           // tokens an owner handles at most
         // where the pushed rows land, [source rank][owner's token][128] float32: beside the stages (16 tokens) or
@@ -1655,7 +1656,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* out, int out_mode
     if (!SWAP && (cl || out_mode == OUT_SWIGLU || out_mode == OUT_QKV)) return GG_ERR_ARG;      // forms the normal orientation does not have
     // eight warps only where they save an owner's tokens a round over six (4,096 x 2,048, K in eight: 33 tokens, five an owner, 7.4 us with six
     // warps and 7.8 with eight; 64, eight an owner, 8.7)
-    constexpr int most = decode_threads<BN, SWAP, MINB>();
+    constexpr int most = decode_threads<BN, SWAP>();
     const int owned = ((M < BN ? M : BN) + (cl ? splits : 1) - 1) / (cl ? splits : 1);
     const int threads = (owned + 7) / 8 < (owned + 5) / 6 ? most : NUM_THREADS;
     return gg_launch(kern, grid, dim3(threads), smem, stream, cl ? splits : 1, ta, tb, out, out_mode, ldo, M, N, K,
@@ -1759,11 +1760,7 @@ static int gemm_tc_impl(const void* x, const void* w, void* out, int out_mode, i
         // to run as one wave.  GOGGUF_B200_GEMM_DEEP=0 always takes the three-per-SM forms.
         const long long ctas = (long long)((N + BM - 1) / BM) * ((M + bn - 1) / bn) * splits;
         // (33 to 64 tokens: see gg_gemm_tc_splits; above, three per SM always)
-        // A CTA of one or two slabs of K has no use for the ring: where there is one an SM, the next kernel's CTAs come in earlier beside a
-        // smaller one (33 tokens, 1,024 x 1,024 4.9 us, in the deeper ring 5.2; 2,048 x 1,024 5.5, 5.7; from 49 tokens on the eight warps of
-        // the other form count for more: 64 tokens 6.1, 5.6 and 6.9, 6.4).
-        const bool deep = gemm_deep() && (bn <= 32 ? ctas <= 296 : bn == 64 && cluster && two_per_sm_at_64((N + BM - 1) / BM, K)
-                                                                   && !(ctas <= 148 && per <= 2 && (M + splits - 1) / splits <= 6));
+        const bool deep = gemm_deep() && (bn <= 32 ? ctas <= 296 : bn == 64 && cluster && two_per_sm_at_64((N + BM - 1) / BM, K));
 #define GG_DECODE_AS(BN_, ST_, MINB_, X_) launch<BN_, ST_, true, MINB_, X_>(ta, tb, out, out_mode, ldo, M, N, K, splits, per, scratch, \
                                                                           cluster, status, nio, qio, stream)
 #define GG_DECODE(BN_, ST_, MINB_) (nio.xielu ? GG_DECODE_AS(BN_, ST_, MINB_, true) : GG_DECODE_AS(BN_, ST_, MINB_, false))
